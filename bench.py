@@ -587,7 +587,7 @@ def main():
     finish_bytes = int(coded - f_coded - f_stored - p.stream_jobs["src_len"].sum()
                        + p.stream_jobs["n"].sum() + fin_plain + p.base_bytes)
     kbytes = {"stream_decode": stream_bytes, "finish": finish_bytes, "fused": fused_bytes}
-    kname = {"stream_decode": "k_rans / k_stream<bytes>",
+    kname = {"stream_decode": "k_stream<bytes>",
              "finish": "k_stream<delta> + k_finish" if p.delta_jobs.size else "k_finish",
              "fused": "k_stream<f32>" if p.n_fused_f32 * 2 > fj.size + tj.size else
                       "k_stream<bf16, shared tables>" if tj.size > fj.size else "k_stream<bf16>"}
@@ -789,7 +789,7 @@ def run_stress(a, rank: int):
                    "l2": "the largest cells stream up to 17 GB per launch; small cells fit the 126 MB L2 and are launch-bound"},
         "clocks": clk.summary(),
         "e2e": None, "gpu_launches": len(cells) * 8,
-        "roofline": {"bound": "hbm", "kernel": "k_stream<bytes> / k_rans", "achieved": round(best_cell["moved"] / best_cell["ms"] / 1e6, 1),
+        "roofline": {"bound": "hbm", "kernel": "k_stream<bytes>", "achieved": round(best_cell["moved"] / best_cell["ms"] / 1e6, 1),
                      "peak": peak, "unit": "GB/s", "frac": best_cell["hbm_frac"], "traffic": None,
                      "cell": {k: best_cell[k] for k in ("dist", "len", "batch", "tables")}},
         "cpu_baseline": cpu,

@@ -61,7 +61,7 @@ int lmz_gpu_validate(const void *streams, const void *off, unsigned nstr);
  * shared by all streams (each stream then starts at its 8 states) or NULL.
  * d_streams must be 16-byte aligned with lmz_gpu_pad_bytes() of slack after
  * the last stream.  Asynchronous on cuda_stream (NULL = default); `tpb` is
- * accepted and ignored.  Unlike the reference's, a batch of 9472 streams or more
+ * accepted and ignored.  Unlike the reference's, a batch of more than 76 streams per SM
  * with per-stream tables takes (nstr + 2) * 4 bytes of stream-ordered memory from
  * a pool this library keeps per device, for an index list that sorts the streams
  * by alphabet size; lmz_gpu_decode_batch_dev_noalloc never does. */
@@ -83,12 +83,10 @@ int lmz_gpu_decode_batch(const void *hdr, const void *streams, size_t nbytes, co
 int lmz_gpu_set_device(int device);
 
 /* No counterpart in the reference: choose the per-stream decode-table layout for
- * streams that carry their own table.  -1 = by batch size (default), 0 = narrow
- * (5 KiB per stream), 2 = compact (2 KiB, the most streams per SM), 3 = a wide
- * 16 KiB table per stream (one lookup per symbol; 12 streams per SM, for launches
- * small enough to be bound by per-symbol latency), 4 = the same with 13 streams per SM
- * and every symbol stored straight to its output byte.  A tuning and testing knob;
- * results are identical. */
+ * streams that carry their own table.  -1 = by batch size (default), 0 or 2 = compact
+ * (1 KiB and a word per symbol, the most streams per SM), 3 or 4 = a wide 16 KiB table
+ * per stream (one lookup per symbol; 12 streams per SM, for launches small enough to be
+ * bound by per-symbol latency).  A tuning and testing knob; results are identical. */
 int lmz_gpu_set_table_mode(int mode);
 
 /* One stream to decode; mirrors struct lmz::StreamJob.  32 bytes. */

@@ -298,7 +298,6 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
             ta.piece_crc = (uint32_t *)p->d_piece_crc;
             ta.tabs = (const CrcTables *)p->d_crc_tables;
             ta.tables = (const uint8_t *)p->d_tables;
-            ta.per_cta = F_SHARED_SINK_WARPS * 4;
             if (!ta.tables) return fail_msg(LMZ_GPU_EUNSUPPORTED, "shared-table chunks without d_tables");
             rc = p->d_piece_crc ? launch_stream<SINK_BF16, true, -1>(ta, fs)
                                 : launch_stream<SINK_BF16, false, -1>(ta, fs);

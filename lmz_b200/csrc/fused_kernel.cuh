@@ -1,5 +1,5 @@
-// k_stream: the throughput kernel.  One 8-lane group per rANS stream, compact
-// per-stream tables, and the stream's consumer fused into the decode loop:
+// k_stream: the decode kernel.  One 8-lane group per rANS stream and the stream's consumer
+// fused into the decode loop:
 //
 //   SINK_BYTES  the decoded plane is written as is (decode_batch, scratch planes)
 //   SINK_BF16   a CODEC_BF16 chunk whose exponent plane is rANS and whose
@@ -17,28 +17,37 @@
 //               in the output space, written once and checksummed (CFN = 192: a 128-entry
 //               level 2 for the first plane, a 256-entry one for the second)
 //
-// Differences from k_rans that buy instructions and occupancy:
-//   * shared memory is laid out by kind (all level-1 tables, all level-2 tables,
-//     all rings ...) so each table base is aligned to its size and an address is
-//     (index bits) | base in one logic op; a warp's four level-1 tables interleave
-//     word by word, which drops the index shift and keeps the four streams' lookups
-//     in different banks
-//   * the input ring (4 x 128 B) is followed by a mirror of its first 272 bytes,
-//     filled by the same bulk copies, so a tile reads linearly with no wrap masks
+// What bounds it: a symbol depends on the one before it, so the time of a launch is (steps of
+// a stream) x (latency of a step) x (waves of streams), and the chip is filled with as many
+// streams as shared memory and registers hold.  A step is a table lookup on the state's low
+// 12 bits, the state update, and -- for the lanes whose state fell below 2^16 -- a refill with
+// the next 16-bit word of the stream, whose place a vote over the group gives.  Done in that
+// order a refilled lane's lookup waits for update, vote, popcount, word and then the table.
+// Here the words are looked up before anyone asks for them: while the group decodes, each of its
+// lanes also translates two of the next sixteen words (their place in the table is known: a
+// refilled state's low 12 bits ARE the word's) and leaves word and lookup result together in a
+// ring in shared memory.  A refilled lane finds its next table entry in the word it fetches, the
+// other lanes look theirs up meanwhile, and the two halves of the old chain run side by side.
+//
+//   * compressed words come straight from global memory into registers, two aligned 32-bit
+//     loads per lane and 16 words (any byte alignment: a funnel shift), one round ahead
+//   * the ring holds 64 translated words and a copy of its first 32 behind them, so a block of
+//     four steps reads linearly; a round of 16 is translated every eight steps where there is
+//     room, and a loop before each block tops up streams that consume more than that
 //   * refill offsets come from a 4-step history of the group's votes: one
 //     byte-permute and one popcount per step instead of two popcounts
+//   * a warp's four level-1 tables interleave word by word: the lookup address is the state's
+//     bits 4-11 unshifted, and the four streams' lookups stay in different banks
 //   * CFN = 128: level 2 has 128 slots, the four streams of a warp rotated 8
 //     entries apart so their popular symbols sit in different banks; streams with
 //     more than 104 live symbols must be given to the CFN = 256 instance
-//   * CFN = 0: no levels, a 16 KiB slot -> entry table per stream and 12 streams per
-//     CTA, 256-symbol tiles: for launches so small that only the length of a symbol's
-//     dependent chain counts (one lookup instead of two and a popcount)
-//   * CFN = 0 with a fourth warp: 13 streams per CTA -- the tables on 16 KiB boundaries, the rings
-//     (shorter) in what is left below the first and above the last -- and every symbol stored
-//     straight to its output byte (no staging row)
-//   * CFN = -1: the same wide table once per CTA, for batches whose streams share one
-//     516-byte table (lmz_gpu_decode_batch's d_hdr) or for the chunks of a shared-table
-//     archive (StreamArgs.tables); a stream is then states + words
+//   * TR8: a ring entry is word and table entry (8 bytes); otherwise word and level-2 offset
+//     (4 bytes, half the space: more streams per SM for one more lookup in a refilled lane's step)
+//   * CFN = 0: a 16 KiB slot -> entry table per stream; CFN = -1: one such table per CTA, for
+//     batches whose streams share one 516-byte table (lmz_gpu_decode_batch's d_hdr) or for the
+//     chunks of a shared-table archive (StreamArgs.tables); a stream is then states + words
+//   * warps are independent: each takes four streams, then the next four, ...; a launch is
+//     at most one CTA per SM, with no more warps than its streams need
 #pragma once
 #include "chunk_kernels.cuh"
 #include "rans.cuh"
@@ -46,30 +55,9 @@
 namespace lmz {
 
 enum : int { SINK_BYTES = 0, SINK_BF16 = 1, SINK_F32 = 2, SINK_DELTA = 3 };
-constexpr uint32_t F_SLOT = 128, F_NSLOT = 4, F_RING = F_SLOT * F_NSLOT;
-constexpr uint32_t F_MIRROR = 272;                 // a tile reads at most 256 + 2 bytes ahead
-constexpr uint32_t F_RING_BYTES = F_RING + F_MIRROR;        // 784
-constexpr uint32_t F_STAGE = 144;                  // 128 + 16: groups land 4 banks apart
-// The per-stream wide instance (CFN = 0) runs one warp per scheduler, where every
-// instruction of tile bookkeeping is paid in full, and has shared memory to spare beside
-// its 12 tables: its tiles are twice as long (256 symbols) and its ring twice as deep.
-__host__ __device__ constexpr bool stream_long_tiles(int cfn, int warps) { return cfn == 0 && (warps == 3 || warps == 4); }
-// The same with a thirteenth stream (a fourth warp that carries one): thirteen tables on 16 KiB
-// boundaries leave 19 KiB in two pieces, under the first and above the last, enough for rings of six
-// slots instead of eight and for no staging rows -- every symbol goes straight to its byte of the output.  For launches of 12 x SMs + 1 ... 13 x SMs
-// streams (the 1915 long streams of an 8B model at the reference's default chunking, on 148 SMs).
-__host__ __device__ constexpr bool stream_direct(int cfn, int warps) { return cfn == 0 && warps == 4; }
-constexpr uint32_t F_DIRECT_GROUPS = 13;
-__host__ __device__ constexpr uint32_t stream_tile(int cfn, int warps) { return stream_long_tiles(cfn, warps) ? 256u : 128u; }
-__host__ __device__ constexpr uint32_t stream_nslot(int cfn, int warps) { return stream_direct(cfn, warps) ? 6u : stream_long_tiles(cfn, warps) ? 8u : F_NSLOT; }
-__host__ __device__ constexpr uint32_t stream_mirror(int cfn, int warps) { return stream_long_tiles(cfn, warps) ? 528u : F_MIRROR; }
-__host__ __device__ constexpr uint32_t stream_ring_bytes(int cfn, int warps)
-{
-    return F_SLOT * stream_nslot(cfn, warps) + stream_mirror(cfn, warps);
-}
-__host__ __device__ constexpr uint32_t stream_stage(int cfn, int warps) { return stream_direct(cfn, warps) ? 0u : stream_long_tiles(cfn, warps) ? 272u : F_STAGE; }
-constexpr uint32_t F_LOGS = 3;                     // eight copies of the CRC slice tables (32 KiB), one per lane of a group: see CrcQuarters
-constexpr uint32_t F_CRC_BYTES = (4096u << F_LOGS) + 4096u;   // + the row-advance tables, once
+constexpr uint32_t F_STAGE = 144;                  // a tile's 128 symbols + 16: groups land 4 banks apart
+constexpr uint32_t TR_N = 64, TR_MIRROR = 32;      // ring of translated words; a block of four steps reads at most 32
+constexpr uint32_t TR_ROUND = 16;                  // words translated at a time, two per lane
 constexpr uint32_t F_ROW = 256, F_UNIT = 32;       // bytes of BF16 one group / one lane emits per tile
 constexpr int F_SMALL_CFN = 128;                   // level-2 slots of the dense instance
 constexpr int F_HYBRID_CFN = 192;                  // delta sink: 128-entry tables for first planes, 256-entry for second planes
@@ -123,145 +111,168 @@ struct StreamArgs {
     const uint32_t *order;
     const uint32_t *count;
     uint32_t order_from_back;
-    // Streams per CTA (a multiple of 4, at most the instance's capacity; 0 = the capacity):
-    // the launcher spreads a launch evenly over its waves of CTAs, so that a launch of 3.03
-    // waves runs as four waves of three quarters the streams instead of three full waves
-    // and one nearly empty one, and a small launch uses every SM.
-    uint32_t per_cta;
 };
 
-constexpr uint32_t F_WIDE_BYTES = PROB_SCALE * 4;   // CFN = 0: one 16 KiB slot -> entry table per stream
-constexpr int F_WIDE_GROUPS = 12;                   // three full warps; 13 tables would fit, but not their rings
-__host__ __device__ constexpr uint32_t stream_group_bytes(int cfn)
-{
-    return (cfn > 0 ? 1024 + 4 * cfn : cfn == 0 ? F_WIDE_BYTES : 0) + F_RING_BYTES + F_STAGE + 32;   // 3008 / 2496 / 17344 / 960
-}
-constexpr int F_SHARED_WARPS = 16;                  // CFN = -1: one table per CTA, two CTAs per SM (64 registers a thread)
+constexpr uint32_t F_WIDE_BYTES = PROB_SCALE * 4;   // a slot -> entry table
 constexpr uint32_t F_TABLE_STRIDE = 528;            // 516 rounded up to 16
-constexpr int F_SHARED_SINK_WARPS = 20;             // CFN = -1 with the BF16 sink: one CTA per SM, 80 chunks sharing its table
-// Streams are carved from the bottom of the CTA's shared memory and the CRC tables
-// from the top (slice tables 8 KiB aligned, row-advance tables above them), so the
-// launch asks for everything the device lets one CTA have: 227 KiB that start
-// F_SMEM_BASE bytes into the shared window (the launcher checks that reservation).
+constexpr uint32_t F_SHARED_SINK_WARPS = 20;        // chunks of a shared-table archive: 80 per CTA share its table
+constexpr uint32_t F_CRC_BYTES = 32768;             // four slice tables x 256 entries x eight copies (CrcQuarters)
+// The launch's shared memory starts F_SMEM_BASE bytes into the CTA's window (the launcher checks
+// that reservation); at most F_SMEM_DYN bytes of it are to be had.
 constexpr uint32_t F_SMEM_BASE = 1024, F_SMEM_DYN = 232448;
-__host__ __device__ constexpr uint32_t stream_crc_adv(uint32_t top) { return (top - 4096u) & ~1023u; }
-__host__ __device__ constexpr uint32_t stream_crc_slice(uint32_t top)
+
+// Where a CTA of W warps keeps what, as addresses in the shared window.  The CRC tables sit on a
+// 32 KiB boundary (a table index is OR-ed onto the base) and level-1 tables on 4 KiB boundaries;
+// what fits goes below the CRC tables, chosen so that the whole is shortest.
+struct StreamSmem {
+    uint32_t cf, stage, tr, l1, crc, adv, poison, end;
+};
+__host__ __device__ constexpr uint32_t tr_entry(bool tr8) { return tr8 ? 8u : 4u; }
+__host__ __device__ constexpr uint32_t tr_group(bool tr8) { return (TR_N + TR_MIRROR) * tr_entry(tr8); }
+__host__ __device__ constexpr StreamSmem stream_smem_with(int cfn, bool crc, int sink, bool tr8, uint32_t W, bool low_stage, bool low_tr)
 {
-    return (stream_crc_adv(top) - (4096u << F_LOGS)) & ~((1024u << F_LOGS) - 1u);
+    StreamSmem m{};
+    uint32_t p = F_SMEM_BASE;
+    m.poison = p; p += 16;
+    const uint32_t cf = cfn > 0 ? W * 16u * (uint32_t)cfn : 0u, stage = W * 4u * F_STAGE, tr = W * 4u * tr_group(tr8);
+    m.cf = p; p += cf;
+    if (low_stage) { m.stage = p; p += stage; }
+    if (low_tr) { m.tr = p; p += tr; }
+    if (crc) {
+        p = (p + F_CRC_BYTES - 1) & ~(F_CRC_BYTES - 1);
+        m.crc = p; p += F_CRC_BYTES;
+        if (sink == SINK_F32) { m.adv = p; p += 4096; }
+    }
+    const uint32_t align = cfn > 0 ? 4096u : F_WIDE_BYTES;
+    p = (p + align - 1) & ~(align - 1);
+    m.l1 = p; p += cfn > 0 ? W * 4096u : cfn == 0 ? W * 4u * F_WIDE_BYTES : F_WIDE_BYTES;
+    if (!low_tr) { m.tr = p; p += tr; }
+    if (!low_stage) { m.stage = p; p += stage; }
+    m.end = p;
+    return m;
 }
-// The BF16 sink's checksum needs no row-advance tables (see k_stream), so the 4 KiB they
-// would take, above the slice tables, hold the level-1 tables of the CTA's last warp.
-__host__ __device__ constexpr bool stream_top_l1(int sink, bool crc, int cfn) { return (sink == SINK_BF16 || sink == SINK_DELTA) && crc && cfn > 0; }
-__host__ __device__ constexpr int stream_warps(int cfn, bool crc, int sink = SINK_BYTES)
+__host__ __device__ constexpr StreamSmem stream_smem(int cfn, bool crc, int sink, bool tr8, uint32_t W)
 {
-    constexpr uint32_t top = F_SMEM_BASE + F_SMEM_DYN;
-    if (cfn == 0) return F_WIDE_GROUPS / 4;
-    if (cfn < 0) return sink == SINK_BF16 ? F_SHARED_SINK_WARPS : F_SHARED_WARPS;
-    const uint32_t room = (crc ? stream_crc_slice(top) : top) - F_SMEM_BASE + (stream_top_l1(sink, crc, cfn) ? 4096u : 0u);
-    int w = (int)(room / (4u * stream_group_bytes(cfn)));
-    // Registers are shared per scheduler: a 21st warp would put six on one of the four and cut every
-    // thread from 96 registers to 80 (which this kernel does not fit in), so 20 is the most.
-    if (crc && w > 20) w = 20;
+    StreamSmem best = stream_smem_with(cfn, crc, sink, tr8, W, false, false);
+    for (int i = 1; i < 4; i++) {
+        const StreamSmem m = stream_smem_with(cfn, crc, sink, tr8, W, (i & 1) != 0, (i & 2) != 0);
+        if (m.end < best.end) best = m;
+    }
+    return best;
+}
+// The most warps of an instance: what shared memory holds, and registers (96 a thread up to 20
+// warps, 80 up to 24).
+__host__ __device__ constexpr uint32_t stream_warps(int cfn, bool crc, int sink, bool tr8)
+{
+    if (cfn < 0 && sink == SINK_BF16) return F_SHARED_SINK_WARPS;
+    uint32_t w = cfn < 0 ? 32u : 24u;
+    while (stream_smem(cfn, crc, sink, tr8, w).end > F_SMEM_BASE + F_SMEM_DYN) w--;
     return w;
 }
-__host__ __device__ constexpr unsigned stream_groups(int cfn, int warps) { return warps * 4; }
-static_assert(F_LOGS == 3 && stream_crc_slice(F_SMEM_BASE + F_SMEM_DYN) % 32768u == 0,
-              "crc_feed4q ORs a 32 KiB table's offsets onto its base");
-static_assert(stream_warps(128, true) == 19 && stream_warps(256, true) == 16 &&
-              stream_warps(128, false) == 23 && stream_warps(256, false) == 19 &&
-              stream_warps(128, true, SINK_BF16) >= 19 && stream_warps(256, true, SINK_BF16) == 16, "shared memory budget");
 
-__device__ __forceinline__ void bulk_g2s_sa(uint32_t dst_sa, const void *src, uint32_t bytes,
-                                            uint32_t bar_sa)
+// ---- the ring of translated words ------------------------------------------------------------
+// A slot's table entry: its level-2 byte offset from the stream's first entry (compact), or the
+// address of the entry itself (wide).
+template <int CFN>
+__device__ __forceinline__ uint32_t slot_ref(uint32_t x, uint32_t l1_sa)
 {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-        ::"r"(dst_sa), "l"(src), "r"(bytes), "r"(bar_sa) : "memory");
+    if (CFN <= 0) return ((x << 2) & 0x3ffcu) | l1_sa;         // the table is 16 KiB aligned
+    // the warp's four level-1 tables are interleaved word by word, so bucket b of this group
+    // sits 16 * b bytes in -- the slot's bits 4-11, unshifted
+    const uint32_t e1 = lds_u32((x & 0xff0u) | l1_sa);
+    return (e1 >> 16) + 4u * __popc(e1 << ((~x & 15u) | 16u));
 }
+template <int CFN>
+__device__ __forceinline__ uint32_t ref_addr(uint32_t ref, uint32_t cf_sa) { return CFN <= 0 ? ref : cf_sa + ref; }
 
-// Input ring with a mirror of its head behind it.  Offsets are bytes from `abase`.
-template <uint32_t NSLOT_, uint32_t MIRROR_>
-struct MRingT {
-    static constexpr uint32_t F_NSLOT = NSLOT_, F_RING = F_SLOT * NSLOT_, F_MIRROR = MIRROR_;
-    uint32_t sa;           // shared address of the ring
-    uint64_t *bars;
-    const uint8_t *abase;
-    uint32_t valid_slots, issued, ready;
-    bool dead;
+// Positions are in bytes of ring entries and only grow; the ring index is the position modulo the ring.
+template <int CFN, bool TR8>
+struct Words {
+    static constexpr uint32_t ES = tr_entry(TR8), RB = TR_N * ES, LOW = TR_MIRROR * ES;
+    static_assert(TR8 || CFN > 0, "a wide table's entry does not fit a 4-byte ring entry");
+    uint32_t sa;             // the ring
+    uint32_t rd, wr;         // words consumed / translated so far
+    uint32_t lo, hi, sh;     // this lane's next two words: aligned loads and the shift between them
+    const uint32_t *next;
+    int32_t left;            // rounds of the stream that have not been requested
 
-    // Every lane of the group keeps `issued` (so the usual "nothing to request" costs no
-    // divergent branch); only the leader touches the barrier and starts the copies.
-    __device__ __forceinline__ void issue(uint32_t cursor, bool leader)
+    // This lane's next two words, if the stream has them and `want`.  No branch: the loads are
+    // predicated.  A stream is read front to back in 32-byte pieces: the L2 is asked for 256 bytes
+    // at a time, so that most requests wait for the L2 and not for HBM.
+    __device__ __forceinline__ void request(bool want)
     {
-        uint32_t lim = cursor / F_SLOT + F_NSLOT;
-        if (lim > valid_slots) lim = valid_slots;
-        while (issued < lim) {
-            if (leader) {
-                uint32_t j = issued % F_NSLOT;
-                uint32_t m = j * F_SLOT < F_MIRROR ? min(F_SLOT, F_MIRROR - j * F_SLOT) : 0u;
-                const uint8_t *g = abase + (size_t)issued * F_SLOT;
-                mbar_expect_tx(&bars[j], F_SLOT + m);
-                bulk_g2s_sa(sa + j * F_SLOT, g, F_SLOT, smem_addr(&bars[j]));
-                if (m) bulk_g2s_sa(sa + F_RING + j * F_SLOT, g, m, smem_addr(&bars[j]));
-            }
-            issued++;
-        }
+        const int32_t go = want ? left : 0;
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.gt.s32 p, %3, 0;\n\t"
+                     "@p ld.global.nc.L2::256B.u32 %0, [%2];\n\t@p ld.global.nc.u32 %1, [%2+4];\n\t}"
+                     : "+r"(lo), "+r"(hi) : "l"(next), "r"(go));
+        next += want ? TR_ROUND / 2 : 0;
+        left -= want ? 1 : 0;
     }
-    __device__ __forceinline__ void require(uint32_t upto)
+    __device__ __forceinline__ uint32_t block() const { return sa + (rd & (RB - 1)); }
+    __device__ __forceinline__ bool low() const { return wr - rd < LOW; }
+    // A group that only runs along asks for no more words (and writes none: there is never room).
+    __device__ __forceinline__ void retire() { wr = rd + 0x40000000u; }
+
+    // A round in three parts, so that the steps of the decode run between them.
+    uint32_t v, r0, r1;
+    bool room;
+    __device__ __forceinline__ void part1()
     {
-        uint32_t need = (upto + F_SLOT - 1) / F_SLOT;
-        if (need > valid_slots) need = valid_slots;
-        while (ready < need) {
-            if (!dead && !mbar_wait(&bars[ready % F_NSLOT], (ready / F_NSLOT) & 1u)) dead = true;
-            ready++;
-        }
+        room = wr - rd <= RB - TR_ROUND * ES;
+        v = __funnelshift_r(lo, hi, sh);
     }
-    __device__ __forceinline__ uint32_t byte_at(uint32_t o) const { return lds_u8(sa + (o & (F_RING - 1))); }
-    __device__ __forceinline__ uint32_t u16_at(uint32_t o) const { return byte_at(o) | (byte_at(o + 1) << 8); }
-    __device__ __forceinline__ uint32_t u32_at(uint32_t o) const { return u16_at(o) | (u16_at(o + 2) << 16); }
+    __device__ __forceinline__ void part2(uint32_t l1_sa)
+    {
+        r0 = slot_ref<CFN>(v, l1_sa);
+        r1 = slot_ref<CFN>(v >> 16, l1_sa);
+    }
+    __device__ __forceinline__ void part3(uint32_t cf_sa, uint32_t k)
+    {
+        const uint32_t at = sa + (wr & (RB - 1)) + 2u * ES * k;
+        const uint32_t keep = room, again = room && !(wr & LOW);
+        if (TR8) {
+            const uint32_t e0 = lds_u32(ref_addr<CFN>(r0, cf_sa)), e1 = lds_u32(ref_addr<CFN>(r1, cf_sa));
+            sts_u128_if(keep, at, e0, v, e1, v >> 16);
+            sts_u128_if(again, at + RB, e0, v, e1, v >> 16);
+        } else {
+            const uint32_t t0 = __byte_perm(v, r0, 0x5410), t1 = __byte_perm(v, r1, 0x5432);
+            sts_u64_if(keep, at, t0, t1);
+            sts_u64_if(again, at + RB, t0, t1);
+        }
+        wr += room ? TR_ROUND * ES : 0;
+        request(room);
+    }
+    __device__ __forceinline__ void round(uint32_t l1_sa, uint32_t cf_sa, uint32_t k)
+    {
+        part1();
+        part2(l1_sa);
+        part3(cf_sa, k);
+    }
 };
 
-// Table lookups and the state update of one decode step, before the refill.
-// Returns the level-2 entry (its low byte is the symbol); x2 is the new state.
-template <int CFN>
-__device__ __forceinline__ uint32_t stream_advance(uint32_t x, uint32_t l1_sa, uint32_t cf_sa, uint32_t &x2)
+__device__ __forceinline__ uint32_t rans_update(uint32_t x, uint32_t e)
 {
-    uint32_t e;
-    if (CFN <= 0) {
-        // wide table at l1_sa (the stream's own, or the CTA's shared one), 16 KiB aligned: one
-        // lookup, the index OR-ed onto the base
-        e = lds_u32(((x << 2) & 0x3ffcu) | l1_sa);
-    } else {
-        // level 1: the warp's four tables are interleaved word by word, so bucket b of
-        // this group sits 16 * b bytes in -- the slot's bits 4-11, unshifted
-        const uint32_t e1 = lds_u32((x & 0xff0u) | l1_sa);
-        const uint32_t upto = 0xffffffffu >> ((~x) & 15u);             // bits 0 .. 16 + (slot & 15)
-        const uint32_t pc = __popc(e1 & upto & 0xffff0000u);
-        constexpr uint32_t IDX = 4u * (uint32_t)(CFN > 0 ? CFN : 1) - 4u;   // byte offset field of level 1
-        e = lds_u32(((e1 & IDX) | cf_sa) + (pc << 2));
-    }
     // f * (x >> 12) + slot - start  ==  x - (x >> 12) * (4096 - f) - start
-    x2 = x - ((x >> PROB_BITS) * (e >> 20) + ((e >> 8) & 0xfffu));
-    return e;
+    return x - ((x >> PROB_BITS) * (e >> 20) + ((e >> 8) & 0xfffu));
 }
 
-// One decode step, any lane mix.  `caddr` is the shared address of the cursor
-// (linear within a tile thanks to the mirror).
-template <int CFN>
-__device__ __forceinline__ uint32_t stream_step(uint32_t &x, uint32_t &caddr, uint32_t l1_sa,
-                                                uint32_t cf_sa, uint32_t lt_mask, uint32_t grp_mask,
-                                                bool active)
+// The second half of a step: x2 is the updated state; a lane that needs a refill takes the ring
+// entry at word_sa, the others look their slot up.  `e` leaves as the entry of the new state's slot.
+template <int CFN, bool TR8>
+__device__ __forceinline__ void refill(uint32_t &x, uint32_t &e, uint32_t x2, bool need, uint32_t word_sa, uint32_t l1_sa,
+                                       uint32_t cf_sa)
 {
-    uint32_t x2;
-    const uint32_t e = stream_advance<CFN>(x, l1_sa, cf_sa, x2);
-    const bool need = active && x2 < RANS_LOW;
-    const uint32_t vote = __ballot_sync(0xffffffffu, need);
-    const uint32_t addr = caddr + 2 * __popc(vote & lt_mask);
-    const uint32_t lo = lds_u8(addr), hi = lds_u8_1(addr);
-    if (need) x2 = ((x2 << 8) + hi << 8) + lo;
-    if (active) x = x2;
-    caddr += 2 * __popc(vote & grp_mask);
-    return e;
+    uint32_t a = ref_addr<CFN>(slot_ref<CFN>(x2, l1_sa), cf_sa);
+    if (TR8) {
+        e = lds_u32(a);
+        const uint2 w = lds_u64(word_sa);
+        if (need) { e = w.x; x2 = __byte_perm(w.y, x2, 0x5410); }
+    } else {
+        const uint32_t w = lds_u32(word_sa);
+        if (need) { a = cf_sa + (w >> 16); x2 = __byte_perm(w, x2, 0x5410); }
+        e = lds_u32(a);
+    }
+    x = x2;
 }
 
 // One step of a full tile, four to a block.  `hist` collects the group's votes of
@@ -269,26 +280,34 @@ __device__ __forceinline__ uint32_t stream_step(uint32_t &x, uint32_t &caddr, ui
 // the warp vote and shifts the older ones up); refills consumed before this
 // lane's = bits of the older bytes plus the lanes below it in the newest, so one
 // popcount of hist & below (= 0xffffff00 | lanes below) gives the offset from
-// the block's cursor.  The caller adds 2 * popc(hist) to `cbase` after step 3.
-template <int CFN, bool FIRST>
-__device__ __forceinline__ uint32_t stream_step4(uint32_t &x, uint32_t &hist, uint32_t cbase,
-                                                 uint32_t l1_sa, uint32_t cf_sa, uint32_t below,
-                                                 uint32_t vsel)
+// the block's start.
+template <int CFN, bool TR8, bool FIRST>
+__device__ __forceinline__ void stream_step4(uint32_t &x, uint32_t &e, uint32_t &hist, uint32_t base, uint32_t l1_sa,
+                                             uint32_t cf_sa, uint32_t below, uint32_t vsel)
 {
-    uint32_t x2;
-    const uint32_t e = stream_advance<CFN>(x, l1_sa, cf_sa, x2);
+    const uint32_t x2 = rans_update(x, e);
     const bool need = x2 < RANS_LOW;
     const uint32_t vote = __ballot_sync(0xffffffffu, need);
     hist = __byte_perm(vote, FIRST ? 0u : hist, vsel);
-    const uint32_t addr = cbase + 2 * __popc(hist & below);
-    const uint32_t lo = lds_u8(addr), hi = lds_u8_1(addr);
-    if (need) x2 = ((x2 << 8) + hi << 8) + lo;       // two predicated shift-adds, no select
-    x = x2;
-    return e;
+    refill<CFN, TR8>(x, e, x2, need, base + tr_entry(TR8) * __popc(hist & below), l1_sa, cf_sa);
 }
 
-template <int SINK, bool CRC, int WARPS, int CFN>
-__global__ void __launch_bounds__(WARPS * 32, CFN < 0 && SINK == SINK_BYTES ? 2 : 1) k_stream(StreamArgs a)
+// One step of a ragged tile, any lane mix: lanes past the end keep their state.
+template <int CFN, bool TR8>
+__device__ __forceinline__ void stream_step(uint32_t &x, uint32_t &e, uint32_t &base, uint32_t l1_sa, uint32_t cf_sa,
+                                            uint32_t lt_mask, uint32_t grp_mask, bool active)
+{
+    const uint32_t x2 = rans_update(x, e);
+    const bool need = active && x2 < RANS_LOW;
+    const uint32_t vote = __ballot_sync(0xffffffffu, need);
+    uint32_t nx = x, ne = e;
+    refill<CFN, TR8>(nx, ne, x2, need, base + tr_entry(TR8) * __popc(vote & lt_mask), l1_sa, cf_sa);
+    if (active) { x = nx; e = ne; }
+    base += tr_entry(TR8) * __popc(vote & grp_mask);
+}
+
+template <int SINK, bool CRC, int CFN, bool TR8>
+__global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, TR8) * 32, 1) k_stream(StreamArgs a)
 {
     // SINK_BF16 checksums: lane k keeps one running value per word of its 32-byte unit,
     // ra[i] = sum over the piece's rows so far of word i * x^(2048 * rows since); a row
@@ -297,85 +316,77 @@ __global__ void __launch_bounds__(WARPS * 32, CFN < 0 && SINK == SINK_BYTES ? 2 
     // word_mul[k][i] carry them to the piece's end.
     constexpr bool ROWMUL = (SINK == SINK_BF16 || SINK == SINK_DELTA) && CRC;
     constexpr int NRA = SINK == SINK_DELTA ? 4 : 8;        // running values per lane: words of its unit of a row
-    constexpr bool TOPL1 = stream_top_l1(SINK, CRC, CFN);
     extern __shared__ __align__(16) uint8_t ssm[];
     constexpr bool WIDE = CFN <= 0, SHARED = CFN < 0;
-    constexpr bool DIRECT = stream_direct(CFN, WARPS);
-    static_assert(!DIRECT || SINK == SINK_BYTES, "the 13-stream instance writes bytes only");
     // SINK_DELTA with CFN = 192: the two planes of a chunk have level-2 tables of different sizes, 128
     // entries for the exponent differences (a handful of symbols) and 256 for the sign/mantissa
-    // differences, 768 bytes a stream on average; the decode steps are those of the 256-entry instance.
+    // differences, 768 bytes a stream on average.
     constexpr bool HYB = SINK == SINK_DELTA && CFN == F_HYBRID_CFN;
-    constexpr int CFN_STEP = HYB ? 256 : CFN;
-    constexpr uint32_t G = DIRECT ? F_DIRECT_GROUPS : stream_groups(CFN, WARPS), CFB = WIDE ? 16u : 4u * CFN;
-    constexpr uint32_t CF_ALIGN = HYB ? 1024u : CFB;
     static_assert(CFN != F_HYBRID_CFN || SINK == SINK_DELTA, "mixed table sizes are the delta sink's");
     constexpr uint32_t LEAD = (SHARED ? 0u : HDR_BYTES) + STATE_BYTES;
-    constexpr uint32_t MAX_LIVE = CFN > 0 && CFN < 256 ? (uint32_t)CFN - 24u : 256u;
-    constexpr uint32_t TS = stream_tile(CFN, WARPS), NSL = stream_nslot(CFN, WARPS), RB = stream_ring_bytes(CFN, WARPS);
-    constexpr uint32_t STG = stream_stage(CFN, WARPS), RINGB = F_SLOT * NSL;
-    constexpr uint32_t HS = NSL != F_NSLOT ? 160u : 144u;     // header staging copy: four of them cover 548 + 15 bytes
-    static_assert(CFN != 0 || !CRC, "the per-stream wide instance has no room for CRC tables");
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    // DIRECT: the fourth warp carries one stream; its other three groups shadow it (same tables,
-    // ring and states, no copies requested, nothing stored) so that the warp decodes full tiles
-    const uint32_t k = lane & 7u, g = lane >> 3, gi = DIRECT ? min(warp * 4 + g, G - 1) : warp * 4 + g;
-    const bool shadow = DIRECT && warp * 4 + g > gi;
+    constexpr uint32_t TS = TILE;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, W = blockDim.x >> 5, G = W * 4;
+    const uint32_t k = lane & 7u, g = lane >> 3, gi = warp * 4 + g;
     const uint32_t grp_mask = 0xffu << (g * 8), lt_mask = ((1u << k) - 1u) << (g * 8);
     const uint32_t below = 0xffffff00u | ((1u << k) - 1u), vsel = 0x6540u + g;
 
-    // ---- carve shared memory (addresses are 32-bit shared-space addresses) --------
-    // small per-stream pieces from the bottom; level-1 tables (4 KiB per warp, the
-    // four streams interleaved) end where the CRC tables begin, or at the top
-    const uint32_t s0 = smem_addr(ssm), top = s0 + dynamic_smem_bytes();
-    const uint32_t adv0 = stream_crc_adv(top), tab0 = stream_crc_slice(top);
-    const uint32_t bars_0 = (s0 + 15u) & ~15u;
-    const uint32_t stage_0 = bars_0 + G * 8 * NSL;
-    const uint32_t ring_0 = stage_0 + G * STG;
-    // DIRECT: thirteen 16 KiB tables leave 19 KiB of the window, some of it below the first 16 KiB
-    // boundary and some above the last table: the tables sit on boundaries (an index is OR-ed onto the
-    // base, which is what makes the step as short as the 12-stream instance's) and the rings fill both
-    // remainders, `ring_below` of them under the tables.
-    const uint32_t dl1_0 = (ring_0 + F_WIDE_BYTES - 1) & ~(F_WIDE_BYTES - 1);
-    const uint32_t ring_below = DIRECT ? min(G, (dl1_0 - ring_0) / RB) : G;
-    const uint32_t ring_above_0 = dl1_0 + G * F_WIDE_BYTES;
-    auto ring_of = [&](uint32_t grp) { return DIRECT && grp >= ring_below ? ring_above_0 + (grp - ring_below) * RB : ring_0 + grp * RB; };
-    const uint32_t cf_0 = (ring_0 + G * RB + CF_ALIGN - 1) & ~(CF_ALIGN - 1);
-    // compact: level 1 at the top; wide: 16 KiB tables from the first 16 KiB boundary up
-    const uint32_t l1_0 = DIRECT ? dl1_0 : WIDE ? (cf_0 + F_WIDE_BYTES - 1) & ~(F_WIDE_BYTES - 1)
-                               : ((CRC ? tab0 : top) & ~4095u) - (WARPS - (TOPL1 ? 1 : 0)) * 4096u;
-    // compact: this warp's 4 KiB of level 1 (the last warp's sits where the row-advance tables would)
-    auto l1_of = [&](uint32_t w) { return TOPL1 && w == WARPS - 1 ? adv0 : l1_0 + w * 4096u; };
-    const bool fits = DIRECT ? ring_above_0 + (G - ring_below) * RB <= top
-                    : WIDE ? l1_0 + (SHARED ? 1u : G) * F_WIDE_BYTES <= (CRC ? tab0 : top)
-                           : cf_0 + G * CFB <= l1_0 && (!TOPL1 || (adv0 & 4095u) == 0);
+    // ---- shared memory (addresses are 32-bit shared-space addresses) ----------------------
+    const uint32_t s0 = smem_addr(ssm);
+    const StreamSmem m_ = stream_smem(CFN, CRC, SINK, TR8, W);
+    const bool fits = s0 == F_SMEM_BASE && m_.end <= s0 + dynamic_smem_bytes();
     auto gen = [&](uint32_t sa) { return ssm + (sa - s0); };
-    const uint32_t l1_sa = SHARED ? l1_0 : WIDE ? l1_0 + gi * F_WIDE_BYTES : l1_of(warp) + g * 4;
+    const uint32_t tab0 = m_.crc;
+    const uint32_t l1_sa = SHARED ? m_.l1 : WIDE ? m_.l1 + gi * F_WIDE_BYTES : m_.l1 + warp * 4096u + g * 4;
     // (mixed sizes: the 1 KiB tables of the second planes first, then the half-KiB tables of the first planes)
-    auto cf_of = [&](uint32_t grp) { return HYB ? ((grp & 1u) ? cf_0 + (grp >> 1) * 1024u : cf_0 + (G / 2) * 1024u + (grp >> 1) * 512u)
-                                               : cf_0 + grp * CFB; };
+    auto cf_of = [&](uint32_t grp) { return HYB ? ((grp & 1u) ? m_.cf + (grp >> 1) * 1024u : m_.cf + (G / 2) * 1024u + (grp >> 1) * 512u)
+                                               : m_.cf + grp * (WIDE ? 0u : 4u * CFN); };
     const uint32_t cf_sa = cf_of(gi);
-    const uint32_t stage_sa = stage_0 + gi * STG;
+    const uint32_t stage_sa = m_.stage + gi * F_STAGE;
     // byte (i + g) & 3 of a state word goes through slice table 3 - ((i + g) & 3)
     CrcQuarters cq;
 #pragma unroll
     for (uint32_t i = 0; i < 4; i++) cq.b[i] = tab0 + 32u * (3u - ((i + g) & 3u)) + 4u * k;
     cq.rot = 8u * g;
-    const uint32_t tla = adv0 - 4096u;                              // crc_advance<0> adds 4 .. 7 KiB
+    const uint32_t tla = m_.adv - 4096u;                            // crc_advance<0> adds 4 .. 7 KiB
 
-    MRingT<NSL, stream_mirror(CFN, WARPS)> ring;
-    ring.sa = ring_of(gi);
-    ring.bars = reinterpret_cast<uint64_t *>(gen(bars_0)) + gi * NSL;
-
-    // ---- this group's stream ------------------------------------------------------
-    const uint32_t per_cta = a.per_cta ? a.per_cta : G;
-    const uint32_t idx = blockIdx.x * per_cta + gi;
     uint32_t limit = a.njobs;
-    if (a.count) {
-        limit = SINK == SINK_DELTA ? 2u * *a.count : *a.count;     // (delta: the count is of chunks, two streams each)
-        if (blockIdx.x * per_cta >= limit) return;    // the whole CTA: nothing of this class is left
+    if (a.count) limit = SINK == SINK_DELTA ? 2u * *a.count : *a.count;     // (delta: the count is of chunks, two streams each)
+    // A CTA of a shared-table archive takes one table's next 80 jobs; every other launch deals
+    // fours of jobs to warps, over the CTAs first.
+    const bool by_table = SHARED && a.tables != nullptr;
+    if (blockIdx.x * (by_table ? G : 4u) >= limit) return;          // the whole CTA has nothing to do
+
+    if (CRC && fits) {
+        // slice-by-4 tables, eight copies in the bank-quartered layout of CrcQuarters; then
+        // "advance by one row minus one lane unit"
+        uint32_t *ts = reinterpret_cast<uint32_t *>(gen(tab0));
+        // (crc_feed4q sends byte m of a state through table 3 - m, crc_word's order; the
+        // row multiplication is in crc_apply's order, byte m through table m)
+        for (uint32_t i = threadIdx.x; i < F_CRC_BYTES / 4; i += blockDim.x)
+            ts[i] = ROWMUL ? a.tabs->mul_row[3u - ((i >> 3) & 3u)][i >> 5] : a.tabs->slice[(i >> 3) & 3u][i >> 5];
+        if (SINK == SINK_F32) {
+            uint32_t *ta = reinterpret_cast<uint32_t *>(gen(m_.adv));
+            for (uint32_t i = threadIdx.x; i < 1024u; i += blockDim.x) ta[i] = (&a.tabs->adv_row4[0][0])[i];
+        }
     }
-    const bool have = gi < per_cta && idx < limit;
+    if (SHARED && fits && warp == 0) {
+        // one table for the CTA, built by its first warp: the launch's, or the one this CTA's chunks
+        // name (a shared-table archive); a table that does not validate fails every stream of the CTA
+        const uint8_t *h = by_table ? a.tables + (size_t)a.jobs[blockIdx.x * G].flags * F_TABLE_STRIDE : a.shared_hdr;
+        uint32_t f[8];
+        load_freqs(h, lane, f);
+        bool ok = build_table<true>(f, reinterpret_cast<uint32_t *>(gen(m_.l1)), nullptr, lane);
+        if (lane == 0) *reinterpret_cast<uint32_t *>(gen(m_.poison)) = (ok && h[0] == 'R' && h[1] == '1') ? 0u : 1u;
+    }
+    __syncthreads();
+    const bool poisoned = SHARED && fits && lds_u32(m_.poison) != 0;
+
+    const uint32_t quads = limit / 4 + ((limit & 3u) != 0), q_step = gridDim.x * W;       // (a by-table launch has one each)
+#pragma unroll 1
+    for (uint32_t quad = by_table ? blockIdx.x * W + warp : blockIdx.x + gridDim.x * warp; quad < quads; quad += q_step) {
+    // ---- this group's stream ------------------------------------------------------
+    const uint32_t idx = quad * 4 + g;
+    const bool have = idx < limit;
     // (SINK_DELTA: `order` lists chunks; stream 2c + p is plane p of chunk c)
     const uint32_t job = !(have && a.order) ? idx
                        : SINK == SINK_DELTA ? 2u * a.order[a.order_from_back ? a.njobs / 2 - 1 - (idx >> 1) : idx >> 1] + (idx & 1u)
@@ -384,7 +395,7 @@ __global__ void __launch_bounds__(WARPS * 32, CFN < 0 && SINK == SINK_BYTES ? 2 
     uint32_t slen = 0, n = 0, piece0 = 0;
     if (have) {
         if (SINK == SINK_DELTA) {
-            // groups 2c and 2c + 1 of the CTA take the two planes of its chunk c
+            // groups 2c and 2c + 1 of the warp take the two planes of its chunk c
             const DeltaJob j = a.djobs[job >> 1];
             soff = (job & 1u) ? j.src_b : j.src_a; slen = (job & 1u) ? j.len_b : j.len_a;
             doff = j.dst_off; moff = j.base_off; n = j.n; piece0 = j.piece0;
@@ -402,100 +413,76 @@ __global__ void __launch_bounds__(WARPS * 32, CFN < 0 && SINK == SINK_BYTES ? 2 
     }
     uint32_t st = ST_OK;
     if (!fits) { st = ST_BAD_SHAPE; n = 0; }          // the launch gave less shared memory than the layout needs
-    if (n != 0 && slen < LEAD) { st = ST_BAD_HEADER; n = 0; }
+    if (n != 0 && (slen < LEAD || poisoned)) { st = ST_BAD_HEADER; n = 0; }
     if (n == 0) slen = 0;
     const uint8_t *sbase = a.src + soff;
-    const uint32_t skew = (uint32_t)(reinterpret_cast<uintptr_t>(sbase) & 15u);
-    ring.abase = sbase - skew;
-    ring.valid_slots = n ? (skew + slen + F_SLOT - 1) / F_SLOT : 0;
-    ring.issued = 0; ring.ready = 0; ring.dead = false;
 
-    if (k == 0 && !shadow)
-        for (uint32_t j = 0; j < NSL; j++) mbar_init(&ring.bars[j], 1);
-    mbar_fence_init();
-    if (CRC && fits) {
-        // slice-by-4 tables, eight copies in the bank-quartered layout of CrcQuarters; then
-        // "advance by one row minus one lane unit"
-        uint32_t *ts = reinterpret_cast<uint32_t *>(gen(tab0)), *ta = reinterpret_cast<uint32_t *>(gen(adv0));
-        // (crc_feed4q sends byte m of a state through table 3 - m, crc_word's order; the
-        // row multiplication is in crc_apply's order, byte m through table m)
-        for (uint32_t i = threadIdx.x; i < 1024u << F_LOGS; i += WARPS * 32)
-            ts[i] = ROWMUL ? a.tabs->mul_row[3u - ((i >> 3) & 3u)][i >> 5] : a.tabs->slice[(i >> 3) & 3u][i >> 5];
-        const uint32_t *row_adv = SINK == SINK_F32 ? &a.tabs->adv_row4[0][0] : &a.tabs->adv_row[0][0];
-        if (!ROWMUL)
-            for (uint32_t i = threadIdx.x; i < 1024u; i += WARPS * 32) ta[i] = row_adv[i];
-    }
-    __syncthreads();
-
-    if (SHARED) {
-        // one table for the CTA, built by its first warp; a table that does not validate
-        // fails every stream of the CTA
-        uint32_t *poison = reinterpret_cast<uint32_t *>(gen(cf_0));
-        if (warp == 0) {
-            // one table for the launch, or the one this CTA's chunks name (a shared-table archive)
-            const uint8_t *h = (a.tables && a.jobs) ? a.tables + (size_t)a.jobs[blockIdx.x * per_cta].flags * F_TABLE_STRIDE : a.shared_hdr;
-            Tables tb{};
-            tb.wide = reinterpret_cast<uint32_t *>(gen(l1_0));
-            bool ok = fits && build_table<T_WIDE1>(
-                [&](uint32_t s) { return (uint32_t)h[4 + 2 * s] | ((uint32_t)h[5 + 2 * s] << 8); }, tb, lane);
-            if (lane == 0) *poison = (ok && h[0] == 'R' && h[1] == '1') ? 0u : 1u;
+    // the words follow table and states; the first four rounds are requested before the table is
+    // built, which hides their latency
+    Words<CFN, TR8> wd;
+    wd.sa = m_.tr + gi * tr_group(TR8);
+    wd.rd = wd.wr = 0;
+    wd.lo = wd.hi = 0;
+    uint32_t first[4][2];
+    uint32_t x = 0;
+    {
+        const uintptr_t at = reinterpret_cast<uintptr_t>(sbase + LEAD);
+        wd.sh = (uint32_t)(at & 3u) * 8u;
+        wd.next = reinterpret_cast<const uint32_t *>(at & ~uintptr_t(3)) + k;
+        const uint32_t words = n ? (slen - LEAD) / 2 : 0;
+        wd.left = (int32_t)((words + TR_ROUND - 1) / TR_ROUND);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            wd.request(true);
+            first[j][0] = wd.lo; first[j][1] = wd.hi;
         }
-        __syncthreads();
-        if (*poison && n) { st = ST_BAD_HEADER; n = 0; }
-        // the ring starts cold: slots 0..3 are requested the ordinary way
-        ring.valid_slots = n ? ring.valid_slots : 0;
-        __syncwarp();
+        wd.request(true);
         if (n) {
-            ring.issue(0, k == 0);
-            ring.require(skew + LEAD);
+            uint32_t s[1];
+            load_words_nc<1>(sbase + LEAD - STATE_BYTES + 4 * k, s);
+            x = s[0];
         }
-    }
-    // The stream's first 576 bytes or more (table + states, wherever the 16-byte
-    // boundary falls) land linearly from the ring's start: four copies, one on each of
-    // the first four slot barriers, which have then completed one phase -- as if ring
-    // slots 0..3 had been filled and consumed -- when normal ring operation takes over.
-    if (!SHARED && k == 0 && n && !shadow) {
-        for (uint32_t j = 0; j < 4; j++) {
-            mbar_expect_tx(&ring.bars[j], HS);
-            bulk_g2s_sa(ring.sa + HS * j, ring.abase + HS * j, HS, smem_addr(&ring.bars[j]));
-        }
-    }
-    __syncwarp();
-    if (!SHARED) {
-        if (n)
-            for (uint32_t j = 0; j < 4; j++)
-                if (!ring.dead && !mbar_wait(&ring.bars[j], 0)) ring.dead = true;
-        // the bytes of ring slots 0..3 are in place and their barriers are one phase on; a
-        // deeper ring's other slots and barriers are untouched
-        ring.issued = ring.ready = 4;
     }
 
     // ---- per-stream tables, built by the whole warp one stream at a time ------------
-#pragma unroll 1
-    for (uint32_t gg = 0; !SHARED && gg < 4; gg++) {
-        uint32_t on = __shfl_sync(0xffffffffu, n, gg * 8);
-        if (!on || (DIRECT && warp * 4 + gg >= G)) continue;
-        uint32_t sk = __shfl_sync(0xffffffffu, skew, gg * 8);
-        const uint32_t rsa = ring_of(warp * 4 + gg);
-        auto rd = [&](uint32_t o) { return lds_u8(rsa + o); };     // header sits in the first 548+15 bytes
-        Tables tb{};
-        auto freq_of = [&](uint32_t s) { return rd(sk + 4 + 2 * s) | (rd(sk + 5 + 2 * s) << 8); };
-        uint32_t nlive = 0, max_live = MAX_LIVE;
-        bool ok;
-        if (WIDE) {
-            tb.wide = reinterpret_cast<uint32_t *>(gen(l1_0 + (warp * 4 + gg) * F_WIDE_BYTES));
-            ok = build_table<T_WIDE1>(freq_of, tb, lane);
-        } else {
-            tb.l1 = reinterpret_cast<uint32_t *>(gen(l1_of(warp) + gg * 4));
-            tb.cf = reinterpret_cast<uint32_t *>(gen(cf_of(warp * 4 + gg)));
-            max_live = HYB ? ((gg & 1u) ? 256u : F_SMALL_LIVE) : MAX_LIVE;
-            ok = build_table<T_COMPACT, 4>(freq_of, tb, lane, (HYB ? !(gg & 1u) : CFN < 256) ? 8u * gg : 0u, &nlive, max_live);
+    if (!SHARED) {
+        uint32_t fr[4][8], magic[4];
+#pragma unroll
+        for (uint32_t gg = 0; gg < 4; gg++) {
+            const uint32_t on = __shfl_sync(0xffffffffu, n, gg * 8);
+            const uint8_t *h = reinterpret_cast<const uint8_t *>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(sbase), gg * 8));
+            magic[gg] = 0;
+#pragma unroll
+            for (int i = 0; i < 8; i++) fr[gg][i] = 0;
+            if (on) {
+                load_freqs(h, lane, fr[gg]);
+                magic[gg] = (uint32_t)h[0] | ((uint32_t)h[1] << 8);
+            }
         }
-        ok = ok && rd(sk) == 'R' && rd(sk + 1) == '1';
-        // an alphabet too large for this instance is the caller's mistake, not the stream's
-        if (!ok && gi == warp * 4 + gg) { st = nlive > max_live ? ST_BAD_SHAPE : ST_BAD_HEADER; n = 0; }
+#pragma unroll
+        for (uint32_t gg = 0; gg < 4; gg++) {
+            const uint32_t on = __shfl_sync(0xffffffffu, n, gg * 8);
+            uint32_t nlive = 0, max_live = 256;
+            bool ok = false;
+            uint32_t *tab = reinterpret_cast<uint32_t *>(gen(WIDE ? m_.l1 + (warp * 4 + gg) * F_WIDE_BYTES : m_.l1 + warp * 4096u + gg * 4));
+            if (WIDE) {
+                if (on) ok = build_table<true>(fr[gg], tab, nullptr, lane);
+            } else {
+                const bool small = HYB ? !(gg & 1u) : CFN < 256;
+                max_live = small ? F_SMALL_LIVE : 256u;
+                if (on)
+                    ok = build_table<false, 4>(fr[gg], tab, reinterpret_cast<uint32_t *>(gen(cf_of(warp * 4 + gg))), lane,
+                                               small ? 8u * gg : 0u, &nlive, max_live);
+                // a group without a stream runs along in full tiles: its lookups must stay in its tables
+                if (!ok && fits)
+                    for (uint32_t i = lane; i < 256; i += 32) tab[i * 4] = 0;
+            }
+            ok = ok && magic[gg] == ('R' | ('1' << 8));
+            // an alphabet too large for this instance is the caller's mistake, not the stream's
+            if (on && !ok && g == gg) { st = nlive > max_live ? ST_BAD_SHAPE : ST_BAD_HEADER; n = 0; }
+        }
+        __syncwarp();
     }
-    __syncwarp();
     if (SINK == SINK_DELTA) {
         // The two groups of a chunk walk its tiles together (they share the merge, and the
         // checksum is folded over both with shuffles): when one plane has been refused, the
@@ -503,10 +490,23 @@ __global__ void __launch_bounds__(WARPS * 32, CFN < 0 && SINK == SINK_BYTES ? 2 
         const uint32_t partner_n = __shfl_xor_sync(0xffffffffu, n, 8);
         if (partner_n == 0) n = 0;
     }
-
-    const uint32_t xo = ring.sa + skew + (SHARED ? 0u : HDR_BYTES) + 4 * k;
-    uint32_t x = lds_u8(xo) | (lds_u8(xo + 1) << 8) | (lds_u8(xo + 2) << 16) | (lds_u8(xo + 3) << 24);
-    uint32_t cursor = skew + LEAD;
+    uint32_t e = 0;
+    if (__any_sync(0xffffffffu, n != 0)) {
+        // the whole ring, so that a group without a stream finds nothing but bounded entries in it
+        const uint32_t lo = wd.lo, hi = wd.hi;
+        const uint32_t *next = wd.next;
+        const int32_t left = wd.left;
+        wd.left = 0;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            wd.lo = first[j][0]; wd.hi = first[j][1];
+            wd.round(l1_sa, cf_sa, k);
+        }
+        wd.lo = lo; wd.hi = hi; wd.next = next; wd.left = left;
+        if (n == 0) wd.retire();
+        e = lds_u32(ref_addr<CFN>(slot_ref<CFN>(x, l1_sa), cf_sa));
+        __syncwarp();
+    }
     uint8_t *out = a.dst + doff;
     const uint32_t al = (uint32_t)(reinterpret_cast<uintptr_t>(out) & 15u);
 
@@ -529,6 +529,7 @@ __global__ void __launch_bounds__(WARPS * 32, CFN < 0 && SINK == SINK_BYTES ? 2 
     // NEXT tile decodes (32 independent table lookups that hide behind the decode chain),
     // then that tile's words are XORed in.  SINK_F32 keeps one value, `acc`.
     uint32_t acc = 0, ra[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    uint32_t last_x = x, last_rd = 0;             // state and words consumed at the stream's end
 
     // ---- tiles of 128 symbols ---------------------------------------------------------
     const uint32_t warp_tiles = __reduce_max_sync(0xffffffffu, my_tiles);
@@ -537,14 +538,10 @@ __global__ void __launch_bounds__(WARPS * 32, CFN < 0 && SINK == SINK_BYTES ? 2 
         const uint32_t done = t * TS;
         const uint32_t rem = n > done ? n - done : 0;
         __syncwarp();
-        if (rem) {
-            ring.issue(cursor, k == 0 && !shadow);
-            ring.require(cursor + 2 * TS);         // every lane sees the completion itself
-        }
         // SINK_F32: the tile's stored bytes are requested before the decode, which hides
         // their latency (lane k: elements 16k .. 16k+15 of each of the three planes)
         uint32_t pr[SINK == SINK_F32 ? 3 : 1][5];
-        if (SINK == SINK_F32) {
+        if constexpr (SINK == SINK_F32) {
             const bool mine = rem > 16 * k;
 #pragma unroll
             for (int j = 0; j < 3; j++) {
@@ -554,51 +551,81 @@ __global__ void __launch_bounds__(WARPS * 32, CFN < 0 && SINK == SINK_BYTES ? 2 
                 for (int i = 0; i < 5; i++) pr[j][i] = mine ? __ldg(pq + i) : 0u;
             }
         }
-        const uint32_t caddr0 = ring.sa + ((RINGB & (RINGB - 1)) == 0 ? cursor & (RINGB - 1) : cursor % RINGB);
-        uint32_t caddr = caddr0;
-        // (lanes that never had a stream run along in full tiles; nothing of theirs is kept)
-        const bool full = __all_sync(0xffffffffu, rem >= TS);
-        // a decoded symbol goes to the group's staging row, or (DIRECT) straight to its output byte
-        uint8_t *const orow = out + done + k;
-        auto put = [&](uint32_t step, uint32_t e) {
-            if (DIRECT) { if (!shadow) orow[step * NLANES] = (uint8_t)e; }
-            else sts_u8(stage_sa + step * NLANES + k, e);
+        auto top_up = [&]() {
+            while (__any_sync(0xffffffffu, wd.low())) {
+                wd.round(l1_sa, cf_sa, k);
+                __syncwarp();
+            }
         };
+        auto put = [&](uint32_t step) { sts_u8(stage_sa + step * NLANES + k, e); };
+        auto fold = [&](uint32_t i) {
+            if (ROWMUL && i < NRA) ra[i] = crc_feed4q(cq, ra[i]);
+        };
+        // (a group that has no stream, or is done with it, runs along in the others' full tiles;
+        // nothing of its is kept)
+        const bool full = __all_sync(0xffffffffu, rem >= TS || rem == 0);
         if (full) {
 #pragma unroll
-            for (uint32_t s4 = 0; s4 < TS / NLANES; s4 += 4) {
-                uint32_t hist = 0, e;
-                e = stream_step4<CFN_STEP, true>(x, hist, caddr, l1_sa, cf_sa, below, vsel);
-                put(s4, e);
-                e = stream_step4<CFN_STEP, false>(x, hist, caddr, l1_sa, cf_sa, below, vsel);
-                put(s4 + 1, e);
-                if (ROWMUL && (s4 >> 1) < NRA) ra[s4 >> 1] = crc_feed4q(cq, ra[s4 >> 1]);
-                e = stream_step4<CFN_STEP, false>(x, hist, caddr, l1_sa, cf_sa, below, vsel);
-                put(s4 + 2, e);
-                e = stream_step4<CFN_STEP, false>(x, hist, caddr, l1_sa, cf_sa, below, vsel);
-                put(s4 + 3, e);
-                if (ROWMUL && (s4 >> 1) < NRA) ra[(s4 >> 1) + 1] = crc_feed4q(cq, ra[(s4 >> 1) + 1]);
-                caddr += 2 * __popc(hist);
+            for (uint32_t s8 = 0; s8 < TS / NLANES; s8 += 8) {
+                // eight steps: two blocks, and where warps are few a round of translation between the
+                // steps of the first (where they are many, top_up does all of them: fewer instructions)
+                constexpr bool WOVEN = TR8;
+                top_up();
+                uint32_t base = wd.block(), hist = 0;
+                if (WOVEN) wd.part1();
+                put(s8);
+                stream_step4<CFN, TR8, true>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                if (WOVEN) wd.part2(l1_sa);
+                put(s8 + 1);
+                stream_step4<CFN, TR8, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                fold(s8 / 2);
+                put(s8 + 2);
+                stream_step4<CFN, TR8, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                if (WOVEN) wd.part3(cf_sa, k);
+                put(s8 + 3);
+                stream_step4<CFN, TR8, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                fold(s8 / 2 + 1);
+                wd.rd += tr_entry(TR8) * __popc(hist);
+                __syncwarp();
+                top_up();
+                base = wd.block();
+                hist = 0;
+                put(s8 + 4);
+                stream_step4<CFN, TR8, true>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                put(s8 + 5);
+                stream_step4<CFN, TR8, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                fold(s8 / 2 + 2);
+                put(s8 + 6);
+                stream_step4<CFN, TR8, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                put(s8 + 7);
+                stream_step4<CFN, TR8, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                fold(s8 / 2 + 3);
+                wd.rd += tr_entry(TR8) * __popc(hist);
             }
         } else {
-            if (ROWMUL) {
 #pragma unroll
-                for (int i = 0; i < NRA; i++) ra[i] = crc_feed4q(cq, ra[i]);
-            }
+            for (int i = 0; i < NRA; i++) fold(i);
 #pragma unroll 1
-            for (uint32_t s = 0; s < TS / NLANES; s++) {
-                bool active = s * NLANES + k < rem;
-                uint32_t e = stream_step<CFN_STEP>(x, caddr, l1_sa, cf_sa, lt_mask, grp_mask, active);
-                if (active) put(s, e);
+            for (uint32_t s4 = 0; s4 < TS / NLANES; s4 += 4) {
+                top_up();
+                uint32_t base = wd.block();
+                const uint32_t base0 = base;
+#pragma unroll 1
+                for (uint32_t s = s4; s < s4 + 4; s++) {
+                    const bool active = s * NLANES + k < rem;
+                    if (active) put(s);
+                    stream_step<CFN, TR8>(x, e, base, l1_sa, cf_sa, lt_mask, grp_mask, active);
+                }
+                wd.rd += base - base0;
             }
         }
-        cursor += caddr - caddr0;
         __syncwarp();
-        if (!rem || DIRECT) continue;
+        if (t + 1 == my_tiles) { last_x = x; last_rd = wd.rd; wd.retire(); }
+        if (!rem) continue;
         if (SINK == SINK_DELTA) {
             // ---- both planes' symbols of this lane's eight elements, merge, XOR the base, write, checksum
-            const uint32_t pair_sa = stage_0 + (gi & ~1u) * STG + 8u * j16;
-            const uint2 ea = lds_u64(pair_sa), eb = lds_u64(pair_sa + STG);
+            const uint32_t pair_sa = m_.stage + (gi & ~1u) * F_STAGE + 8u * j16;
+            const uint2 ea = lds_u64(pair_sa), eb = lds_u64(pair_sa + F_STAGE);
             uint32_t w[4];
             bf16_merge4(ea.x, eb.x, w[0], w[1]);
             bf16_merge4(ea.y, eb.y, w[2], w[3]);
@@ -656,33 +683,21 @@ __global__ void __launch_bounds__(WARPS * 32, CFN < 0 && SINK == SINK_BYTES ? 2 
             }
             continue;
         }
-        constexpr uint32_t PER = TS / NLANES;                  // this lane's symbols of the tile: 16 or 32
-        uint4 evs[PER / 16];
-#pragma unroll
-        for (uint32_t q = 0; q < PER / 16; q++) evs[q] = lds_u128(stage_sa + PER * k + 16 * q);
-        const uint4 ev = evs[0];
-
+        const uint4 ev = lds_u128(stage_sa + 16 * k);
+        const uint32_t ew[4] = {ev.x, ev.y, ev.z, ev.w};
         if (SINK == SINK_BYTES) {
             if (rem >= TS && al == 0) {
-#pragma unroll
-                for (uint32_t q = 0; q < PER / 16; q++)
-                    *reinterpret_cast<uint4 *>(out + done + k * PER + 16 * q) = evs[q];
+                *reinterpret_cast<uint4 *>(out + done + 16 * k) = ev;
             } else {
                 const uint32_t cnt = rem < TS ? rem : TS;
 #pragma unroll
-                for (uint32_t q = 0; q < PER / 16; q++) {
-                    const uint32_t ew[4] = {evs[q].x, evs[q].y, evs[q].z, evs[q].w};
-#pragma unroll
-                    for (uint32_t i = 0; i < 16; i++)
-                        if (k * PER + 16 * q + i < cnt)
-                            out[done + k * PER + 16 * q + i] = (uint8_t)(ew[i >> 2] >> (8 * (i & 3)));
-                }
+                for (uint32_t i = 0; i < 16; i++)
+                    if (16 * k + i < cnt) out[done + 16 * k + i] = (uint8_t)(ew[i >> 2] >> (8 * (i & 3)));
             }
             continue;
         }
 
-        const uint32_t ew[4] = {ev.x, ev.y, ev.z, ev.w};
-        if (SINK == SINK_F32) {
+        if constexpr (SINK == SINK_F32) {
             // ---- interleave with the three stored planes, write, checksum ------------
             const uint32_t ve = rem > 16 * k ? min(rem - 16 * k, 16u) : 0u;   // valid elements of this lane
             uint32_t pw[3][4];
@@ -812,17 +827,18 @@ __global__ void __launch_bounds__(WARPS * 32, CFN < 0 && SINK == SINK_BYTES ? 2 
     }
 
     // ---- verdict -----------------------------------------------------------------------
-    const uint32_t all_rest = __ballot_sync(0xffffffffu, x == RANS_LOW) & grp_mask;
-    if (have && k == 0 && !shadow) {
+    const uint32_t all_rest = __ballot_sync(0xffffffffu, last_x == RANS_LOW) & grp_mask;
+    if (have && k == 0) {
         if (st == ST_OK && n) {
-            const uint32_t used = cursor - skew;
-            if (ring.dead) st = ST_TIMEOUT;
-            else if (used > slen) st = ST_OVERRUN;
+            const uint32_t used = LEAD + 2 * (last_rd / tr_entry(TR8));
+            if (used > slen) st = ST_OVERRUN;
             else if (used != slen || all_rest != grp_mask) st = ST_SLACK;
         }
         if (a.status) a.status[job] = st;
         if (a.any_bad && st != ST_OK && st != ST_SLACK) atomicOr(a.any_bad, 1u);
     }
+    __syncwarp();
+    }   // the warp's next four streams
 }
 
 // Sort a launch's streams by alphabet size, on the device: one warp per stream counts the

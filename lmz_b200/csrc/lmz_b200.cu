@@ -13,7 +13,6 @@
 #include <mutex>
 
 #include "../../include/lmz_b200.h"
-#include "rans_kernel.cuh"
 #include "chunk_kernels.cuh"
 #include "cond_kernels.cuh"
 #include "fused_kernel.cuh"
@@ -75,26 +74,6 @@ static int opt_in_smem(K kernel, uint32_t bytes, bool *done /* [64] by device */
     return LMZ_GPU_OK;
 }
 
-constexpr int WARPS_NARROW = 4;    // 2 CTAs/SM: 32 streams resident
-constexpr int WARPS_WIDE = 8;
-// Batches at least this large are occupancy-bound and take the compact tables;
-// smaller ones are latency-bound per stream and keep the shorter narrow lookup.
-constexpr unsigned COMPACT_MIN_JOBS = 148 * 32 * 2;
-
-template <int MODE, int WARPS>
-static int launch_rans_mode(const RansArgs &a, cudaStream_t cs)
-{
-    static bool done[64];
-    constexpr uint32_t shm = rans_smem_bytes<MODE>(WARPS);
-    int rc = opt_in_smem(k_rans<MODE, WARPS>, shm, done);
-    if (rc) return rc;
-    unsigned blocks = (a.njobs + WARPS * 4 - 1) / (WARPS * 4);
-    k_rans<MODE, WARPS><<<blocks, WARPS * 32, shm, cs>>>(a);
-    cudaError_t le = cudaGetLastError();
-    if (le != cudaSuccess) return fail_cuda("launch k_rans", le);
-    return LMZ_GPU_OK;
-}
-
 // k_stream takes all the shared memory one CTA may have and lays its tables out from
 // both ends, counting on the window starting F_SMEM_BASE bytes in (what the
 // driver reserves per CTA on this architecture).
@@ -115,52 +94,67 @@ static int stream_smem_ok()
     return LMZ_GPU_OK;
 }
 
-// CFN = 128 is for streams the caller knows to have at most F_SMALL_LIVE live symbols;
-// CFN = 0 is the per-stream wide table (12 streams per SM), CFN = -1 one wide table per CTA.
 static int sm_count(int *out);
 
-template <int SINK, bool CRC, int CFN, int WARPS_ = 0>
-static int launch_stream(const StreamArgs &a0, cudaStream_t cs)
+template <int SINK, bool CRC, int CFN, bool TR8>
+static int launch_stream_as(const StreamArgs &a, uint32_t grid, uint32_t W, cudaStream_t cs)
 {
-    if (a0.njobs == 0) return LMZ_GPU_OK;
-    StreamArgs a = a0;
-    constexpr int WARPS = WARPS_ ? WARPS_ : stream_warps(CFN, CRC, SINK);
     static bool done[64];
-    int rc = stream_smem_ok();
+    const uint32_t shm = stream_smem(CFN, CRC, SINK, TR8, W).end - F_SMEM_BASE;
+    int rc = opt_in_smem(k_stream<SINK, CRC, CFN, TR8>, F_SMEM_DYN, done);
     if (rc) return rc;
-    // the shared-table instance needs little shared memory and runs two CTAs per SM
-    constexpr bool PAIRED = CFN < 0 && SINK == SINK_BYTES;      // two CTAs per SM
-    constexpr uint32_t shm = PAIRED ? 2u * F_WIDE_BYTES + WARPS * 4 * stream_group_bytes(CFN) : F_SMEM_DYN;
-    rc = opt_in_smem(k_stream<SINK, CRC, WARPS, CFN>, shm, done);
-    if (rc) return rc;
-    constexpr bool DIRECT = stream_direct(CFN, WARPS);
-    constexpr unsigned groups = DIRECT ? F_DIRECT_GROUPS : stream_groups(CFN, WARPS);
-    unsigned per = groups;
-    if (a.per_cta) {
-        per = a.per_cta;          // the caller's job list is laid out for this many streams per CTA
-    } else {
-        // as many waves of CTAs as full CTAs would need, the streams spread evenly over them
-        // (when the device holds the count, as if every job of the launch were of this class)
-        int sms = 0;
-        rc = sm_count(&sms);
-        if (rc) return rc;
-        const unsigned slots = (unsigned)sms * (PAIRED ? 2u : 1u);
-        const unsigned waves = (a.njobs + slots * groups - 1) / (slots * groups);
-        per = (a.njobs + waves * slots - 1) / (waves * slots);
-        if (!DIRECT) per = (per + 3u) & ~3u;
-        if (per > groups) per = groups;
-    }
-    a.per_cta = per;
-    unsigned blocks = (a.njobs + per - 1) / per;
-    k_stream<SINK, CRC, WARPS, CFN><<<blocks, WARPS * 32, shm, cs>>>(a);
+    k_stream<SINK, CRC, CFN, TR8><<<grid, W * 32, shm, cs>>>(a);
     cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) return fail_cuda("launch k_stream", le);
     return LMZ_GPU_OK;
 }
 
+// CFN = 128 is for streams the caller knows to have at most F_SMALL_LIVE live symbols;
+// CFN = 0 is the per-stream wide table, CFN = -1 one wide table per CTA.
+template <int SINK, bool CRC, int CFN>
+static int launch_stream(const StreamArgs &a, cudaStream_t cs)
+{
+    if (a.njobs == 0) return LMZ_GPU_OK;
+    int rc = stream_smem_ok();
+    if (rc) return rc;
+    int sms = 0;
+    rc = sm_count(&sms);
+    if (rc) return rc;
+    if (CFN < 0 && a.tables)          // the job list is laid out 80 to a CTA
+        return launch_stream_as<SINK, CRC, CFN, true>(a, a.njobs / (F_SHARED_SINK_WARPS * 4), F_SHARED_SINK_WARPS, cs);
+    // At most one CTA per SM; its warps take four streams at a time.  As many rounds of fours as the
+    // fullest CTA would need, the warps of a CTA just enough for them (when the device holds the count,
+    // as if every job of the launch were of this class).
+    const uint32_t quads = (a.njobs + 3) / 4, grid = quads < (uint32_t)sms ? quads : (uint32_t)sms;
+    auto waves = [&](uint32_t most) { return (quads + grid * most - 1) / (grid * most); };
+    auto warps = [&](uint32_t most) { return (quads + grid * waves(most) - 1) / (grid * waves(most)); };
+    // 8-byte ring entries make the shorter step, 4-byte ones leave room for more warps: those are
+    // taken where they save a round (one B200, 64 KiB BF16 chunks with checksums, 8-byte against
+    // 4-byte entries: 180 chunks per SM 2160 against 1880 us, 34 per SM 605 against 675).
+    constexpr uint32_t most8 = stream_warps(CFN, CRC, SINK, true);
+    if constexpr (CFN > 0) {
+        constexpr uint32_t most4 = stream_warps(CFN, CRC, SINK, false);
+        if (waves(most4) < waves(most8)) return launch_stream_as<SINK, CRC, CFN, false>(a, grid, warps(most4), cs);
+    }
+    return launch_stream_as<SINK, CRC, CFN, true>(a, grid, warps(most8), cs);
+}
+
 // `force_mode` < 0 picks by batch size.
 static std::atomic<int> g_force_table_mode{-1};
 
+
+// A batch of streams to decode to bytes.
+struct RansArgs {
+    const uint8_t *src;         // compressed bytes (16-byte aligned base, PAD_BYTES of slack after)
+    const StreamJob *jobs;      // njobs descriptors, or NULL to use `offs`/`plane`
+    const uint64_t *offs;       // reference layout: (offset, length) pairs
+    uint32_t plane;             // symbols per stream when `offs` is used
+    uint32_t njobs;
+    uint8_t *dst;
+    const uint8_t *shared_hdr;  // 516-byte table shared by every stream
+    uint32_t *status;           // one word per job, may be NULL
+    uint32_t *any_bad;          // set non-zero when a job fails hard, may be NULL
+};
 
 static StreamArgs as_stream_args(const RansArgs &a)
 {
@@ -235,40 +229,28 @@ static int launch_compact_sorted(const RansArgs &a, cudaStream_t cs)
     return rc;
 }
 
-// A launch that gives every stream an SM slot at once with 12 streams per SM is bound by
-// the length of the per-symbol dependent chain alone, and a wide table per stream shortens
-// it by one shared-memory round trip.  (13 such tables fit an SM too, but then not the long
-// tiles that pay for the instance: above 12 per SM the narrow tables are faster.)
+// Streams that carry their own table.  Up to 12 per SM a wide table each fits, and a step is one
+// lookup shorter; up to 76 per SM the full-size compact tables take the launch in one round,
+// whatever the alphabets; above that small alphabets go to the denser instance.
+constexpr unsigned WIDE_PER_SM = 4 * stream_warps(0, false, SINK_BYTES, true);
+constexpr unsigned COMPACT_PER_SM = 4 * stream_warps(256, false, SINK_BYTES, true);
+
 static int launch_rans(const RansArgs &a, cudaStream_t cs, bool may_alloc = true)
 {
     if (a.njobs == 0) return LMZ_GPU_OK;
     int sms = 0;
     int rc = sm_count(&sms);
     if (rc) return rc;
-    if (a.shared_hdr) {
-        // one table for the whole launch: the k_stream instance (128 streams per SM, leaner
-        // steps) once every SM is full, the plain kernel (shorter chain on a lone warp) below
-        const int forced = g_force_table_mode.load(std::memory_order_relaxed);
-        const bool plain = forced == T_NARROW || (forced < 0 && a.njobs < (unsigned)sms * 128u);
-        return plain ? launch_rans_mode<T_WIDE, WARPS_WIDE>(a, cs)
-                     : launch_stream<SINK_BYTES, false, -1>(as_stream_args(a), cs);
-    }
+    const StreamArgs sa = as_stream_args(a);
+    if (a.shared_hdr) return launch_stream<SINK_BYTES, false, -1>(sa, cs);
     const int forced = g_force_table_mode.load(std::memory_order_relaxed);
-    int mode = forced;
-    if (mode < 0)
-        mode = a.njobs <= (unsigned)sms * F_WIDE_GROUPS ? T_WIDE1
-             : a.njobs <= (unsigned)sms * F_DIRECT_GROUPS ? T_WIDE13
-             : a.njobs >= COMPACT_MIN_JOBS ? T_COMPACT : T_NARROW;
-    if (mode == T_WIDE1) return launch_stream<SINK_BYTES, false, 0>(as_stream_args(a), cs);
-    if (mode == T_WIDE13) return launch_stream<SINK_BYTES, false, 0, 4>(as_stream_args(a), cs);
-    if (mode == T_COMPACT) {
-        if (may_alloc && forced < 0) {
-            int rc = launch_compact_sorted(a, cs);
-            if (rc != 1) return rc;
-        }
-        return launch_stream<SINK_BYTES, false, 256>(as_stream_args(a), cs);
+    const bool wide = forced < 0 ? a.njobs <= (unsigned)sms * WIDE_PER_SM : forced == T_WIDE1 || forced == T_WIDE13;
+    if (wide) return launch_stream<SINK_BYTES, false, 0>(sa, cs);
+    if (may_alloc && forced < 0 && a.njobs > (unsigned)sms * COMPACT_PER_SM) {
+        rc = launch_compact_sorted(a, cs);
+        if (rc != 1) return rc;
     }
-    return launch_rans_mode<T_NARROW, WARPS_NARROW>(a, cs);
+    return launch_stream<SINK_BYTES, false, 256>(sa, cs);
 }
 
 // ------------------------------------------------------- the reference's nine
@@ -396,7 +378,7 @@ API int lmz_gpu_set_table_mode(int mode)
 {
     if (mode != -1 && mode != T_NARROW && mode != T_COMPACT && mode != T_WIDE1 && mode != T_WIDE13)
         return fail_msg(LMZ_GPU_EUNSUPPORTED,
-                        "table mode must be -1 (auto), 0 (narrow), 2 (compact), 3 (wide per stream) or 4 (wide, 13 per SM)");
+                        "table mode must be -1 (auto), 0 or 2 (compact), 3 or 4 (wide per stream)");
     g_force_table_mode.store(mode, std::memory_order_relaxed);
     return LMZ_GPU_OK;
 }
