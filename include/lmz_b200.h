@@ -69,10 +69,11 @@ int lmz_gpu_decode_batch_dev(const void *d_hdr, const void *d_streams, const voi
                              unsigned nstr, unsigned plane, void *d_out, void *cuda_stream,
                              unsigned tpb);
 
-/* lmz/gpu/lmzgpu.cu:478-527 -- the same for host memory: allocate, copy in,
- * decode, synchronise, copy out, free.  A stream that is malformed or
- * truncated returns LMZ_GPU_EBADSTREAM (the reference detects the former on
- * the host and returns garbage for the latter). */
+/* lmz/gpu/lmzgpu.cu:478-527 -- the same for host memory: copy in, decode, copy out,
+ * wait.  A stream that is malformed or truncated returns LMZ_GPU_EBADSTREAM (the
+ * reference detects the former on the host and returns garbage for the latter); `out`
+ * is then as it was, unless it came from lmz_gpu_host_alloc.  Device memory and stream of
+ * a call are kept for the next one, within bounds (see lmz_gpu_trim). */
 int lmz_gpu_decode_batch(const void *hdr, const void *streams, size_t nbytes, const void *off,
                          unsigned nstr, unsigned plane, void *out);
 
@@ -81,6 +82,18 @@ int lmz_gpu_decode_batch(const void *hdr, const void *streams, size_t nbytes, co
 /* No counterpart in the reference (which always uses device 0): make `device`
  * current for this thread.  All other calls act on the current device. */
 int lmz_gpu_set_device(int device);
+
+/* No counterpart in the reference.  Page-locked host memory for results: as `out` of
+ * lmz_gpu_decode_batch it is written by the copy engine directly.  NULL when there is
+ * none.  Freed memory is kept for the next call, at most 512 MiB of it; any thread may
+ * free it. */
+void *lmz_gpu_host_alloc(size_t bytes);
+void lmz_gpu_host_free(void *p);
+
+/* No counterpart in the reference.  Give back what the host-memory entry points keep
+ * between calls: idle result memory, and per device up to four idle workspaces with
+ * device buffers of at most 256 MiB each. */
+void lmz_gpu_trim(void);
 
 /* No counterpart in the reference: choose the per-stream decode-table layout for
  * streams that carry their own table.  -1 = by batch size (default), 0 or 2 = compact

@@ -1,0 +1,245 @@
+// lmz_gpu_decode_batch for host memory (included by lmz_b200.cu), and the memory it keeps.
+//
+// A call of a few planes decodes in tens of microseconds, while allocating and freeing its
+// buffers took 0.8 ms (one B200, 7 streams of 4 KiB: 830 us a call, of which 60 us kernel).
+// So a call borrows a workspace -- a stream, a device buffer, a small page-locked block -- and
+// gives it back; results that this library's callers do not bring a buffer for come in
+// page-locked memory that the copy engine writes itself.  Both are bounded: at most
+// KEPT_WORKSPACES idle workspaces per device with device buffers of at most KEPT_DEVICE_BYTES,
+// at most KEPT_HOST_BYTES of idle result memory; what is over goes back to the driver at once,
+// and lmz_gpu_trim() returns the rest.  A workspace belongs to one call at a time.
+
+namespace {
+
+constexpr size_t KEPT_DEVICE_BYTES = (size_t)256 << 20;
+constexpr size_t KEPT_HOST_BYTES = (size_t)512 << 20;
+constexpr size_t KEPT_WORKSPACES = 4;
+
+size_t size_class(size_t bytes)
+{
+    size_t c = 4096;
+    while (c < bytes) c <<= 1;
+    return c;
+}
+
+struct Workspace {
+    int device = -1;
+    cudaStream_t stream = nullptr;
+    uint8_t *dev = nullptr;
+    size_t dev_bytes = 0;
+    uint8_t *pin = nullptr;          // offsets in, verdict out
+    size_t pin_bytes = 0;
+
+    cudaError_t need(size_t device_bytes, size_t pinned_bytes)
+    {
+        cudaError_t e = cudaSuccess;
+        if (!stream) e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+        if (e == cudaSuccess && dev_bytes < device_bytes) {
+            if (dev) cudaFree(dev);
+            dev = nullptr; dev_bytes = 0;
+            const size_t c = device_bytes <= KEPT_DEVICE_BYTES ? size_class(device_bytes) : device_bytes;
+            e = cudaMalloc((void **)&dev, c);
+            if (e == cudaSuccess) dev_bytes = c;
+        }
+        if (e == cudaSuccess && pin_bytes < pinned_bytes) {
+            if (pin) cudaFreeHost(pin);
+            pin = nullptr; pin_bytes = 0;
+            const size_t c = size_class(pinned_bytes);
+            e = cudaMallocHost((void **)&pin, c);
+            if (e == cudaSuccess) pin_bytes = c;
+        }
+        return e;
+    }
+    void drop()
+    {
+        if (dev) cudaFree(dev);
+        if (pin) cudaFreeHost(pin);
+        if (stream) cudaStreamDestroy(stream);
+        *this = Workspace{};
+    }
+};
+
+struct HostPool {
+    std::mutex mu;
+    std::vector<Workspace> idle;
+    std::unordered_map<void *, size_t> lent;               // result memory in callers' hands
+    std::unordered_multimap<size_t, void *> spare;         // idle result memory by size class
+    size_t spare_bytes = 0;
+};
+HostPool &host_pool()
+{
+    static HostPool *p = new HostPool;      // (never destroyed: calls may still run while the process exits)
+    return *p;
+}
+
+// A workspace for one call, given back when the call ends -- with its stream idle.
+struct Borrowed {
+    Workspace w;
+    bool sound = false;
+    explicit Borrowed(int device)
+    {
+        HostPool &p = host_pool();
+        std::lock_guard<std::mutex> lock(p.mu);
+        for (size_t i = 0; i < p.idle.size(); i++)
+            if (p.idle[i].device == device) {
+                w = p.idle[i];
+                p.idle.erase(p.idle.begin() + i);
+                break;
+            }
+        w.device = device;
+    }
+    ~Borrowed()
+    {
+        if (w.stream) cudaStreamSynchronize(w.stream);
+        if (sound && w.dev_bytes <= KEPT_DEVICE_BYTES) {
+            HostPool &p = host_pool();
+            std::lock_guard<std::mutex> lock(p.mu);
+            size_t mine = 0;
+            for (const Workspace &o : p.idle) mine += o.device == w.device;
+            if (mine < KEPT_WORKSPACES) {
+                p.idle.push_back(w);
+                return;
+            }
+        }
+        w.drop();
+    }
+};
+
+bool is_lent(const void *p, size_t bytes)
+{
+    HostPool &pool = host_pool();
+    std::lock_guard<std::mutex> lock(pool.mu);
+    auto it = pool.lent.find(const_cast<void *>(p));
+    return it != pool.lent.end() && it->second >= bytes;
+}
+
+}  // namespace
+
+API void *lmz_gpu_host_alloc(size_t bytes)
+{
+    const size_t c = size_class(bytes);
+    HostPool &p = host_pool();
+    {
+        std::lock_guard<std::mutex> lock(p.mu);
+        auto it = p.spare.find(c);
+        if (it != p.spare.end()) {
+            void *q = it->second;
+            p.spare.erase(it);
+            p.spare_bytes -= c;
+            p.lent[q] = c;
+            return q;
+        }
+    }
+    void *q = nullptr;
+    if (cudaHostAlloc(&q, c, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    std::lock_guard<std::mutex> lock(p.mu);
+    p.lent[q] = c;
+    return q;
+}
+
+API void lmz_gpu_host_free(void *q)
+{
+    HostPool &p = host_pool();
+    {
+        std::lock_guard<std::mutex> lock(p.mu);
+        auto it = p.lent.find(q);
+        if (it == p.lent.end()) return;
+        const size_t c = it->second;
+        p.lent.erase(it);
+        if (p.spare_bytes + c <= KEPT_HOST_BYTES) {
+            p.spare.emplace(c, q);
+            p.spare_bytes += c;
+            return;
+        }
+    }
+    cudaFreeHost(q);
+}
+
+API void lmz_gpu_trim(void)
+{
+    HostPool &p = host_pool();
+    std::vector<Workspace> idle;
+    std::vector<void *> spare;
+    {
+        std::lock_guard<std::mutex> lock(p.mu);
+        idle.swap(p.idle);
+        for (auto &kv : p.spare) spare.push_back(kv.second);
+        p.spare.clear();
+        p.spare_bytes = 0;
+    }
+    int dev = 0;
+    const bool had = cudaGetDevice(&dev) == cudaSuccess;
+    for (Workspace &w : idle) {
+        cudaSetDevice(w.device);
+        w.drop();
+    }
+    if (had) cudaSetDevice(dev);
+    for (void *q : spare) cudaFreeHost(q);
+}
+
+API int lmz_gpu_decode_batch(const void *hdr, const void *streams, size_t nbytes, const void *off,
+                             unsigned nstr, unsigned plane, void *out)
+{
+    if (nstr == 0) return LMZ_GPU_OK;
+    if (plane == 0) return fail_msg(LMZ_GPU_EUNSUPPORTED, "plane is zero");
+    if (int rc = device_ready()) return rc;
+    // every (offset, length) pair must lie inside the buffer, and a length must fit the
+    // 32 bits the kernels carry it in
+    const uint64_t *pairs = static_cast<const uint64_t *>(off);
+    for (unsigned i = 0; i < nstr; i++) {
+        const uint64_t at = pairs[2 * i], len = pairs[2 * i + 1];
+        if (at > nbytes || len > nbytes - at) return fail_msg(LMZ_GPU_EBADSTREAM, "a stream lies outside the buffer");
+        if (len >> 32) return fail_msg(LMZ_GPU_EUNSUPPORTED, "a stream is 4 GiB or longer");
+    }
+    int device = 0;
+    CK("cudaGetDevice", cudaGetDevice(&device));
+
+    // device buffer: offsets | shared table | verdict | streams + slack | plaintext + its verdict
+    auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
+    const size_t out_bytes = (size_t)nstr * plane, table_bytes = (size_t)nstr * 16;
+    const size_t at_hdr = table_bytes, at_verdict = (at_hdr + (hdr ? HDR_BYTES : 0) + 15) & ~(size_t)15;
+    const size_t head_bytes = at_verdict + 16, at_src = up(head_bytes), at_out = up(at_src + nbytes + PAD_BYTES);
+    Borrowed b(device);
+    Workspace &w = b.w;
+    if (cudaError_t e = w.need(at_out + out_bytes, head_bytes + 16)) {
+        cudaGetLastError();
+        return fail_cuda("memory for the batch", e);
+    }
+    uint8_t *d = w.dev;
+    memcpy(w.pin, off, table_bytes);
+    if (hdr) memcpy(w.pin + at_hdr, hdr, HDR_BYTES);
+    memset(w.pin + at_verdict, 0, 16);
+    uint32_t *verdict = reinterpret_cast<uint32_t *>(w.pin + head_bytes);
+    *verdict = 0;
+    CK("copy offsets in", cudaMemcpyAsync(d, w.pin, head_bytes, cudaMemcpyHostToDevice, w.stream));
+    CK("copy streams in", cudaMemcpyAsync(d + at_src, streams, nbytes, cudaMemcpyHostToDevice, w.stream));
+    RansArgs a{};
+    a.src = d + at_src;
+    a.offs = reinterpret_cast<const uint64_t *>(d);
+    a.plane = plane;
+    a.njobs = nstr;
+    a.dst = d + at_out;
+    a.shared_hdr = hdr ? d + at_hdr : nullptr;
+    a.any_bad = reinterpret_cast<uint32_t *>(d + at_verdict);
+    if (int rc = launch_rans(a, w.stream)) return rc;
+    CK("copy the verdict out", cudaMemcpyAsync(verdict, d + at_verdict, 4, cudaMemcpyDeviceToHost, w.stream));
+    // memory of this library's own takes the plaintext at once; a caller's buffer only if all is well
+    const bool direct = is_lent(out, out_bytes);
+    if (direct) CK("copy plaintext out", cudaMemcpyAsync(out, d + at_out, out_bytes, cudaMemcpyDeviceToHost, w.stream));
+    CK("decode", cudaStreamSynchronize(w.stream));
+    b.sound = true;
+    if (*verdict) {
+        // (the device's word is enough to refuse the batch; the host looks again for the reason)
+        if (!hdr)
+            if (int rc = lmz_gpu_validate(streams, off, nstr)) return rc;
+        return fail_msg(LMZ_GPU_EBADSTREAM, "a stream is malformed or truncated");
+    }
+    if (!direct) {
+        CK("copy plaintext out", cudaMemcpyAsync(out, d + at_out, out_bytes, cudaMemcpyDeviceToHost, w.stream));
+        CK("copy plaintext out", cudaStreamSynchronize(w.stream));
+    }
+    return LMZ_GPU_OK;
+}

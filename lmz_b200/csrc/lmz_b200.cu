@@ -11,6 +11,8 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <unordered_map>
+#include <vector>
 
 #include "../../include/lmz_b200.h"
 #include "chunk_kernels.cuh"
@@ -314,63 +316,7 @@ API int lmz_gpu_decode_batch_dev(const void *d_hdr, const void *d_streams, const
     return launch_rans(a, (cudaStream_t)cuda_stream);
 }
 
-namespace {
-// Device memory that lives as long as one host-form call.
-struct Transient {
-    void *p = nullptr;
-    ~Transient() { if (p) cudaFree(p); }
-    cudaError_t take(size_t bytes) { return cudaMalloc(&p, bytes ? bytes : 1); }
-    template <class T> T *as() const { return static_cast<T *>(p); }
-};
-}  // namespace
-
-API int lmz_gpu_decode_batch(const void *hdr, const void *streams, size_t nbytes, const void *off,
-                             unsigned nstr, unsigned plane, void *out)
-{
-    if (nstr == 0) return LMZ_GPU_OK;
-    if (plane == 0) return fail_msg(LMZ_GPU_EUNSUPPORTED, "plane is zero");
-    if (int rc = device_ready()) return rc;
-    // every (offset, length) pair must lie inside the buffer, and a length must fit the
-    // 32 bits the kernels carry it in
-    const uint64_t *pairs = static_cast<const uint64_t *>(off);
-    for (unsigned i = 0; i < nstr; i++) {
-        const uint64_t at = pairs[2 * i], len = pairs[2 * i + 1];
-        if (at > nbytes || len > nbytes - at) return fail_msg(LMZ_GPU_EBADSTREAM, "a stream lies outside the buffer");
-        if (len >> 32) return fail_msg(LMZ_GPU_EUNSUPPORTED, "a stream is 4 GiB or longer");
-    }
-    if (!hdr)
-        if (int rc = lmz_gpu_validate(streams, off, nstr)) return rc;
-
-    const size_t out_bytes = (size_t)nstr * plane, table_bytes = (size_t)nstr * 16;
-    Transient coded, table, plain, verdict, shared;
-    CK("cudaMalloc(streams)", coded.take(nbytes + PAD_BYTES));
-    CK("cudaMalloc(offsets)", table.take(table_bytes));
-    CK("cudaMalloc(out)", plain.take(out_bytes));
-    CK("cudaMalloc(verdict)", verdict.take(sizeof(uint32_t)));
-    CK("copy streams in", cudaMemcpy(coded.p, streams, nbytes, cudaMemcpyHostToDevice));
-    CK("clear the slack", cudaMemset(coded.as<uint8_t>() + nbytes, 0, PAD_BYTES));
-    CK("copy offsets in", cudaMemcpy(table.p, off, table_bytes, cudaMemcpyHostToDevice));
-    CK("clear the verdict", cudaMemset(verdict.p, 0, sizeof(uint32_t)));
-    if (hdr) {
-        CK("cudaMalloc(table)", shared.take(HDR_BYTES));
-        CK("copy table in", cudaMemcpy(shared.p, hdr, HDR_BYTES, cudaMemcpyHostToDevice));
-    }
-    RansArgs a{};
-    a.src = coded.as<uint8_t>();
-    a.offs = table.as<uint64_t>();
-    a.plane = plane;
-    a.njobs = nstr;
-    a.dst = plain.as<uint8_t>();
-    a.shared_hdr = shared.as<uint8_t>();
-    a.any_bad = verdict.as<uint32_t>();
-    if (int rc = launch_rans(a, 0)) return rc;
-    CK("cudaDeviceSynchronize", cudaDeviceSynchronize());
-    uint32_t any_bad = 0;
-    CK("copy the verdict out", cudaMemcpy(&any_bad, verdict.p, sizeof any_bad, cudaMemcpyDeviceToHost));
-    if (any_bad) return fail_msg(LMZ_GPU_EBADSTREAM, "a stream is malformed or truncated");
-    CK("copy plaintext out", cudaMemcpy(out, plain.p, out_bytes, cudaMemcpyDeviceToHost));
-    return LMZ_GPU_OK;
-}
+#include "host_batch.inl"
 
 // ------------------------------------------------------------------- additive
 

@@ -46,6 +46,9 @@ _SIGNATURES = {
     "lmz_gpu_decode_batch_dev_noalloc": (_C.c_int, [_C.c_void_p] * 3 + [_C.c_uint, _C.c_uint, _C.c_void_p,
                                                                          _C.c_void_p, _C.c_void_p]),
     "lmz_gpu_set_device": (_C.c_int, [_C.c_int]),
+    "lmz_gpu_host_alloc": (_C.c_void_p, [_C.c_size_t]),
+    "lmz_gpu_host_free": (None, [_C.c_void_p]),
+    "lmz_gpu_trim": (None, []),
     "lmz_gpu_set_table_mode": (_C.c_int, [_C.c_int]),
     "lmz_gpu_decode_streams_dev": (_C.c_int, [_C.c_void_p, _C.c_uint] + [_C.c_void_p] * 6),
     "lmz_gpu_encode_slot_bytes": (_C.c_int, [_C.c_uint]),
@@ -165,6 +168,21 @@ def _host_view(buf, writable: bool = False):
     return arr
 
 
+def _result_memory(lib, size: int):
+    """A writable numpy uint8 array of `size` bytes for a result.  Page-locked where the
+    library has some to lend (the copy engine then writes it, and a fresh result costs no
+    page faults); it goes back to the library when the last view of it is dropped."""
+    import weakref
+
+    import numpy as np
+    at = lib.lmz_gpu_host_alloc(size)
+    if not at:
+        return np.zeros(size, dtype=np.uint8)
+    block = (ctypes.c_uint8 * size).from_address(at)
+    weakref.finalize(block, lib.lmz_gpu_host_free, at).atexit = False
+    return np.frombuffer(block, dtype=np.uint8)
+
+
 def _addr(view):
     return view.ctypes.data if view is not None and view.size else None
 
@@ -270,8 +288,7 @@ def decode_batch(streams, offsets, nstr: int, plane: int, out=None, header=None)
     if out is not None and len(out) >= size:
         held, dst = out, _host_view(out, writable=True)
     else:
-        held = bytearray(size)
-        dst = _host_view(held)
+        held = dst = _result_memory(lib, size)
     rc = lib.lmz_gpu_decode_batch(_addr(shared), _addr(src), src.size, _addr(table), nstr, plane,
                                   _addr(dst))
     if rc == EBADSTREAM:

@@ -149,3 +149,26 @@ def test_stress_extremes_long_streams_and_wide_batches(gpu, orc, dist, table_mod
     out = np.frombuffer(gpu.decode_batch(blob, offs, 4096, 4096, header=header),
                         dtype=np.uint8).reshape(4096, 4096)
     assert (out == np.stack(plains)).all()
+
+
+@pytest.mark.parametrize("nstr,plane", [(1, 1), (3, 4097), (40, 65537)])
+def test_results_in_lent_memory_stay_their_callers_own(gpu, orc, nstr, plane, table_mode):
+    """Results of host batches come in memory the library takes back when they are dropped:
+    one that is still held must not change under later calls, from this thread or others."""
+    if table_mode != -1:
+        pytest.skip("the memory does not depend on the table layout")
+    from concurrent.futures import ThreadPoolExecutor
+    sets = []
+    for s in range(4):
+        plains = [shaped("skewed", plane, 31 * s + i) for i in range(nstr)]
+        sets.append((pack_streams([orc.rans_encode(p) for p in plains]), b"".join(p.tobytes() for p in plains)))
+    held = [gpu.decode_batch(*sets[s][0], nstr, plane) for s in range(2)]
+    with ThreadPoolExecutor(6) as pool:
+        got = list(pool.map(lambda i: bytes(gpu.decode_batch(*sets[i % 4][0], nstr, plane)), range(24)))
+    assert all(g == sets[i % 4][1] for i, g in enumerate(got))
+    assert [bytes(h) for h in held] == [sets[0][1], sets[1][1]]
+    part = held[0][:1]
+    del held
+    gpu.library().lmz_gpu_trim()
+    gpu.decode_batch(*sets[2][0], nstr, plane)
+    assert bytes(part) == sets[0][1][:1]
