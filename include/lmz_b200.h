@@ -220,6 +220,45 @@ int lmz_gpu_crc_tables(void *host_dst, size_t cap);
  * counted in n_fused_small. */
 int lmz_host_alphabet_sizes(const void *base, const uint64_t *offs, size_t n, uint16_t *out);
 
+/* Host helper for planners: n pieces of `width` bytes at offs[i] of a file (fd >= 0) or of
+ * memory of `size` bytes, one after the other into `out`; bytes past `size` read as zero.
+ * Several threads: the headers in front of an archive's chunks lie one to a page. */
+int lmz_host_gather(int fd, const void *host, uint64_t size, const uint64_t *offs, size_t n, unsigned width, void *out);
+
+/* Host helper for planners: the job arrays of an archive whose chunks are stored, one-stream,
+ * byte-plane or BF16 chunks without references (lmz_b200/plan.py says what each array holds and
+ * how large it must be).  `heads`: lmz_host_plan_head_bytes() bytes from the start of every
+ * chunk's payload.  Returns 0, or 1 when a record is of another kind or not as it should be;
+ * plan.py's own planner then takes the archive or says what is wrong with it. */
+int lmz_host_plan_head_bytes(void);
+int lmz_host_plan(const void *records, const int64_t *select, size_t n, const uint64_t *ranges, const void *heads,
+                  int fuse, unsigned fuse_f32_min, void *chunks, void *fused, void *delta, void *streams, int64_t *owner,
+                  uint32_t *piece_chunk, int64_t *general, uint64_t *counts);
+
+/* ---- files and HBM ----------------------------------------------------------
+ * No counterpart in the reference.  A staging is `depth` page-locked blocks of `block` bytes and
+ * `threads` threads (fewer than blocks) that fill or empty them; one may serve any number of
+ * transfers.  A transfer is a run of ranges that cross in the background, on a stream of its
+ * own that starts behind `cuda_stream`'s work so far (current device).
+ *   upload    len bytes at `off` of a file (fd >= 0) or of host memory -> d_dst
+ *   download  len bytes at d_src, as cuda_stream's work so far leaves them -> `off` of a mapping
+ *             (map != NULL) or of a file
+ * Both return the range's number, negative on failure.  wait() returns when a range has been
+ * issued whole (upload: cuda_stream then waits for its arrival) or written (download); free()
+ * waits for all.  An error ends every later block of the transfer. */
+void *lmz_gpu_staging_new(size_t block, unsigned depth, unsigned threads);
+void lmz_gpu_staging_free(void *staging);
+void *lmz_gpu_transfer_new(void *staging, void *cuda_stream);
+int lmz_gpu_transfer_upload(void *transfer, int fd, const void *host, uint64_t off, uint64_t len, void *d_dst);
+int lmz_gpu_transfer_download(void *transfer, const void *d_src, uint64_t len, int fd, void *map, uint64_t off,
+                              void *cuda_stream);
+int lmz_gpu_transfer_wait(void *transfer, int range, void *cuda_stream);
+int lmz_gpu_transfer_free(void *transfer);
+/* [off, off + len) of a file on a memory-backed file system as writable memory with its space
+ * reserved, or NULL (another file system, no space, off not a multiple of 4096). */
+void *lmz_host_map_file(int fd, uint64_t off, uint64_t len);
+int lmz_host_unmap_file(void *p, uint64_t len);
+
 /* Everything lmz_gpu_decode_chunks_dev needs.  All pointers are device pointers.
  * Layouts of the job arrays are those of csrc/common.cuh and csrc/chunk_kernels.cuh;
  * lmz_b200/plan.py builds them. */

@@ -29,3 +29,19 @@ def bind(lib) -> None:
     lib.lmz_host_alphabet_sizes.argtypes = [_v, _v, ctypes.c_size_t, _v]
     lib.lmz_gpu_decode_chunks_dev.restype = ctypes.c_int
     lib.lmz_gpu_decode_chunks_dev.argtypes = [ctypes.POINTER(DecodePlan), _v]
+    _u64, _int, _uns = ctypes.c_uint64, ctypes.c_int, ctypes.c_uint
+    for name, res, args in (
+            ("lmz_gpu_staging_new", _v, [ctypes.c_size_t, _uns, _uns]),
+            ("lmz_gpu_staging_free", None, [_v]),
+            ("lmz_gpu_transfer_new", _v, [_v, _v]),
+            ("lmz_gpu_transfer_upload", _int, [_v, _int, _v, _u64, _u64, _v]),
+            ("lmz_gpu_transfer_download", _int, [_v, _v, _u64, _int, _v, _u64, _v]),
+            ("lmz_gpu_transfer_wait", _int, [_v, _int, _v]),
+            ("lmz_gpu_transfer_free", _int, [_v]),
+            ("lmz_host_gather", _int, [_int, _v, _u64, _v, ctypes.c_size_t, _uns, _v]),
+            ("lmz_host_map_file", _v, [_int, _u64, _u64]),
+            ("lmz_host_unmap_file", _int, [_v, _u64]),
+            ("lmz_host_plan_head_bytes", _int, []),
+            ("lmz_host_plan", _int, [_v, _v, ctypes.c_size_t, _v, _v, _int, _uns] + [_v] * 8)):
+        fn = getattr(lib, name)
+        fn.restype, fn.argtypes = res, args

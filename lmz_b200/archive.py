@@ -67,15 +67,44 @@ def inflate_tail(raw: bytes) -> bytes:
         raise CorruptArchive(f"archive index failed to inflate: {exc}") from exc
 
 
+class MappedFile(np.memmap):
+    """A file's bytes, mapped, not read: only what is touched is.  `fd` is the file while it is open."""
+
+    fd = -1
+
+
+def open_blob(path):
+    """The bytes of an archive: a path is mapped; an array or bytes-like object is used as it is."""
+    if isinstance(path, (str, os.PathLike)):
+        f = open(path, "rb")
+        blob = np.memmap(f, dtype=np.uint8, mode="r").view(MappedFile)
+        blob.fd, blob.file = f.fileno(), f
+        return blob
+    return path if isinstance(path, np.ndarray) else np.frombuffer(path, dtype=np.uint8)
+
+
+def payload_end(b) -> int:
+    """Where the payload region of an archive's bytes ends and its index begins, from the footer."""
+    if b.size < HEADER.size + FOOTER.size:
+        raise FormatError("file is too small to be an lmz archive")
+    if bytes(b[:4]) != MAGIC:
+        raise FormatError("not an lmz archive (bad magic)")
+    toff, tlen, _moff, _mlen, tail = FOOTER.unpack_from(b, b.size - FOOTER.size)
+    if tail != TAIL:
+        raise FormatError("archive is truncated or corrupt (bad footer)")
+    if toff < HEADER.size or toff + tlen > b.size:
+        raise FormatError("chunk table points outside the file")
+    return int(toff)
+
+
 class Archive:
     """Header, manifest and chunk records of one archive held in host memory."""
 
+    fd = -1                                # the archive's file while it is open, or -1: held in memory
+
     def __init__(self, blob):
-        if isinstance(blob, (str, os.PathLike)):
-            # a file is mapped, not read: only the index at its end is touched here, and the
-            # payload pages are read when they are uploaded
-            blob = np.memmap(blob, dtype=np.uint8, mode="r")
-        self.blob = blob if isinstance(blob, np.ndarray) else np.frombuffer(blob, dtype=np.uint8)
+        self.blob = open_blob(blob)
+        self.fd = getattr(self.blob, "fd", -1)
         b = self.blob
         if b.size < HEADER.size + FOOTER.size:
             raise FormatError("file is too small to be an lmz archive")

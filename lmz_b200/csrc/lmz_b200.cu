@@ -5,6 +5,7 @@
 // with the same names, argument meaning, return codes and error behaviour; the
 // rest are additive entry points for whole-archive decode.  Declarations and
 // the per-function contract live in include/lmz_b200.h.
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -317,6 +318,8 @@ API int lmz_gpu_decode_batch_dev(const void *d_hdr, const void *d_streams, const
 }
 
 #include "host_batch.inl"
+#include "host_io.inl"
+#include "host_plan.inl"
 
 // ------------------------------------------------------------------- additive
 

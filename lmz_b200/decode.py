@@ -24,10 +24,51 @@ _TORCH_DTYPES = {"BF16": "bfloat16", "F16": "float16", "F32": "float32", "F64": 
                  "BOOL": "bool"}
 
 
-def _dev(arr: np.ndarray, device):
-    import torch
-    t = torch.from_numpy(np.ascontiguousarray(arr).view(np.uint8).reshape(-1).copy())
-    return t.to(device, non_blocking=False)
+class _Arena:
+    """Many small device arrays in two allocations: job arrays, which come over in one copy from one
+    page-locked block, and work arrays, cleared by one memset."""
+
+    def __init__(self, lib, device):
+        self.lib, self.device = lib, device
+        self.jobs, self.work = {}, {}
+        self.host = None
+
+    def job(self, name, arr):
+        self.jobs[name] = np.ascontiguousarray(arr).view(np.uint8).reshape(-1)
+
+    def words(self, name, count, kind="int32"):
+        self.work[name] = (max(1, int(count)), kind)
+
+    def place(self):
+        """{name: tensor} of everything asked for."""
+        import torch
+        out, at = {}, 0
+        spans = {}
+        for name, a in self.jobs.items():
+            spans[name] = at
+            at += (a.size + 255) & ~255
+        self.host = gpu.result_memory(self.lib, max(at, 1))
+        for name, a in self.jobs.items():
+            self.host[spans[name]:spans[name] + a.size] = a
+        work = {}
+        total = 0
+        size = {"int32": 4, "int16": 2, "uint8": 1}
+        for name, (count, kind) in self.work.items():
+            work[name] = total
+            total += (count * size[kind] + 255) & ~255
+        dev = torch.empty(max(at, 1) + total, dtype=torch.uint8, device=self.device)
+        dev[:at].copy_(torch.from_numpy(self.host[:at]), non_blocking=True)
+        dev[at:].zero_()
+        for name, a in self.jobs.items():
+            out[name] = dev[spans[name]:spans[name] + a.size]
+        for name, (count, kind) in self.work.items():
+            lo = at + work[name]
+            out[name] = dev[lo:lo + count * size[kind]].view(getattr(torch, kind))
+        return out
+
+    def arrived(self):
+        """The copy has been waited for: the host block may go."""
+        self.host = None
 
 
 _tables = {}
@@ -45,6 +86,24 @@ def _crc_tables(lib, device):
     return _tables[key]
 
 
+_layouts_of = set()
+
+
+def _check_layouts(lib):
+    """The library's job layouts are the planner's (asked once)."""
+    if id(lib) in _layouts_of:
+        return
+    sizes = (ctypes.c_uint * 5)()
+    lib.lmz_gpu_struct_sizes(ctypes.byref(sizes))
+    want = (planner.STREAM_JOB.itemsize, planner.CHUNK_JOB.itemsize,
+            planner.COND_JOB.itemsize, planner.COND_STATE_BYTES, planner.FUSED_JOB.itemsize)
+    if tuple(sizes) != want or lib.lmz_gpu_piece_bytes() != planner.PIECE or \
+            lib.lmz_gpu_shared_group() != planner.T_GROUP or \
+            lib.lmz_gpu_delta_job_bytes() != planner.DELTA_JOB.itemsize:
+        raise RuntimeError("the CUDA library and the planner disagree on job layouts")
+    _layouts_of.add(id(lib))
+
+
 class ArchiveDecoder:
     """An archive planned and resident on `device`, ready to decode repeatedly.
 
@@ -53,22 +112,16 @@ class ArchiveDecoder:
     `verify_checksums=False`).  `payload` may be given as a CUDA uint8 tensor with room
     for `plan.payload`, the plan's host-inflated header chunks and `gpu.pad_bytes()` of
     slack; the caller then brings the payload bytes there itself (`upload`, or copies of
-    its own) before `run`."""
+    its own) before `run`.  With `settle=False` the job arrays may still be on their way when the
+    constructor returns: `run` must then be on the stream that was current here."""
 
     def __init__(self, ar, device=None, checksum: bool = True, out=None, plan=None,
-                 fuse=True, payload=None):
+                 fuse=True, payload=None, *, settle: bool = True):
         import torch
 
         lib = gpu.library()
         self.lib = lib
-        sizes = (ctypes.c_uint * 5)()
-        lib.lmz_gpu_struct_sizes(ctypes.byref(sizes))
-        want = (planner.STREAM_JOB.itemsize, planner.CHUNK_JOB.itemsize,
-                planner.COND_JOB.itemsize, planner.COND_STATE_BYTES, planner.FUSED_JOB.itemsize)
-        if tuple(sizes) != want or lib.lmz_gpu_piece_bytes() != planner.PIECE or \
-                lib.lmz_gpu_shared_group() != planner.T_GROUP or \
-                lib.lmz_gpu_delta_job_bytes() != planner.DELTA_JOB.itemsize:
-            raise RuntimeError("the CUDA library and the planner disagree on job layouts")
+        _check_layouts(lib)
         self.archive = ar if isinstance(ar, fmt.Archive) else fmt.Archive(ar)
         self.plan = p = plan if plan is not None else planner.build_plan(self.archive, fuse=fuse)
         self.device = torch.device(device if device is not None else
@@ -77,50 +130,48 @@ class ArchiveDecoder:
         d = self.device
         with torch.cuda.device(d):
             pad = gpu.pad_bytes()
-            nbytes = p.payload.size + p.extras.size
+            nbytes = p.extras_at + p.extras.size
             if payload is not None and payload.numel() < nbytes + pad:
                 raise ValueError("the payload buffer is smaller than the plan's payload, header chunks and slack")
             self.d_payload = payload if payload is not None else \
                 torch.empty(nbytes + pad, dtype=torch.uint8, device=d)
-            self.h2d_bytes = int(nbytes)
-            self.d_payload[nbytes:].zero_()
-            if p.extras.size:
-                self.d_payload[p.payload.size:nbytes].copy_(torch.from_numpy(p.extras.copy()))
-            if payload is None:
-                self.upload()
+            self.h2d_bytes = int(p.payload.size + p.extras.size)
+            self.d_payload[nbytes:nbytes + pad].zero_()
+            up = self._start_upload() if payload is None else None      # under the rest of this
             self.d_scratch = torch.empty(max(p.scratch_bytes, 64), dtype=torch.uint8, device=d)
             self.d_out = out if out is not None else \
                 torch.empty(p.total + 64, dtype=torch.uint8, device=d)
             if self.d_out.numel() < p.total + 64:
                 raise ValueError("the output buffer needs total + 64 bytes")
-            self.d_stream_jobs = _dev(p.stream_jobs, d)
-            self.d_seg_jobs = _dev(p.seg_jobs, d)
-            self.d_fused_jobs = _dev(p.fused_jobs, d)
-            self.d_delta_jobs = _dev(p.delta_jobs, d)
-            self.d_chunks = _dev(p.chunks, d)
-            self.d_piece_chunk = _dev(p.piece_chunk, d)
-            self.d_cond_jobs = _dev(p.cond_jobs, d)
-            self.d_cond_pieces = _dev(p.cond_pieces, d)
-            ncond = p.cond_jobs.size
-            u32 = dict(dtype=torch.int32, device=d)
-            self.d_cond_state = torch.zeros(max(1, ncond * planner.COND_STATE_BYTES),
-                                            dtype=torch.uint8, device=d)
-            self.d_hist = torch.zeros(max(1, ncond * 256), **u32)
-            self.d_piece_cnt = torch.zeros(max(1, p.n_pieces * 16), **u32)
-            self.d_piece_wcnt = torch.zeros(max(1, p.n_pieces * 64 if ncond else 1), dtype=torch.int16, device=d)
-            self.d_piece_lcnt = torch.empty(max(1, p.cond_pieces.size * 2048), **u32)
-            self.d_piece_crc = torch.zeros(max(1, p.n_pieces), **u32)
-            self.d_stream_status = torch.zeros(max(1, p.stream_jobs.size), **u32)
-            self.d_seg_status = torch.zeros(max(1, p.seg_jobs.size), **u32)
-            self.d_fused_status = torch.zeros(max(1, p.fused_jobs.size), **u32)
-            self.d_delta_status = torch.zeros(max(1, 2 * p.delta_jobs.size), **u32)
-            self.d_delta_order = torch.zeros(p.delta_jobs.size + 4, **u32)
-            self.d_chunk_status = torch.zeros(max(1, p.chunks.size), **u32)
-            self.d_chunk_crc = torch.zeros(max(1, p.chunks.size), **u32)
-            self.d_any_bad = torch.zeros(1, **u32)
-            self.d_fused_order = torch.zeros(p.n_fused + 4, **u32) if p.device_classify else None
-            self.d_tables = _dev(p.tables, d) if p.n_fused_t else None
+            ncond, nchunks, npieces = p.cond_jobs.size, p.chunks.size, p.n_pieces
+            self._arena = a = _Arena(lib, d)
+            for name in ("stream_jobs", "seg_jobs", "fused_jobs", "delta_jobs", "chunks", "piece_chunk",
+                         "cond_jobs", "cond_pieces", "extras"):
+                a.job("d_" + name, getattr(p, name))
+            if p.n_fused_t:
+                a.job("d_tables", p.tables)
+            a.words("d_cond_state", ncond * planner.COND_STATE_BYTES, "uint8")
+            for name, count in (("hist", ncond * 256), ("piece_cnt", npieces * 16 if ncond else 1), ("piece_crc", npieces),
+                                ("stream_status", p.stream_jobs.size), ("seg_status", p.seg_jobs.size),
+                                ("fused_status", p.fused_jobs.size), ("delta_status", 2 * p.delta_jobs.size),
+                                ("delta_order", p.delta_jobs.size + 4), ("chunk_status", nchunks), ("chunk_crc", nchunks),
+                                ("any_bad", 1), ("fused_order", p.n_fused + 4)):
+                a.words("d_" + name, count)
+            a.words("d_piece_wcnt", npieces * 64 if ncond else 1, "int16")
+            self.d_tables = None
+            for name, t in a.place().items():
+                setattr(self, name, t)
+            if not p.device_classify:
+                self.d_fused_order = None
+            if p.extras.size:
+                self.d_payload[p.extras_at:nbytes].copy_(self.d_extras)
+            self.d_piece_lcnt = torch.empty(max(1, p.cond_pieces.size * 2048), dtype=torch.int32, device=d)
             self.d_tabs = _crc_tables(lib, d)
+            if up is not None:
+                self._finish_upload(up)
+            if settle:
+                torch.cuda.current_stream(d).synchronize()
+                self._arena.arrived()
         c = _chunks.DecodePlan()
         c.d_payload, c.d_scratch = self.d_payload.data_ptr(), self.d_scratch.data_ptr()
         c.d_out = self.d_out.data_ptr()
@@ -169,14 +220,25 @@ class ArchiveDecoder:
     def upload(self, pinned=None, non_blocking: bool = False):
         """Copy the archive's payload region host -> device (from `pinned`, a host
         uint8 tensor of `plan.payload.size` bytes, if given)."""
-        import warnings
-
         import torch
-        if pinned is None:
-            with warnings.catch_warnings():
-                warnings.simplefilter("ignore")          # read-only numpy views are fine to read
-                pinned = torch.from_numpy(self.plan.payload)
-        self.d_payload[:self.plan.payload.size].copy_(pinned, non_blocking=non_blocking)
+        n = self.plan.payload.size
+        if pinned is not None:
+            self.d_payload[:n].copy_(pinned, non_blocking=non_blocking)
+            return
+        with torch.cuda.device(self.device):
+            self._finish_upload(self._start_upload())
+            torch.cuda.current_stream(self.device).synchronize()
+
+    def _start_upload(self):
+        up = _Uploader(self.archive.blob, self.device)
+        n = self.plan.payload.size
+        lo = n and self.plan.payload.ctypes.data - self.archive.blob.ctypes.data
+        up.send(lo, lo + n, self.d_payload)
+        return up
+
+    def _finish_upload(self, up):
+        up.wait(0)
+        up.close()
 
     def run(self, stream=None, phases: int = 0):
         """Launch the decode on `stream` (default: torch's current). Asynchronous.
@@ -201,6 +263,7 @@ class ArchiveDecoder:
         """Synchronise and raise CorruptArchive if any stream or chunk failed."""
         import torch
         torch.cuda.synchronize(self.device)
+        self._arena.arrived()
         if int(self.d_any_bad.item()) == 0:
             return
         p = self.plan
@@ -304,12 +367,11 @@ class PipelinedDecoder:
         cache, ordinary memory): see `load_archive`, which also plans under the copies."""
         import torch
         compute = stream if stream is not None else torch.cuda.current_stream(self.device)
-        up = _Uploader(self.archive.blob, self.device, staging)
-        up.copy_stream.wait_stream(compute)
+        up = _Uploader(self.archive.blob, self.device, staging, compute)
         for dec, (lo, hi) in zip(self.slices, self.ranges):
             up.send(lo, hi, dec.d_payload)
         for si, dec in enumerate(self.slices):
-            compute.wait_event(up.wait(si))
+            up.wait(si)
             dec.run(stream=compute)
         up.close()
         return self.d_out[:self.archive.total]
@@ -320,22 +382,22 @@ class PipelinedDecoder:
 
 
 class Staging:
-    """Page-locked staging between a file and the device: `depth` buffers of `block`
-    bytes and the threads that fill and send them.  (Six threads: on a 16-core host four
-    leave the link idle at times and eight or more slow the planning that runs beside them.)"""
+    """Page-locked staging between a file and the device: `depth` blocks of `block` bytes and
+    the library's threads that fill and send them (csrc/host_io.inl).  Twelve threads: the copy out
+    of the page cache bounds a load, and a dozen reach the host memory's rate."""
 
     _shared = None
 
-    def __init__(self, block: int = 32 << 20, depth: int = 8, threads: int = 6):
-        import concurrent.futures
-
-        import torch
+    def __init__(self, block: int = 2 << 20, depth: int = 24, threads: int = 12):
+        import weakref
         if threads >= depth:
             raise ValueError("staging needs more buffers than threads")
+        lib = gpu.library()
         self.block, self.depth = block, depth
-        self.buffers = [torch.empty(block, dtype=torch.uint8).pin_memory() for _ in range(depth)]
-        self.views = [b.numpy() for b in self.buffers]
-        self.pool = concurrent.futures.ThreadPoolExecutor(threads)
+        self.handle = lib.lmz_gpu_staging_new(block, depth, threads)
+        if not self.handle:
+            raise RuntimeError(gpu.last_error())
+        weakref.finalize(self, lib.lmz_gpu_staging_free, self.handle).atexit = False
 
     @classmethod
     def shared(cls):
@@ -345,96 +407,46 @@ class Staging:
 
 
 class _Uploader:
-    """Byte ranges of a host array -> device tensors through `Staging`, in the background.
+    """Byte ranges of an archive -> device memory through `Staging`, in the background.
 
-    `send(lo, hi, dst)` queues one range ("a slice"); worker threads copy it block by
-    block into page-locked buffers and start each block's host -> device copy themselves on
-    one copy stream, so the caller is free to plan and launch meanwhile.  `wait(i)` blocks
-    until every block of the i-th range has been issued and returns a CUDA event that
-    completes when they have all arrived."""
+    `send(lo, hi, dst)` queues one range; the staging's threads copy it block by block while
+    the caller plans and launches.  `wait(i)` blocks until the i-th range has been issued
+    whole and makes `stream` (default: torch's current) wait for its arrival."""
 
-    def __init__(self, blob, device, staging=None):
-        import threading
-
+    def __init__(self, blob, device, staging=None, stream=None):
         import torch
-        self.blob, self.device = blob, device
-        self.st = staging if staging is not None else Staging.shared()
-        self.copy_stream = torch.cuda.Stream(device)
-        self.lock = threading.Lock()
-        self.turn = threading.Condition()
-        self.slot_free = [None] * self.st.depth        # CUDA event: the slot's last copy has left it
-        self.slot_round = [0] * self.st.depth          # blocks that have been through each buffer
-        self.nblocks = 0
-        self.failed = False
-        self.left, self.ready, self.events, self.tasks = [], [], [], []
+        self.blob, self.fd, self.lib = blob, getattr(blob, "fd", -1), gpu.library()
+        self.staging = staging if staging is not None else Staging.shared()
+        self.stream = stream if stream is not None else torch.cuda.current_stream(device)
+        self.device = device
+        with torch.cuda.device(device):
+            self.handle = self.lib.lmz_gpu_transfer_new(self.staging.handle, self.stream.cuda_stream)
+        if not self.handle:
+            raise RuntimeError(gpu.last_error())
 
-    def send(self, lo: int, hi: int, dst):
-        import threading
-        si = len(self.left)
-        spans = [(b, min(b + self.st.block, hi)) for b in range(lo, hi, self.st.block)]
-        self.left.append(len(spans))
-        self.ready.append(threading.Event())
-        self.events.append(None)
-        if not spans:
-            self._finish(si)
-        for b, e in spans:
-            self.tasks.append(self.st.pool.submit(self._block, si, self.nblocks, b, e, dst[b - lo:e - lo]))
-            self.nblocks += 1
-        return si
-
-    def _finish(self, si):
+    def send(self, lo: int, hi: int, dst) -> int:
         import torch
-        with torch.cuda.stream(self.copy_stream):
-            ev = torch.cuda.Event()
-            ev.record(self.copy_stream)
-        self.events[si] = ev
-        self.ready[si].set()
+        with torch.cuda.device(self.device):
+            r = self.lib.lmz_gpu_transfer_upload(self.handle, self.fd, self.blob.ctypes.data, int(lo), int(hi - lo),
+                                                 dst.data_ptr())
+        if r < 0:
+            raise RuntimeError(gpu.last_error())
+        return r
 
-    def _block(self, si, index, lo, hi, dst):
-        import torch
-        try:
-            slot, rnd = index % self.st.depth, index // self.st.depth
-            with torch.cuda.device(self.device):
-                # a buffer takes its blocks strictly in turn: block `index` may fill it only after
-                # block `index - depth` has issued its copy (tasks start in order but may finish in
-                # any) and that copy has left the buffer
-                with self.turn:
-                    self.turn.wait_for(lambda: self.slot_round[slot] == rnd or self.failed)
-                if self.failed:
-                    raise RuntimeError("an earlier upload block failed")
-                if self.slot_free[slot] is not None:
-                    self.slot_free[slot].synchronize()
-                np.copyto(self.st.views[slot][:hi - lo], self.blob[lo:hi])
-                with self.lock:                      # one issuer at a time keeps stream order = event order
-                    with torch.cuda.stream(self.copy_stream):
-                        dst.copy_(self.st.buffers[slot][:hi - lo], non_blocking=True)
-                        ev = torch.cuda.Event()
-                        ev.record(self.copy_stream)
-                    self.slot_free[slot] = ev
-                    self.left[si] -= 1
-                    if self.left[si] == 0:
-                        self._finish(si)
-                with self.turn:
-                    self.slot_round[slot] = rnd + 1
-                    self.turn.notify_all()
-        except BaseException:
-            self.failed = True
-            with self.turn:
-                self.turn.notify_all()
-            self.ready[si].set()                     # wake the waiter; result() re-raises below
-            raise
+    def wait(self, si: int) -> None:
+        if self.lib.lmz_gpu_transfer_wait(self.handle, si, self.stream.cuda_stream) != gpu.OK:
+            raise RuntimeError(f"an upload failed: {gpu.last_error()}")
 
-    def wait(self, si):
-        self.ready[si].wait()
-        if self.events[si] is None:
-            for t in self.tasks:
-                t.result()                           # surfaces the worker's exception
-            raise RuntimeError("an upload block failed")
-        return self.events[si]
+    def close(self) -> None:
+        """Wait for every range and let go; the memory sent to must live until then."""
+        if self.handle:
+            handle, self.handle = self.handle, None
+            if self.lib.lmz_gpu_transfer_free(handle) != gpu.OK:
+                raise RuntimeError(f"an upload failed: {gpu.last_error()}")
 
-    def close(self):
-        for t in self.tasks:
-            t.result()
+    def __del__(self):
+        if getattr(self, "handle", None):
+            self.lib.lmz_gpu_transfer_free(self.handle)
 
 
 def _slice_groups(ar, nslices):
@@ -452,60 +464,101 @@ def _slice_groups(ar, nslices):
     return [g for g in np.split(order, cuts) if g.size]
 
 
+def _upload_cuts(table_off: int, nslices):
+    """Where an archive's payload region is cut into ranges that are uploaded (and decoded) one after
+    the other: as many as asked for, or one per 192 MiB, at most eight.  (A range is decoded
+    under the upload of the next, but a decode has a smallest duration, that of one stream.)"""
+    n = nslices if nslices is not None else min(8, -(-table_off // (192 << 20)))
+    n = max(1, min(int(n), max(1, table_off)))
+    return [table_off * i // n for i in range(n + 1)]
+
+
 def load_archive(path, device=None, checksum: bool = True, nslices=None, stats=None, staging=None):
     """File on disk -> verified plaintext in HBM (the load the reference times as "cold
-    disk -> VRAM", README.md:79-84).  The archive is mapped and its index read; its chunks
-    are cut into slices of consecutive payload bytes; background threads stream slice
-    after slice through page-locked staging to the device; each slice is planned while it
-    is on its way (after the copy has brought its pages in, so the planner's reads of the
-    in-payload headers cost nothing) and decoded as soon as it has arrived, under the
-    copies of the next; every chunk's verdict is checked at the end.  Returns the decoded
-    output space as a device tensor.  `stats`, a dict, receives `open_s` (map + index),
-    `run_s` (everything else), `plan_s` (planning inside run_s), `h2d_bytes`, `slices`."""
+    disk -> VRAM", README.md:79-84).  The upload of the payload region starts before the index is
+    read: the library's threads stream it range after range through page-locked staging to the
+    device, while this thread reads the index, plans each range's chunks and, as soon as the
+    range has been issued, launches their decode behind it; every chunk's verdict is checked at the
+    end.  Returns the decoded output space as a device tensor.  `stats`, a dict, receives `open_s`
+    (until the upload has been started), `run_s` (everything else), `plan_s` (reading the index and
+    planning inside run_s), `h2d_bytes`, `slices`."""
     import time
 
     import torch
     t0 = time.perf_counter()
-    ar = fmt.Archive(path)
-    ar.check_coverage()
+    blob = fmt.open_blob(path)
+    table_off = fmt.payload_end(blob)
     dev = torch.device(device if device is not None else f"cuda:{torch.cuda.current_device()}")
-    r = ar.records
-    groups = _slice_groups(ar, nslices)
-    t1 = time.perf_counter()
     with torch.cuda.device(dev):
-        out = torch.empty(ar.total + 64, dtype=torch.uint8, device=dev)
         compute = torch.cuda.current_stream(dev)
-        up = _Uploader(ar.blob, dev, staging)
         pad = gpu.pad_bytes()
-        spans, payloads = [], []
-        for g in groups:
-            lo = int(r["off"][g].min())
-            hi = int((r["off"][g].astype(np.int64) + r["clen"][g]).max())
-            # room behind the payload for header chunks the planner inflates on the host
-            general = (r["codec"][g] == fmt.CODEC_ZSTD) & np.isin(r["flags"][g] & 3, (fmt.METHOD_ZSTD, fmt.METHOD_DEFLATE))
-            extra = int(r["rlen"][g][general].sum())
-            d = torch.empty(hi - lo + extra + pad, dtype=torch.uint8, device=dev)
-            spans.append((lo, hi))
-            payloads.append(d)
-            up.send(lo, hi, d)
-        decs, plan_s = [], 0.0
-        for si, g in enumerate(groups):
-            arrived = up.wait(si)                    # every block of the slice has been read and issued
-            tp = time.perf_counter()
-            p = planner.build_plan(ar, select=g, payload_range=spans[si])
-            dec = ArchiveDecoder(ar, device=dev, checksum=checksum, out=out, plan=p, payload=payloads[si])
-            plan_s += time.perf_counter() - tp
-            compute.wait_event(arrived)
-            dec.run(stream=compute)
-            decs.append(dec)
-        up.close()
+        # (room behind the payload for header chunks that are inflated on the host)
+        room = (1 << 20) + table_off // 256
+        payload = torch.empty(table_off + room + pad, dtype=torch.uint8, device=dev)
+        cuts = _upload_cuts(table_off, nslices)
+
+        def start():
+            up = _Uploader(blob, dev, staging, compute)
+            return up, [up.send(lo, hi, payload[lo:]) for lo, hi in zip(cuts, cuts[1:])]
+
+        up, sent = start()
+        t1 = time.perf_counter()
+        try:
+            ar = fmt.Archive(blob)
+            ar.check_coverage()
+            r = ar.records
+            general = (r["codec"] == fmt.CODEC_ZSTD) & ((r["flags"] & 3) != fmt.METHOD_STORED) & \
+                      ((r["flags"] & 3) != fmt.METHOD_RANS)
+            inflated = int(r["rlen"][general].sum()) if general.any() else 0
+            if inflated > room:                          # (or a reference's delta of one: rare, and checked below)
+                up.close()
+                payload = torch.empty(table_off + inflated + pad, dtype=torch.uint8, device=dev)
+                up, sent = start()
+            out = torch.empty(ar.total + 64, dtype=torch.uint8, device=dev)
+            decs, plan_s, extras_at, tp = [], 0.0, table_off, t1
+            for upto, group in _range_groups(ar, cuts, nslices):
+                p = planner.build_plan(ar, select=group, payload_range=(0, table_off), extras_at=extras_at)
+                extras_at += p.extras.size
+                dec = ArchiveDecoder(ar, device=dev, checksum=checksum, out=out, plan=p, payload=payload, settle=False)
+                plan_s += time.perf_counter() - tp
+                for si in sent[:upto]:
+                    up.wait(si)
+                tp = time.perf_counter()
+                dec.run(stream=compute)
+                decs.append(dec)
+        finally:
+            up.close()
         for dec in decs:
             dec.check()
         torch.cuda.synchronize(dev)
     if stats is not None:
         stats.update(open_s=t1 - t0, run_s=time.perf_counter() - t1, plan_s=plan_s,
-                     h2d_bytes=sum(hi - lo for lo, hi in spans), slices=len(groups))
+                     h2d_bytes=table_off, slices=len(decs))
     return out[:ar.total]
+
+
+def _range_groups(ar, cuts, nslices):
+    """[(ranges needed, record indices or None for all)]: the chunks each uploaded range completes.
+    One group where chunks read other chunks' output, and for chunks of a megabyte or more, whose
+    decode time is the latency of one long stream whatever their number, one per ~1900 of them."""
+    r, n = ar.records, len(cuts) - 1
+    if np.isin(r["codec"], (fmt.CODEC_REF, fmt.CODEC_DELTA)).any():
+        n = 1
+    elif nslices is None:
+        big = int((r["rlen"] >= (1 << 20)).sum())
+        n = min(n, max(1, big // 1900)) if big else n
+    if n <= 1 or r.size < n:
+        return [(len(cuts) - 1, None)]
+    end = r["off"].astype(np.int64) + r["clen"]
+    step = (len(cuts) - 1) / n
+    out, done = [], 0
+    for i in range(1, n + 1):
+        upto = len(cuts) - 1 if i == n else int(i * step)
+        mine = np.nonzero((end > done) & (end <= cuts[upto]))[0] if i < n else np.nonzero(end > done)[0]
+        done = cuts[upto]
+        if mine.size:
+            out.append((upto, mine))
+    return out
 
 
 def decode_tensors(ar, names, device=None, checksum: bool = True):
@@ -542,7 +595,7 @@ def decode_tensors(ar, names, device=None, checksum: bool = True):
     pay_lo = int(r["off"].min()) & ~15
     pay_hi = int((r["off"].astype(np.int64) + r["clen"]).max())
     p = planner.build_plan(ar, select=select, payload_range=(pay_lo, pay_hi), out_range=(out_lo, out_hi))
-    dec = ArchiveDecoder(ar, device=device, checksum=checksum, plan=p)
+    dec = ArchiveDecoder(ar, device=device, checksum=checksum, plan=p, settle=False)
     dec.run()
     dec.check()
     out = {}

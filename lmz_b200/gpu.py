@@ -168,7 +168,7 @@ def _host_view(buf, writable: bool = False):
     return arr
 
 
-def _result_memory(lib, size: int):
+def result_memory(lib, size: int):
     """A writable numpy uint8 array of `size` bytes for a result.  Page-locked where the
     library has some to lend (the copy engine then writes it, and a fresh result costs no
     page faults); it goes back to the library when the last view of it is dropped."""
@@ -288,7 +288,7 @@ def decode_batch(streams, offsets, nstr: int, plane: int, out=None, header=None)
     if out is not None and len(out) >= size:
         held, dst = out, _host_view(out, writable=True)
     else:
-        held = dst = _result_memory(lib, size)
+        held = dst = result_memory(lib, size)
     rc = lib.lmz_gpu_decode_batch(_addr(shared), _addr(src), src.size, _addr(table), nstr, plane,
                                   _addr(dst))
     if rc == EBADSTREAM:

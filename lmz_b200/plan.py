@@ -80,6 +80,7 @@ class Plan:
     delta_jobs: np.ndarray = field(default=None)   # chunks with both BF16 planes coded: decoded, merged, a delta undone
                                                    # and checksummed by one kernel; the first n_delta_plain have no base
     n_delta_plain: int = 0
+    extras_at: int = 0             # where `extras` go, bytes from the payload buffer's start
     tables: np.ndarray = field(default=None)   # the shared tables, TABLE_STRIDE bytes apart
 
     @property
@@ -93,8 +94,19 @@ class Plan:
         return int(self.piece_chunk.size)
 
 
-def _gather(blob: np.ndarray, offs: np.ndarray, width: int) -> np.ndarray:
-    return blob[offs[:, None] + np.arange(width, dtype=np.int64)[None, :]]
+def _gather(ar: fmt.Archive, lo: int, offs: np.ndarray, width: int) -> np.ndarray:
+    """[len(offs), width]: the bytes at each of `offs`, counted from byte `lo` of the archive.  Through
+    the library's threads where it is loaded (one page of a file per chunk: reading them is what
+    planning a large archive would otherwise wait for)."""
+    from . import gpu
+    lib = gpu.loaded_library()
+    if lib is not None and ar.blob.flags.c_contiguous:
+        at = np.ascontiguousarray(offs + lo, dtype=np.uint64)
+        out = np.empty((at.size, width), dtype=np.uint8)
+        if lib.lmz_host_gather(ar.fd, ar.blob.ctypes.data, ar.blob.size, at.ctypes.data, at.size, width,
+                               out.ctypes.data) == gpu.OK:
+            return out
+    return ar.blob[lo:][offs[:, None] + np.arange(width, dtype=np.int64)[None, :]]
 
 
 # Fewest 4-byte-element chunks worth the fused kernel: a launch that cannot fill the SMs'
@@ -126,7 +138,7 @@ def _align16(x):
 
 
 def build_plan(ar: fmt.Archive, fuse=True, select=None, payload_range=None,
-               out_range=None, classify: str = "device") -> Plan:
+               out_range=None, classify: str = "device", extras_at: int | None = None) -> Plan:
     """`fuse` routes BF16 chunks whose exponent plane is rANS and whose sign/mantissa
     plane is stored to the fused decode+merge+checksum kernel (no scratch plane),
     4-byte-element chunks whose top byte plane alone is coded likewise when there are
@@ -143,10 +155,16 @@ def build_plan(ar: fmt.Archive, fuse=True, select=None, payload_range=None,
     `classify`: which side counts the live symbols of each fused stream's table to give
     small alphabets the denser kernel instance -- "device" (a kernel, after the upload; the
     host then never touches the payload's stream headers) or "host" (here, with numpy or
-    the library's host helper)."""
+    the library's host helper).
+    `extras_at`: where in the payload buffer the host-inflated header chunks will be (default:
+    right behind the payload range)."""
     ar.check_coverage()
-    r = ar.records if select is None else ar.records[np.asarray(select, dtype=np.int64)]
     lo, hi = (0, int(ar.table_off)) if payload_range is None else map(int, payload_range)
+    if classify == "device":
+        p = _plan_natively(ar, fuse, select, (lo, hi), out_range, extras_at)
+        if p is not None:
+            return p
+    r = ar.records if select is None else ar.records[np.asarray(select, dtype=np.int64)]
     blob = ar.blob[lo:]
     N = r.size
     codec = r["codec"].astype(np.int64)
@@ -171,7 +189,7 @@ def build_plan(ar: fmt.Archive, fuse=True, select=None, payload_range=None,
     if di.size:
         if (clen[di] < 9).any():
             raise CorruptArchive("delta chunk is truncated")           # lmz/codec.py:1036
-        h = _gather(blob, off[di], 9)
+        h = _gather(ar, lo, off[di], 9)
         base[di] = np.ascontiguousarray(h[:, :8]).view("<u8")[:, 0].astype(np.int64) - out_lo
         inner = h[:, 8].astype(np.int64)
         if np.isin(inner, (fmt.CODEC_REF, fmt.CODEC_DELTA)).any():
@@ -181,7 +199,7 @@ def build_plan(ar: fmt.Archive, fuse=True, select=None, payload_range=None,
     if ri.size:
         if (clen[ri] != 8).any():
             raise CorruptArchive("ref chunk payload must be 8 bytes")  # lmz/api.py:873
-        ref_src[ri] = np.ascontiguousarray(_gather(blob, off[ri], 8)).view("<u8")[:, 0].astype(np.int64) - out_lo
+        ref_src[ri] = np.ascontiguousarray(_gather(ar, lo, off[ri], 8)).view("<u8")[:, 0].astype(np.int64) - out_lo
     pass2 = is_delta | is_ref
     src = np.where(is_ref, ref_src, base)
     si = np.nonzero(pass2)[0]
@@ -199,7 +217,8 @@ def build_plan(ar: fmt.Archive, fuse=True, select=None, payload_range=None,
     plane_off = np.zeros((N, 8), dtype=np.uint64)
     scratch_mask = np.zeros(N, dtype=np.uint8)
     src_is_out = np.zeros(N, dtype=np.uint8)
-    extras, extra_pos = [], hi - lo
+    extras_at = hi - lo if extras_at is None else int(extras_at)
+    extras, extra_pos = [], extras_at
     # stream jobs, collected as columns; dst assigned once all are known
     sj_src, sj_len, sj_n, sj_owner, sj_plane = [], [], [], [], []
 
@@ -239,13 +258,9 @@ def build_plan(ar: fmt.Archive, fuse=True, select=None, payload_range=None,
         for j in i[(m == fmt.METHOD_ZSTD) | (m == fmt.METHOD_DEFLATE)]:
             # General-purpose streams are tiny container headers; they are inflated
             # here and travel to the device as stored bytes.
-            raw = blob[eoff[j]:eoff[j] + eclen[j]].tobytes()
-            data = fmt.inflate_tail(raw) if (flags[j] & 3) == fmt.METHOD_ZSTD else _inflate(raw)
-            if len(data) != rlen[j]:
-                raise CorruptArchive(f"chunk decoded to {len(data)} bytes, expected {rlen[j]}")
             plane_off[j, 0] = extra_pos
-            extras.append(np.frombuffer(data, dtype=np.uint8))
-            extra_pos += len(data)
+            extras.append(_general(ar, r[j]))
+            extra_pos += extras[-1].size
         known[i] = True
 
     # byte-plane and BF16 field splits (lmz/codec.py:1176-1223, lmzcore.c:1553-1598)
@@ -264,7 +279,7 @@ def build_plan(ar: fmt.Archive, fuse=True, select=None, payload_range=None,
                 continue
             if (eclen[i] < 4 * npl).any():
                 raise CorruptArchive("split chunk is truncated")
-            lens = np.ascontiguousarray(_gather(blob, eoff[i], 4 * npl)).view("<u4").astype(np.int64)
+            lens = np.ascontiguousarray(_gather(ar, lo, eoff[i], 4 * npl)).view("<u4").astype(np.int64)
             meth = (flags[i][:, None] >> (2 * np.arange(npl))[None, :]) & 3
             nelem = rlen[i] // npl
             starts = eoff[i][:, None] + 4 * npl + np.cumsum(lens, axis=1) - lens
@@ -315,7 +330,7 @@ def build_plan(ar: fmt.Archive, fuse=True, select=None, payload_range=None,
             raise FormatError("a delta whose difference is shared-table coded is not something any writer produces")
         if (esize[ti] != 2).any() or (rlen[ti] % 2).any() or (eclen[ti] < 16).any():
             raise CorruptArchive("a shared-table bf16 chunk is malformed")
-        h = np.ascontiguousarray(_gather(blob, eoff[ti], 16)).view(BF16T_HDR)[:, 0]
+        h = np.ascontiguousarray(_gather(ar, lo, eoff[ti], 16)).view(BF16T_HDR)[:, 0]
         len0, len1 = h["len0"].astype(np.int64), h["len1"].astype(np.int64)
         nelem = rlen[ti] // 2
         if (16 + len0 + len1 > eclen[ti]).any() or (len1 != nelem).any():
@@ -325,7 +340,7 @@ def build_plan(ar: fmt.Archive, fuse=True, select=None, payload_range=None,
             raise CorruptArchive("a shared-table bf16 chunk names a table outside the payload region")
         uniq, inv = np.unique(toff, return_inverse=True)
         tables = np.zeros((uniq.size, TABLE_STRIDE), dtype=np.uint8)
-        tables[:, :fmt.TABLE_BYTES] = _gather(ar.blob, uniq, fmt.TABLE_BYTES)      # read from the file itself: a
+        tables[:, :fmt.TABLE_BYTES] = _gather(ar, 0, uniq, fmt.TABLE_BYTES)      # read from the file itself: a
         table_of[ti] = inv                                                         # table may lie outside this plan's payload range
         kind[ti] = K_BF16
         plane_off[ti, 0], plane_off[ti, 1] = eoff[ti] + 16, eoff[ti] + 16 + len0
@@ -345,7 +360,7 @@ def build_plan(ar: fmt.Archive, fuse=True, select=None, payload_range=None,
             raise CorruptArchive("a conditioned bf16 chunk must have 2-byte elements")
         if (eclen[ci] < 46).any():
             raise CorruptArchive("conditioned bf16 chunk is truncated")
-        h = np.ascontiguousarray(_gather(blob, eoff[ci], 46)).view(BF16C_HDR)[:, 0]
+        h = np.ascontiguousarray(_gather(ar, lo, eoff[ci], 46)).view(BF16C_HDR)[:, 0]
         if (h["k"] != 8).any():
             raise CorruptArchive("conditioned bf16 chunk does not declare 8 buckets")
         nelem = rlen[ci] // 2
@@ -497,7 +512,63 @@ def build_plan(ar: fmt.Archive, fuse=True, select=None, payload_range=None,
                 n_fused_f32_small=int((wide4 & small).sum()),
                 coded_bytes=int(clen.sum()), base_bytes=int(rlen[is_delta].sum()),
                 device_classify=classify != "host", n_fused_t=n_fused_t, tables=tables,
-                delta_jobs=delta_jobs, n_delta_plain=n_delta_plain)
+                delta_jobs=delta_jobs, n_delta_plain=n_delta_plain, extras_at=extras_at)
+
+
+def _general(ar: fmt.Archive, rec) -> np.ndarray:
+    """The bytes of a chunk that is coded with a general-purpose compressor (a container's header)."""
+    raw = ar.blob[int(rec["off"]):int(rec["off"]) + int(rec["clen"])].tobytes()
+    data = fmt.inflate_tail(raw) if (int(rec["flags"]) & 3) == fmt.METHOD_ZSTD else _inflate(raw)
+    if len(data) != rec["rlen"]:
+        raise CorruptArchive(f"chunk decoded to {len(data)} bytes, expected {rec['rlen']}")
+    return np.frombuffer(data, dtype=np.uint8)
+
+
+def _plan_natively(ar: fmt.Archive, fuse, select, payload_range, out_range, extras_at):
+    """The plan of an archive without references or conditioned chunks by the library's own planner,
+    or None: the library is not loaded, or the archive wants (or deserves) the planner in
+    `build_plan`, whose results are the same."""
+    from . import gpu
+    lib = gpu.loaded_library()
+    if lib is None or not ar.blob.flags.c_contiguous:
+        return None
+    r = np.ascontiguousarray(ar.records)
+    sel = None if select is None else np.ascontiguousarray(select, dtype=np.int64)
+    n = int(r.size if sel is None else sel.size)
+    off, rlen = (r["off"], r["rlen"]) if sel is None else (r["off"][sel], r["rlen"][sel])
+    lo, hi = payload_range
+    out_lo, out_hi = (0, int(ar.total)) if out_range is None else map(int, out_range)
+    if not n or lo < 0 or hi < lo or out_lo < 0 or out_hi < out_lo:
+        return None
+    heads = _gather(ar, 0, off, lib.lmz_host_plan_head_bytes())
+    npieces = int((rlen.astype(np.int64) + (PIECE - 1) >> 16).sum())
+    chunks, fused = np.empty(n, dtype=CHUNK_JOB), np.empty(n, dtype=FUSED_JOB)
+    delta, streams = np.empty(n, dtype=DELTA_JOB), np.empty(8 * n, dtype=STREAM_JOB)
+    owner, general = np.empty(8 * n, dtype=np.int64), np.empty(n, dtype=np.int64)
+    piece_chunk = np.empty(max(npieces, 1), dtype=np.uint32)
+    ranges = np.array([lo, hi, out_lo, out_hi], dtype=np.uint64)
+    counts = np.zeros(10, dtype=np.uint64)
+    rc = lib.lmz_host_plan(r.ctypes.data, sel.ctypes.data if sel is not None else None, n, ranges.ctypes.data,
+                           heads.ctypes.data, 2 if fuse == "all" else int(bool(fuse)), FUSE_F32_MIN, chunks.ctypes.data,
+                           fused.ctypes.data, delta.ctypes.data, streams.ctypes.data, owner.ctypes.data,
+                           piece_chunk.ctypes.data, general.ctypes.data, counts.ctypes.data)
+    if rc != gpu.OK:
+        return None
+    nfused, nf32, npair, nstreams, npieces, nplain, ngeneral, nextra, scratch, coded = (int(c) for c in counts)
+    extras = [_general(ar, r[int(i) if sel is None else int(sel[i])]) for i in general[:ngeneral]]
+    at = hi - lo if extras_at is None else int(extras_at)
+    if at != hi - lo and ngeneral:
+        pos = np.empty(n, dtype=np.int64)
+        pos[chunks["record"]] = np.arange(n)
+        chunks["plane_off"][pos[general[:ngeneral]], 0] += np.uint64(at - (hi - lo))
+    return Plan(payload=ar.blob[lo:hi], extras=np.concatenate(extras) if extras else np.zeros(0, dtype=np.uint8),
+                total=out_hi - out_lo, scratch_bytes=scratch + 64, stream_jobs=streams[:nstreams],
+                seg_jobs=np.zeros(0, dtype=STREAM_JOB), chunks=chunks, piece_chunk=piece_chunk[:npieces],
+                piece_split=np.array([0, 0, nplain, npieces, npieces, npieces], dtype=np.uint32),
+                cond_jobs=np.zeros(0, dtype=COND_JOB), cond_pieces=np.zeros(0, dtype=np.uint32),
+                fused_jobs=fused[:nfused], n_fused_f32=nf32, stream_owner=owner[:nstreams], coded_bytes=coded,
+                device_classify=True, delta_jobs=delta[:npair], n_delta_plain=npair, extras_at=at,
+                tables=np.zeros((0, TABLE_STRIDE), dtype=np.uint8))
 
 
 def _inflate(raw: bytes) -> bytes:

@@ -24,6 +24,7 @@ from __future__ import annotations
 
 import ctypes
 import json
+import os
 import struct
 import zlib
 
@@ -33,7 +34,9 @@ from . import archive as fmt, gpu
 
 MIN_GAIN_FLOOR = 1024            # lmz/codec.py:396-398: a coded stream must save max(1024, n >> 8) bytes
 COND_MIN_BYTES = 2 << 20         # chunks of a mebi-element or more are exponent-conditioned by the reference
-BATCH_BYTES = 512 << 20          # BF16 bytes framed per round of kernel launches
+BATCH_BYTES = 64 << 20           # BF16 bytes framed per round of kernel launches: small enough that the first
+                                 # round is on its way to the file early, the others are coded under its writing
+IN_FLIGHT = 4                    # rounds whose payload may be on its way to the file
 
 
 def _safetensors_layout(head: bytes):
@@ -66,20 +69,87 @@ def save_archive(path, members, chunk_size: int = 64 << 10, mapped: bool = True,
     """Write `members` = [(member path, CUDA uint8 tensor holding a BF16 safetensors file)] as
     an lmz archive.  Every tensor must be BF16.  Returns the number of bytes written.
     `stats`, a dict, receives `device_s` (the kernels: split + encode + frame + checksum, timed
-    with CUDA events) and `payload_bytes`.  The framed payload comes back through a page-locked
-    buffer that the module keeps between calls and goes to the file batch by batch."""
+    with CUDA events) and `payload_bytes`.  The framed payload leaves the device in batches, through
+    the page-locked blocks and the threads that loads use (csrc/host_io.inl); what bounds a save is
+    the file system's side of that.  An existing file is overwritten in place and cut to length."""
     if chunk_size < (64 << 10) or chunk_size >= COND_MIN_BYTES or chunk_size % 2:
         raise ValueError("chunk_size must be even, at least 64 KiB and below 2 MiB")
-    with open(path, "wb") as f:
-        return _write_archive(f, members, chunk_size, mapped, stats)
+    fd = os.open(path, os.O_RDWR | os.O_CREAT, 0o666)
+    try:
+        try:
+            return _write_archive(fd, members, chunk_size, mapped, stats)
+        except BaseException:
+            os.ftruncate(fd, 0)
+            raise
+    finally:
+        os.close(fd)
 
 
-def _write_archive(f, members, chunk_size, mapped, stats):
+class _FileWriter:
+    """Device memory -> a file, in the background, from one position to the next.  On a memory-backed
+    file system the bytes are stored through a mapping by all threads at once, elsewhere written."""
+
+    def __init__(self, lib, fd, device):
+        import torch
+        from . import decode
+        self.lib, self.fd, self.device = lib, fd, device
+        self.stream = torch.cuda.current_stream(device).cuda_stream
+        with torch.cuda.device(device):
+            self.handle = lib.lmz_gpu_transfer_new(decode.Staging.shared().handle, self.stream)
+        if not self.handle:
+            raise RuntimeError(gpu.last_error())
+        self.pending = []
+
+    def send(self, data, pos: int) -> None:
+        import torch
+        n = int(data.numel())
+        if not n:
+            return
+        lead = pos & 4095
+        at = self.lib.lmz_host_map_file(self.fd, pos - lead, n + lead)
+        with torch.cuda.device(self.device):
+            r = self.lib.lmz_gpu_transfer_download(self.handle, data.data_ptr(), n, self.fd, at, lead if at else pos, self.stream)
+        if r < 0:
+            raise RuntimeError(gpu.last_error())
+        self.pending.append((r, data, at, n + lead))
+        while len(self.pending) > IN_FLIGHT:
+            self._first_done()
+
+    def _first_done(self):
+        r, _data, at, n = self.pending.pop(0)
+        rc = self.lib.lmz_gpu_transfer_wait(self.handle, r, self.stream)
+        if at:
+            self.lib.lmz_host_unmap_file(at, n)
+        if rc != gpu.OK:
+            raise OSError(f"writing the archive failed: {gpu.last_error()}")
+
+    def close(self):
+        try:
+            while self.pending:
+                self._first_done()
+        finally:
+            handle, self.handle = self.handle, None
+            if handle:
+                self.lib.lmz_gpu_transfer_free(handle)          # (waits for whatever is still under way)
+            for _r, _data, at, n in self.pending:
+                if at:
+                    self.lib.lmz_host_unmap_file(at, n)
+
+
+def _put(fd, data: bytes, pos: int) -> int:
+    view = memoryview(data)
+    while view.nbytes:
+        n = os.pwrite(fd, view, pos)
+        view, pos = view[n:], pos + n
+    return pos
+
+
+def _write_archive(fd, members, chunk_size, mapped, stats):
     import torch
     lib = gpu.library()
     recs_parts, metas, base = [], [], 0                      # record arrays, in file order
-    device_s = 0.0
-    f.write(bytes(fmt.HEADER.size))                          # the header goes in last: it holds the total size
+    timed, pos = [], fmt.HEADER.size                         # the header goes in last: it holds the total size
+    writers = {}
 
     def add_records(dst, rlen, crc, codec, esize, flags, clen):
         part = np.zeros(len(dst), dtype=fmt.RECORD)
@@ -87,76 +157,76 @@ def _write_archive(f, members, chunk_size, mapped, stats):
         part["esize"], part["flags"], part["clen"] = esize, flags, clen
         recs_parts.append(part)
 
-    for mpath, data in members:
-        if not (type(data).__module__.startswith("torch") and data.is_cuda and data.dtype == torch.uint8):
-            raise ValueError("a member must be a CUDA uint8 tensor")
-        flat = data.reshape(-1)
-        size = int(flat.numel())
-        head = bytes(flat[:min(size, 8)].cpu().numpy())
-        hlen = struct.unpack("<Q", head)[0] if len(head) == 8 else 0
-        head = bytes(flat[:min(size, 8 + hlen)].cpu().numpy())
-        start, tensors = _safetensors_layout(head)
-        if any(t["dtype"] != "BF16" for t in tensors.values()):
-            raise ValueError("this writer takes BF16 members only")
-        if (size - start) % 2:
-            raise ValueError("a BF16 data area has an odd number of bytes")
-        # the header: byte chunks of at most chunk_size (lmz/planner.py:582-652)
-        for s in range(0, start, chunk_size):
-            raw = head[s:min(s + chunk_size, start)]
-            payload, codec, flags = _header_chunk(raw)
-            add_records([base + s], [len(raw)], [zlib.crc32(raw) & 0xFFFFFFFF], [codec], [1], [flags], [len(payload)])
-            f.write(payload)
-        # the data area: BF16 chunks, framed on the device
-        body = flat[start:]
-        nbytes = int(body.numel())
-        # (in batches: the coder's slots take a little over twice the bytes they code)
-        batch = max(1, BATCH_BYTES // chunk_size) * chunk_size
-        for b0 in range(0, nbytes, batch):
-            part = body[b0:min(b0 + batch, nbytes)]
-            payload, clen, codec, flags, crc, kernel_s = _frame_bf16(lib, part, chunk_size)
-            device_s += kernel_s
-            at = np.arange(clen.size, dtype=np.int64) * chunk_size
-            add_records(base + start + b0 + at, np.minimum(chunk_size, int(part.numel()) - at), crc, codec,
-                        np.full(clen.size, 2), flags, clen)
-            f.write(memoryview(payload))                      # the chunks' payloads back to back, in record order
-        metas.append({"path": mpath, "size": size, "dst": base, "kind": "safetensors", "mode": 0o644, "crc": 0,
-                      "tensors": {k: dict(v) for k, v in tensors.items()}})
-        base += size
-    recs = np.concatenate(recs_parts) if recs_parts else np.zeros(0, dtype=fmt.RECORD)
-    clens = recs["clen"].astype(np.int64)
-    recs["off"] = fmt.HEADER.size + np.cumsum(clens) - clens
-    off = fmt.HEADER.size + int(clens.sum())
-    manifest = {"version": 1, "tool": "lmz-b200 device writer", "level": 1, "chunk_size": chunk_size,
-                "mapped": bool(mapped), "aligned": False, "entropy": "deflate", "checksum": "crc32",
-                "total_size": base, "members": metas, "chunks": int(recs.size), "table_raw_len": int(recs.nbytes)}
-    table_c = zlib.compress(recs.tobytes(), 3)
-    man_c = zlib.compress(json.dumps(manifest, separators=(",", ":")).encode(), 3)
-    f.write(table_c)
-    f.write(man_c)
-    f.write(fmt.FOOTER.pack(off, len(table_c), off + len(table_c), len(man_c), fmt.TAIL))
-    f.seek(0)
-    f.write(fmt.HEADER.pack(fmt.MAGIC, 6, fmt.FLAG_PAGE_MAPPED if mapped else 0, base, 0, 0))
+    try:
+        for mpath, data in members:
+            if not (type(data).__module__.startswith("torch") and data.is_cuda and data.dtype == torch.uint8):
+                raise ValueError("a member must be a CUDA uint8 tensor")
+            flat = data.reshape(-1)
+            size = int(flat.numel())
+            head = bytes(flat[:min(size, 8)].cpu().numpy())
+            hlen = struct.unpack("<Q", head)[0] if len(head) == 8 else 0
+            head = bytes(flat[:min(size, 8 + hlen)].cpu().numpy())
+            start, tensors = _safetensors_layout(head)
+            if any(t["dtype"] != "BF16" for t in tensors.values()):
+                raise ValueError("this writer takes BF16 members only")
+            if (size - start) % 2:
+                raise ValueError("a BF16 data area has an odd number of bytes")
+            # the header: byte chunks of at most chunk_size (lmz/planner.py:582-652)
+            for s in range(0, start, chunk_size):
+                raw = head[s:min(s + chunk_size, start)]
+                payload, codec, flags = _header_chunk(raw)
+                add_records([base + s], [len(raw)], [zlib.crc32(raw) & 0xFFFFFFFF], [codec], [1], [flags], [len(payload)])
+                pos = _put(fd, payload, pos)
+            # the data area: BF16 chunks, framed on the device
+            body = flat[start:]
+            nbytes = int(body.numel())
+            # (in batches: the coder's slots take a little over twice the bytes they code)
+            batch = max(1, BATCH_BYTES // chunk_size) * chunk_size
+            if data.device not in writers:
+                writers[data.device] = _FileWriter(lib, fd, data.device)
+            for b0 in range(0, nbytes, batch):
+                part = body[b0:min(b0 + batch, nbytes)]
+                payload, clen, codec, flags, crc, events = _frame_bf16(lib, part, chunk_size)
+                timed.append(events)
+                at = np.arange(clen.size, dtype=np.int64) * chunk_size
+                add_records(base + start + b0 + at, np.minimum(chunk_size, int(part.numel()) - at), crc, codec,
+                            np.full(clen.size, 2), flags, clen)
+                writers[data.device].send(payload, pos)           # the chunks' payloads back to back, in record order
+                pos += int(payload.numel())
+            metas.append({"path": mpath, "size": size, "dst": base, "kind": "safetensors", "mode": 0o644, "crc": 0,
+                          "tensors": {k: dict(v) for k, v in tensors.items()}})
+            base += size
+        recs = np.concatenate(recs_parts) if recs_parts else np.zeros(0, dtype=fmt.RECORD)
+        clens = recs["clen"].astype(np.int64)
+        recs["off"] = fmt.HEADER.size + np.cumsum(clens) - clens
+        off = fmt.HEADER.size + int(clens.sum())
+        manifest = {"version": 1, "tool": "lmz-b200 device writer", "level": 1, "chunk_size": chunk_size,
+                    "mapped": bool(mapped), "aligned": False, "entropy": "deflate", "checksum": "crc32",
+                    "total_size": base, "members": metas, "chunks": int(recs.size), "table_raw_len": int(recs.nbytes)}
+        table_c = zlib.compress(recs.tobytes(), 3)
+        man_c = zlib.compress(json.dumps(manifest, separators=(",", ":")).encode(), 3)
+        end = _put(fd, table_c + man_c + fmt.FOOTER.pack(off, len(table_c), off + len(table_c), len(man_c), fmt.TAIL), off)
+    finally:
+        errors = []
+        for w in writers.values():
+            try:
+                w.close()
+            except Exception as exc:
+                errors.append(exc)
+    if errors:
+        raise errors[0]
+    _put(fd, fmt.HEADER.pack(fmt.MAGIC, 6, fmt.FLAG_PAGE_MAPPED if mapped else 0, base, 0, 0), 0)
+    os.ftruncate(fd, end)
     if stats is not None:
-        stats.update(device_s=device_s, payload_bytes=off - fmt.HEADER.size)
-    return off + len(table_c) + len(man_c) + fmt.FOOTER.size
-
-
-_host = {}
-
-
-def _host_buffer(nbytes: int):
-    """A page-locked host buffer of at least `nbytes`, kept between calls (allocating one is slow)."""
-    import torch
-    buf = _host.get("buf")
-    if buf is None or buf.numel() < nbytes:
-        _host["buf"] = buf = torch.empty(max(nbytes, 64 << 20), dtype=torch.uint8).pin_memory()
-    return buf
+        stats.update(device_s=sum(e0.elapsed_time(e1) + e2.elapsed_time(e3) for e0, e1, e2, e3 in timed) / 1e3,
+                     payload_bytes=off - fmt.HEADER.size)
+    return end
 
 
 def _frame_bf16(lib, body, chunk_size: int):
-    """Chunk payloads of one BF16 data area, on the device.  Returns host arrays: the payload
-    bytes of all chunks back to back (a view of the module's page-locked buffer: use it before
-    the next call), per chunk its length, codec id, flags and crc32, and the kernels' seconds."""
+    """Chunk payloads of one BF16 data area, on the device: the payload bytes of all chunks back to
+    back (a device tensor, written by work on the current stream), per chunk its length, codec id,
+    flags and crc32 (host arrays), and the events around the two stretches of kernels."""
     import torch
     dev = body.device
     nbytes = int(body.numel())
@@ -189,10 +259,17 @@ def _frame_bf16(lib, body, chunk_size: int):
                                         None, None, None, None, cs)              # pass 1: sizes and choices
         if rc != gpu.OK:
             raise RuntimeError(f"chunk framing failed ({rc}): {gpu.last_error()}")
+        from . import decode
+        tabs = decode._crc_tables(lib, dev)
+        rc = lib.lmz_gpu_crc32_chunks_dev(body.data_ptr(), nbytes, chunk_size, tabs.data_ptr(),
+                                          meta.data_ptr(), cs)
+        if rc != gpu.OK:
+            raise RuntimeError(f"chunk checksum failed ({rc}): {gpu.last_error()}")
         clen = meta[:, 0].to(torch.int64)
         offs = (torch.cumsum(clen, 0) - clen).contiguous()
         e1.record()
-        total = int(clen.sum())                                                  # (the host needs the size: a sync)
+        m = meta.cpu().numpy()                                                   # (the host needs the sizes: a sync)
+        total = int(m[:, 0].astype(np.int64).sum())
         out = torch.empty(total + 16, dtype=torch.uint8, device=dev)
         e2.record()
         rc = lib.lmz_gpu_frame_bf16_dev(body.data_ptr(), nbytes, chunk_size, lens.data_ptr(), meta.data_ptr(),
@@ -200,17 +277,6 @@ def _frame_bf16(lib, body, chunk_size: int):
                                         out.data_ptr(), cs)                      # pass 2: the bytes
         if rc != gpu.OK:
             raise RuntimeError(f"chunk framing failed ({rc}): {gpu.last_error()}")
-        from . import decode
-        tabs = decode._crc_tables(lib, dev)
-        rc = lib.lmz_gpu_crc32_chunks_dev(body.data_ptr(), nbytes, chunk_size, tabs.data_ptr(),
-                                          meta.data_ptr(), cs)
-        if rc != gpu.OK:
-            raise RuntimeError(f"chunk checksum failed ({rc}): {gpu.last_error()}")
         e3.record()
-        host = _host_buffer(total)[:total]
-        host.copy_(out[:total], non_blocking=True)
-        torch.cuda.current_stream(dev).synchronize()
-        m = meta.cpu().numpy()
-        kernel_s = (e0.elapsed_time(e1) + e2.elapsed_time(e3)) / 1e3
-        return (host.numpy(), m[:, 0].astype(np.int64), m[:, 1], m[:, 2],
-                m[:, 3].astype(np.int64) & 0xFFFFFFFF, kernel_s)
+        return (out[:total], m[:, 0].astype(np.int64), m[:, 1], m[:, 2],
+                m[:, 3].astype(np.int64) & 0xFFFFFFFF, (e0, e1, e2, e3))

@@ -165,6 +165,60 @@ def test_planner_lists_fp32_chunks_after_bf16_in_the_fused_jobs(shard):
     assert plan.build_plan(ar, fuse=False).fused_jobs.size == 0
 
 
+@pytest.fixture
+def native_planner(lib_path, monkeypatch):
+    """The built library as if it had been loaded (its planner needs no GPU)."""
+    from lmz_b200 import _chunks, gpu
+    lib = ctypes.CDLL(lib_path)
+    _chunks.bind(lib)
+    monkeypatch.setattr(gpu._loader, "lib", lib)
+    return lib
+
+
+@pytest.mark.parametrize("fuse", [True, False, "all"])
+@pytest.mark.parametrize("layout", ["mapped", "1MiB", "f32+i64", "both planes", "from a file, sliced"])
+def test_native_planner_gives_the_same_plan(shard, native_planner, monkeypatch, tmp_path, layout, fuse):
+    """Every array and number of the plan, against the planner in Python."""
+    from lmz_b200 import archive, gpu, plan
+    rng = np.random.default_rng(3)
+    kw = dict(mapped=True)
+    if layout == "1MiB":
+        blob = oa.write_archive([("m.safetensors", shard)], chunk_size=1 << 20)
+    elif layout == "f32+i64":
+        f = synth.safetensors_bytes([("w", "F32", (50000,), (rng.standard_normal(50000) * 0.02).astype("<f4").view(np.uint8)),
+                                     ("i", "I64", (9001,), rng.integers(0, 70000, 9001).astype("<i8").view(np.uint8)),
+                                     ("h", "I16", (40000,), rng.integers(0, 50, 40000).astype("<i2").view(np.uint8)),
+                                     ("b", "BF16", (33333,), synth.normal_bf16((33333,), 4))])
+        blob = oa.write_archive([("f.safetensors", f), ("raw.bin", rng.integers(0, 9, 70001).astype(np.uint8))], **kw)
+    elif layout == "both planes":
+        b = synth.safetensors_bytes([("n", "BF16", (90000,), np.repeat(synth.normal_bf16((900,), 5).view("<u2"), 100).view(np.uint8)),
+                                     ("w", "BF16", (90000,), synth.normal_bf16((90000,), 6))])
+        blob = oa.write_archive([("b.safetensors", b)], **kw)
+    else:
+        blob = oa.write_archive([("m.safetensors", shard)], **kw)
+    args = [dict(fuse=fuse)]
+    if layout.startswith("from"):
+        (tmp_path / "a.lmz").write_bytes(blob)
+        blob = str(tmp_path / "a.lmz")
+        r = archive.Archive(blob).records
+        for select in (np.arange(3, r.size - 2), np.array([r.size - 1, 0, 5])):
+            off, dst = r["off"][select].astype(np.int64), r["dst"][select].astype(np.int64)
+            pay = (int(off.min()), int((off + r["clen"][select]).max()))
+            out = (int(dst.min()) & ~15, int((dst + r["rlen"][select]).max()))
+            args += [dict(fuse=fuse, select=select, payload_range=pay, out_range=out),
+                     dict(fuse=fuse, select=select, extras_at=1 << 33)]
+    for kw in args:
+        monkeypatch.setattr(gpu._loader, "lib", native_planner)
+        got = plan._plan_natively(archive.Archive(blob), kw["fuse"], kw.get("select"),
+                                  kw.get("payload_range", (0, archive.Archive(blob).table_off)), kw.get("out_range"), kw.get("extras_at"))
+        assert got is not None
+        monkeypatch.setattr(gpu._loader, "lib", None)
+        want = plan.build_plan(archive.Archive(blob), **kw)
+        for name in want.__dataclass_fields__:
+            a, b = getattr(got, name), getattr(want, name)
+            assert np.array_equal(a, b) if isinstance(b, np.ndarray) else a == b, name
+
+
 def test_planner_gives_two_plane_deltas_jobs_of_their_own(shard):
     """A delta chunk whose difference is a BF16 chunk with both planes coded gets a job for
     the kernel that decodes both planes and undoes the delta in one pass: no scratch streams,
