@@ -141,6 +141,14 @@ int lmz_gpu_decode_batch_dev_noalloc(const void *d_hdr, const void *d_streams, c
                                      unsigned nstr, unsigned plane, void *d_out,
                                      void *cuda_stream, uint32_t *h_status);
 
+/* No counterpart in the reference.  lmz_gpu_decode_batch_dev with every check made and the answer
+ * waited for: each (offset, length) pair against the buffer's `nbytes`, magic, frequencies and
+ * truncation.  d_work: lmz_gpu_batch_work_bytes(nstr) bytes, 256-byte aligned.  64 bytes after the
+ * buffer's end must be readable (fetched, never used); d_streams may start anywhere. */
+int lmz_gpu_batch_work_bytes(unsigned nstr);
+int lmz_gpu_decode_batch_checked_dev(const void *d_hdr, const void *d_streams, uint64_t nbytes, const void *d_off,
+                                     unsigned nstr, unsigned plane, void *d_out, void *d_work, void *cuda_stream);
+
 /* ---- batch encode -----------------------------------------------------------
  * No counterpart in the reference's GPU library (its encoder is CPU code,
  * lmz/native/lmzcore.c:882-937 and :958-979, :1318-1383).  Stream i is byte-identical
@@ -154,6 +162,11 @@ int lmz_gpu_decode_batch_dev_noalloc(const void *d_hdr, const void *d_streams, c
 int lmz_gpu_encode_slot_bytes(unsigned plane);
 int lmz_gpu_encode_batch_dev(const void *d_planes, unsigned nstr, unsigned plane, void *d_slots,
                              void *d_lengths, void *cuda_stream);
+/* The offset table of the streams packed back to back (d_offsets, 2 * nstr uint64) from their
+ * lengths, their total size and how many planes could not be coded; waits for cuda_stream.
+ * d_work: 16 bytes. */
+int lmz_gpu_pack_offsets_dev(const void *d_lengths, unsigned nstr, void *d_offsets, void *d_work, uint64_t *h_total,
+                             unsigned *h_failed, void *cuda_stream);
 /* Copy the streams out of their slots into one buffer: d_offsets = 2*nstr uint64
  * (byte offset in d_out, length) - the layout lmz_gpu_decode_batch_dev reads. */
 int lmz_gpu_pack_streams_dev(const void *d_slots, unsigned plane, const void *d_offsets, unsigned nstr,

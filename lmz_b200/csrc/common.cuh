@@ -106,6 +106,11 @@ __device__ __forceinline__ uint2 lds_u64(uint32_t a)
 }
 
 // The same where `on`, without a branch.
+__device__ __forceinline__ void sts_u16_if(uint32_t on, uint32_t a, uint32_t v)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.shared.u16 [%0], %1;\n\t}"
+                 ::"r"(a), "r"(v), "r"(on) : "memory");
+}
 __device__ __forceinline__ void sts_u64_if(uint32_t on, uint32_t a, uint32_t x, uint32_t y)
 {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\t@p st.shared.v2.u32 [%0], {%1,%2};\n\t}"

@@ -111,6 +111,8 @@ struct StreamArgs {
     const uint32_t *order;
     const uint32_t *count;
     uint32_t order_from_back;
+    uint32_t most_ctas;         // for the launcher: fewer CTAs than there are SMs (0 = one per SM), as something
+                                // else runs beside this launch
 };
 
 constexpr uint32_t F_WIDE_BYTES = PROB_SCALE * 4;   // a slot -> entry table
@@ -876,6 +878,23 @@ __global__ void k_classify(StreamArgs a, uint32_t small_live, uint32_t *order, u
         const uint32_t pos = atomicAdd(&counts[small ? 0 : 1], 1u);
         order[small ? pos : a.njobs - 1 - pos] = job;
     }
+}
+
+// (offset, length) pairs -> stream jobs of `plane` symbols each, in order in the output.  A stream
+// outside the `nbytes` of the buffer gets an empty job and bit 1 of *bad.
+__global__ void k_batch_jobs(const uint64_t *pairs, uint64_t nbytes, uint32_t nstr, uint32_t plane, StreamJob *jobs, uint32_t *bad)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nstr) return;
+    const uint64_t at = pairs[2 * (size_t)i], len = pairs[2 * (size_t)i + 1];
+    const bool inside = at <= nbytes && len <= nbytes - at && len >> 32 == 0;
+    StreamJob j{};
+    j.src_off = inside ? at : 0;
+    j.dst_off = (uint64_t)i * plane;
+    j.src_len = inside ? (uint32_t)len : 0u;
+    j.n = inside ? plane : 0u;
+    jobs[i] = j;
+    if (!inside) atomicOr(bad, 2u);
 }
 
 }  // namespace lmz

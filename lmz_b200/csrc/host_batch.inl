@@ -243,3 +243,71 @@ API int lmz_gpu_decode_batch(const void *hdr, const void *streams, size_t nbytes
     }
     return LMZ_GPU_OK;
 }
+
+// ---- batches in device memory, with the answer ------------------------------------------------
+
+API int lmz_gpu_batch_work_bytes(unsigned nstr)
+{
+    const uint64_t b = (uint64_t)nstr * sizeof(StreamJob) + 256;
+    return b > 0x7fffffffu ? 0 : (int)b;
+}
+
+API int lmz_gpu_decode_batch_checked_dev(const void *d_hdr, const void *d_streams, uint64_t nbytes, const void *d_off,
+                                         unsigned nstr, unsigned plane, void *d_out, void *d_work, void *cuda_stream)
+{
+    if (nstr == 0) return LMZ_GPU_OK;
+    if (plane == 0) return fail_msg(LMZ_GPU_EUNSUPPORTED, "plane is zero");
+    if (int rc = device_ready()) return rc;
+    int device = 0;
+    CK("cudaGetDevice", cudaGetDevice(&device));
+    cudaStream_t cs = (cudaStream_t)cuda_stream;
+    uint32_t *d_verdict = static_cast<uint32_t *>(d_work);
+    StreamJob *jobs = reinterpret_cast<StreamJob *>(static_cast<uint8_t *>(d_work) + 256);
+    Borrowed b(device);
+    CK("a page-locked word", b.w.need(0, 64));
+    volatile uint32_t *verdict = reinterpret_cast<volatile uint32_t *>(b.w.pin);
+    CK("clear the verdict", cudaMemsetAsync(d_verdict, 0, 4, cs));
+    k_batch_jobs<<<(nstr + 255) / 256, 256, 0, cs>>>(static_cast<const uint64_t *>(d_off), nbytes, nstr, plane, jobs, d_verdict);
+    cudaError_t le = cudaGetLastError();
+    if (le != cudaSuccess) return fail_cuda("launch k_batch_jobs", le);
+    RansArgs a{};
+    a.src = static_cast<const uint8_t *>(d_streams);
+    a.jobs = jobs;
+    a.njobs = nstr;
+    a.dst = static_cast<uint8_t *>(d_out);
+    a.shared_hdr = static_cast<const uint8_t *>(d_hdr);
+    a.any_bad = d_verdict;
+    if (int rc = launch_rans(a, cs)) return rc;
+    CK("copy the verdict out", cudaMemcpyAsync(b.w.pin, d_verdict, 4, cudaMemcpyDeviceToHost, cs));
+    CK("decode", cudaStreamSynchronize(cs));
+    b.sound = true;
+    if (*verdict & 2u) return fail_msg(LMZ_GPU_EBADSTREAM, "a stream lies outside the buffer");
+    if (*verdict) return fail_msg(LMZ_GPU_EBADSTREAM, "a stream is malformed or truncated");
+    return LMZ_GPU_OK;
+}
+
+API int lmz_gpu_pack_offsets_dev(const void *d_lengths, unsigned nstr, void *d_offsets, void *d_work, uint64_t *h_total,
+                                 unsigned *h_failed, void *cuda_stream)
+{
+    if (int rc = device_ready()) return rc;
+    *h_total = 0;
+    *h_failed = 0;
+    if (nstr == 0) return LMZ_GPU_OK;
+    if (!d_lengths || !d_offsets || !d_work) return fail_msg(LMZ_GPU_EUNSUPPORTED, "null argument");
+    int device = 0;
+    CK("cudaGetDevice", cudaGetDevice(&device));
+    cudaStream_t cs = (cudaStream_t)cuda_stream;
+    Borrowed b(device);
+    CK("a page-locked block", b.w.need(0, 64));
+    k_pack_offsets<<<1, 1024, 0, cs>>>(static_cast<const uint32_t *>(d_lengths), nstr, static_cast<uint64_t *>(d_offsets),
+                                       static_cast<uint64_t *>(d_work));
+    cudaError_t le = cudaGetLastError();
+    if (le != cudaSuccess) return fail_cuda("launch k_pack_offsets", le);
+    CK("copy the sizes out", cudaMemcpyAsync(b.w.pin, d_work, 16, cudaMemcpyDeviceToHost, cs));
+    CK("encode", cudaStreamSynchronize(cs));
+    b.sound = true;
+    const volatile uint64_t *got = reinterpret_cast<const volatile uint64_t *>(b.w.pin);
+    *h_total = got[0];
+    *h_failed = (unsigned)got[1];
+    return LMZ_GPU_OK;
+}

@@ -128,7 +128,8 @@ static int launch_stream(const StreamArgs &a, cudaStream_t cs)
     // At most one CTA per SM; its warps take four streams at a time.  As many rounds of fours as the
     // fullest CTA would need, the warps of a CTA just enough for them (when the device holds the count,
     // as if every job of the launch were of this class).
-    const uint32_t quads = (a.njobs + 3) / 4, grid = quads < (uint32_t)sms ? quads : (uint32_t)sms;
+    const uint32_t quads = (a.njobs + 3) / 4, room = a.most_ctas ? a.most_ctas : (uint32_t)sms;
+    const uint32_t grid = quads < room ? quads : room;
     auto waves = [&](uint32_t most) { return (quads + grid * most - 1) / (grid * most); };
     auto warps = [&](uint32_t most) { return (quads + grid * waves(most) - 1) / (grid * waves(most)); };
     // 8-byte ring entries make the shorter step, 4-byte ones leave room for more warps: those are
@@ -350,11 +351,7 @@ API int lmz_gpu_encode_batch_dev(const void *d_planes, unsigned nstr, unsigned p
     if (!d_planes || !d_slots || !d_lengths) return fail_msg(LMZ_GPU_EUNSUPPORTED, "null argument");
     if (plane == 0 || plane > ENCODE_MAX_PLANE) return fail_msg(LMZ_GPU_EUNSUPPORTED, "plane must be 1 .. 2^29 bytes");
     if ((uintptr_t)d_slots & 511u) return fail_msg(LMZ_GPU_EUNSUPPORTED, "the slot buffer must be 512-byte aligned");
-    constexpr int WARPS = 4;      // 43 KiB of shared memory a CTA: five CTAs (80 streams) per SM
-    static bool done[64];
-    constexpr uint32_t shm = encode_smem_bytes(WARPS);
-    rc = opt_in_smem(k_encode<WARPS>, shm, done);
-    if (rc) return rc;
+    constexpr uint32_t shm = encode_smem_bytes();
     EncodeArgs a{};
     a.src = (const uint8_t *)d_planes;
     a.plane = plane;
@@ -362,7 +359,7 @@ API int lmz_gpu_encode_batch_dev(const void *d_planes, unsigned nstr, unsigned p
     a.slots = (uint8_t *)d_slots;
     a.slot_bytes = encode_slot_bytes(plane);
     a.lengths = (uint32_t *)d_lengths;
-    k_encode<WARPS><<<(nstr + WARPS * 4 - 1) / (WARPS * 4), WARPS * 32, shm, (cudaStream_t)cuda_stream>>>(a);
+    k_encode<<<(nstr + 3) / 4, 32, shm, (cudaStream_t)cuda_stream>>>(a);
     cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) return fail_cuda("launch k_encode", le);
     return LMZ_GPU_OK;

@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(256) k_frame_pack(const uint8_t *src, uint64_t
     const FrameMeta m = meta[c];
     if (m.codec == CODEC_ID_STORED) {
         const uint8_t *s = src + (uint64_t)c * chunk;
-        for (uint32_t i = threadIdx.x; i < len; i += 256) d[i] = s[i];
+        copy_bytes(d, s, len, threadIdx.x, 256);
         return;
     }
     uint32_t plen[2];
@@ -109,8 +109,8 @@ __global__ void __launch_bounds__(256) k_frame_pack(const uint8_t *src, uint64_t
         const uint32_t v = plen[threadIdx.x >> 2];
         d[threadIdx.x] = (uint8_t)(v >> (8 * (threadIdx.x & 3)));
     }
-    for (uint32_t i = threadIdx.x; i < plen[0]; i += 256) d[8 + i] = from[0][i];
-    for (uint32_t i = threadIdx.x; i < plen[1]; i += 256) d[8 + plen[0] + i] = from[1][i];
+    copy_bytes(d + 8, from[0], plen[0], threadIdx.x, 256);
+    copy_bytes(d + 8 + plen[0], from[1], plen[1], threadIdx.x, 256);
 }
 
 // crc32 of every chunk: 256 threads per chunk, each over its own contiguous run (table lookups

@@ -46,6 +46,10 @@ _SIGNATURES = {
     "lmz_gpu_decode_batch_dev_noalloc": (_C.c_int, [_C.c_void_p] * 3 + [_C.c_uint, _C.c_uint, _C.c_void_p,
                                                                          _C.c_void_p, _C.c_void_p]),
     "lmz_gpu_set_device": (_C.c_int, [_C.c_int]),
+    "lmz_gpu_batch_work_bytes": (_C.c_int, [_C.c_uint]),
+    "lmz_gpu_decode_batch_checked_dev": (_C.c_int, [_C.c_void_p, _C.c_void_p, _C.c_uint64, _C.c_void_p, _C.c_uint,
+                                                    _C.c_uint] + [_C.c_void_p] * 3),
+    "lmz_gpu_pack_offsets_dev": (_C.c_int, [_C.c_void_p, _C.c_uint] + [_C.c_void_p] * 5),
     "lmz_gpu_host_alloc": (_C.c_void_p, [_C.c_size_t]),
     "lmz_gpu_host_free": (None, [_C.c_void_p]),
     "lmz_gpu_trim": (None, []),
@@ -296,16 +300,18 @@ def decode_batch(streams, offsets, nstr: int, plane: int, out=None, header=None)
     return memoryview(held)[:size] if rc == OK else None
 
 
+_READ_AHEAD = 64             # bytes the decode kernel may fetch past the last stream
+
+
 def _decode_batch_cuda(lib, streams, offsets, nstr, plane, out, header):
-    """Device-to-device decode with per-stream verdicts.  The offset table is checked
-    against the buffer before anything is launched, and the kernels report bad magic, bad
-    frequency sums and truncation per stream, so hostile input ends in ValueError."""
+    """Device-to-device decode.  The offset table is checked against the buffer, and magic, frequency
+    sums and truncation per stream, on the device; one word comes back, so hostile input ends in
+    ValueError."""
     import torch
 
     dev = streams.device
     with torch.cuda.device(dev):
-        flat = streams.reshape(-1)
-        pad = pad_bytes()
+        flat = streams.reshape(-1).view(torch.uint8)
         if _is_cuda_tensor(offsets):
             offs = offsets.reshape(-1).view(torch.int64)
         else:
@@ -315,15 +321,14 @@ def _decode_batch_cuda(lib, streams, offsets, nstr, plane, out, header):
             offs = torch.frombuffer(bytearray(table[:16 * nstr]), dtype=torch.int64).to(dev)
         if offs.numel() < 2 * nstr:
             raise ValueError("offsets is too short")
-        pairs = offs[:2 * nstr].reshape(nstr, 2)
-        start, length = pairs[:, 0], pairs[:, 1]
-        inside = (start >= 0) & (length >= 0) & (length < (1 << 32)) & (start <= flat.numel()) & \
-                 (length <= flat.numel() - start)
-        if not bool(inside.all()):
-            raise ValueError("a stream lies outside the buffer")
-        buf = torch.empty(flat.numel() + pad, dtype=torch.uint8, device=dev)
-        buf[:flat.numel()].copy_(flat)
-        buf[flat.numel():].zero_()
+        offs = offs.contiguous()
+        # the kernel reads a little past the last stream: only a tensor that ends where its memory
+        # does has to be copied for that
+        if flat.untyped_storage().nbytes() - flat.storage_offset() - flat.numel() < _READ_AHEAD:
+            buf = torch.empty(flat.numel() + _READ_AHEAD, dtype=torch.uint8, device=dev)
+            buf[:flat.numel()].copy_(flat)
+        else:
+            buf = flat
         hdr = None
         if header is not None:
             hdr = header if _is_cuda_tensor(header) else \
@@ -331,24 +336,14 @@ def _decode_batch_cuda(lib, streams, offsets, nstr, plane, out, header):
         size = nstr * plane
         dst = out if (out is not None and _is_cuda_tensor(out) and out.numel() >= size) \
             else torch.empty(size, dtype=torch.uint8, device=dev)
-        # one 32-byte job per stream (include/lmz_b200.h, lmz_stream_job): source offset,
-        # destination offset, then length and symbol count packed into the third word
-        jobs = torch.zeros((nstr, 4), dtype=torch.int64, device=dev)
-        jobs[:, 0] = start
-        jobs[:, 1] = torch.arange(nstr, dtype=torch.int64, device=dev) * plane
-        jobs[:, 2] = length | (plane << 32)
-        verdicts = torch.zeros(nstr + 1, dtype=torch.int32, device=dev)      # [nstr] = any bad
-        cs = torch.cuda.current_stream(dev)
-        rc = lib.lmz_gpu_decode_streams_dev(jobs.data_ptr(), nstr, buf.data_ptr(), dst.data_ptr(),
-                                            hdr.data_ptr() if hdr is not None else None,
-                                            verdicts.data_ptr(), verdicts[nstr:].data_ptr(),
-                                            cs.cuda_stream)
-        if rc != OK:
-            return None
-        cs.synchronize()             # also keeps the inputs alive until the kernels have read them
-        if int(verdicts[nstr].item()) != 0:
-            raise ValueError("malformed rANS stream")
-        return dst[:size]
+        work = torch.empty(nstr * 32 + 256, dtype=torch.uint8, device=dev)
+        # (synchronous, which also keeps the inputs alive until the kernels have read them)
+        rc = lib.lmz_gpu_decode_batch_checked_dev(hdr.data_ptr() if hdr is not None else None, buf.data_ptr(), flat.numel(),
+                                                  offs.data_ptr(), nstr, plane, dst.data_ptr(), work.data_ptr(),
+                                                  torch.cuda.current_stream(dev).cuda_stream)
+        if rc == EBADSTREAM:
+            raise ValueError((lib.lmz_gpu_last_error() or b"malformed rANS stream").decode(errors="replace"))
+        return dst[:size] if rc == OK else None
 
 
 def encode_batch(planes, nstr: int, plane: int):
@@ -383,21 +378,26 @@ def encode_batch(planes, nstr: int, plane: int):
         if slot <= 0:
             raise ValueError("plane must be at most 2^29 bytes")
         slots = torch.empty(nstr * slot, dtype=torch.uint8, device=dev)       # the allocator aligns to 512
-        lens = torch.zeros(nstr, dtype=torch.int32, device=dev)
+        lens = torch.empty(nstr, dtype=torch.int32, device=dev)
         cs = torch.cuda.current_stream(dev).cuda_stream
         rc = lib.lmz_gpu_encode_batch_dev(src.data_ptr(), nstr, plane, slots.data_ptr(), lens.data_ptr(), cs)
         if rc != OK:
             return None
-        lens64 = lens.to(torch.int64)
-        if bool((lens64 == 0).any()):
+        offs = torch.empty(2 * nstr, dtype=torch.int64, device=dev)
+        sums = torch.empty(2, dtype=torch.int64, device=dev)
+        total, failed = ctypes.c_uint64(), ctypes.c_uint()
+        rc = lib.lmz_gpu_pack_offsets_dev(lens.data_ptr(), nstr, offs.data_ptr(), sums.data_ptr(), ctypes.byref(total),
+                                          ctypes.byref(failed), cs)
+        if rc != OK:
+            return None
+        if failed.value:
             raise ValueError("a plane could not be coded")
-        offs = torch.stack((torch.cumsum(lens64, 0) - lens64, lens64), dim=1).reshape(-1).contiguous()
-        total = int(lens64.sum())
-        out = torch.zeros(total + pad_bytes(), dtype=torch.uint8, device=dev)
+        total = total.value
+        out = torch.empty(total + pad_bytes(), dtype=torch.uint8, device=dev)
+        out[total:].zero_()
         rc = lib.lmz_gpu_pack_streams_dev(slots.data_ptr(), plane, offs.data_ptr(), nstr, out.data_ptr(), cs)
         if rc != OK:
             return None
-        torch.cuda.current_stream(dev).synchronize()
         if on_device:
             return out[:total], offs
         return out[:total].cpu().numpy().tobytes(), offs.cpu().numpy().astype("<u8").tobytes()

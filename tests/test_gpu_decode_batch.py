@@ -172,3 +172,25 @@ def test_results_in_lent_memory_stay_their_callers_own(gpu, orc, nstr, plane, ta
     gpu.library().lmz_gpu_trim()
     gpu.decode_batch(*sets[2][0], nstr, plane)
     assert bytes(part) == sets[0][1][:1]
+
+
+@pytest.mark.parametrize("lead,tail", [(0, 0), (0, 63), (0, 64), (1, 0), (3, 200), (16, 64)])
+def test_device_batches_wherever_they_lie(gpu, orc, lead, tail, table_mode):
+    """A tensor that starts anywhere in its memory and ends where that does (it is then copied
+    for the kernel's reading ahead) or before; offsets outside it are refused."""
+    if table_mode != -1:
+        pytest.skip("where the bytes lie does not depend on the table layout")
+    import torch
+    plains = [shaped("skewed", 1001, i) for i in range(9)]
+    blob, offs = pack_streams([orc.rans_encode(p) for p in plains])
+    whole = torch.zeros(lead + len(blob) + tail, dtype=torch.uint8, device="cuda")
+    t = whole[lead:lead + len(blob)]
+    t.copy_(torch.frombuffer(bytearray(blob), dtype=torch.uint8))
+    out = gpu.decode_batch(t, offs, 9, 1001)
+    assert out.cpu().numpy().tobytes() == b"".join(p.tobytes() for p in plains)
+    table = np.frombuffer(offs, dtype="<u8").copy()
+    for at, value in ((16, len(blob) - 100), (16, 1 << 63), (17, len(blob) - int(table[16]) + 1), (17, 1 << 32)):
+        bad = table.copy()
+        bad[at] = value
+        with pytest.raises(ValueError):
+            gpu.decode_batch(t, bad.tobytes(), 9, 1001)

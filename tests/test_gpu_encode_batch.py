@@ -87,3 +87,11 @@ def test_random_round_trips(gpu, orc):
             assert bytes(gpu.decode_batch(streams, offsets, nstr, plane)) == data.tobytes(), (trial, plane, nstr, live)
     finally:
         lib.lmz_gpu_set_table_mode(-1)
+
+
+@pytest.mark.parametrize("plane", [511_999, 512_000, 512_001, 1_024_016])
+@pytest.mark.parametrize("dist", ["single", "two", "uniform"])
+def test_counts_past_one_stretch_of_the_lanes_counters(gpu, orc, dist, plane):
+    """Planes around the lengths at which the encoder sums its 16-bit counters: all of one
+    symbol (a lane's counter at its fullest), next to all of one, and every symbol."""
+    _check(gpu, orc, [distribution(dist, plane, 5 * i + plane) for i in range(3)])
