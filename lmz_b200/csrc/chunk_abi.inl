@@ -148,7 +148,8 @@ API int lmz_host_alphabet_sizes(const void *base, const uint64_t *offs, size_t n
 // Chunks whose two BF16 planes are both coded, jobs [first, first + count) of the plan's list: alphabets
 // counted on the device, then chunks whose first plane has a small one (the rule) to the instance with
 // mixed table sizes (72 streams per SM), the others to the one with full-size tables for both planes (64).
-static int launch_two_plane(const lmz_decode_plan *p, uint32_t first, uint32_t count, cudaStream_t cs)
+// `most_ctas`: see StreamArgs::most_ctas.
+static int launch_two_plane(const lmz_decode_plan *p, uint32_t first, uint32_t count, uint32_t most_ctas, cudaStream_t cs)
 {
     if (count == 0) return LMZ_GPU_OK;
     if (!p->d_delta_jobs || !p->d_delta_status || !p->d_delta_order)
@@ -157,6 +158,7 @@ static int launch_two_plane(const lmz_decode_plan *p, uint32_t first, uint32_t c
     da.src = (const uint8_t *)p->d_payload;
     da.djobs = (const DeltaJob *)p->d_delta_jobs + first;
     da.njobs = 2 * count;
+    da.most_ctas = most_ctas;
     da.dst = (uint8_t *)p->d_out;
     da.status = (uint32_t *)p->d_delta_status + 2 * (size_t)first;
     da.any_bad = (uint32_t *)p->d_any_bad;
@@ -205,9 +207,19 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
     SideScope scope;
     if (p->n_fused_t % (F_SHARED_SINK_WARPS * 4u))
         return fail_msg(LMZ_GPU_EUNSUPPORTED, "n_fused_t is not a multiple of lmz_gpu_shared_group()");
-    const bool other_work = p->n_stream_jobs || p->n_cond || p->piece_split[2] > p->piece_split[0] ||
+    const bool other_work = p->n_stream_jobs || p->n_cond || p->n_delta_plain || p->piece_split[2] > p->piece_split[0] ||
                             p->piece_split[5] > p->piece_split[3];
     if (p->n_delta_plain > p->n_delta) return fail_msg(LMZ_GPU_EUNSUPPORTED, "n_delta_plain exceeds n_delta");
+    // Plain chunks with both planes coded: the two-plane kernel without a base.  Few chunks are of this
+    // shape (29 of an 8B model's 245 069) but one takes as long as any other, so they go first and beside
+    // the fused kernel, packed into a few CTAs (eight warps: 16 chunks) with as many SMs left to them.
+    // Behind it they had the chip to themselves: four 8B decoder layers with one such chunk took
+    // 2.5 ms where the fused kernel takes 1.9.
+    uint32_t pairs_ctas = 0;
+    if (p->n_delta_plain && (ph & 1u) && (p->n_fused || p->n_fused_t) && (ph & 16u)) {
+        pairs_ctas = (p->n_delta_plain + 15) / 16;
+        if (pairs_ctas > (uint32_t)sms / 4) pairs_ctas = 0;          // a large part of the work: no corner of its own
+    }
     if ((p->n_fused || p->n_fused_t) && (ph & 16u)) {
         cudaStream_t fs = cs;
         if (ph == 0x1fu && other_work) {        // whole decode: run the fused kernel beside the rest
@@ -218,7 +230,14 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
                 fs = side->stream;
             }
         }
+        if (pairs_ctas && fs != cs) {
+            rc = launch_two_plane(p, 0, p->n_delta_plain, pairs_ctas, cs);
+            if (rc) return rc;
+        } else {
+            pairs_ctas = 0;
+        }
         StreamArgs sa{};
+        sa.most_ctas = pairs_ctas ? (uint32_t)sms - pairs_ctas : 0;
         sa.src = (const uint8_t *)p->d_payload;
         sa.jobs = (const FusedJob *)p->d_fused_jobs;
         sa.njobs = p->n_fused;
@@ -305,14 +324,13 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
         }
     }
 
-    // 1. plain chunks with both planes coded: the two-plane kernel without a base (few chunks are of this
-    //    shape: a short launch, beside the fused kernel when that one has a stream of its own)
-    if (p->n_delta_plain && (ph & 1u)) {
-        rc = launch_two_plane(p, 0, p->n_delta_plain, cs);
+    // 1. (those two-plane chunks, where they have not gone ahead)
+    if (p->n_delta_plain && (ph & 1u) && !pairs_ctas) {
+        rc = launch_two_plane(p, 0, p->n_delta_plain, 0, cs);
         if (rc) return rc;
     }
 
-    //    and every rANS stream whose length is known up front, into scratch
+    //    every rANS stream whose length is known up front, into scratch
     if (p->n_stream_jobs && (ph & 1u)) {
         RansArgs a{};
         a.src = (const uint8_t *)p->d_payload;
@@ -397,7 +415,7 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
             // pass 2 (and the verdicts) read what the fused kernel wrote
             CK("join the side stream", scope.join());
             // delta chunks with both planes coded, now that the chunks they are differences against are in place
-            rc = launch_two_plane(p, p->n_delta_plain, p->n_delta - p->n_delta_plain, cs);
+            rc = launch_two_plane(p, p->n_delta_plain, p->n_delta - p->n_delta_plain, 0, cs);
             if (rc) return rc;
             continue;
         }

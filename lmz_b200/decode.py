@@ -594,8 +594,27 @@ def decode_tensors(ar, names, device=None, checksum: bool = True):
     out_hi = int((r["dst"].astype(np.int64) + r["rlen"]).max())
     pay_lo = int(r["off"].min()) & ~15
     pay_hi = int((r["off"].astype(np.int64) + r["clen"]).max())
-    p = planner.build_plan(ar, select=select, payload_range=(pay_lo, pay_hi), out_range=(out_lo, out_hi))
-    dec = ArchiveDecoder(ar, device=device, checksum=checksum, plan=p, settle=False)
+    dev = torch.device(device if device is not None else f"cuda:{torch.cuda.current_device()}")
+    with torch.cuda.device(dev):
+        # only what the chunks hold crosses, to its place in a buffer that spans all of it, while the
+        # chunks are planned (gaps below 256 KiB are not worth a range of their own)
+        general = (r["codec"] == fmt.CODEC_ZSTD) & ((r["flags"] & 3) != fmt.METHOD_STORED) & ((r["flags"] & 3) != fmt.METHOD_RANS)
+        room = pay_hi - pay_lo + int(r["rlen"][general].sum()) + gpu.pad_bytes()
+        payload = torch.empty(room, dtype=torch.uint8, device=dev)
+        up = _Uploader(ar.blob, dev)
+        order = np.argsort(r["off"], kind="stable")
+        lo = r["off"][order].astype(np.int64)
+        hi = np.maximum.accumulate(lo + r["clen"][order])
+        first = np.concatenate(([True], lo[1:] > hi[:-1] + (256 << 10)))
+        last = np.concatenate((first[1:], [True]))
+        sent = [up.send(a, b, payload[a - pay_lo:]) for a, b in zip(lo[first].tolist(), hi[last].tolist())]
+        try:
+            p = planner.build_plan(ar, select=select, payload_range=(pay_lo, pay_hi), out_range=(out_lo, out_hi))
+            dec = ArchiveDecoder(ar, device=dev, checksum=checksum, plan=p, payload=payload, settle=False)
+            for si in sent:
+                up.wait(si)
+        finally:
+            up.close()
     dec.run()
     dec.check()
     out = {}
