@@ -125,17 +125,25 @@ constexpr uint32_t PADDED_PIECE = PIECE_ELEMS + (PIECE_ELEMS >> 7) * 4;
 // CRC tables in the bank-quartered layout (k_stream, k_cond_finish), laid out so that the warp's 32 lookups of one load never
 // share a bank: entry i of table j, copy r sits at word 32 i + 8 j + r -- a table owns a
 // quarter of the banks and each of its eight copies one bank of that quarter.  Lane k of
-// group g uses copy k, and the groups take the four bytes of a state word in rotated order
-// (group g starts at byte g), so in each of the four loads the groups are in four different
-// tables, i.e. bank quarters.  b[i] = table base + this lane's word for load i; rot = 8 g.
+// group g uses copy k, and load i of group g takes byte i ^ g of a state word, so in each of
+// the four loads the groups are in four different tables, i.e. bank quarters.  b[i] = table
+// base + this lane's word for load i; rot = the byte permutation.
 struct CrcQuarters {
     uint32_t b[4], rot;
 };
+__device__ __forceinline__ uint32_t mad128(uint32_t a, uint32_t b)
+{
+    uint32_t v;
+    asm("mad.lo.u32 %0, %1, 128, %2;" : "=r"(v) : "r"(a), "r"(b));
+    return v;
+}
 __device__ __forceinline__ uint32_t crc_feed4q(const CrcQuarters &q, uint32_t s)
 {
-    const uint32_t r = __funnelshift_r(s, s, q.rot);     // byte i of r = byte (i + g) & 3 of s
-    return lds_u32(((r << 7) & 0x7f80u) | q.b[0]) ^ lds_u32(((r >> 1) & 0x7f80u) | q.b[1]) ^
-           lds_u32(((r >> 9) & 0x7f80u) | q.b[2]) ^ lds_u32(((r >> 17) & 0x7f80u) | q.b[3]);
+    // (a byte permute and a multiply-add per lookup: half of the work on the multiplier's pipe, where a
+    // shift and a mask would both be the integer pipe's, which is the busy one in k_stream)
+    const uint32_t r = __byte_perm(s, 0u, q.rot);        // byte i of r = byte i ^ g of s
+    return lds_u32(mad128(__byte_perm(r, 0u, 0x4440u), q.b[0])) ^ lds_u32(mad128(__byte_perm(r, 0u, 0x4441u), q.b[1])) ^
+           lds_u32(mad128(__byte_perm(r, 0u, 0x4442u), q.b[2])) ^ lds_u32(mad128(__byte_perm(r, 0u, 0x4443u), q.b[3]));
 }
 
 struct FinishArgs {
@@ -226,8 +234,8 @@ __global__ void __launch_bounds__(FINISH_THREADS * SUBS) k_finish(FinishArgs a)
     {
         const uint32_t k = lane & 7u, g = lane >> 3;
 #pragma unroll
-        for (uint32_t i = 0; i < 4; i++) cq.b[i] = tab0 + 32u * (3u - ((i + g) & 3u)) + 4u * k;
-        cq.rot = 8u * g;
+        for (uint32_t i = 0; i < 4; i++) cq.b[i] = tab0 + 32u * (3u - (i ^ g)) + 4u * k;
+        cq.rot = 0x3210u ^ (0x1111u * g);
     }
     auto sub_sync = [&]() {
         if (SUBS == 1) __syncthreads();

@@ -285,8 +285,8 @@ __global__ void __launch_bounds__(CF_THREADS, 1) k_cond_finish(FinishArgs a)
     // through table 3 - m, which crc_feed4q looks for in slot m
     const uint32_t k = lane & 7u, g = lane >> 3;
 #pragma unroll
-    for (uint32_t i = 0; i < 4; i++) sh.cq.b[i] = tab0 + 32u * (3u - ((i + g) & 3u)) + 4u * k;
-    sh.cq.rot = 8u * g;
+    for (uint32_t i = 0; i < 4; i++) sh.cq.b[i] = tab0 + 32u * (3u - (i ^ g)) + 4u * k;
+    sh.cq.rot = 0x3210u ^ (0x1111u * g);
     if (a.piece_crc && fits) {
         uint32_t *tw = reinterpret_cast<uint32_t *>(csm + (tab0 - s0));
         for (uint32_t i = threadIdx.x; i < CF_TABLE_BYTES / 4; i += CF_THREADS)

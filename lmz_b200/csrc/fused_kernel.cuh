@@ -344,11 +344,11 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, TR8) * 32, 1) k_s
                                                : m_.cf + grp * (WIDE ? 0u : 4u * CFN); };
     const uint32_t cf_sa = cf_of(gi);
     const uint32_t stage_sa = m_.stage + gi * F_STAGE;
-    // byte (i + g) & 3 of a state word goes through slice table 3 - ((i + g) & 3)
+    // byte i ^ g of a state word goes through slice table 3 - (i ^ g)
     CrcQuarters cq;
 #pragma unroll
-    for (uint32_t i = 0; i < 4; i++) cq.b[i] = tab0 + 32u * (3u - ((i + g) & 3u)) + 4u * k;
-    cq.rot = 8u * g;
+    for (uint32_t i = 0; i < 4; i++) cq.b[i] = tab0 + 32u * (3u - (i ^ g)) + 4u * k;
+    cq.rot = 0x3210u ^ (0x1111u * g);
     const uint32_t tla = m_.adv - 4096u;                            // crc_advance<0> adds 4 .. 7 KiB
 
     uint32_t limit = a.njobs;
