@@ -105,6 +105,11 @@ __device__ __forceinline__ uint2 lds_u64(uint32_t a)
     return v;
 }
 
+__device__ __forceinline__ void prefetch_l2(const void *p)
+{
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
 // The same where `on`, without a branch.
 __device__ __forceinline__ void sts_u16_if(uint32_t on, uint32_t a, uint32_t v)
 {

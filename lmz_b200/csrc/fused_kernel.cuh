@@ -41,8 +41,8 @@
 //   * CFN = 128: level 2 has 128 slots, the four streams of a warp rotated 8
 //     entries apart so their popular symbols sit in different banks; streams with
 //     more than 104 live symbols must be given to the CFN = 256 instance
-//   * TR8: a ring entry is word and table entry (8 bytes); otherwise word and level-2 offset
-//     (4 bytes, half the space: more streams per SM for one more lookup in a refilled lane's step)
+//   * a ring entry is word and table entry (8 bytes), or word and level-2 offset (TR_4: 4 bytes, half
+//     the space: more streams per SM for one more lookup in a refilled lane's step)
 //   * CFN = 0: a 16 KiB slot -> entry table per stream; CFN = -1: one such table per CTA, for
 //     batches whose streams share one 516-byte table (lmz_gpu_decode_batch's d_hdr) or for the
 //     chunks of a shared-table archive (StreamArgs.tables); a stream is then states + words
@@ -55,6 +55,11 @@
 namespace lmz {
 
 enum : int { SINK_BYTES = 0, SINK_BF16 = 1, SINK_F32 = 2, SINK_DELTA = 3 };
+// How a kernel instance keeps its translated words, and how many warps it is for (see Words):
+//   TR_FEW  8-byte ring entries, data brought to the L2 early: up to 16 warps
+//   TR_8    8-byte ring entries
+//   TR_4    4-byte ring entries: the most warps
+enum : int { TR_4 = 0, TR_8 = 1, TR_FEW = 2 };
 constexpr uint32_t F_STAGE = 144;                  // a tile's 128 symbols + 16: groups land 4 banks apart
 constexpr uint32_t TR_N = 64, TR_MIRROR = 32;      // ring of translated words; a block of four steps reads at most 32
 constexpr uint32_t TR_ROUND = 16;                  // words translated at a time, two per lane
@@ -129,14 +134,14 @@ constexpr uint32_t F_SMEM_BASE = 1024, F_SMEM_DYN = 232448;
 struct StreamSmem {
     uint32_t cf, stage, tr, l1, crc, adv, poison, end;
 };
-__host__ __device__ constexpr uint32_t tr_entry(bool tr8) { return tr8 ? 8u : 4u; }
-__host__ __device__ constexpr uint32_t tr_group(bool tr8) { return (TR_N + TR_MIRROR) * tr_entry(tr8); }
-__host__ __device__ constexpr StreamSmem stream_smem_with(int cfn, bool crc, int sink, bool tr8, uint32_t W, bool low_stage, bool low_tr)
+__host__ __device__ constexpr uint32_t tr_entry(int mode) { return mode == TR_4 ? 4u : 8u; }
+__host__ __device__ constexpr uint32_t tr_group(int mode) { return (TR_N + TR_MIRROR) * tr_entry(mode); }
+__host__ __device__ constexpr StreamSmem stream_smem_with(int cfn, bool crc, int sink, int mode, uint32_t W, bool low_stage, bool low_tr)
 {
     StreamSmem m{};
     uint32_t p = F_SMEM_BASE;
     m.poison = p; p += 16;
-    const uint32_t cf = cfn > 0 ? W * 16u * (uint32_t)cfn : 0u, stage = W * 4u * F_STAGE, tr = W * 4u * tr_group(tr8);
+    const uint32_t cf = cfn > 0 ? W * 16u * (uint32_t)cfn : 0u, stage = W * 4u * F_STAGE, tr = W * 4u * tr_group(mode);
     m.cf = p; p += cf;
     if (low_stage) { m.stage = p; p += stage; }
     if (low_tr) { m.tr = p; p += tr; }
@@ -153,22 +158,22 @@ __host__ __device__ constexpr StreamSmem stream_smem_with(int cfn, bool crc, int
     m.end = p;
     return m;
 }
-__host__ __device__ constexpr StreamSmem stream_smem(int cfn, bool crc, int sink, bool tr8, uint32_t W)
+__host__ __device__ constexpr StreamSmem stream_smem(int cfn, bool crc, int sink, int mode, uint32_t W)
 {
-    StreamSmem best = stream_smem_with(cfn, crc, sink, tr8, W, false, false);
+    StreamSmem best = stream_smem_with(cfn, crc, sink, mode, W, false, false);
     for (int i = 1; i < 4; i++) {
-        const StreamSmem m = stream_smem_with(cfn, crc, sink, tr8, W, (i & 1) != 0, (i & 2) != 0);
+        const StreamSmem m = stream_smem_with(cfn, crc, sink, mode, W, (i & 1) != 0, (i & 2) != 0);
         if (m.end < best.end) best = m;
     }
     return best;
 }
-// The most warps of an instance: what shared memory holds, and registers (96 a thread up to 20
-// warps, 80 up to 24).
-__host__ __device__ constexpr uint32_t stream_warps(int cfn, bool crc, int sink, bool tr8)
+// The most warps of an instance: what shared memory holds, and registers (128 a thread up to 16
+// warps, 96 up to 20, 80 up to 24).
+__host__ __device__ constexpr uint32_t stream_warps(int cfn, bool crc, int sink, int mode)
 {
     if (cfn < 0 && sink == SINK_BF16) return F_SHARED_SINK_WARPS;
-    uint32_t w = cfn < 0 ? 32u : 24u;
-    while (stream_smem(cfn, crc, sink, tr8, w).end > F_SMEM_BASE + F_SMEM_DYN) w--;
+    uint32_t w = cfn < 0 ? 32u : mode == TR_FEW ? 16u : 24u;
+    while (stream_smem(cfn, crc, sink, mode, w).end > F_SMEM_BASE + F_SMEM_DYN) w--;
     return w;
 }
 
@@ -188,13 +193,23 @@ template <int CFN>
 __device__ __forceinline__ uint32_t ref_addr(uint32_t ref, uint32_t cf_sa) { return CFN <= 0 ? ref : cf_sa + ref; }
 
 // Positions are in bytes of ring entries and only grow; the ring index is the position modulo the ring.
-template <int CFN, bool TR8>
+//
+// A warp that waits for one load waits for all that the compiler counts on the same counter, however
+// long ago they were requested, so where warps are few every load in flight is a stall (one B200, 12
+// streams per SM: a third of the time; bulk copies through a raw ring cost as much as they saved).
+// TR_FEW has the L2 fetch words 512 bytes ahead, and the stored bytes that a sink merges four tiles
+// ahead.  On one B200: a 4096 x 14336 BF16 tensor's kernel 583 -> 456 us, the delta kernel of a
+// three-checkpoint chain 1190 -> 1070 us.
+template <int CFN, int MODE>
 struct Words {
-    static constexpr uint32_t ES = tr_entry(TR8), RB = TR_N * ES, LOW = TR_MIRROR * ES;
+    static constexpr bool TR8 = MODE != TR_4;
+    static constexpr int AHEAD = MODE == TR_FEW ? 2 : 1;
+    static constexpr uint32_t ES = tr_entry(MODE), RB = TR_N * ES, LOW = TR_MIRROR * ES;
     static_assert(TR8 || CFN > 0, "a wide table's entry does not fit a 4-byte ring entry");
     uint32_t sa;             // the ring
     uint32_t rd, wr;         // words consumed / translated so far
     uint32_t lo, hi, sh;     // this lane's next two words: aligned loads and the shift between them
+    uint32_t lo2, hi2;       // TR_FEW: and the two after those
     const uint32_t *next;
     int32_t left;            // rounds of the stream that have not been requested
 
@@ -204,14 +219,29 @@ struct Words {
     __device__ __forceinline__ void request(bool want)
     {
         const int32_t go = want ? left : 0;
-        asm volatile("{\n\t.reg .pred p;\n\tsetp.gt.s32 p, %3, 0;\n\t"
-                     "@p ld.global.nc.L2::256B.u32 %0, [%2];\n\t@p ld.global.nc.u32 %1, [%2+4];\n\t}"
-                     : "+r"(lo), "+r"(hi) : "l"(next), "r"(go));
+        if constexpr (MODE == TR_FEW) {
+            if (want) { lo = lo2; hi = hi2; }
+            asm volatile("{\n\t.reg .pred p;\n\tsetp.gt.s32 p, %3, 0;\n\t"
+                         "@p ld.global.nc.u32 %0, [%2];\n\t@p ld.global.nc.u32 %1, [%2+4];\n\t}"
+                         : "+r"(lo2), "+r"(hi2) : "l"(next), "r"(go));
+            if (go > 20 && !(reinterpret_cast<uintptr_t>(next) & 64u)) prefetch_l2(next + 128);
+        } else {
+            asm volatile("{\n\t.reg .pred p;\n\tsetp.gt.s32 p, %3, 0;\n\t"
+                         "@p ld.global.nc.L2::256B.u32 %0, [%2];\n\t@p ld.global.nc.u32 %1, [%2+4];\n\t}"
+                         : "+r"(lo), "+r"(hi) : "l"(next), "r"(go));
+        }
         next += want ? TR_ROUND / 2 : 0;
         left -= want ? 1 : 0;
     }
     __device__ __forceinline__ uint32_t block() const { return sa + (rd & (RB - 1)); }
     __device__ __forceinline__ bool low() const { return wr - rd < LOW; }
+    // Words consumed so far of a stream of that many bytes.  (Positions are 32-bit bytes of ring entries
+    // and wrap in a stream of half a Gi words; the rounds do not.  AHEAD rounds are loaded ahead of `wr`.)
+    __device__ __forceinline__ uint32_t taken(uint32_t bytes) const
+    {
+        const int32_t rounds = (int32_t)((bytes / 2 + TR_ROUND - 1) / TR_ROUND) - left - AHEAD;
+        return TR_ROUND * (uint32_t)rounds - (wr - rd) / ES;
+    }
     // A group that only runs along asks for no more words (and writes none: there is never room).
     __device__ __forceinline__ void retire() { wr = rd + 0x40000000u; }
 
@@ -260,12 +290,12 @@ __device__ __forceinline__ uint32_t rans_update(uint32_t x, uint32_t e)
 
 // The second half of a step: x2 is the updated state; a lane that needs a refill takes the ring
 // entry at word_sa, the others look their slot up.  `e` leaves as the entry of the new state's slot.
-template <int CFN, bool TR8>
+template <int CFN, int MODE>
 __device__ __forceinline__ void refill(uint32_t &x, uint32_t &e, uint32_t x2, bool need, uint32_t word_sa, uint32_t l1_sa,
                                        uint32_t cf_sa)
 {
     uint32_t a = ref_addr<CFN>(slot_ref<CFN>(x2, l1_sa), cf_sa);
-    if (TR8) {
+    if (MODE != TR_4) {
         e = lds_u32(a);
         const uint2 w = lds_u64(word_sa);
         if (need) { e = w.x; x2 = __byte_perm(w.y, x2, 0x5410); }
@@ -283,7 +313,7 @@ __device__ __forceinline__ void refill(uint32_t &x, uint32_t &e, uint32_t x2, bo
 // lane's = bits of the older bytes plus the lanes below it in the newest, so one
 // popcount of hist & below (= 0xffffff00 | lanes below) gives the offset from
 // the block's start.
-template <int CFN, bool TR8, bool FIRST>
+template <int CFN, int MODE, bool FIRST>
 __device__ __forceinline__ void stream_step4(uint32_t &x, uint32_t &e, uint32_t &hist, uint32_t base, uint32_t l1_sa,
                                              uint32_t cf_sa, uint32_t below, uint32_t vsel)
 {
@@ -291,11 +321,11 @@ __device__ __forceinline__ void stream_step4(uint32_t &x, uint32_t &e, uint32_t 
     const bool need = x2 < RANS_LOW;
     const uint32_t vote = __ballot_sync(0xffffffffu, need);
     hist = __byte_perm(vote, FIRST ? 0u : hist, vsel);
-    refill<CFN, TR8>(x, e, x2, need, base + tr_entry(TR8) * __popc(hist & below), l1_sa, cf_sa);
+    refill<CFN, MODE>(x, e, x2, need, base + tr_entry(MODE) * __popc(hist & below), l1_sa, cf_sa);
 }
 
 // One step of a ragged tile, any lane mix: lanes past the end keep their state.
-template <int CFN, bool TR8>
+template <int CFN, int MODE>
 __device__ __forceinline__ void stream_step(uint32_t &x, uint32_t &e, uint32_t &base, uint32_t l1_sa, uint32_t cf_sa,
                                             uint32_t lt_mask, uint32_t grp_mask, bool active)
 {
@@ -303,13 +333,13 @@ __device__ __forceinline__ void stream_step(uint32_t &x, uint32_t &e, uint32_t &
     const bool need = active && x2 < RANS_LOW;
     const uint32_t vote = __ballot_sync(0xffffffffu, need);
     uint32_t nx = x, ne = e;
-    refill<CFN, TR8>(nx, ne, x2, need, base + tr_entry(TR8) * __popc(vote & lt_mask), l1_sa, cf_sa);
+    refill<CFN, MODE>(nx, ne, x2, need, base + tr_entry(MODE) * __popc(vote & lt_mask), l1_sa, cf_sa);
     if (active) { x = nx; e = ne; }
-    base += tr_entry(TR8) * __popc(vote & grp_mask);
+    base += tr_entry(MODE) * __popc(vote & grp_mask);
 }
 
-template <int SINK, bool CRC, int CFN, bool TR8>
-__global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, TR8) * 32, 1) k_stream(StreamArgs a)
+template <int SINK, bool CRC, int CFN, int MODE>
+__global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_stream(StreamArgs a)
 {
     // SINK_BF16 checksums: lane k keeps one running value per word of its 32-byte unit,
     // ra[i] = sum over the piece's rows so far of word i * x^(2048 * rows since); a row
@@ -334,7 +364,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, TR8) * 32, 1) k_s
 
     // ---- shared memory (addresses are 32-bit shared-space addresses) ----------------------
     const uint32_t s0 = smem_addr(ssm);
-    const StreamSmem m_ = stream_smem(CFN, CRC, SINK, TR8, W);
+    const StreamSmem m_ = stream_smem(CFN, CRC, SINK, MODE, W);
     const bool fits = s0 == F_SMEM_BASE && m_.end <= s0 + dynamic_smem_bytes();
     auto gen = [&](uint32_t sa) { return ssm + (sa - s0); };
     const uint32_t tab0 = m_.crc;
@@ -421,10 +451,10 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, TR8) * 32, 1) k_s
 
     // the words follow table and states; the first four rounds are requested before the table is
     // built, which hides their latency
-    Words<CFN, TR8> wd;
-    wd.sa = m_.tr + gi * tr_group(TR8);
+    Words<CFN, MODE> wd;
+    wd.sa = m_.tr + gi * tr_group(MODE);
     wd.rd = wd.wr = 0;
-    wd.lo = wd.hi = 0;
+    wd.lo = wd.hi = wd.lo2 = wd.hi2 = 0;
     uint32_t first[4][2];
     uint32_t x = 0;
     {
@@ -436,9 +466,9 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, TR8) * 32, 1) k_s
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             wd.request(true);
-            first[j][0] = wd.lo; first[j][1] = wd.hi;
+            first[j][0] = MODE == TR_FEW ? wd.lo2 : wd.lo; first[j][1] = MODE == TR_FEW ? wd.hi2 : wd.hi;
         }
-        wd.request(true);
+        for (int j = 0; j < wd.AHEAD; j++) wd.request(true);
         if (n) {
             uint32_t s[1];
             load_words_nc<1>(sbase + LEAD - STATE_BYTES + 4 * k, s);
@@ -495,7 +525,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, TR8) * 32, 1) k_s
     uint32_t e = 0;
     if (__any_sync(0xffffffffu, n != 0)) {
         // the whole ring, so that a group without a stream finds nothing but bounded entries in it
-        const uint32_t lo = wd.lo, hi = wd.hi;
+        const uint32_t lo = wd.lo, hi = wd.hi, lo2 = wd.lo2, hi2 = wd.hi2;
         const uint32_t *next = wd.next;
         const int32_t left = wd.left;
         wd.left = 0;
@@ -504,7 +534,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, TR8) * 32, 1) k_s
             wd.lo = first[j][0]; wd.hi = first[j][1];
             wd.round(l1_sa, cf_sa, k);
         }
-        wd.lo = lo; wd.hi = hi; wd.next = next; wd.left = left;
+        wd.lo = lo; wd.hi = hi; wd.lo2 = lo2; wd.hi2 = hi2; wd.next = next; wd.left = left;
         if (n == 0) wd.retire();
         e = lds_u32(ref_addr<CFN>(slot_ref<CFN>(x, l1_sa), cf_sa));
         __syncwarp();
@@ -531,7 +561,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, TR8) * 32, 1) k_s
     // NEXT tile decodes (32 independent table lookups that hide behind the decode chain),
     // then that tile's words are XORed in.  SINK_F32 keeps one value, `acc`.
     uint32_t acc = 0, ra[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    uint32_t last_x = x, last_rd = 0;             // state and words consumed at the stream's end
+    uint32_t last_x = x, taken = 0;               // state and words consumed at the stream's end
 
     // ---- tiles of 128 symbols ---------------------------------------------------------
     const uint32_t warp_tiles = __reduce_max_sync(0xffffffffu, my_tiles);
@@ -551,6 +581,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, TR8) * 32, 1) k_s
                 const uint32_t *pq = reinterpret_cast<const uint32_t *>(reinterpret_cast<uintptr_t>(pp) & ~uintptr_t(3));
 #pragma unroll
                 for (int i = 0; i < 5; i++) pr[j][i] = mine ? __ldg(pq + i) : 0u;
+                if (MODE == TR_FEW && rem > 5 * TS) prefetch_l2(pq + 4 * TS / 4);
             }
         }
         auto top_up = [&]() {
@@ -571,38 +602,38 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, TR8) * 32, 1) k_s
             for (uint32_t s8 = 0; s8 < TS / NLANES; s8 += 8) {
                 // eight steps: two blocks, and where warps are few a round of translation between the
                 // steps of the first (where they are many, top_up does all of them: fewer instructions)
-                constexpr bool WOVEN = TR8;
+                constexpr bool WOVEN = MODE != TR_4;
                 top_up();
                 uint32_t base = wd.block(), hist = 0;
                 if (WOVEN) wd.part1();
                 put(s8);
-                stream_step4<CFN, TR8, true>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                stream_step4<CFN, MODE, true>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
                 if (WOVEN) wd.part2(l1_sa);
                 put(s8 + 1);
-                stream_step4<CFN, TR8, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                stream_step4<CFN, MODE, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
                 fold(s8 / 2);
                 put(s8 + 2);
-                stream_step4<CFN, TR8, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                stream_step4<CFN, MODE, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
                 if (WOVEN) wd.part3(cf_sa, k);
                 put(s8 + 3);
-                stream_step4<CFN, TR8, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                stream_step4<CFN, MODE, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
                 fold(s8 / 2 + 1);
-                wd.rd += tr_entry(TR8) * __popc(hist);
+                wd.rd += tr_entry(MODE) * __popc(hist);
                 __syncwarp();
                 top_up();
                 base = wd.block();
                 hist = 0;
                 put(s8 + 4);
-                stream_step4<CFN, TR8, true>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                stream_step4<CFN, MODE, true>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
                 put(s8 + 5);
-                stream_step4<CFN, TR8, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                stream_step4<CFN, MODE, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
                 fold(s8 / 2 + 2);
                 put(s8 + 6);
-                stream_step4<CFN, TR8, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                stream_step4<CFN, MODE, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
                 put(s8 + 7);
-                stream_step4<CFN, TR8, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                stream_step4<CFN, MODE, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
                 fold(s8 / 2 + 3);
-                wd.rd += tr_entry(TR8) * __popc(hist);
+                wd.rd += tr_entry(MODE) * __popc(hist);
             }
         } else {
 #pragma unroll
@@ -616,13 +647,13 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, TR8) * 32, 1) k_s
                 for (uint32_t s = s4; s < s4 + 4; s++) {
                     const bool active = s * NLANES + k < rem;
                     if (active) put(s);
-                    stream_step<CFN, TR8>(x, e, base, l1_sa, cf_sa, lt_mask, grp_mask, active);
+                    stream_step<CFN, MODE>(x, e, base, l1_sa, cf_sa, lt_mask, grp_mask, active);
                 }
                 wd.rd += base - base0;
             }
         }
         __syncwarp();
-        if (t + 1 == my_tiles) { last_x = x; last_rd = wd.rd; wd.retire(); }
+        if (t + 1 == my_tiles) { last_x = x; taken = wd.taken(slen - LEAD); wd.retire(); }
         if (!rem) continue;
         if (SINK == SINK_DELTA) {
             // ---- both planes' symbols of this lane's eight elements, merge, XOR the base, write, checksum
@@ -636,6 +667,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, TR8) * 32, 1) k_s
             if (has_base && n > (t + 1) * TS + 8u * j16) {         // next tile's base bytes, if this lane has any
 #pragma unroll
                 for (int i = 0; i < 5; i++) m[i] = __ldg(mq + (size_t)(t + 1) * (2 * TS / 4) + i);
+                if (MODE == TR_FEW && t + 4 < my_tiles) prefetch_l2(mq + (size_t)(t + 4) * (2 * TS / 4));
             }
             uint8_t *d = out + (size_t)done * 2 + 16u * j16;
             const uint32_t ve = rem > 8u * j16 ? min(rem - 8u * j16, 8u) : 0u;   // valid elements of this lane
@@ -776,6 +808,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, TR8) * 32, 1) k_s
         if (t + 1 < my_tiles) {                                // next tile's stored bytes
 #pragma unroll
             for (int i = 0; i < 5; i++) m[i] = __ldg(mq + (size_t)(t + 1) * (TILE / 4) + i);
+            if (MODE == TR_FEW && t + 5 < my_tiles) prefetch_l2(mq + (size_t)(t + 5) * (TILE / 4));
         }
         uint8_t *d = out + (size_t)done * 2 + k * F_UNIT;
         const uint32_t ve = rem > 16 * k ? min(rem - 16 * k, 16u) : 0u;   // valid elements of this lane
@@ -832,7 +865,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, TR8) * 32, 1) k_s
     const uint32_t all_rest = __ballot_sync(0xffffffffu, last_x == RANS_LOW) & grp_mask;
     if (have && k == 0) {
         if (st == ST_OK && n) {
-            const uint32_t used = LEAD + 2 * (last_rd / tr_entry(TR8));
+            const uint64_t used = LEAD + 2 * (uint64_t)taken;
             if (used > slen) st = ST_OVERRUN;
             else if (used != slen || all_rest != grp_mask) st = ST_SLACK;
         }

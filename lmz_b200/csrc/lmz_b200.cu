@@ -99,14 +99,14 @@ static int stream_smem_ok()
 
 static int sm_count(int *out);
 
-template <int SINK, bool CRC, int CFN, bool TR8>
+template <int SINK, bool CRC, int CFN, int MODE>
 static int launch_stream_as(const StreamArgs &a, uint32_t grid, uint32_t W, cudaStream_t cs)
 {
     static bool done[64];
-    const uint32_t shm = stream_smem(CFN, CRC, SINK, TR8, W).end - F_SMEM_BASE;
-    int rc = opt_in_smem(k_stream<SINK, CRC, CFN, TR8>, F_SMEM_DYN, done);
+    const uint32_t shm = stream_smem(CFN, CRC, SINK, MODE, W).end - F_SMEM_BASE;
+    int rc = opt_in_smem(k_stream<SINK, CRC, CFN, MODE>, F_SMEM_DYN, done);
     if (rc) return rc;
-    k_stream<SINK, CRC, CFN, TR8><<<grid, W * 32, shm, cs>>>(a);
+    k_stream<SINK, CRC, CFN, MODE><<<grid, W * 32, shm, cs>>>(a);
     cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) return fail_cuda("launch k_stream", le);
     return LMZ_GPU_OK;
@@ -124,7 +124,7 @@ static int launch_stream(const StreamArgs &a, cudaStream_t cs)
     rc = sm_count(&sms);
     if (rc) return rc;
     if (CFN < 0 && a.tables)          // the job list is laid out 80 to a CTA
-        return launch_stream_as<SINK, CRC, CFN, true>(a, a.njobs / (F_SHARED_SINK_WARPS * 4), F_SHARED_SINK_WARPS, cs);
+        return launch_stream_as<SINK, CRC, CFN, TR_8>(a, a.njobs / (F_SHARED_SINK_WARPS * 4), F_SHARED_SINK_WARPS, cs);
     // At most one CTA per SM; its warps take four streams at a time.  As many rounds of fours as the
     // fullest CTA would need, the warps of a CTA just enough for them (when the device holds the count,
     // as if every job of the launch were of this class).
@@ -132,15 +132,23 @@ static int launch_stream(const StreamArgs &a, cudaStream_t cs)
     const uint32_t grid = quads < room ? quads : room;
     auto waves = [&](uint32_t most) { return (quads + grid * most - 1) / (grid * most); };
     auto warps = [&](uint32_t most) { return (quads + grid * waves(most) - 1) / (grid * waves(most)); };
-    // 8-byte ring entries make the shorter step, 4-byte ones leave room for more warps: those are
-    // taken where they save a round (one B200, 64 KiB BF16 chunks with checksums, 8-byte against
-    // 4-byte entries: 180 chunks per SM 2160 against 1880 us, 34 per SM 605 against 675).
-    constexpr uint32_t most8 = stream_warps(CFN, CRC, SINK, true);
+    // TR_FEW makes the shortest step, TR_4 has room for the most warps: that is taken where it saves a
+    // round (one B200, 64 KiB BF16 chunks with checksums, TR_8 against TR_4: 180 chunks per SM
+    // 2160 against 1880 us, 34 per SM 605 against 675).  Streams of bytes alone, with no checksum tables to
+    // make room for, run as many warps of TR_8 as of TR_4, and faster (193 streams per SM 1490 against
+    // 1535 us).  A wide table's three warps have nothing to gain from the L2 (50.4 ms against 50.2).
     if constexpr (CFN > 0) {
-        constexpr uint32_t most4 = stream_warps(CFN, CRC, SINK, false);
-        if (waves(most4) < waves(most8)) return launch_stream_as<SINK, CRC, CFN, false>(a, grid, warps(most4), cs);
+        constexpr uint32_t few = stream_warps(CFN, CRC, SINK, TR_FEW), most4 = stream_warps(CFN, CRC, SINK, TR_4);
+        if constexpr (SINK == SINK_BYTES) {
+            constexpr uint32_t most8 = stream_warps(CFN, CRC, SINK, TR_8);
+            if (waves(most8) <= waves(most4) && waves(most8) < waves(few))
+                return launch_stream_as<SINK, CRC, CFN, TR_8>(a, grid, warps(most8), cs);
+        }
+        if (waves(most4) < waves(few)) return launch_stream_as<SINK, CRC, CFN, TR_4>(a, grid, warps(most4), cs);
+        return launch_stream_as<SINK, CRC, CFN, TR_FEW>(a, grid, warps(few), cs);
+    } else {
+        return launch_stream_as<SINK, CRC, CFN, TR_8>(a, grid, warps(stream_warps(CFN, CRC, SINK, TR_8)), cs);
     }
-    return launch_stream_as<SINK, CRC, CFN, true>(a, grid, warps(most8), cs);
 }
 
 // `force_mode` < 0 picks by batch size.
@@ -236,8 +244,8 @@ static int launch_compact_sorted(const RansArgs &a, cudaStream_t cs)
 // Streams that carry their own table.  Up to 12 per SM a wide table each fits, and a step is one
 // lookup shorter; up to 76 per SM the full-size compact tables take the launch in one round,
 // whatever the alphabets; above that small alphabets go to the denser instance.
-constexpr unsigned WIDE_PER_SM = 4 * stream_warps(0, false, SINK_BYTES, true);
-constexpr unsigned COMPACT_PER_SM = 4 * stream_warps(256, false, SINK_BYTES, true);
+constexpr unsigned WIDE_PER_SM = 4 * stream_warps(0, false, SINK_BYTES, TR_8);
+constexpr unsigned COMPACT_PER_SM = 4 * stream_warps(256, false, SINK_BYTES, TR_8);
 
 static int launch_rans(const RansArgs &a, cudaStream_t cs, bool may_alloc = true)
 {
