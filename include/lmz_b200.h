@@ -108,8 +108,9 @@ typedef struct lmz_stream_job {
     uint64_t dst_off; /* first output byte, bytes from d_dst */
     uint32_t src_len; /* stream length */
     uint32_t n;       /* symbols to decode */
-    uint32_t flags;   /* 0 */
-    uint32_t aux;     /* 0 */
+    uint32_t flags;   /* 0; 1: n is only a bound -- the stream is decoded until its words run out, which is
+                       * then no failure */
+    uint32_t aux;     /* 0; with flags 1 the kernel writes how many symbols the words were good for */
 } lmz_stream_job;
 
 /* Generalises lmz_gpu_decode_batch_dev (lmz/gpu/lmzgpu.cu:412-467) to streams
@@ -280,7 +281,8 @@ typedef struct lmz_decode_plan {
     void *d_scratch;            /* decoded planes and segments */
     void *d_out;                /* the concatenated output space, 64 bytes of slack */
     const void *d_stream_jobs;  /* rANS streams whose decoded size the host knows */
-    void *d_seg_jobs;           /* 8 per conditioned chunk, sized on the device */
+    void *d_seg_jobs;           /* coded segments of conditioned chunks, sized on the device; those of a chunk
+                                 * marked `open` are stream jobs of their own (flags 1) instead */
     void *d_stream_status;      /* uint32 per stream job */
     void *d_seg_status;         /* uint32 per segment job */
     const void *d_fused_jobs;   /* chunks decoded, merged and checksummed by one kernel: BF16 chunks

@@ -359,6 +359,7 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
         c.piece_wcnt = (uint16_t *)p->d_piece_wcnt;
         c.piece_lcnt = (uint32_t *)p->d_piece_lcnt;
         c.seg_jobs = (StreamJob *)p->d_seg_jobs;
+        c.stream_jobs = (const StreamJob *)p->d_stream_jobs;
         c.payload = (const uint8_t *)p->d_payload;
         c.scratch = (const uint8_t *)p->d_scratch;
         CK("memset hist", cudaMemsetAsync(p->d_hist, 0, (size_t)p->n_cond * 1024, cs));

@@ -43,15 +43,18 @@ static_assert(sizeof(ChunkJob) == 104, "ChunkJob layout is shared with the host"
 struct CondJob {
     uint64_t exp_off;        // exponent plane: scratch offset, or payload offset when stored
     uint64_t seg_src[8];     // coded segment b in the payload
-    uint64_t seg_scratch;    // where decoded rANS segments go (scratch)
+    uint64_t seg_scratch;    // where decoded rANS segments go (scratch), back to back; where they are open
+                             // streams (see STREAM_OPEN), seg_stride bytes apart
     uint32_t seg_len[8];
     uint32_t nelem;
-    uint32_t seg_job0;       // first of the chunk's 8 StreamJob slots
+    uint32_t seg_job0;       // first of the chunk's segment jobs (open: among the stream jobs)
     uint32_t piece0;
     uint32_t chunk;
     uint8_t seg_method[8];
     uint8_t exp_in_scratch;
-    uint8_t pad_[7];
+    uint8_t open;            // the segments are decoded beside the exponent planes, as open streams
+    uint8_t pad_[2];
+    uint32_t seg_stride;
 };
 static_assert(sizeof(CondJob) == 144, "CondJob layout is shared with the host");
 

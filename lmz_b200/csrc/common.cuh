@@ -35,9 +35,13 @@ struct StreamJob {
     uint64_t dst_off;   // first output byte, bytes from the destination base
     uint32_t src_len;   // stream length in bytes
     uint32_t n;         // symbols to produce
-    uint32_t flags;     // reserved
-    uint32_t aux;       // reserved
+    uint32_t flags;     // STREAM_OPEN: see below
+    uint32_t aux;       // written for STREAM_OPEN: how many symbols the stream's words were good for
 };
+// A stream whose length is not known yet, only a bound (`n`): decoded until it asks for a word it has
+// not got, which a sound one does right behind its last symbol.  Running out is no failure; who
+// learns the length compares it with `aux`.
+constexpr uint32_t STREAM_OPEN = 1;
 static_assert(sizeof(StreamJob) == 32, "StreamJob layout is shared with the host");
 
 // ---- PTX wrappers ------------------------------------------------------------

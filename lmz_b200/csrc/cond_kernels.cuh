@@ -20,6 +20,7 @@ struct CondArgs {
                                    // 32 consecutive elements one lane of k_cond_finish takes, as 8-bit fields
                                    // (buckets 0, 2, 4, 6 in the first word, 1, 3, 5, 7 in the second)
     StreamJob *seg_jobs;           // one slot per rANS-coded segment, sized by k_cond_plan
+    const StreamJob *stream_jobs;  // open segments among them: aux says how many symbols each was good for
     const uint8_t *payload;
     const uint8_t *scratch;
 };
@@ -122,11 +123,16 @@ __global__ void k_cond_plan(CondArgs a)
         cs.seg_ptr[j] = cj.seg_src[j];
         // the host made one job slot per rANS-coded, non-empty segment, in bucket order
         const bool slot = m == 3 && ln != 0;
-        if (slot) a.seg_jobs[cj.seg_job0 + nj].n = 0;
+        if (slot && !cj.open) a.seg_jobs[cj.seg_job0 + nj].n = 0;
         if (want == 0) {
             if (ln) status = ST_BAD_SHAPE;
         } else if (m == 0) {
             if (ln != want) status = ST_BAD_SHAPE;
+        } else if (slot && cj.open) {
+            // already decoded, as far as its words went
+            cs.seg_ptr[j] = cj.seg_scratch + (uint64_t)nj * cj.seg_stride;
+            in_scratch |= 1u << j;
+            if (want > a.stream_jobs[cj.seg_job0 + nj].aux) status = ST_OVERRUN;
         } else if (slot) {
             StreamJob &sj = a.seg_jobs[cj.seg_job0 + nj];
             cs.seg_ptr[j] = cj.seg_scratch + run;
@@ -139,7 +145,7 @@ __global__ void k_cond_plan(CondArgs a)
         }
         nj += slot;
     }
-    if (status != ST_OK)
+    if (status != ST_OK && !cj.open)
         for (uint32_t j = 0; j < nj; j++) a.seg_jobs[cj.seg_job0 + j].n = 0;
     cs.seg_in_scratch = in_scratch;
     cs.status = status;

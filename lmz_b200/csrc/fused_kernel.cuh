@@ -324,18 +324,23 @@ __device__ __forceinline__ void stream_step4(uint32_t &x, uint32_t &e, uint32_t 
     refill<CFN, MODE>(x, e, x2, need, base + tr_entry(MODE) * __popc(hist & below), l1_sa, cf_sa);
 }
 
-// One step of a ragged tile, any lane mix: lanes past the end keep their state.
+// One step of a ragged tile, any lane mix: lanes past the end keep their state.  `base` is where the
+// block's next word lies; returns how many of the block's words had been taken when this lane took
+// one, NONE32 if it took none.
+constexpr uint32_t NONE32 = 0xffffffffu;
 template <int CFN, int MODE>
-__device__ __forceinline__ void stream_step(uint32_t &x, uint32_t &e, uint32_t &base, uint32_t l1_sa, uint32_t cf_sa,
-                                            uint32_t lt_mask, uint32_t grp_mask, bool active)
+__device__ __forceinline__ uint32_t stream_step(uint32_t &x, uint32_t &e, uint32_t &base, uint32_t base0, uint32_t l1_sa, uint32_t cf_sa,
+                                                uint32_t lt_mask, uint32_t grp_mask, bool active)
 {
     const uint32_t x2 = rans_update(x, e);
     const bool need = active && x2 < RANS_LOW;
     const uint32_t vote = __ballot_sync(0xffffffffu, need);
+    const uint32_t at = base + tr_entry(MODE) * __popc(vote & lt_mask);
     uint32_t nx = x, ne = e;
-    refill<CFN, MODE>(nx, ne, x2, need, base + tr_entry(MODE) * __popc(vote & lt_mask), l1_sa, cf_sa);
+    refill<CFN, MODE>(nx, ne, x2, need, at, l1_sa, cf_sa);
     if (active) { x = nx; e = ne; }
     base += tr_entry(MODE) * __popc(vote & grp_mask);
+    return need ? (at - base0) / tr_entry(MODE) : NONE32;
 }
 
 template <int SINK, bool CRC, int CFN, int MODE>
@@ -425,6 +430,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
                                             : a.order[a.order_from_back ? a.njobs - 1 - idx : idx];
     uint64_t soff = 0, doff = 0, moff = 0;
     uint32_t slen = 0, n = 0, piece0 = 0;
+    bool open = false;
     if (have) {
         if (SINK == SINK_DELTA) {
             // groups 2c and 2c + 1 of the warp take the two planes of its chunk c
@@ -438,6 +444,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
         } else if (a.sjobs) {
             StreamJob j = a.sjobs[job];
             soff = j.src_off; doff = j.dst_off; slen = j.src_len; n = j.n;
+            open = SINK == SINK_BYTES && (j.flags & STREAM_OPEN);
         } else {
             soff = a.offs[2 * job]; slen = (uint32_t)a.offs[2 * job + 1];
             n = a.plane; doff = (uint64_t)job * a.plane;
@@ -551,7 +558,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
     const uint32_t msh = (uint32_t)(reinterpret_cast<uintptr_t>(mant) & 3u) * 8u;
     const uint32_t *mq = reinterpret_cast<const uint32_t *>(reinterpret_cast<uintptr_t>(mant) & ~uintptr_t(3));
     uint32_t m[5] = {0, 0, 0, 0, 0};
-    const uint32_t my_tiles = (n + TS - 1) / TS;
+    uint32_t my_tiles = (n + TS - 1) / TS;
     const bool has_base = SINK == SINK_DELTA && moff != NONE64;      // (a plain two-plane chunk has none: m stays zero)
     if ((SINK == SINK_BF16 && my_tiles) || (has_base && n > 8 * j16)) {
 #pragma unroll
@@ -561,14 +568,16 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
     // NEXT tile decodes (32 independent table lookups that hide behind the decode chain),
     // then that tile's words are XORed in.  SINK_F32 keeps one value, `acc`.
     uint32_t acc = 0, ra[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    const bool was_open = open;
+    uint32_t open_got = n;
     uint32_t last_x = x, taken = 0;               // state and words consumed at the stream's end
 
     // ---- tiles of 128 symbols ---------------------------------------------------------
-    const uint32_t warp_tiles = __reduce_max_sync(0xffffffffu, my_tiles);
+    uint32_t warp_tiles = __reduce_max_sync(0xffffffffu, my_tiles);
 #pragma unroll 1
     for (uint32_t t = 0; t < warp_tiles; t++) {
         const uint32_t done = t * TS;
-        const uint32_t rem = n > done ? n - done : 0;
+        uint32_t rem = n > done ? n - done : 0;
         __syncwarp();
         // SINK_F32: the tile's stored bytes are requested before the decode, which hides
         // their latency (lane k: elements 16k .. 16k+15 of each of the three planes)
@@ -596,7 +605,9 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
         };
         // (a group that has no stream, or is done with it, runs along in the others' full tiles;
         // nothing of its is kept)
-        const bool full = __all_sync(0xffffffffu, rem >= TS || rem == 0);
+        // (an open stream that may run out of words in this tile -- fewer than eight rounds of sixteen
+        // are left to load -- is watched step by step)
+        const bool full = __all_sync(0xffffffffu, (rem >= TS && !(SINK == SINK_BYTES && open && wd.left < 8)) || rem == 0);
         if (full) {
 #pragma unroll
             for (uint32_t s8 = 0; s8 < TS / NLANES; s8 += 8) {
@@ -647,12 +658,25 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
                 for (uint32_t s = s4; s < s4 + 4; s++) {
                     const bool active = s * NLANES + k < rem;
                     if (active) put(s);
-                    stream_step<CFN, MODE>(x, e, base, l1_sa, cf_sa, lt_mask, grp_mask, active);
+                    const uint32_t ahead = stream_step<CFN, MODE>(x, e, base, base0, l1_sa, cf_sa, lt_mask, grp_mask, active);
+                    if (SINK == SINK_BYTES) {
+                        // the first lane that took a word the stream has not got ends an open stream:
+                        // `ahead` words had been taken in this block before it took its own
+                        const bool out = open && ahead != NONE32 && wd.taken(slen - LEAD) + ahead >= (slen - LEAD) / 2;
+                        const uint32_t outs = __ballot_sync(0xffffffffu, out) & grp_mask;
+                        if (outs) {
+                            open_got = n = done + s * NLANES + (uint32_t)__ffs((int)(outs >> (8 * g))) - 1;
+                            rem = n - done;
+                            my_tiles = t + 1;
+                            open = false;
+                        }
+                    }
                 }
                 wd.rd += base - base0;
             }
         }
         __syncwarp();
+        if (SINK == SINK_BYTES && !full) warp_tiles = __reduce_max_sync(0xffffffffu, my_tiles);
         if (t + 1 == my_tiles) { last_x = x; taken = wd.taken(slen - LEAD); wd.retire(); }
         if (!rem) continue;
         if (SINK == SINK_DELTA) {
@@ -864,7 +888,9 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
     // ---- verdict -----------------------------------------------------------------------
     const uint32_t all_rest = __ballot_sync(0xffffffffu, last_x == RANS_LOW) & grp_mask;
     if (have && k == 0) {
-        if (st == ST_OK && n) {
+        if (SINK == SINK_BYTES && was_open) {
+            const_cast<StreamJob *>(a.sjobs)[job].aux = st == ST_OK ? open_got : 0u;
+        } else if (st == ST_OK && n) {
             const uint64_t used = LEAD + 2 * (uint64_t)taken;
             if (used > slen) st = ST_OVERRUN;
             else if (used != slen || all_rest != grp_mask) st = ST_SLACK;

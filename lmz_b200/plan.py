@@ -39,7 +39,7 @@ CHUNK_JOB = np.dtype([("dst_off", "<u8"), ("base_off", "<u8"), ("plane_off", "<u
 COND_JOB = np.dtype([("exp_off", "<u8"), ("seg_src", "<u8", 8), ("seg_scratch", "<u8"),
                      ("seg_len", "<u4", 8), ("nelem", "<u4"), ("seg_job0", "<u4"),
                      ("piece0", "<u4"), ("chunk", "<u4"), ("seg_method", "u1", 8),
-                     ("exp_in_scratch", "u1"), ("pad", "u1", 7)])
+                     ("exp_in_scratch", "u1"), ("open", "u1"), ("pad", "u1", 2), ("seg_stride", "<u4")])
 FUSED_JOB = np.dtype([("src_off", "<u8"), ("mant_off", "<u8"), ("dst_off", "<u8"),
                       ("src_len", "<u4"), ("n", "<u4"), ("piece0", "<u4"), ("flags", "<u4")])
 COND_STATE_BYTES = 360
@@ -131,6 +131,15 @@ def _alphabet_sizes(blob: np.ndarray, offs: np.ndarray) -> np.ndarray:
         o = offs[i:i + 8192, None].astype(np.int64) + 4 + cols
         out[i:i + 8192] = ((blob[o] | blob[o + 1]) != 0).sum(1)
     return out
+
+
+# Conditioned chunks with at most this many coded segments have them decoded beside the exponent planes:
+# a segment's length is known only when the exponent plane is, but it is not needed to decode, only
+# room for the longest it could be (every coded segment the size of all of them: twice the room at
+# most).  The exponent plane is the longest stream of such a chunk, so its segments then cost no time of
+# their own (one B200, a 117 MB tensor in 8 MiB chunks: 17 of 50 ms).
+OPEN_SEGMENTS = 2
+STREAM_OPEN = 1                # StreamJob.flags (csrc/common.cuh)
 
 
 def _align16(x):
@@ -415,22 +424,37 @@ def build_plan(ar: fmt.Archive, fuse=True, select=None, payload_range=None,
         cond_of[ci] = np.arange(ci.size)
         ex = ~pl
         cond["exp_off"][cond_of[s_owner[ex]]] = s_dst[ex]
-        seg_sizes = _align16(seg_rans_total)
-        cond["seg_scratch"] = scratch_pos + np.cumsum(seg_sizes) - seg_sizes
-        scratch_pos += int(seg_sizes.sum())
         is_job = (cond["seg_method"] == fmt.METHOD_RANS) & (cond["seg_len"] > 0)
         per = is_job.sum(axis=1)
-        cond["seg_job0"] = np.cumsum(per) - per
-    order = np.argsort(-s_n, kind="stable")         # long streams first
+        is_open = (per > 0) & (per <= OPEN_SEGMENTS)
+        stride = _align16(seg_rans_total)
+        seg_sizes = stride * np.where(is_open, per, 1)
+        cond["seg_scratch"] = scratch_pos + np.cumsum(seg_sizes) - seg_sizes
+        scratch_pos += int(seg_sizes.sum())
+        cond["open"], cond["seg_stride"] = is_open, stride
+        sized = np.where(is_open, 0, per)
+        opened = np.where(is_open, per, 0)
+        cond["seg_job0"] = np.where(is_open, s_n.size + np.cumsum(opened) - opened, np.cumsum(sized) - sized)
+    order = np.argsort(-s_n, kind="stable")         # long streams first, open segments last
     stream_jobs = np.zeros(s_n.size, dtype=STREAM_JOB)
     stream_jobs["src_off"], stream_jobs["dst_off"] = s_src[order], s_dst[order]
     stream_jobs["src_len"], stream_jobs["n"] = s_len[order], s_n[order]
+    stream_owner = s_owner[order]
+    seg_jobs = np.zeros(0, dtype=STREAM_JOB)
     if ci.size:
-        seg_jobs = np.zeros(int(is_job.sum()), dtype=STREAM_JOB)
-        seg_jobs["src_off"] = cond["seg_src"][is_job]        # row-major: chunk, then bucket
-        seg_jobs["src_len"] = cond["seg_len"][is_job]
-    else:
-        seg_jobs = np.zeros(0, dtype=STREAM_JOB)
+        late = is_job & ~is_open[:, None]
+        seg_jobs = np.zeros(int(late.sum()), dtype=STREAM_JOB)
+        seg_jobs["src_off"] = cond["seg_src"][late]          # row-major: chunk, then bucket
+        seg_jobs["src_len"] = cond["seg_len"][late]
+        early = is_job & is_open[:, None]
+        row = np.nonzero(early)[0]
+        jobs = np.zeros(row.size, dtype=STREAM_JOB)
+        jobs["src_off"], jobs["src_len"] = cond["seg_src"][early], cond["seg_len"][early]
+        nth = np.arange(row.size) - (np.cumsum(opened) - opened)[row]
+        jobs["dst_off"] = cond["seg_scratch"][row] + (nth * stride[row]).astype(np.uint64)
+        jobs["n"], jobs["flags"] = seg_rans_total[row], STREAM_OPEN
+        stream_jobs = np.concatenate((stream_jobs, jobs))
+        stream_owner = np.concatenate((stream_owner, ci[row]))
 
     # ---- chunk jobs in launch order ----------------------------------------------
     group = np.where(pass2, 3, 0) + (kind != K_COND) + (fused & ~pass2)
@@ -507,7 +531,7 @@ def build_plan(ar: fmt.Archive, fuse=True, select=None, payload_range=None,
     return Plan(payload=payload, extras=extra, total=out_hi - out_lo, scratch_bytes=scratch_pos + 64,
                 stream_jobs=stream_jobs, seg_jobs=seg_jobs, chunks=chunks,
                 piece_chunk=piece_chunk, piece_split=split, cond_jobs=cond,
-                cond_pieces=cond_pieces, stream_owner=s_owner[order], fused_jobs=fused_jobs,
+                cond_pieces=cond_pieces, stream_owner=stream_owner, fused_jobs=fused_jobs,
                 n_fused_small=int((~wide4 & small).sum()), n_fused_f32=int(wide4.sum()),
                 n_fused_f32_small=int((wide4 & small).sum()),
                 coded_bytes=int(clen.sum()), base_bytes=int(rlen[is_delta].sum()),

@@ -478,3 +478,45 @@ def test_host_and_device_classification_agree(shard):
         dec.run()
         dec.check()
         assert (dec.output.cpu().numpy() == both).all()
+
+
+def _conditioned(coded, n=(1 << 20) + 88):
+    """BF16 bytes whose exponents fall into eight even buckets, the sign/mantissa bytes of the first
+    `coded` of them skewed (they will be coded), of the others uniform (stored)."""
+    rng = np.random.default_rng(coded)
+    bucket = rng.permutation(np.repeat(np.arange(8), n // 8))
+    skewed = np.minimum(rng.geometric(0.2 + 0.1 * (bucket % 3), n) - 1, 255)
+    sm = np.where(bucket < coded, skewed, rng.integers(0, 256, n)).astype(np.uint16)
+    return (((sm & 0x80) << 8) | ((100 + bucket).astype(np.uint16) << 7) | (sm & 0x7F)).astype("<u2").view(np.uint8)
+
+
+@pytest.mark.parametrize("coded", [0, 1, 2, 3, 8])
+def test_conditioned_chunks_by_number_of_coded_segments(gpu, coded):
+    """Up to two coded segments are decoded beside the exponent plane before their lengths are
+    known, more of them after; a segment that is a word short is refused either way, also
+    without checksums."""
+    from lmz_b200 import archive, decode, plan
+    raw = _conditioned(coded)
+    blob = oa.write_archive([("m.safetensors", synth.safetensors_bytes([("w", "BF16", (raw.size // 2,), raw)]))])
+    ar = archive.Archive(blob)
+    p = plan.build_plan(ar)
+    r = ar.records[ar.records["codec"] == 5]
+    if r.size == 0:
+        assert coded == 0                          # nothing to gain: a plain chunk
+    for c in p.cond_jobs:
+        per = int(((c["seg_method"] == 3) & (c["seg_len"] > 0)).sum())
+        assert per == coded and bool(c["open"]) == (0 < per <= plan.OPEN_SEGMENTS)
+    got = decode.decode_archive(blob).cpu().numpy()
+    assert (got[-raw.size:] == raw).all()
+    if not coded:
+        return
+    # the last coded segment of the first conditioned chunk gives its final word to the next bucket's bytes
+    head = int(r["off"][0])
+    bad = bytearray(blob)
+    at = head + 14 + 4 * (coded - 1)
+    short = int.from_bytes(bad[at:at + 4], "little") - 2
+    bad[at:at + 4] = short.to_bytes(4, "little")
+    dec = decode.ArchiveDecoder(bytes(bad), checksum=False)
+    dec.run()
+    with pytest.raises(archive.CorruptArchive):
+        dec.check()
