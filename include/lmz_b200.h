@@ -108,8 +108,8 @@ typedef struct lmz_stream_job {
     uint64_t dst_off; /* first output byte, bytes from d_dst */
     uint32_t src_len; /* stream length */
     uint32_t n;       /* symbols to decode */
-    uint32_t flags;   /* 0; 1: n is only a bound -- the stream is decoded until its words run out, which is
-                       * then no failure */
+    uint32_t flags;   /* 0; among the stream jobs of a plan with conditioned chunks also 1: n is only a bound, the
+                       * stream is decoded until its words run out, which is then no failure */
     uint32_t aux;     /* 0; with flags 1 the kernel writes how many symbols the words were good for */
 } lmz_stream_job;
 

@@ -2,6 +2,8 @@
 // fused into the decode loop:
 //
 //   SINK_BYTES  the decoded plane is written as is (decode_batch, scratch planes)
+//   SINK_OPEN   the same where open streams (STREAM_OPEN) may be among them; an instance of its own, as
+//               the watch for their ends costs the others 8 %
 //   SINK_BF16   a CODEC_BF16 chunk whose exponent plane is rANS and whose
 //               sign/mantissa plane is stored: each 128-symbol tile is merged with
 //               128 stored bytes (lmz/native/lmzcore.c:439-447), written once as
@@ -54,7 +56,7 @@
 
 namespace lmz {
 
-enum : int { SINK_BYTES = 0, SINK_BF16 = 1, SINK_F32 = 2, SINK_DELTA = 3 };
+enum : int { SINK_BYTES = 0, SINK_BF16 = 1, SINK_F32 = 2, SINK_DELTA = 3, SINK_OPEN = 4 };
 // How a kernel instance keeps its translated words, and how many warps it is for (see Words):
 //   TR_FEW  8-byte ring entries, data brought to the L2 early: up to 16 warps
 //   TR_8    8-byte ring entries
@@ -444,7 +446,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
         } else if (a.sjobs) {
             StreamJob j = a.sjobs[job];
             soff = j.src_off; doff = j.dst_off; slen = j.src_len; n = j.n;
-            open = SINK == SINK_BYTES && (j.flags & STREAM_OPEN);
+            open = SINK == SINK_OPEN && (j.flags & STREAM_OPEN);
         } else {
             soff = a.offs[2 * job]; slen = (uint32_t)a.offs[2 * job + 1];
             n = a.plane; doff = (uint64_t)job * a.plane;
@@ -607,7 +609,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
         // nothing of its is kept)
         // (an open stream that may run out of words in this tile -- fewer than eight rounds of sixteen
         // are left to load -- is watched step by step)
-        const bool full = __all_sync(0xffffffffu, (rem >= TS && !(SINK == SINK_BYTES && open && wd.left < 8)) || rem == 0);
+        const bool full = __all_sync(0xffffffffu, (rem >= TS && !(SINK == SINK_OPEN && open && wd.left < 8)) || rem == 0);
         if (full) {
 #pragma unroll
             for (uint32_t s8 = 0; s8 < TS / NLANES; s8 += 8) {
@@ -659,7 +661,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
                     const bool active = s * NLANES + k < rem;
                     if (active) put(s);
                     const uint32_t ahead = stream_step<CFN, MODE>(x, e, base, base0, l1_sa, cf_sa, lt_mask, grp_mask, active);
-                    if (SINK == SINK_BYTES) {
+                    if (SINK == SINK_OPEN) {
                         // the first lane that took a word the stream has not got ends an open stream:
                         // `ahead` words had been taken in this block before it took its own
                         const bool out = open && ahead != NONE32 && wd.taken(slen - LEAD) + ahead >= (slen - LEAD) / 2;
@@ -676,7 +678,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
             }
         }
         __syncwarp();
-        if (SINK == SINK_BYTES && !full) warp_tiles = __reduce_max_sync(0xffffffffu, my_tiles);
+        if (SINK == SINK_OPEN && !full) warp_tiles = __reduce_max_sync(0xffffffffu, my_tiles);
         if (t + 1 == my_tiles) { last_x = x; taken = wd.taken(slen - LEAD); wd.retire(); }
         if (!rem) continue;
         if (SINK == SINK_DELTA) {
@@ -743,7 +745,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
         }
         const uint4 ev = lds_u128(stage_sa + 16 * k);
         const uint32_t ew[4] = {ev.x, ev.y, ev.z, ev.w};
-        if (SINK == SINK_BYTES) {
+        if (SINK == SINK_BYTES || SINK == SINK_OPEN) {
             if (rem >= TS && al == 0) {
                 *reinterpret_cast<uint4 *>(out + done + 16 * k) = ev;
             } else {
@@ -888,7 +890,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
     // ---- verdict -----------------------------------------------------------------------
     const uint32_t all_rest = __ballot_sync(0xffffffffu, last_x == RANS_LOW) & grp_mask;
     if (have && k == 0) {
-        if (SINK == SINK_BYTES && was_open) {
+        if (SINK == SINK_OPEN && was_open) {
             const_cast<StreamJob *>(a.sjobs)[job].aux = st == ST_OK ? open_got : 0u;
         } else if (st == ST_OK && n) {
             const uint64_t used = LEAD + 2 * (uint64_t)taken;

@@ -166,6 +166,7 @@ struct RansArgs {
     const uint8_t *shared_hdr;  // 516-byte table shared by every stream
     uint32_t *status;           // one word per job, may be NULL
     uint32_t *any_bad;          // set non-zero when a job fails hard, may be NULL
+    bool open;                  // open streams may be among the jobs
 };
 
 static StreamArgs as_stream_args(const RansArgs &a)
@@ -257,6 +258,7 @@ static int launch_rans(const RansArgs &a, cudaStream_t cs, bool may_alloc = true
     if (a.shared_hdr) return launch_stream<SINK_BYTES, false, -1>(sa, cs);
     const int forced = g_force_table_mode.load(std::memory_order_relaxed);
     const bool wide = forced < 0 ? a.njobs <= (unsigned)sms * WIDE_PER_SM : forced == T_WIDE1 || forced == T_WIDE13;
+    if (a.open) return wide ? launch_stream<SINK_OPEN, false, 0>(sa, cs) : launch_stream<SINK_OPEN, false, 256>(sa, cs);
     if (wide) return launch_stream<SINK_BYTES, false, 0>(sa, cs);
     if (may_alloc && forced < 0 && a.njobs > (unsigned)sms * COMPACT_PER_SM) {
         rc = launch_compact_sorted(a, cs);

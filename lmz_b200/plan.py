@@ -434,7 +434,10 @@ def build_plan(ar: fmt.Archive, fuse=True, select=None, payload_range=None,
         cond["open"], cond["seg_stride"] = is_open, stride
         sized = np.where(is_open, 0, per)
         opened = np.where(is_open, per, 0)
-        cond["seg_job0"] = np.where(is_open, s_n.size + np.cumsum(opened) - opened, np.cumsum(sized) - sized)
+        # (open segments start a group of four jobs of their own: a warp goes at the pace of its slowest
+        # stream, and theirs are bytes of near eight bits each)
+        pad = -s_n.size % 4 if opened.any() else 0
+        cond["seg_job0"] = np.where(is_open, s_n.size + pad + np.cumsum(opened) - opened, np.cumsum(sized) - sized)
     order = np.argsort(-s_n, kind="stable")         # long streams first, open segments last
     stream_jobs = np.zeros(s_n.size, dtype=STREAM_JOB)
     stream_jobs["src_off"], stream_jobs["dst_off"] = s_src[order], s_dst[order]
@@ -453,8 +456,8 @@ def build_plan(ar: fmt.Archive, fuse=True, select=None, payload_range=None,
         nth = np.arange(row.size) - (np.cumsum(opened) - opened)[row]
         jobs["dst_off"] = cond["seg_scratch"][row] + (nth * stride[row]).astype(np.uint64)
         jobs["n"], jobs["flags"] = seg_rans_total[row], STREAM_OPEN
-        stream_jobs = np.concatenate((stream_jobs, jobs))
-        stream_owner = np.concatenate((stream_owner, ci[row]))
+        stream_jobs = np.concatenate((stream_jobs, np.zeros(pad, dtype=STREAM_JOB), jobs))
+        stream_owner = np.concatenate((stream_owner, np.zeros(pad, dtype=np.int64), ci[row]))
 
     # ---- chunk jobs in launch order ----------------------------------------------
     group = np.where(pass2, 3, 0) + (kind != K_COND) + (fused & ~pass2)
