@@ -571,13 +571,14 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
     // then that tile's words are XORed in.  SINK_F32 keeps one value, `acc`.
     uint32_t acc = 0, ra[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     const bool was_open = open;
-    uint32_t open_got = n;
     uint32_t last_x = x, taken = 0;               // state and words consumed at the stream's end
 
     // ---- tiles of 128 symbols ---------------------------------------------------------
-    uint32_t warp_tiles = __reduce_max_sync(0xffffffffu, my_tiles);
-#pragma unroll 1
-    for (uint32_t t = 0; t < warp_tiles; t++) {
+    // FULL: every group of the warp that has symbols left has a whole tile of them.  (A group that has no
+    // stream, or is done with it, runs along; nothing of its is kept.)
+    uint32_t t = 0;
+    auto tile = [&](auto full_c) {
+        constexpr bool FULL = decltype(full_c)::value;
         const uint32_t done = t * TS;
         uint32_t rem = n > done ? n - done : 0;
         __syncwarp();
@@ -585,7 +586,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
         // their latency (lane k: elements 16k .. 16k+15 of each of the three planes)
         uint32_t pr[SINK == SINK_F32 ? 3 : 1][5];
         if constexpr (SINK == SINK_F32) {
-            const bool mine = rem > 16 * k;
+            const bool mine = FULL ? rem != 0 : rem > 16 * k;
 #pragma unroll
             for (int j = 0; j < 3; j++) {
                 const uint8_t *pp = a.src + moff + (size_t)j * n + done + 16 * k;
@@ -605,12 +606,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
         auto fold = [&](uint32_t i) {
             if (ROWMUL && i < NRA) ra[i] = crc_feed4q(cq, ra[i]);
         };
-        // (a group that has no stream, or is done with it, runs along in the others' full tiles;
-        // nothing of its is kept)
-        // (an open stream that may run out of words in this tile -- fewer than eight rounds of sixteen
-        // are left to load -- is watched step by step)
-        const bool full = __all_sync(0xffffffffu, (rem >= TS && !(SINK == SINK_OPEN && open && wd.left < 8)) || rem == 0);
-        if (full) {
+        if constexpr (FULL) {
 #pragma unroll
             for (uint32_t s8 = 0; s8 < TS / NLANES; s8 += 8) {
                 // eight steps: two blocks, and where warps are few a round of translation between the
@@ -667,7 +663,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
                         const bool out = open && ahead != NONE32 && wd.taken(slen - LEAD) + ahead >= (slen - LEAD) / 2;
                         const uint32_t outs = __ballot_sync(0xffffffffu, out) & grp_mask;
                         if (outs) {
-                            open_got = n = done + s * NLANES + (uint32_t)__ffs((int)(outs >> (8 * g))) - 1;
+                            n = done + s * NLANES + (uint32_t)__ffs((int)(outs >> (8 * g))) - 1;
                             rem = n - done;
                             my_tiles = t + 1;
                             open = false;
@@ -678,9 +674,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
             }
         }
         __syncwarp();
-        if (SINK == SINK_OPEN && !full) warp_tiles = __reduce_max_sync(0xffffffffu, my_tiles);
-        if (t + 1 == my_tiles) { last_x = x; taken = wd.taken(slen - LEAD); wd.retire(); }
-        if (!rem) continue;
+        if (!rem) return;
         if (SINK == SINK_DELTA) {
             // ---- both planes' symbols of this lane's eight elements, merge, XOR the base, write, checksum
             const uint32_t pair_sa = m_.stage + (gi & ~1u) * F_STAGE + 8u * j16;
@@ -696,7 +690,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
                 if (MODE == TR_FEW && t + 4 < my_tiles) prefetch_l2(mq + (size_t)(t + 4) * (2 * TS / 4));
             }
             uint8_t *d = out + (size_t)done * 2 + 16u * j16;
-            const uint32_t ve = rem > 8u * j16 ? min(rem - 8u * j16, 8u) : 0u;   // valid elements of this lane
+            const uint32_t ve = FULL ? 8u : rem > 8u * j16 ? min(rem - 8u * j16, 8u) : 0u;   // valid elements of this lane
             if (ve == 8) {
                 if (al == 0) *reinterpret_cast<uint4 *>(d) = make_uint4(w[0], w[1], w[2], w[3]);
                 else if ((al & 3) == 0) {
@@ -741,25 +735,25 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
                     }
                 }
             }
-            continue;
+            return;
         }
         const uint4 ev = lds_u128(stage_sa + 16 * k);
         const uint32_t ew[4] = {ev.x, ev.y, ev.z, ev.w};
         if (SINK == SINK_BYTES || SINK == SINK_OPEN) {
-            if (rem >= TS && al == 0) {
+            if ((FULL || rem >= TS) && al == 0) {
                 *reinterpret_cast<uint4 *>(out + done + 16 * k) = ev;
             } else {
-                const uint32_t cnt = rem < TS ? rem : TS;
+                const uint32_t cnt = FULL || rem >= TS ? TS : rem;
 #pragma unroll
                 for (uint32_t i = 0; i < 16; i++)
                     if (16 * k + i < cnt) out[done + 16 * k + i] = (uint8_t)(ew[i >> 2] >> (8 * (i & 3)));
             }
-            continue;
+            return;
         }
 
         if constexpr (SINK == SINK_F32) {
             // ---- interleave with the three stored planes, write, checksum ------------
-            const uint32_t ve = rem > 16 * k ? min(rem - 16 * k, 16u) : 0u;   // valid elements of this lane
+            const uint32_t ve = FULL ? 16u : rem > 16 * k ? min(rem - 16 * k, 16u) : 0u;   // valid elements of this lane
             uint32_t pw[3][4];
 #pragma unroll
             for (int j = 0; j < 3; j++) {
@@ -823,7 +817,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
                     acc = 0;
                 }
             }
-            continue;
+            return;
         }
 
         // ---- SINK_BF16: merge with the stored plane, write, checksum ------------------
@@ -837,7 +831,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
             if (MODE == TR_FEW && t + 5 < my_tiles) prefetch_l2(mq + (size_t)(t + 5) * (TILE / 4));
         }
         uint8_t *d = out + (size_t)done * 2 + k * F_UNIT;
-        const uint32_t ve = rem > 16 * k ? min(rem - 16 * k, 16u) : 0u;   // valid elements of this lane
+        const uint32_t ve = FULL ? 16u : rem > 16 * k ? min(rem - 16 * k, 16u) : 0u;   // valid elements of this lane
         if (ve == 16) {
             if (al == 0) {
                 reinterpret_cast<uint4 *>(d)[0] = make_uint4(w[0], w[1], w[2], w[3]);
@@ -885,13 +879,44 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
                 }
             }
         }
+    };
+    if constexpr (SINK == SINK_BYTES) {
+        const uint32_t warp_tiles = __reduce_max_sync(0xffffffffu, my_tiles);
+#pragma unroll 1
+        for (; t < warp_tiles;) {
+            const uint32_t done = t * TS;
+            if (__all_sync(0xffffffffu, n <= done || n - done >= TS)) tile(std::true_type{});
+            else tile(std::false_type{});
+            t++;
+            if (t == my_tiles) { last_x = x; taken = wd.taken(slen - LEAD); wd.retire(); }
+        }
+    } else {
+    // Tiles are decoded in runs of whole ones, with nothing to watch inside a run: as many as the
+    // group with the fewest has, and what an open stream's unloaded rounds of sixteen words are sure to be
+    // enough for (a tile takes eight of them at most).  Where there is none, one tile step by step.
+    for (;;) {
+        const uint32_t done = t * TS;
+        uint32_t whole = n > done ? (n - done) / TS : 0xffffffffu;
+        if (SINK == SINK_OPEN && open && n > done) whole = min(whole, wd.left > 0 ? (uint32_t)wd.left / 8 : 0u);
+        const uint32_t run = __reduce_min_sync(0xffffffffu, whole);
+        if (run == 0xffffffffu) break;                            // nobody has anything left
+        const uint32_t stop = t + max(run, 1u);
+        if (run) {
+#pragma unroll 1
+            for (; t < stop; t++) tile(std::true_type{});
+        } else {
+            tile(std::false_type{});
+            t++;
+        }
+        if (t == my_tiles) { last_x = x; taken = wd.taken(slen - LEAD); wd.retire(); }
+    }
     }
 
     // ---- verdict -----------------------------------------------------------------------
     const uint32_t all_rest = __ballot_sync(0xffffffffu, last_x == RANS_LOW) & grp_mask;
     if (have && k == 0) {
         if (SINK == SINK_OPEN && was_open) {
-            const_cast<StreamJob *>(a.sjobs)[job].aux = st == ST_OK ? open_got : 0u;
+            const_cast<StreamJob *>(a.sjobs)[job].aux = st == ST_OK ? n : 0u;
         } else if (st == ST_OK && n) {
             const uint64_t used = LEAD + 2 * (uint64_t)taken;
             if (used > slen) st = ST_OVERRUN;

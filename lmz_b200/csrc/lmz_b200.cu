@@ -123,9 +123,9 @@ static int launch_stream(const StreamArgs &a, cudaStream_t cs)
     int sms = 0;
     rc = sm_count(&sms);
     if (rc) return rc;
-    if (CFN < 0 && a.tables)          // the job list is laid out 80 to a CTA
+    if constexpr (CFN < 0 && SINK == SINK_BF16)     // the job list is laid out 80 to a CTA
         return launch_stream_as<SINK, CRC, CFN, TR_8>(a, a.njobs / (F_SHARED_SINK_WARPS * 4), F_SHARED_SINK_WARPS, cs);
-    // At most one CTA per SM; its warps take four streams at a time.  As many rounds of fours as the
+    // Else at most one CTA per SM; its warps take four streams at a time.  As many rounds of fours as the
     // fullest CTA would need, the warps of a CTA just enough for them (when the device holds the count,
     // as if every job of the launch were of this class).
     const uint32_t quads = (a.njobs + 3) / 4, room = a.most_ctas ? a.most_ctas : (uint32_t)sms;
