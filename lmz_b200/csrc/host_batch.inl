@@ -14,6 +14,10 @@ namespace {
 constexpr size_t KEPT_DEVICE_BYTES = (size_t)256 << 20;
 constexpr size_t KEPT_HOST_BYTES = (size_t)512 << 20;
 constexpr size_t KEPT_WORKSPACES = 4;
+// A large call runs in slices of its streams, so that streams go in, are decoded and plaintext comes out
+// at the same time: at most MOST_SLICES, of at least SLICE_BYTES in and out.
+constexpr unsigned MOST_SLICES = 8, LANES = 4;
+constexpr size_t SLICE_BYTES = (size_t)4 << 20;
 
 size_t size_class(size_t bytes)
 {
@@ -29,6 +33,26 @@ struct Workspace {
     size_t dev_bytes = 0;
     uint8_t *pin = nullptr;          // offsets in, verdict out
     size_t pin_bytes = 0;
+    cudaStream_t lane[LANES] = {};   // sliced calls: decode and copy out
+    cudaEvent_t here[MOST_SLICES] = {}, done[LANES] = {};
+
+    cudaError_t need_lanes()
+    {
+        cudaError_t e = cudaSuccess;
+        for (unsigned i = 0; i < LANES && e == cudaSuccess; i++) {
+            if (!lane[i]) e = cudaStreamCreateWithFlags(&lane[i], cudaStreamNonBlocking);
+            if (e == cudaSuccess && !done[i]) e = cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming);
+        }
+        for (unsigned i = 0; i < MOST_SLICES && e == cudaSuccess; i++)
+            if (!here[i]) e = cudaEventCreateWithFlags(&here[i], cudaEventDisableTiming);
+        return e;
+    }
+    void idle()
+    {
+        if (stream) cudaStreamSynchronize(stream);
+        for (cudaStream_t l : lane)
+            if (l) cudaStreamSynchronize(l);
+    }
 
     cudaError_t need(size_t device_bytes, size_t pinned_bytes)
     {
@@ -55,6 +79,12 @@ struct Workspace {
         if (dev) cudaFree(dev);
         if (pin) cudaFreeHost(pin);
         if (stream) cudaStreamDestroy(stream);
+        for (cudaStream_t l : lane)
+            if (l) cudaStreamDestroy(l);
+        for (cudaEvent_t e : here)
+            if (e) cudaEventDestroy(e);
+        for (cudaEvent_t e : done)
+            if (e) cudaEventDestroy(e);
         *this = Workspace{};
     }
 };
@@ -90,7 +120,7 @@ struct Borrowed {
     }
     ~Borrowed()
     {
-        if (w.stream) cudaStreamSynchronize(w.stream);
+        w.idle();
         if (sound && w.dev_bytes <= KEPT_DEVICE_BYTES) {
             HostPool &p = host_pool();
             std::lock_guard<std::mutex> lock(p.mu);
@@ -189,10 +219,12 @@ API int lmz_gpu_decode_batch(const void *hdr, const void *streams, size_t nbytes
     // every (offset, length) pair must lie inside the buffer, and a length must fit the
     // 32 bits the kernels carry it in
     const uint64_t *pairs = static_cast<const uint64_t *>(off);
+    bool in_order = true;
     for (unsigned i = 0; i < nstr; i++) {
         const uint64_t at = pairs[2 * i], len = pairs[2 * i + 1];
         if (at > nbytes || len > nbytes - at) return fail_msg(LMZ_GPU_EBADSTREAM, "a stream lies outside the buffer");
         if (len >> 32) return fail_msg(LMZ_GPU_EUNSUPPORTED, "a stream is 4 GiB or longer");
+        in_order = in_order && (i == 0 || pairs[2 * (size_t)i - 2] + pairs[2 * (size_t)i - 1] <= at);
     }
     int device = 0;
     CK("cudaGetDevice", cudaGetDevice(&device));
@@ -215,20 +247,44 @@ API int lmz_gpu_decode_batch(const void *hdr, const void *streams, size_t nbytes
     uint32_t *verdict = reinterpret_cast<uint32_t *>(w.pin + head_bytes);
     *verdict = 0;
     CK("copy offsets in", cudaMemcpyAsync(d, w.pin, head_bytes, cudaMemcpyHostToDevice, w.stream));
-    CK("copy streams in", cudaMemcpyAsync(d + at_src, streams, nbytes, cudaMemcpyHostToDevice, w.stream));
-    RansArgs a{};
-    a.src = d + at_src;
-    a.offs = reinterpret_cast<const uint64_t *>(d);
-    a.plane = plane;
-    a.njobs = nstr;
-    a.dst = d + at_out;
-    a.shared_hdr = hdr ? d + at_hdr : nullptr;
-    a.any_bad = reinterpret_cast<uint32_t *>(d + at_verdict);
-    if (int rc = launch_rans(a, w.stream)) return rc;
-    CK("copy the verdict out", cudaMemcpyAsync(verdict, d + at_verdict, 4, cudaMemcpyDeviceToHost, w.stream));
     // memory of this library's own takes the plaintext at once; a caller's buffer only if all is well
     const bool direct = is_lent(out, out_bytes);
-    if (direct) CK("copy plaintext out", cudaMemcpyAsync(out, d + at_out, out_bytes, cudaMemcpyDeviceToHost, w.stream));
+    RansArgs a{};
+    a.src = d + at_src;
+    a.plane = plane;
+    a.shared_hdr = hdr ? d + at_hdr : nullptr;
+    a.any_bad = reinterpret_cast<uint32_t *>(d + at_verdict);
+    // slices want each its own stretch of the streams, and plaintext that may leave before the verdict
+    size_t slices = direct && in_order ? (nbytes + out_bytes) / SLICE_BYTES : 1;
+    slices = std::max<size_t>(1, std::min<size_t>(slices, std::min<size_t>(MOST_SLICES, nstr)));
+    if (slices > 1) CK("streams for the batch", w.need_lanes());
+    size_t from = 0;
+    for (size_t j = 0; j < slices; j++) {
+        const size_t first = nstr * j / slices, last = nstr * (j + 1) / slices;
+        const size_t upto = last == nstr ? nbytes : (size_t)pairs[2 * last];
+        if (upto > from)
+            CK("copy streams in", cudaMemcpyAsync(d + at_src + from, static_cast<const uint8_t *>(streams) + from, upto - from,
+                                                  cudaMemcpyHostToDevice, w.stream));
+        from = upto;
+        cudaStream_t cs = w.stream;
+        if (slices > 1) {
+            cs = w.lane[j % LANES];
+            CK("slice of the batch", cudaEventRecord(w.here[j], w.stream));
+            CK("slice of the batch", cudaStreamWaitEvent(cs, w.here[j], 0));
+        }
+        a.offs = reinterpret_cast<const uint64_t *>(d) + 2 * first;
+        a.njobs = (uint32_t)(last - first);
+        const size_t at = first * plane, bytes = (size_t)a.njobs * plane;
+        a.dst = d + at_out + at;
+        if (int rc = launch_rans(a, cs)) return rc;
+        if (direct)
+            CK("copy plaintext out", cudaMemcpyAsync(static_cast<uint8_t *>(out) + at, d + at_out + at, bytes, cudaMemcpyDeviceToHost, cs));
+    }
+    for (size_t l = 0; slices > 1 && l < std::min<size_t>(slices, LANES); l++) {
+        CK("end of the batch", cudaEventRecord(w.done[l], w.lane[l]));
+        CK("end of the batch", cudaStreamWaitEvent(w.stream, w.done[l], 0));
+    }
+    CK("copy the verdict out", cudaMemcpyAsync(verdict, d + at_verdict, 4, cudaMemcpyDeviceToHost, w.stream));
     CK("decode", cudaStreamSynchronize(w.stream));
     b.sound = true;
     if (*verdict) {
