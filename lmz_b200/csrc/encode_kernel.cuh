@@ -26,7 +26,7 @@
 // the state needs them, and the division by the symbol's frequency is exact in one multiply-add
 // and a shift (a multiplier and an addend per frequency: N. Robison's choice between rounding the
 // reciprocal up and rounding it down, of which one always works), with no correction after it.
-// A warp is a CTA: 19.5 KiB of shared memory, eleven per SM, dealt out one by one, so that a batch
+// A warp is a CTA: 19 KiB of shared memory, eleven per SM, dealt out one by one, so that a batch
 // spreads evenly.  4096 planes of 32 KiB of BF16 exponents on one B200: 943 -> 518 us
 // (142 -> 259 GB/s of symbols).
 #pragma once
@@ -43,7 +43,7 @@ struct EncodeArgs {
     uint32_t *lengths;      // per stream: bytes written at the end of its slot, 0 = failed
 };
 
-constexpr uint32_t E_RING = 512, E_TILE = 256;
+constexpr uint32_t E_RING = 512, E_TILE = 128;
 constexpr uint32_t E_TABLE = 4096;                    // 256 entries of 16 bytes; until then the group's share of the counters
 constexpr uint32_t E_GROUP_BYTES = E_TABLE + E_RING + E_TILE;
 constexpr uint32_t E_COUNT_MAX = 8u * 64000u;         // symbols counted before the lanes' 16-bit counters are summed
@@ -239,9 +239,7 @@ __global__ void __launch_bounds__(32) k_encode(EncodeArgs a)
     const uint32_t tiles = (T + 15) / 16;
     const uint32_t warp_tiles = __reduce_max_sync(0xffffffffu, tiles);
     uint32_t x = RANS_LOW, emitted = 0, flushed = 0;    // bytes, counted back from the slot's end
-    // a tile's 128 symbols (lane k: bytes 16 k .. 16 k + 15); two tiles are requested at a time, two ahead (a
-    // warp waits for its loads about a quarter of the time however early they are asked for, as whatever it
-    // waits for next waits for them too: fewer requests are fewer waits)
+    // a tile's 128 symbols (lane k: bytes 16 k .. 16 k + 15), requested a tile ahead
     const bool aligned = (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
     auto fetch = [&](uint32_t tt) {
         uint4 v = make_uint4(0, 0, 0, 0);
@@ -267,28 +265,17 @@ __global__ void __launch_bounds__(32) k_encode(EncodeArgs a)
         }
         return v;
     };
-    uint4 next0 = make_uint4(0, 0, 0, 0), next1 = next0;
-    if (warp_tiles) {
-        next0 = fetch((warp_tiles - 1) & ~1u);
-        next1 = fetch((warp_tiles - 1) | 1u);
-    }
+    uint4 next = warp_tiles ? fetch(warp_tiles - 1) : make_uint4(0, 0, 0, 0);
 #pragma unroll 1
     for (uint32_t tt = warp_tiles; tt-- > 0;) {
         const bool mine_tile = tt < tiles;
-        if ((tt & 1u) || tt + 1 == warp_tiles) {
-            __syncwarp();
-            sts_u128_if(1, tile_sa + 16 * k, next0.x, next0.y, next0.z, next0.w);
-            sts_u128_if(1, tile_sa + 128 + 16 * k, next1.x, next1.y, next1.z, next1.w);
-            if (tt >= 2) {
-                next0 = fetch((tt & ~1u) - 2);
-                next1 = fetch((tt & ~1u) - 1);
-            }
-            __syncwarp();
-        }
-        const uint32_t row = tile_sa + (tt & 1u) * 128 + k;
+        __syncwarp();
+        sts_u128_if(1, tile_sa + 16 * k, next.x, next.y, next.z, next.w);
+        if (tt) next = fetch(tt - 1);
+        __syncwarp();
         uint32_t at[16];
 #pragma unroll
-        for (int s = 15; s >= 0; s--) at[s] = tab_sa + 16 * lds_u8(row + s * 8);
+        for (int s = 15; s >= 0; s--) at[s] = tab_sa + 16 * lds_u8(tile_sa + s * 8 + k);
         uint4 e0 = lds_u128(at[15]), e1 = lds_u128(at[14]);
         const bool full = __all_sync(0xffffffffu, mine_tile && tt * 128 + 128 <= n);
         auto step = [&](int s, bool active) {
