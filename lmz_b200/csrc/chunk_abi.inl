@@ -167,6 +167,12 @@ static int launch_two_plane(const lmz_decode_plan *p, uint32_t first, uint32_t c
     // work space: `count` indices and two counters, at 2 * first + ... so the two passes never share it
     uint32_t *order = (uint32_t *)p->d_delta_order + (first ? first + 2 : 0);
     uint32_t *counts = order + count;
+    const bool crc = p->d_piece_crc != nullptr;
+    int sms = 0;
+    if (int rc = sm_count(&sms)) return rc;
+    const uint32_t per = crc ? wide_per_sm<SINK_DELTA, true>() : wide_per_sm<SINK_DELTA, false>();
+    if (da.njobs <= per * (most_ctas ? most_ctas : (uint32_t)sms))      // wide tables: nothing to sort by
+        return crc ? launch_stream<SINK_DELTA, true, 256>(da, cs) : launch_stream<SINK_DELTA, false, 256>(da, cs);
     CK("memset two-plane counts", cudaMemsetAsync(counts, 0, 8, cs));
     StreamArgs ca = da;
     ca.njobs = count;
@@ -174,7 +180,6 @@ static int launch_two_plane(const lmz_decode_plan *p, uint32_t first, uint32_t c
     cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) return fail_cuda("launch k_classify", le);
     da.order = order;
-    const bool crc = p->d_piece_crc != nullptr;
     int rc = LMZ_GPU_OK;
     for (int big = 0; big < 2 && !rc; big++) {
         da.count = counts + big;
@@ -212,12 +217,14 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
     if (p->n_delta_plain > p->n_delta) return fail_msg(LMZ_GPU_EUNSUPPORTED, "n_delta_plain exceeds n_delta");
     // Plain chunks with both planes coded: the two-plane kernel without a base.  Few chunks are of this
     // shape (29 of an 8B model's 245 069) but one takes as long as any other, so they go first and beside
-    // the fused kernel, packed into a few CTAs (eight warps: 16 chunks) with as many SMs left to them.
+    // the fused kernel, packed into a few CTAs (wide tables: four chunks; eight warps of compact ones: 16)
+    // with as many SMs left to them.
     // Behind it they had the chip to themselves: four 8B decoder layers with one such chunk took
     // 2.5 ms where the fused kernel takes 1.9.
     uint32_t pairs_ctas = 0;
     if (p->n_delta_plain && (ph & 1u) && (p->n_fused || p->n_fused_t) && (ph & 16u)) {
-        pairs_ctas = (p->n_delta_plain + 15) / 16;
+        pairs_ctas = (p->n_delta_plain + 3) / 4;
+        if (pairs_ctas > (uint32_t)sms / 8) pairs_ctas = (p->n_delta_plain + 15) / 16;
         if (pairs_ctas > (uint32_t)sms / 4) pairs_ctas = 0;          // a large part of the work: no corner of its own
     }
     if ((p->n_fused || p->n_fused_t) && (ph & 16u)) {
@@ -263,7 +270,13 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
                 sa.njobs = group_n[grp];
                 sa.order = nullptr;
                 sa.count = nullptr;
-                if (sa.njobs) {
+                const bool checked = p->d_piece_crc != nullptr;
+                const uint32_t per = checked ? wide_per_sm<SINK_BF16, true>() : wide_per_sm<SINK_BF16, false>();
+                if (grp == 0 && sa.njobs && sa.njobs <= per * (sa.most_ctas ? sa.most_ctas : (uint32_t)sms)) {
+                    // few enough for wide tables: nothing to sort by
+                    rc = checked ? launch_stream<SINK_BF16, true, 256>(sa, fs) : launch_stream<SINK_BF16, false, 256>(sa, fs);
+                    if (rc) return rc;
+                } else if (sa.njobs) {
                     k_classify<<<(sa.njobs + 7) / 8, 256, 0, fs>>>(sa, F_SMALL_LIVE, order, counts);
                     cudaError_t le = cudaGetLastError();
                     if (le != cudaSuccess) return fail_cuda("launch k_classify", le);

@@ -206,13 +206,15 @@ class ArchiveDecoder:
         # totals and the segment decode of conditioned chunks; up to four finish launches; the
         # verdict kernel
         nbf = p.n_fused - p.n_fused_f32
+        # (few enough streams for wide tables: one launch, nothing counted or sorted)
+        few = (8 if checksum else 12) * torch.cuda.get_device_properties(d).multi_processor_count
         if p.device_classify:                # per group: the count kernel and both instances
-            fused_launches = 3 * ((1 if nbf else 0) + (1 if p.n_fused_f32 else 0))
+            fused_launches = (0 if not nbf else 1 if nbf <= few else 3) + (3 if p.n_fused_f32 else 0)
         else:
             fused_launches = (1 if p.n_fused_small else 0) + (1 if nbf > p.n_fused_small else 0) + \
                 (1 if p.n_fused_f32_small else 0) + (1 if p.n_fused_f32 > p.n_fused_f32_small else 0)
-        fused_launches += (1 if p.n_fused_t else 0) + (3 if p.n_delta_plain else 0) + \
-            (3 if p.delta_jobs.size > p.n_delta_plain else 0)
+        fused_launches += (1 if p.n_fused_t else 0) + sum(0 if not n else 1 if 2 * n <= few else 3 for n in (
+            p.n_delta_plain, p.delta_jobs.size - p.n_delta_plain))
         self.launches_per_run = (1 if p.stream_jobs.size else 0) + \
             ((4 + (1 if p.seg_jobs.size else 0)) if ncond else 0) + fused_launches + \
             int(sum(p.piece_split[i + 1] > p.piece_split[i] for i in (0, 1, 3, 4))) + 1
