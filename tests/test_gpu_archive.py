@@ -520,3 +520,42 @@ def test_conditioned_chunks_by_number_of_coded_segments(gpu, coded):
     dec.run()
     with pytest.raises(archive.CorruptArchive):
         dec.check()
+
+
+@pytest.mark.parametrize("nchunks", [1184, 1185, 9473])
+@pytest.mark.parametrize("checksum", [True, False])
+def test_bf16_chunks_by_how_many_there_are(gpu, tmp_path, nchunks, checksum):
+    """Few chunks take wide tables, more of them compact ones in the instance for few warps, many
+    the one for many (the counts are those of 148 SMs); small and large alphabets in each."""
+    import json
+    import struct
+    import torch
+    from lmz_b200 import decode, save
+    n = nchunks * 32768 - 77
+    gen = torch.Generator(device="cuda").manual_seed(nchunks)
+    w = torch.randn(n, generator=gen, device="cuda") * 0.02
+    w[n // 2:n // 2 + (n >> 4)] *= torch.exp2(-torch.empty(n >> 4, device="cuda").geometric_(0.03, generator=gen).clamp_(max=90))
+    data = w.to(torch.bfloat16).view(torch.uint8)
+    del w
+    head = json.dumps({"w": {"dtype": "BF16", "shape": [n], "data_offsets": [0, 2 * n]}}).encode()
+    head += b" " * (-(8 + len(head)) % 8)
+    head = torch.frombuffer(bytearray(struct.pack("<Q", len(head)) + head), dtype=torch.uint8).cuda()
+    member = torch.cat((head, data))
+    path = str(tmp_path / "m.lmz")
+    save.save_archive(path, [("m.safetensors", member)])
+    assert torch.equal(decode.load_archive(path, checksum=checksum), member)
+
+
+@pytest.mark.parametrize("checksum", [True, False])
+def test_many_two_plane_deltas(checksum):
+    """More delta chunks than wide tables take: the instances with compact tables for both planes."""
+    from lmz_b200 import archive, decode
+    n = 910 * 32768 + 5
+    first = synth.normal_bf16((n,), 1)
+    files = [synth.safetensors_bytes([("w", "BF16", (n,), d)]) for d in (first, synth.perturbed_bf16(first, 2))]
+    blob = oa.write_archive([(f"{i}.safetensors", f) for i, f in enumerate(files)], mapped=True, workers=8)
+    dec = decode.ArchiveDecoder(archive.Archive(blob), checksum=checksum)
+    assert dec.plan.delta_jobs.size - dec.plan.n_delta_plain > 888
+    dec.run()
+    dec.check()
+    assert (dec.output.cpu().numpy() == np.concatenate(files)).all()
