@@ -41,16 +41,19 @@ def cover(ar: fmt.Archive, ranges) -> np.ndarray:
     order = np.argsort(r["dst"], kind="stable")
     dst_sorted = r["dst"][order].astype(np.int64)
 
-    def overlapping(pairs):
-        got = [order[max(int(np.searchsorted(dst_sorted, lo, "right")) - 1, 0):
-                     int(np.searchsorted(dst_sorted, hi, "left"))] for lo, hi in pairs if hi > lo]
-        return np.unique(np.concatenate(got)) if got else np.zeros(0, dtype=np.int64)
+    need = np.zeros(r.size, dtype=bool)
 
-    mine = overlapping(ranges)
+    def overlapping(pairs):
+        for lo, hi in pairs:
+            if hi > lo:
+                need[order[max(int(np.searchsorted(dst_sorted, lo, "right")) - 1, 0):
+                           int(np.searchsorted(dst_sorted, hi, "left"))]] = True
+
+    overlapping(ranges)
     src = sources(ar)
-    need = mine[src[mine] >= 0]
-    extra = overlapping([(int(src[i]), int(src[i]) + int(r["rlen"][i])) for i in need])
-    return np.union1d(mine, extra).astype(np.int64)
+    sourced = np.nonzero(need & (src >= 0))[0]
+    overlapping([(int(src[i]), int(src[i]) + int(r["rlen"][i])) for i in sourced])
+    return np.nonzero(need)[0].astype(np.int64)
 
 
 def shard(ar: fmt.Archive, rank: int, world: int):
