@@ -217,14 +217,14 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
     if (p->n_delta_plain > p->n_delta) return fail_msg(LMZ_GPU_EUNSUPPORTED, "n_delta_plain exceeds n_delta");
     // Plain chunks with both planes coded: the two-plane kernel without a base.  Few chunks are of this
     // shape (29 of an 8B model's 245 069) but one takes as long as any other, so they go first and beside
-    // the fused kernel, packed into a few CTAs (wide tables: four chunks; eight warps of compact ones: 16)
-    // with as many SMs left to them.
+    // the fused kernel, packed into a few CTAs (eight warps: 16 chunks) with as many SMs left to them.
+    // (Four chunks to a CTA would let more of them take wide tables, but an 8B model's 29 would keep eight SMs
+    // from its fused kernel: 15.8 against 15.2 ms.)
     // Behind it they had the chip to themselves: four 8B decoder layers with one such chunk took
     // 2.5 ms where the fused kernel takes 1.9.
     uint32_t pairs_ctas = 0;
     if (p->n_delta_plain && (ph & 1u) && (p->n_fused || p->n_fused_t) && (ph & 16u)) {
-        pairs_ctas = (p->n_delta_plain + 3) / 4;
-        if (pairs_ctas > (uint32_t)sms / 8) pairs_ctas = (p->n_delta_plain + 15) / 16;
+        pairs_ctas = (p->n_delta_plain + 15) / 16;
         if (pairs_ctas > (uint32_t)sms / 4) pairs_ctas = 0;          // a large part of the work: no corner of its own
     }
     if ((p->n_fused || p->n_fused_t) && (ph & 16u)) {
