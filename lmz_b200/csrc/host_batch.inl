@@ -19,6 +19,12 @@ constexpr size_t KEPT_WORKSPACES = 4;
 constexpr unsigned MOST_SLICES = 8, LANES = 4;
 constexpr size_t SLICE_BYTES = (size_t)4 << 20;
 
+// Result memory has this much in front of what the caller sees, where a small call's verdict lands.
+constexpr size_t LENT_HEAD = 64, VERDICT = 16;
+// Calls up to here go in by one copy from page-locked memory and out by one, verdict and plaintext
+// together.
+constexpr size_t SMALL_BYTES = (size_t)256 << 10;
+
 size_t size_class(size_t bytes)
 {
     size_t c = 4096;
@@ -140,14 +146,14 @@ bool is_lent(const void *p, size_t bytes)
     HostPool &pool = host_pool();
     std::lock_guard<std::mutex> lock(pool.mu);
     auto it = pool.lent.find(const_cast<void *>(p));
-    return it != pool.lent.end() && it->second >= bytes;
+    return it != pool.lent.end() && it->second - LENT_HEAD >= bytes;
 }
 
 }  // namespace
 
 API void *lmz_gpu_host_alloc(size_t bytes)
 {
-    const size_t c = size_class(bytes);
+    const size_t c = size_class(bytes + LENT_HEAD);
     HostPool &p = host_pool();
     {
         std::lock_guard<std::mutex> lock(p.mu);
@@ -156,6 +162,7 @@ API void *lmz_gpu_host_alloc(size_t bytes)
             void *q = it->second;
             p.spare.erase(it);
             p.spare_bytes -= c;
+            q = static_cast<uint8_t *>(q) + LENT_HEAD;
             p.lent[q] = c;
             return q;
         }
@@ -165,6 +172,7 @@ API void *lmz_gpu_host_alloc(size_t bytes)
         cudaGetLastError();
         return nullptr;
     }
+    q = static_cast<uint8_t *>(q) + LENT_HEAD;
     std::lock_guard<std::mutex> lock(p.mu);
     p.lent[q] = c;
     return q;
@@ -179,6 +187,7 @@ API void lmz_gpu_host_free(void *q)
         if (it == p.lent.end()) return;
         const size_t c = it->second;
         p.lent.erase(it);
+        q = static_cast<uint8_t *>(q) - LENT_HEAD;
         if (p.spare_bytes + c <= KEPT_HOST_BYTES) {
             p.spare.emplace(c, q);
             p.spare_bytes += c;
@@ -233,10 +242,16 @@ API int lmz_gpu_decode_batch(const void *hdr, const void *streams, size_t nbytes
     auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
     const size_t out_bytes = (size_t)nstr * plane, table_bytes = (size_t)nstr * 16;
     const size_t at_hdr = table_bytes, at_verdict = (at_hdr + (hdr ? HDR_BYTES : 0) + 15) & ~(size_t)15;
-    const size_t head_bytes = at_verdict + 16, at_src = up(head_bytes), at_out = up(at_src + nbytes + PAD_BYTES);
+    const size_t head_bytes = at_verdict + 16, at_src = up(head_bytes), at_out = up(at_src + nbytes + PAD_BYTES + VERDICT);
+    // memory of this library's own takes the plaintext at once; a caller's buffer only if all is well
+    const bool direct = is_lent(out, out_bytes);
+    // slices want each its own stretch of the streams, and plaintext that may leave before the verdict
+    size_t slices = direct && in_order ? (nbytes + out_bytes) / SLICE_BYTES : 1;
+    slices = std::max<size_t>(1, std::min<size_t>(slices, std::min<size_t>(MOST_SLICES, nstr)));
+    const bool small = direct && slices == 1 && at_out <= SMALL_BYTES;
     Borrowed b(device);
     Workspace &w = b.w;
-    if (cudaError_t e = w.need(at_out + out_bytes, head_bytes + 16)) {
+    if (cudaError_t e = w.need(at_out + out_bytes, (small ? at_out : head_bytes) + 16)) {
         cudaGetLastError();
         return fail_cuda("memory for the batch", e);
     }
@@ -244,25 +259,28 @@ API int lmz_gpu_decode_batch(const void *hdr, const void *streams, size_t nbytes
     memcpy(w.pin, off, table_bytes);
     if (hdr) memcpy(w.pin + at_hdr, hdr, HDR_BYTES);
     memset(w.pin + at_verdict, 0, 16);
-    uint32_t *verdict = reinterpret_cast<uint32_t *>(w.pin + head_bytes);
-    *verdict = 0;
-    CK("copy offsets in", cudaMemcpyAsync(d, w.pin, head_bytes, cudaMemcpyHostToDevice, w.stream));
-    // memory of this library's own takes the plaintext at once; a caller's buffer only if all is well
-    const bool direct = is_lent(out, out_bytes);
+    // the device's verdict: in the head, or (small) right in front of the plaintext
+    uint8_t *const d_verdict = small ? d + at_out - VERDICT : d + at_verdict;
+    uint32_t *verdict = reinterpret_cast<uint32_t *>(small ? static_cast<uint8_t *>(out) - VERDICT : w.pin + head_bytes);
+    if (small) {
+        memcpy(w.pin + at_src, streams, nbytes);
+        memset(w.pin + at_src + nbytes, 0, at_out - at_src - nbytes);
+        CK("copy the batch in", cudaMemcpyAsync(d, w.pin, at_out, cudaMemcpyHostToDevice, w.stream));
+    } else {
+        *verdict = 0;
+        CK("copy offsets in", cudaMemcpyAsync(d, w.pin, head_bytes, cudaMemcpyHostToDevice, w.stream));
+    }
     RansArgs a{};
     a.src = d + at_src;
     a.plane = plane;
     a.shared_hdr = hdr ? d + at_hdr : nullptr;
-    a.any_bad = reinterpret_cast<uint32_t *>(d + at_verdict);
-    // slices want each its own stretch of the streams, and plaintext that may leave before the verdict
-    size_t slices = direct && in_order ? (nbytes + out_bytes) / SLICE_BYTES : 1;
-    slices = std::max<size_t>(1, std::min<size_t>(slices, std::min<size_t>(MOST_SLICES, nstr)));
+    a.any_bad = reinterpret_cast<uint32_t *>(d_verdict);
     if (slices > 1) CK("streams for the batch", w.need_lanes());
     size_t from = 0;
     for (size_t j = 0; j < slices; j++) {
         const size_t first = nstr * j / slices, last = nstr * (j + 1) / slices;
         const size_t upto = last == nstr ? nbytes : (size_t)pairs[2 * last];
-        if (upto > from)
+        if (upto > from && !small)
             CK("copy streams in", cudaMemcpyAsync(d + at_src + from, static_cast<const uint8_t *>(streams) + from, upto - from,
                                                   cudaMemcpyHostToDevice, w.stream));
         from = upto;
@@ -277,14 +295,17 @@ API int lmz_gpu_decode_batch(const void *hdr, const void *streams, size_t nbytes
         const size_t at = first * plane, bytes = (size_t)a.njobs * plane;
         a.dst = d + at_out + at;
         if (int rc = launch_rans(a, cs)) return rc;
-        if (direct)
+        if (small) {
+            CK("copy verdict and plaintext out", cudaMemcpyAsync(verdict, d_verdict, VERDICT + out_bytes, cudaMemcpyDeviceToHost, cs));
+        } else if (direct) {
             CK("copy plaintext out", cudaMemcpyAsync(static_cast<uint8_t *>(out) + at, d + at_out + at, bytes, cudaMemcpyDeviceToHost, cs));
+        }
     }
     for (size_t l = 0; slices > 1 && l < std::min<size_t>(slices, LANES); l++) {
         CK("end of the batch", cudaEventRecord(w.done[l], w.lane[l]));
         CK("end of the batch", cudaStreamWaitEvent(w.stream, w.done[l], 0));
     }
-    CK("copy the verdict out", cudaMemcpyAsync(verdict, d + at_verdict, 4, cudaMemcpyDeviceToHost, w.stream));
+    if (!small) CK("copy the verdict out", cudaMemcpyAsync(verdict, d_verdict, 4, cudaMemcpyDeviceToHost, w.stream));
     CK("decode", cudaStreamSynchronize(w.stream));
     b.sound = true;
     if (*verdict) {
