@@ -259,7 +259,7 @@ int lmz_host_plan(const void *records, const int64_t *select, size_t n, const ui
  *             (map != NULL) or of a file
  * Both return the range's number, negative on failure.  wait() returns when a range has been
  * issued whole (upload: cuda_stream then waits for its arrival) or written (download); free()
- * waits for all.  An error ends every later block of the transfer. */
+ * returns when all have arrived.  An error ends every later block of the transfer. */
 void *lmz_gpu_staging_new(size_t block, unsigned depth, unsigned threads);
 void lmz_gpu_staging_free(void *staging);
 void *lmz_gpu_transfer_new(void *staging, void *cuda_stream);

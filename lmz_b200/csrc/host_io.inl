@@ -346,6 +346,10 @@ API int lmz_gpu_transfer_free(void *transfer)
         if (t->error[0]) rc = fail_msg(LMZ_GPU_ECUDA, t->error);
     }
     { std::lock_guard<std::mutex> lock(t->issue); }          // the last issuer has let go
+    // Issued is not arrived: a caller that has not waited for every range (an error on its way) gives
+    // the memory back right after this.
+    const cudaError_t e = cudaStreamSynchronize(t->stream);
+    if (e != cudaSuccess && rc == LMZ_GPU_OK) rc = fail_cuda("the copies of a transfer", e);
     for (Transfer::Range &r : t->ranges)
         if (r.event) cudaEventDestroy(r.event);
     cudaStreamDestroy(t->stream);

@@ -421,6 +421,7 @@ class _Uploader:
         self.staging = staging if staging is not None else Staging.shared()
         self.stream = stream if stream is not None else torch.cuda.current_stream(device)
         self.device = device
+        self.sent_to = []                    # held until the copies have arrived
         with torch.cuda.device(device):
             self.handle = self.lib.lmz_gpu_transfer_new(self.staging.handle, self.stream.cuda_stream)
         if not self.handle:
@@ -428,6 +429,7 @@ class _Uploader:
 
     def send(self, lo: int, hi: int, dst) -> int:
         import torch
+        self.sent_to.append(dst)
         with torch.cuda.device(self.device):
             r = self.lib.lmz_gpu_transfer_upload(self.handle, self.fd, self.blob.ctypes.data, int(lo), int(hi - lo),
                                                  dst.data_ptr())
@@ -440,10 +442,12 @@ class _Uploader:
             raise RuntimeError(f"an upload failed: {gpu.last_error()}")
 
     def close(self) -> None:
-        """Wait for every range and let go; the memory sent to must live until then."""
+        """Return when every range has arrived; the memory sent to must live until then."""
         if self.handle:
             handle, self.handle = self.handle, None
-            if self.lib.lmz_gpu_transfer_free(handle) != gpu.OK:
+            rc = self.lib.lmz_gpu_transfer_free(handle)
+            self.sent_to.clear()
+            if rc != gpu.OK:
                 raise RuntimeError(f"an upload failed: {gpu.last_error()}")
 
     def __del__(self):
@@ -615,9 +619,9 @@ def decode_tensors(ar, names, device=None, checksum: bool = True):
             dec = ArchiveDecoder(ar, device=dev, checksum=checksum, plan=p, payload=payload, settle=False)
             for si in sent:
                 up.wait(si)
+            dec.run()
         finally:
             up.close()
-    dec.run()
     dec.check()
     out = {}
     for k in keys:

@@ -559,3 +559,34 @@ def test_many_two_plane_deltas(checksum):
     dec.run()
     dec.check()
     assert (dec.output.cpu().numpy() == np.concatenate(files)).all()
+
+
+@pytest.mark.parametrize("way", ["load_archive", "decode_tensors"])
+def test_a_damaged_index_leaves_no_copy_behind(gpu, shard, tmp_path, way):
+    """The upload has started when the index or a chunk turns out to be damaged: its copies have
+    ended when the error arrives, so memory taken right afterwards stays what its owner makes it."""
+    import torch
+    from lmz_b200 import archive, decode
+    from test_host_logic import _rewrite_table
+    blob = oa.write_archive([("m.safetensors", shard)], mapped=True)
+
+    def spoil(r):
+        r["codec"][-1] = 7
+
+    path = tmp_path / "bad.lmz"
+    path.write_bytes(_rewrite_table(blob, spoil))
+    name = [k for k in archive.Archive(blob).tensor_index()][-1]
+    big = torch.empty(1 << 30, dtype=torch.uint8, device="cuda")
+    for _ in range(3):
+        for _ in range(20):
+            big.add_(1)                          # keeps the stream, and so the uploads behind it, busy
+        with pytest.raises(archive.FormatError):
+            if way == "load_archive":
+                decode.load_archive(str(path))
+            else:
+                decode.decode_tensors(str(path), [name])
+        mine = [torch.full((n,), 0xA5, dtype=torch.uint8, device="cuda") for n in (len(blob) + (1 << 20), len(blob), 4096)]
+        torch.cuda.synchronize()
+        assert all(bool((t == 0xA5).all()) for t in mine)
+    path.write_bytes(blob)
+    assert (decode.load_archive(str(path)).cpu().numpy() == shard).all()
