@@ -512,11 +512,8 @@ def load_archive(path, device=None, checksum: bool = True, nslices=None, stats=N
         try:
             ar = fmt.Archive(blob)
             ar.check_coverage()
-            r = ar.records
-            general = (r["codec"] == fmt.CODEC_ZSTD) & ((r["flags"] & 3) != fmt.METHOD_STORED) & \
-                      ((r["flags"] & 3) != fmt.METHOD_RANS)
-            inflated = int(r["rlen"][general].sum()) if general.any() else 0
-            if inflated > room:                          # (or a reference's delta of one: rare, and checked below)
+            inflated = planner.inflated_bytes(ar.records)
+            if inflated > room:
                 up.close()
                 payload = torch.empty(table_off + inflated + pad, dtype=torch.uint8, device=dev)
                 up, sent = start()
@@ -604,8 +601,7 @@ def decode_tensors(ar, names, device=None, checksum: bool = True):
     with torch.cuda.device(dev):
         # only what the chunks hold crosses, to its place in a buffer that spans all of it, while the
         # chunks are planned (gaps below 256 KiB are not worth a range of their own)
-        general = (r["codec"] == fmt.CODEC_ZSTD) & ((r["flags"] & 3) != fmt.METHOD_STORED) & ((r["flags"] & 3) != fmt.METHOD_RANS)
-        room = pay_hi - pay_lo + int(r["rlen"][general].sum()) + gpu.pad_bytes()
+        room = pay_hi - pay_lo + planner.inflated_bytes(r) + gpu.pad_bytes()
         payload = torch.empty(room, dtype=torch.uint8, device=dev)
         up = _Uploader(ar.blob, dev)
         order = np.argsort(r["off"], kind="stable")

@@ -268,7 +268,7 @@ def build_plan(ar: fmt.Archive, fuse=True, select=None, payload_range=None,
             # General-purpose streams are tiny container headers; they are inflated
             # here and travel to the device as stored bytes.
             plane_off[j, 0] = extra_pos
-            extras.append(_general(ar, r[j]))
+            extras.append(_general(ar, lo + int(eoff[j]), int(eclen[j]), r[j]))
             extra_pos += extras[-1].size
         known[i] = True
 
@@ -542,9 +542,20 @@ def build_plan(ar: fmt.Archive, fuse=True, select=None, payload_range=None,
                 delta_jobs=delta_jobs, n_delta_plain=n_delta_plain, extras_at=extras_at)
 
 
-def _general(ar: fmt.Archive, rec) -> np.ndarray:
-    """The bytes of a chunk that is coded with a general-purpose compressor (a container's header)."""
-    raw = ar.blob[int(rec["off"]):int(rec["off"]) + int(rec["clen"])].tobytes()
+def inflated_bytes(records) -> int:
+    """Bytes the host may have to inflate for these records: one-stream chunks coded with a
+    general-purpose compressor, and deltas whose difference is (the planner refuses any other delta
+    with such a first plane)."""
+    m = records["flags"] & 3
+    general = np.isin(records["codec"], (fmt.CODEC_ZSTD, fmt.CODEC_DELTA)) & \
+        ((m == fmt.METHOD_ZSTD) | (m == fmt.METHOD_DEFLATE))
+    return int(records["rlen"][general].sum(dtype=np.int64))
+
+
+def _general(ar: fmt.Archive, off: int, clen: int, rec) -> np.ndarray:
+    """The bytes of a record whose `clen` bytes at `off` of the archive (a delta's: behind its base) are
+    coded with a general-purpose compressor: a container's header, mostly."""
+    raw = ar.blob[off:off + clen].tobytes()
     data = fmt.inflate_tail(raw) if (int(rec["flags"]) & 3) == fmt.METHOD_ZSTD else _inflate(raw)
     if len(data) != rec["rlen"]:
         raise CorruptArchive(f"chunk decoded to {len(data)} bytes, expected {rec['rlen']}")
@@ -582,7 +593,8 @@ def _plan_natively(ar: fmt.Archive, fuse, select, payload_range, out_range, extr
     if rc != gpu.OK:
         return None
     nfused, nf32, npair, nstreams, npieces, nplain, ngeneral, nextra, scratch, coded = (int(c) for c in counts)
-    extras = [_general(ar, r[int(i) if sel is None else int(sel[i])]) for i in general[:ngeneral]]
+    whole = [r[int(i) if sel is None else int(sel[i])] for i in general[:ngeneral]]
+    extras = [_general(ar, int(rec["off"]), int(rec["clen"]), rec) for rec in whole]
     at = hi - lo if extras_at is None else int(extras_at)
     if at != hi - lo and ngeneral:
         pos = np.empty(n, dtype=np.int64)

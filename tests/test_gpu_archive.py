@@ -575,7 +575,9 @@ def test_a_damaged_index_leaves_no_copy_behind(gpu, shard, tmp_path, way):
 
     path = tmp_path / "bad.lmz"
     path.write_bytes(_rewrite_table(blob, spoil))
-    name = [k for k in archive.Archive(blob).tensor_index()][-1]
+    ar = archive.Archive(blob)
+    at = int(ar.records["dst"][-1])
+    name = next(k for k, (_dt, _shape, s, e) in ar.tensor_index().items() if s <= at < e)
     big = torch.empty(1 << 30, dtype=torch.uint8, device="cuda")
     for _ in range(3):
         for _ in range(20):
@@ -590,3 +592,17 @@ def test_a_damaged_index_leaves_no_copy_behind(gpu, shard, tmp_path, way):
         assert all(bool((t == 0xA5).all()) for t in mine)
     path.write_bytes(blob)
     assert (decode.load_archive(str(path)).cpu().numpy() == shard).all()
+
+
+@pytest.mark.parametrize("n", [1, 3_000_001])
+def test_deltas_with_a_deflated_difference(tmp_path, n):
+    """All three ways in, the difference larger than the room a load sets aside for headers or not."""
+    from helpers import deflated_delta
+    from lmz_b200 import decode
+    blob, plain = deflated_delta(n)
+    path = tmp_path / "d.lmz"
+    path.write_bytes(blob)
+    assert (decode.decode_archive(blob).cpu().numpy() == plain).all()
+    assert (decode.load_archive(str(path)).cpu().numpy() == plain).all()
+    got = decode.decode_tensors(str(path), [("b", "w")])
+    assert (got["b", "w"].cpu().numpy() == plain[n:]).all()

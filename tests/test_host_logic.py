@@ -340,3 +340,19 @@ def test_planner_enforces_single_hop_sources():
     struct.pack_into("<Q", bad, int(recs["off"][delta]), ar.total)
     with pytest.raises(archive.CorruptArchive, match="outside"):
         plan.build_plan(archive.Archive(bytes(bad)))
+
+
+@pytest.mark.parametrize("n", [1, 5000])
+def test_planner_inflates_a_deltas_general_purpose_difference(n):
+    """A delta whose difference is one deflated stream: what is inflated begins behind the base's
+    place and the inner codec, and the room for it is counted."""
+    from helpers import deflated_delta
+    from lmz_b200 import archive, plan
+    blob, plain = deflated_delta(n)
+    assert (oa.decode_archive(blob) == plain).all()
+    ar = archive.Archive(blob)
+    p = plan.build_plan(ar)
+    assert (p.extras == plain[:n] ^ plain[n:]).all()
+    assert plan.inflated_bytes(ar.records) == n
+    late = p.chunks[p.chunks["record"] == 1][0]
+    assert int(late["base_off"]) == 0 and int(late["plane_off"][0]) == ar.table_off
