@@ -31,7 +31,7 @@ class _Arena:
     def __init__(self, lib, device):
         self.lib, self.device = lib, device
         self.jobs, self.work = {}, {}
-        self.host = None
+        self.host = self.copied = None
 
     def job(self, name, arr):
         self.jobs[name] = np.ascontiguousarray(arr).view(np.uint8).reshape(-1)
@@ -58,6 +58,8 @@ class _Arena:
             total += (count * size[kind] + 255) & ~255
         dev = torch.empty(max(at, 1) + total, dtype=torch.uint8, device=self.device)
         dev[:at].copy_(torch.from_numpy(self.host[:at]), non_blocking=True)
+        self.copied = torch.cuda.Event()
+        self.copied.record(torch.cuda.current_stream(self.device))
         dev[at:].zero_()
         for name, a in self.jobs.items():
             out[name] = dev[spans[name]:spans[name] + a.size]
@@ -67,8 +69,14 @@ class _Arena:
         return out
 
     def arrived(self):
-        """The copy has been waited for: the host block may go."""
-        self.host = None
+        """Let the host block go, when the copy out of it has ended: whoever gets it next writes to it at
+        once, and a decode that is already queued would run on what they write."""
+        if self.copied is not None:
+            self.copied.synchronize()
+        self.host = self.copied = None
+
+    def __del__(self):
+        self.arrived()
 
 
 _tables = {}

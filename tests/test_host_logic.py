@@ -356,3 +356,26 @@ def test_planner_inflates_a_deltas_general_purpose_difference(n):
     assert plan.inflated_bytes(ar.records) == n
     late = p.chunks[p.chunks["record"] == 1][0]
     assert int(late["base_off"]) == 0 and int(late["plane_off"][0]) == ar.table_off
+
+
+@pytest.mark.parametrize("settled", [True, False])
+def test_a_decoders_host_block_outlives_its_copy(settled):
+    """The page-locked block that job arrays are copied from goes back only when the copy has ended, also
+    when the decoder is dropped before anybody has waited for it."""
+    from lmz_b200 import decode
+    seen = []
+
+    class Block:
+        def __del__(self):
+            seen.append("block")
+
+    class Event:
+        def synchronize(self):
+            seen.append("copy")
+
+    a = decode._Arena(None, None)
+    a.host, a.copied = Block(), Event()
+    if settled:
+        a.arrived()
+    del a
+    assert seen == ["copy", "block"]
