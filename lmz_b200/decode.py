@@ -138,7 +138,7 @@ class ArchiveDecoder:
         d = self.device
         with torch.cuda.device(d):
             pad = gpu.pad_bytes()
-            nbytes = p.extras_at + p.extras.size
+            nbytes = p.extras_pos + p.extras.size
             if payload is not None and payload.numel() < nbytes + pad:
                 raise ValueError("the payload buffer is smaller than the plan's payload, header chunks and slack")
             self.d_payload = payload if payload is not None else \
@@ -172,7 +172,7 @@ class ArchiveDecoder:
             if not p.device_classify:
                 self.d_fused_order = None
             if p.extras.size:
-                self.d_payload[p.extras_at:nbytes].copy_(self.d_extras)
+                self.d_payload[p.extras_pos:nbytes].copy_(self.d_extras)
             self.d_piece_lcnt = torch.empty(max(1, p.cond_pieces.size * 2048), dtype=torch.int32, device=d)
             self.d_tabs = _crc_tables(lib, d)
             if up is not None:

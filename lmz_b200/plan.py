@@ -80,7 +80,6 @@ class Plan:
     delta_jobs: np.ndarray = field(default=None)   # chunks with both BF16 planes coded: decoded, merged, a delta undone
                                                    # and checksummed by one kernel; the first n_delta_plain have no base
     n_delta_plain: int = 0
-    extras_at: int = 0             # where `extras` go, bytes from the payload buffer's start
     tables: np.ndarray = field(default=None)   # the shared tables, TABLE_STRIDE bytes apart
 
     @property
@@ -88,6 +87,12 @@ class Plan:
         """Fused jobs that carry their own table (BF16, then 4-byte elements)."""
         return int(self.fused_jobs.size) - self.n_fused_t
     base_bytes: int = 0            # bytes of delta bases read back
+    extras_at: int | None = None   # where `extras` go, bytes from the payload buffer's start (None: behind the payload)
+
+    @property
+    def extras_pos(self) -> int:
+        """Where the host-inflated chunks start in the payload buffer."""
+        return int(self.payload.size) if self.extras_at is None else int(self.extras_at)
 
     @property
     def n_pieces(self) -> int:

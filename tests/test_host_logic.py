@@ -379,3 +379,19 @@ def test_a_decoders_host_block_outlives_its_copy(settled):
         a.arrived()
     del a
     assert seen == ["copy", "block"]
+
+
+def test_plans_that_do_not_say_where_their_extras_go(shard):
+    """A plan made or saved without that number, as all were once, has them right behind its payload: the
+    buffer is never sized from a zero."""
+    from lmz_b200 import archive, plan
+    p = plan.build_plan(archive.Archive(oa.write_archive([("m.safetensors", shard)], mapped=True)))
+    state = dict(p.__dict__)
+    assert state.pop("extras_at") == p.payload.size
+    assert plan.Plan(**state).extras_pos == p.payload.size
+    saved = plan.Plan.__new__(plan.Plan)
+    saved.__dict__.update(state)
+    assert saved.extras_pos == p.payload.size
+    assert plan.build_plan(archive.Archive(oa.write_archive([("m.safetensors", shard)])), extras_at=1 << 33).extras_pos == 1 << 33
+    names = list(p.__dataclass_fields__)
+    assert names[names.index("n_delta_plain") + 1] == "tables" and names[-1] == "extras_at"     # (by position, too)
