@@ -112,6 +112,16 @@ def _check_layouts(lib):
     _layouts_of.add(id(lib))
 
 
+def _payload_source(ar, plan):
+    """(bytes, where the plan's payload starts in them): the archive's own, where the payload is a view of
+    them and so may be read from its file; the payload itself where the plan was made of another
+    mapping or copy of the archive."""
+    lo = plan.payload.ctypes.data - ar.blob.ctypes.data
+    if 0 <= lo <= ar.blob.size - plan.payload.size:
+        return ar.blob, lo
+    return np.ascontiguousarray(plan.payload).view(np.ndarray), 0
+
+
 class ArchiveDecoder:
     """An archive planned and resident on `device`, ready to decode repeatedly.
 
@@ -240,10 +250,9 @@ class ArchiveDecoder:
             torch.cuda.current_stream(self.device).synchronize()
 
     def _start_upload(self):
-        up = _Uploader(self.archive.blob, self.device)
-        n = self.plan.payload.size
-        lo = n and self.plan.payload.ctypes.data - self.archive.blob.ctypes.data
-        up.send(lo, lo + n, self.d_payload)
+        blob, lo = _payload_source(self.archive, self.plan)
+        up = _Uploader(blob, self.device)
+        up.send(lo, lo + self.plan.payload.size, self.d_payload)
         return up
 
     def _finish_upload(self, up):

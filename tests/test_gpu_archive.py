@@ -606,3 +606,15 @@ def test_deltas_with_a_deflated_difference(tmp_path, n):
     assert (decode.load_archive(str(path)).cpu().numpy() == plain).all()
     got = decode.decode_tensors(str(path), [("b", "w")])
     assert (got["b", "w"].cpu().numpy() == plain[n:]).all()
+
+
+def test_a_plan_of_another_mapping_of_the_file(shard, tmp_path):
+    from lmz_b200 import archive, decode, plan
+    path = tmp_path / "a.lmz"
+    path.write_bytes(oa.write_archive([("m.safetensors", shard)], mapped=True))
+    dec = decode.ArchiveDecoder(str(path), plan=plan.build_plan(archive.Archive(str(path))))
+    for _ in range(2):
+        dec.run()
+        dec.check()
+        assert (dec.output.cpu().numpy() == shard).all()
+        dec.upload()

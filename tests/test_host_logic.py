@@ -395,3 +395,21 @@ def test_plans_that_do_not_say_where_their_extras_go(shard):
     assert plan.build_plan(archive.Archive(oa.write_archive([("m.safetensors", shard)])), extras_at=1 << 33).extras_pos == 1 << 33
     names = list(p.__dataclass_fields__)
     assert names[names.index("n_delta_plain") + 1] == "tables" and names[-1] == "extras_at"     # (by position, too)
+
+
+def test_a_plan_of_another_mapping_is_uploaded_from_its_own_bytes(shard, tmp_path):
+    """The archive mapped twice, or held in memory and mapped: the plan's payload lies outside the bytes
+    of the archive that the decoder was given, and no place in that archive's file stands for it."""
+    from lmz_b200 import archive, decode, plan
+    blob = oa.write_archive([("m.safetensors", shard)], mapped=True)
+    path = tmp_path / "a.lmz"
+    path.write_bytes(blob)
+    mapped = archive.Archive(str(path))
+    off, end = int(mapped.records["off"][3]), mapped.table_off
+    for other in (str(path), blob):
+        p = plan.build_plan(archive.Archive(other), select=np.arange(3, mapped.records.size), payload_range=(off, end))
+        src, lo = decode._payload_source(mapped, p)
+        assert getattr(src, "fd", -1) == -1 and src.ctypes.data + lo == p.payload.ctypes.data
+    p = plan.build_plan(mapped, select=np.arange(3, mapped.records.size), payload_range=(off, end))
+    src, lo = decode._payload_source(mapped, p)
+    assert src is mapped.blob and src.fd >= 0 and lo == off
