@@ -579,6 +579,8 @@ def _plan_natively(ar: fmt.Archive, fuse, select, payload_range, out_range, extr
     sel = None if select is None else np.ascontiguousarray(select, dtype=np.int64)
     n = int(r.size if sel is None else sel.size)
     off, rlen = (r["off"], r["rlen"]) if sel is None else (r["off"][sel], r["rlen"][sel])
+    if sel is not None and n and int(sel.min()) < 0:
+        sel = np.where(sel < 0, sel + r.size, sel)           # (numpy has refused what lies outside)
     lo, hi = payload_range
     out_lo, out_hi = (0, int(ar.total)) if out_range is None else map(int, out_range)
     if not n or lo < 0 or hi < lo or out_lo < 0 or out_hi < out_lo:

@@ -413,3 +413,17 @@ def test_a_plan_of_another_mapping_is_uploaded_from_its_own_bytes(shard, tmp_pat
     p = plan.build_plan(mapped, select=np.arange(3, mapped.records.size), payload_range=(off, end))
     src, lo = decode._payload_source(mapped, p)
     assert src is mapped.blob and src.fd >= 0 and lo == off
+
+
+def test_native_planner_counts_selected_records_from_the_end_too(shard, native_planner):
+    """Record indices below zero count from the end, as in the planner in Python."""
+    from lmz_b200 import archive, plan
+    ar = archive.Archive(oa.write_archive([("m.safetensors", shard)], mapped=True))
+    n = ar.records.size
+    got = plan.build_plan(ar, select=[-1, 0, 2 - n])
+    want = plan.build_plan(ar, select=[n - 1, 0, 2])
+    for name in want.__dataclass_fields__:
+        a, b = getattr(got, name), getattr(want, name)
+        assert np.array_equal(a, b) if isinstance(b, np.ndarray) else a == b, name
+    with pytest.raises(IndexError):
+        plan.build_plan(ar, select=[-n - 1])
