@@ -112,7 +112,7 @@ API int lmz_host_plan(const void *records, const int64_t *select, size_t n, cons
             c.esize = r.esize;
             c.scratch_mask = own ? 0 : s.coded;
             c.record = (uint32_t)i;
-            for (uint32_t q = 0; q < (r.rlen + PIECE_BYTES - 1) / PIECE_BYTES; q++) piece_chunk[pieces++] = (uint32_t)pos;
+            for (uint64_t q = 0; q < ((uint64_t)r.rlen + PIECE_BYTES - 1) / PIECE_BYTES; q++) piece_chunk[pieces++] = (uint32_t)pos;
             chunks[pos++] = c;
             if (s.way == FUSED || s.way == FUSED4) {
                 FusedJob f{};
@@ -155,7 +155,7 @@ API int lmz_host_plan(const void *records, const int64_t *select, size_t n, cons
                 j.n = r.rlen / (codec == C_ONE ? 1 : planes);
                 j.dst_off = scratch;
                 chunks[place[i]].plane_off[k] = scratch;
-                scratch += (j.n + 15u) & ~15u;
+                scratch += ((uint64_t)j.n + 15) & ~(uint64_t)15;
                 owner[nstreams] = (int64_t)i;
                 streams[nstreams++] = j;
             }

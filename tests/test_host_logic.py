@@ -428,3 +428,20 @@ def test_native_planner_counts_selected_records_from_the_end_too(shard, native_p
         assert np.array_equal(a, b) if isinstance(b, np.ndarray) else a == b, name
     with pytest.raises(IndexError):
         plan.build_plan(ar, select=[-n - 1])
+
+
+@pytest.mark.parametrize("longest", [0xFFFF0000, 0xFFFF0001, 0xFFFFFFF0, 0xFFFFFFFF])
+def test_native_planner_with_chunks_near_four_gib(native_planner, monkeypatch, longest):
+    """Pieces and scratch of chunks whose length leaves no room in 32 bits for rounding up."""
+    from helpers import archive_of
+    from lmz_b200 import archive, gpu, plan
+    sizes = (longest, 5000, longest, 17)
+    blob = archive_of([{"path": "m", "size": sum(sizes), "dst": 0, "kind": "raw"}], [(bytes(600), n, 0, 1, 1, 3) for n in sizes])
+    ar = archive.Archive(blob)
+    got = plan._plan_natively(ar, True, None, (0, ar.table_off), None, None)
+    monkeypatch.setattr(gpu._loader, "lib", None)
+    want = plan.build_plan(ar)
+    assert got is not None and want.piece_chunk.size == sum(-(-n // 65536) for n in sizes)
+    for name in want.__dataclass_fields__:
+        a, b = getattr(got, name), getattr(want, name)
+        assert np.array_equal(a, b) if isinstance(b, np.ndarray) else a == b, name
