@@ -100,11 +100,13 @@ def payload_end(b) -> int:
 class Archive:
     """Header, manifest and chunk records of one archive held in host memory."""
 
-    fd = -1                                # the archive's file while it is open, or -1: held in memory
+    @property
+    def fd(self) -> int:
+        """The archive's file while it is open, or -1: held in memory (a copy's or a pickle's bytes are)."""
+        return getattr(self.blob, "fd", -1)
 
     def __init__(self, blob):
         self.blob = open_blob(blob)
-        self.fd = getattr(self.blob, "fd", -1)
         b = self.blob
         if b.size < HEADER.size + FOOTER.size:
             raise FormatError("file is too small to be an lmz archive")

@@ -445,3 +445,19 @@ def test_native_planner_with_chunks_near_four_gib(native_planner, monkeypatch, l
     for name in want.__dataclass_fields__:
         a, b = getattr(got, name), getattr(want, name)
         assert np.array_equal(a, b) if isinstance(b, np.ndarray) else a == b, name
+
+
+def test_an_archives_file_goes_with_its_mapping(shard, tmp_path):
+    """A copy or pickle of a mapped archive is bytes in memory: it must not name a file descriptor, which
+    by then is another file's or, in another process, never was this one's."""
+    import copy
+    import pickle
+    from lmz_b200 import archive
+    path = tmp_path / "a.lmz"
+    path.write_bytes(oa.write_archive([("m.safetensors", shard)], mapped=True))
+    ar = archive.Archive(str(path))
+    assert ar.fd >= 0 and os.path.samestat(os.fstat(ar.fd), os.stat(path))
+    for other in (copy.deepcopy(ar), pickle.loads(pickle.dumps(ar))):
+        assert other.fd == -1 and (other.blob == ar.blob).all() and (other.records == ar.records).all()
+    assert copy.copy(ar).fd == ar.fd
+    assert archive.Archive(ar.blob[:]).fd == -1 and archive.Archive(path.read_bytes()).fd == -1
