@@ -192,7 +192,10 @@ void upload_block(Transfer *t, size_t r, int fd, const uint8_t *host, uint64_t o
     if (!bad) {
         std::lock_guard<std::mutex> lock(t->issue);
         e = cudaMemcpyAsync(dst, b->p, n, cudaMemcpyHostToDevice, t->stream);
-        if (e == cudaSuccess) e = cudaEventRecord(b->left, t->stream);
+        if (e == cudaSuccess) {
+            e = cudaEventRecord(b->left, t->stream);
+            if (e != cudaSuccess) cudaStreamSynchronize(t->stream);      // (the block is not to be had before its copy has left it)
+        }
         b->busy = e == cudaSuccess;
         if (e == cudaSuccess) {
             // whichever block of the range is issued last records the range's event
@@ -278,19 +281,27 @@ API void *lmz_gpu_transfer_new(void *staging, void *cuda_stream)
     return t.release();
 }
 
+// A range of `n` blocks with its event.  Its blocks count as open from here on, so this comes after every
+// call that can fail: transfer_free waits for each of them.
+static size_t open_range(Transfer *t, size_t n, cudaEvent_t event, bool to_device)
+{
+    std::lock_guard<std::mutex> lock(t->mu);
+    const size_t r = t->ranges.size();
+    t->ranges.emplace_back();
+    t->ranges[r].left = n;
+    t->ranges[r].event = event;
+    t->ranges[r].to_device = to_device;
+    t->open += n;
+    return r;
+}
+
 API int lmz_gpu_transfer_upload(void *transfer, int fd, const void *host, uint64_t off, uint64_t len, void *d_dst)
 {
     Transfer *t = static_cast<Transfer *>(transfer);
     const size_t B = t->pool->block, n = (size_t)((len + B - 1) / B);
-    size_t r;
-    {
-        std::lock_guard<std::mutex> lock(t->mu);
-        r = t->ranges.size();
-        t->ranges.emplace_back();
-        t->ranges[r].left = n;
-        t->open += n;
-        CK("cudaEventCreate", cudaEventCreateWithFlags(&t->ranges[r].event, cudaEventDisableTiming));
-    }
+    cudaEvent_t arrived = nullptr;
+    CK("cudaEventCreate", cudaEventCreateWithFlags(&arrived, cudaEventDisableTiming));
+    const size_t r = open_range(t, n, arrived, true);
     for (uint64_t at = 0; at < len; at += B) {
         const size_t m = (size_t)(len - at < B ? len - at : B);
         uint8_t *dst = static_cast<uint8_t *>(d_dst) + at;
@@ -303,19 +314,13 @@ API int lmz_gpu_transfer_download(void *transfer, const void *d_src, uint64_t le
 {
     Transfer *t = static_cast<Transfer *>(transfer);
     const size_t B = t->pool->block, n = (size_t)((len + B - 1) / B);
-    size_t r;
     cudaEvent_t after = nullptr;
-    {
-        std::lock_guard<std::mutex> lock(t->mu);
-        r = t->ranges.size();
-        t->ranges.emplace_back();
-        t->ranges[r].left = n;
-        t->ranges[r].to_device = false;
-        t->open += n;
-        CK("cudaEventCreate", cudaEventCreateWithFlags(&after, cudaEventDisableTiming));
-        t->ranges[r].event = after;
-        CK("cudaEventRecord", cudaEventRecord(after, (cudaStream_t)cuda_stream));
+    CK("cudaEventCreate", cudaEventCreateWithFlags(&after, cudaEventDisableTiming));
+    if (cudaError_t e = cudaEventRecord(after, (cudaStream_t)cuda_stream); e != cudaSuccess) {
+        cudaEventDestroy(after);
+        return fail_cuda("cudaEventRecord", e);
     }
+    const size_t r = open_range(t, n, after, false);
     for (uint64_t at = 0; at < len; at += B) {
         const size_t m = (size_t)(len - at < B ? len - at : B);
         const uint8_t *src = static_cast<const uint8_t *>(d_src) + at;

@@ -110,6 +110,8 @@ class _FileWriter:
         with torch.cuda.device(self.device):
             r = self.lib.lmz_gpu_transfer_download(self.handle, data.data_ptr(), n, self.fd, at, lead if at else pos, self.stream)
         if r < 0:
+            if at:
+                self.lib.lmz_host_unmap_file(at, n + lead)
             raise RuntimeError(gpu.last_error())
         self.pending.append((r, data, at, n + lead))
         while len(self.pending) > IN_FLIGHT:

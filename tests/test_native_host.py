@@ -24,7 +24,41 @@ def host_io(tmp_path_factory):
     return _compiled(tmp_path_factory, "host_io_check")
 
 
-@pytest.mark.parametrize("check", ["arrived unwaited", "arrived waited"])
+@pytest.mark.parametrize("check", ["arrived unwaited", "arrived waited", "upload without an event",
+                                   "download without an event", "download without a record"])
 def test_transfers(host_io, check):
-    done = subprocess.run([host_io, check], capture_output=True, text=True, timeout=60)
+    done = subprocess.run([host_io, check], capture_output=True, text=True, timeout=20)
     assert done.returncode == 0, done.stderr
+
+
+def test_a_mapping_that_is_not_written_through_is_given_back(monkeypatch):
+    import contextlib
+
+    import torch
+    from lmz_b200 import gpu, save
+    monkeypatch.setattr(torch.cuda, "device", lambda d: contextlib.nullcontext())
+    monkeypatch.setattr(gpu, "last_error", lambda: "made to fail")
+    seen = []
+
+    class Lib:
+        def lmz_host_map_file(self, fd, off, n):
+            return 4096
+
+        def lmz_gpu_transfer_download(self, *a):
+            return gpu.ECUDA
+
+        def lmz_host_unmap_file(self, at, n):
+            seen.append((at, n))
+
+    class Data:
+        def numel(self):
+            return 100
+
+        def data_ptr(self):
+            return 0
+
+    w = save._FileWriter.__new__(save._FileWriter)
+    w.lib, w.fd, w.device, w.stream, w.handle, w.pending = Lib(), 3, None, 0, 1, []
+    with pytest.raises(RuntimeError):
+        w.send(Data(), 4100)
+    assert seen == [(4096, 104)] and not w.pending
