@@ -133,8 +133,11 @@ struct Borrowed {
             size_t mine = 0;
             for (const Workspace &o : p.idle) mine += o.device == w.device;
             if (mine < KEPT_WORKSPACES) {
-                p.idle.push_back(w);
-                return;
+                try {
+                    p.idle.push_back(w);
+                    return;
+                } catch (...) {          // no memory to remember it by
+                }
             }
         }
         w.drop();
@@ -154,28 +157,34 @@ bool is_lent(const void *p, size_t bytes)
 API void *lmz_gpu_host_alloc(size_t bytes)
 {
     const size_t c = size_class(bytes + LENT_HEAD);
-    HostPool &p = host_pool();
-    {
-        std::lock_guard<std::mutex> lock(p.mu);
-        auto it = p.spare.find(c);
-        if (it != p.spare.end()) {
-            void *q = it->second;
-            p.spare.erase(it);
-            p.spare_bytes -= c;
-            q = static_cast<uint8_t *>(q) + LENT_HEAD;
-            p.lent[q] = c;
-            return q;
+    return guarded<void *>(nullptr, [&]() -> void * {
+        HostPool &p = host_pool();
+        {
+            std::lock_guard<std::mutex> lock(p.mu);
+            auto it = p.spare.find(c);
+            if (it != p.spare.end()) {
+                void *q = static_cast<uint8_t *>(it->second) + LENT_HEAD;
+                p.lent[q] = c;
+                p.spare.erase(it);
+                p.spare_bytes -= c;
+                return q;
+            }
         }
-    }
-    void *q = nullptr;
-    if (cudaHostAlloc(&q, c, cudaHostAllocPortable) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    q = static_cast<uint8_t *>(q) + LENT_HEAD;
-    std::lock_guard<std::mutex> lock(p.mu);
-    p.lent[q] = c;
-    return q;
+        void *block = nullptr;
+        if (cudaHostAlloc(&block, c, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        void *q = static_cast<uint8_t *>(block) + LENT_HEAD;
+        std::lock_guard<std::mutex> lock(p.mu);
+        try {
+            p.lent[q] = c;
+        } catch (...) {
+            cudaFreeHost(block);
+            throw;
+        }
+        return q;
+    });
 }
 
 API void lmz_gpu_host_free(void *q)
@@ -189,9 +198,12 @@ API void lmz_gpu_host_free(void *q)
         p.lent.erase(it);
         q = static_cast<uint8_t *>(q) - LENT_HEAD;
         if (p.spare_bytes + c <= KEPT_HOST_BYTES) {
-            p.spare.emplace(c, q);
-            p.spare_bytes += c;
-            return;
+            try {
+                p.spare.emplace(c, q);
+                p.spare_bytes += c;
+                return;
+            } catch (...) {              // no memory to remember it by
+            }
         }
     }
     cudaFreeHost(q);
@@ -201,12 +213,11 @@ API void lmz_gpu_trim(void)
 {
     HostPool &p = host_pool();
     std::vector<Workspace> idle;
-    std::vector<void *> spare;
+    std::unordered_multimap<size_t, void *> spare;
     {
         std::lock_guard<std::mutex> lock(p.mu);
         idle.swap(p.idle);
-        for (auto &kv : p.spare) spare.push_back(kv.second);
-        p.spare.clear();
+        spare.swap(p.spare);
         p.spare_bytes = 0;
     }
     int dev = 0;
@@ -216,7 +227,7 @@ API void lmz_gpu_trim(void)
         w.drop();
     }
     if (had) cudaSetDevice(dev);
-    for (void *q : spare) cudaFreeHost(q);
+    for (auto &kv : spare) cudaFreeHost(kv.second);
 }
 
 API int lmz_gpu_decode_batch(const void *hdr, const void *streams, size_t nbytes, const void *off,

@@ -7,12 +7,16 @@
 // memory), starts its copy on the transfer's stream and takes the next, so several blocks are
 // being filled while others are on the link and no interpreter lock is involved.  Writing a file
 // is the same backwards.
+#include <atomic>
 #include <cerrno>
 #include <condition_variable>
 #include <deque>
 #include <functional>
 #include <memory>
+#include <mutex>
+#include <new>
 #include <thread>
+#include <vector>
 #include <fcntl.h>
 #include <sys/mman.h>
 #include <sys/stat.h>
@@ -31,22 +35,30 @@ struct Workers {
 
     explicit Workers(unsigned n)
     {
-        for (unsigned i = 0; i < n; i++)
-            threads.emplace_back([this] {
-                for (;;) {
-                    std::function<void()> job;
-                    {
-                        std::unique_lock<std::mutex> lock(mu);
-                        wake.wait(lock, [this] { return stop || !jobs.empty(); });
-                        if (jobs.empty()) return;
-                        job = std::move(jobs.front());
-                        jobs.pop_front();
-                    }
-                    job();
-                }
-            });
+        threads.reserve(n);
+        try {
+            for (unsigned i = 0; i < n; i++) threads.emplace_back([this] { run(); });
+        } catch (...) {
+            end();                       // (those that were started must be joined)
+            throw;
+        }
     }
-    ~Workers()
+    ~Workers() { end(); }
+    void run()
+    {
+        for (;;) {
+            std::function<void()> job;
+            {
+                std::unique_lock<std::mutex> lock(mu);
+                wake.wait(lock, [this] { return stop || !jobs.empty(); });
+                if (jobs.empty()) return;
+                job = std::move(jobs.front());
+                jobs.pop_front();
+            }
+            job();
+        }
+    }
+    void end()
     {
         {
             std::lock_guard<std::mutex> lock(mu);
@@ -242,27 +254,33 @@ API void *lmz_gpu_staging_new(size_t block, unsigned depth, unsigned threads)
         fail_msg(LMZ_GPU_EUNSUPPORTED, "staging needs more blocks than threads");
         return nullptr;
     }
-    std::unique_ptr<StagingPool> p(new StagingPool);
-    p->block = block;
-    for (unsigned i = 0; i < depth; i++) {
-        p->blocks.emplace_back(new Block);
-        cudaError_t e = cudaHostAlloc((void **)&p->blocks.back()->p, block, cudaHostAllocPortable);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            fail_cuda("page-locked staging", e);
-            return nullptr;
+    return guarded<void *>(nullptr, [&]() -> void * {
+        std::unique_ptr<StagingPool> p(new StagingPool);
+        p->block = block;
+        for (unsigned i = 0; i < depth; i++) {
+            p->blocks.emplace_back(new Block);
+            cudaError_t e = cudaHostAlloc((void **)&p->blocks.back()->p, block, cudaHostAllocPortable);
+            if (e != cudaSuccess) {
+                cudaGetLastError();
+                fail_cuda("page-locked staging", e);
+                return nullptr;
+            }
+            p->free_blocks.push_back(p->blocks.back().get());
         }
-        p->free_blocks.push_back(p->blocks.back().get());
-    }
-    p->workers.reset(new Workers(threads));
-    return p.release();
+        p->workers.reset(new Workers(threads));
+        return p.release();
+    });
 }
 
 API void lmz_gpu_staging_free(void *staging) { delete static_cast<StagingPool *>(staging); }
 
 API void *lmz_gpu_transfer_new(void *staging, void *cuda_stream)
 {
-    std::unique_ptr<Transfer> t(new Transfer);
+    std::unique_ptr<Transfer> t(new (std::nothrow) Transfer);
+    if (!t) {
+        fail_msg(LMZ_GPU_EUNSUPPORTED, "host resources");
+        return nullptr;
+    }
     t->pool = static_cast<StagingPool *>(staging);
     cudaEvent_t ev = nullptr;
     cudaError_t e = cudaGetDevice(&t->device);
@@ -283,16 +301,32 @@ API void *lmz_gpu_transfer_new(void *staging, void *cuda_stream)
 
 // A range of `n` blocks with its event.  Its blocks count as open from here on, so this comes after every
 // call that can fail: transfer_free waits for each of them.
-static size_t open_range(Transfer *t, size_t n, cudaEvent_t event, bool to_device)
+// -1: no memory, and the event is gone.
+static int open_range(Transfer *t, size_t n, cudaEvent_t event, bool to_device)
 {
-    std::lock_guard<std::mutex> lock(t->mu);
-    const size_t r = t->ranges.size();
-    t->ranges.emplace_back();
-    t->ranges[r].left = n;
-    t->ranges[r].event = event;
-    t->ranges[r].to_device = to_device;
-    t->open += n;
+    const int r = guarded(-1, [&] {
+        std::lock_guard<std::mutex> lock(t->mu);
+        t->ranges.emplace_back();
+        Transfer::Range &range = t->ranges.back();
+        range.left = n;
+        range.event = event;
+        range.to_device = to_device;
+        t->open += n;
+        return (int)t->ranges.size() - 1;
+    });
+    if (r < 0) cudaEventDestroy(event);
     return r;
+}
+
+// A range's block for the workers; one that cannot be handed over ends the transfer like one that failed.
+template <class F>
+static void queue_block(Transfer *t, size_t r, F job)
+{
+    try {
+        t->pool->workers->add(job);
+    } catch (...) {
+        t->finish(r, "no memory for a transfer's block");
+    }
 }
 
 API int lmz_gpu_transfer_upload(void *transfer, int fd, const void *host, uint64_t off, uint64_t len, void *d_dst)
@@ -301,13 +335,14 @@ API int lmz_gpu_transfer_upload(void *transfer, int fd, const void *host, uint64
     const size_t B = t->pool->block, n = (size_t)((len + B - 1) / B);
     cudaEvent_t arrived = nullptr;
     CK("cudaEventCreate", cudaEventCreateWithFlags(&arrived, cudaEventDisableTiming));
-    const size_t r = open_range(t, n, arrived, true);
+    const int r = open_range(t, n, arrived, true);
+    if (r < 0) return LMZ_GPU_EUNSUPPORTED;
     for (uint64_t at = 0; at < len; at += B) {
         const size_t m = (size_t)(len - at < B ? len - at : B);
         uint8_t *dst = static_cast<uint8_t *>(d_dst) + at;
-        t->pool->workers->add([=] { upload_block(t, r, fd, static_cast<const uint8_t *>(host), off + at, m, dst); });
+        queue_block(t, r, [=] { upload_block(t, r, fd, static_cast<const uint8_t *>(host), off + at, m, dst); });
     }
-    return (int)r;
+    return r;
 }
 
 API int lmz_gpu_transfer_download(void *transfer, const void *d_src, uint64_t len, int fd, void *map, uint64_t off, void *cuda_stream)
@@ -320,13 +355,14 @@ API int lmz_gpu_transfer_download(void *transfer, const void *d_src, uint64_t le
         cudaEventDestroy(after);
         return fail_cuda("cudaEventRecord", e);
     }
-    const size_t r = open_range(t, n, after, false);
+    const int r = open_range(t, n, after, false);
+    if (r < 0) return LMZ_GPU_EUNSUPPORTED;
     for (uint64_t at = 0; at < len; at += B) {
         const size_t m = (size_t)(len - at < B ? len - at : B);
         const uint8_t *src = static_cast<const uint8_t *>(d_src) + at;
-        t->pool->workers->add([=] { download_block(t, r, src, m, fd, static_cast<uint8_t *>(map), off + at, after); });
+        queue_block(t, r, [=] { download_block(t, r, src, m, fd, static_cast<uint8_t *>(map), off + at, after); });
     }
-    return (int)r;
+    return r;
 }
 
 API int lmz_gpu_transfer_wait(void *transfer, int range, void *cuda_stream)
@@ -380,10 +416,18 @@ API int lmz_host_gather(int fd, const void *host, uint64_t size, const uint64_t 
         }
     };
     const size_t threads = n < 512 ? 1 : 8, per = (n + threads - 1) / threads;
-    std::vector<std::thread> crew;
-    for (size_t i = 1; i < threads; i++) crew.emplace_back(run, i * per < n ? i * per : n, (i + 1) * per < n ? (i + 1) * per : n);
+    std::thread crew[8];
+    for (size_t i = 1; i < threads; i++) {
+        const size_t lo = i * per < n ? i * per : n, hi = (i + 1) * per < n ? (i + 1) * per : n;
+        try {
+            crew[i] = std::thread(run, lo, hi);
+        } catch (...) {
+            run(lo, hi);                 // no thread to be had: this one's work
+        }
+    }
     run(0, per < n ? per : n);
-    for (std::thread &t : crew) t.join();
+    for (std::thread &t : crew)
+        if (t.joinable()) t.join();
     return bad.load() ? fail_msg(LMZ_GPU_EBADSTREAM, "reading the file failed") : LMZ_GPU_OK;
 }
 

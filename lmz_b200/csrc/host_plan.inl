@@ -22,7 +22,7 @@ enum : unsigned { C_STORED = 0, C_ONE = 1, C_SPLIT = 2, C_BF16 = 3, M_STORED = 0
 
 API int lmz_host_plan_head_bytes(void) { return (int)PLAN_HEAD; }
 
-API int lmz_host_plan(const void *records, const int64_t *select, size_t n, const uint64_t *ranges /* payload lo, hi, output lo, hi */,
+static int plan_chunks(const void *records, const int64_t *select, size_t n, const uint64_t *ranges /* payload lo, hi, output lo, hi */,
                       const void *heads, int fuse /* 0 no, 1 yes, 2 every chunk that can be */, unsigned fuse_f32_min,
                       void *chunks_v, void *fused_v, void *delta_v, void *streams_v, int64_t *owner, uint32_t *piece_chunk,
                       int64_t *general, uint64_t *counts)
@@ -177,4 +177,15 @@ API int lmz_host_plan(const void *records, const int64_t *select, size_t n, cons
     const uint64_t c[] = {nfused + nfused4, nfused4, npair, nstreams, pieces, plain_pieces, ngeneral, extra - pay, scratch, coded_bytes};
     memcpy(counts, c, sizeof c);
     return LMZ_GPU_OK;
+}
+
+API int lmz_host_plan(const void *records, const int64_t *select, size_t n, const uint64_t *ranges /* payload lo, hi, output lo, hi */,
+                      const void *heads, int fuse /* 0 no, 1 yes, 2 every chunk that can be */, unsigned fuse_f32_min,
+                      void *chunks_v, void *fused_v, void *delta_v, void *streams_v, int64_t *owner, uint32_t *piece_chunk,
+                      int64_t *general, uint64_t *counts)
+{
+    return guarded(1, [&] {
+        return plan_chunks(records, select, n, ranges, heads, fuse, fuse_f32_min, chunks_v, fused_v, delta_v, streams_v, owner,
+                           piece_chunk, general, counts);
+    });
 }

@@ -7,7 +7,6 @@
 // the per-function contract live in include/lmz_b200.h.
 #include <algorithm>
 #include <atomic>
-#include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -26,30 +25,7 @@ using namespace lmz;
 
 #define API extern "C" __attribute__((visibility("default")))
 
-// Why the last call on this thread failed (lmz_gpu_last_error).
-static thread_local char g_err[256];
-
-// Record a reason and hand back the code to return.
-static int report(int code, const char *fmt, ...)
-{
-    va_list ap;
-    va_start(ap, fmt);
-    vsnprintf(g_err, sizeof g_err, fmt, ap);
-    va_end(ap);
-    return code;
-}
-
-static int fail_msg(int rc, const char *what) { return report(rc, "%s", what); }
-
-static int fail_cuda(const char *what, cudaError_t e)
-{
-    return report(LMZ_GPU_ECUDA, "%s: %s", what, cudaGetErrorString(e));
-}
-
-// A CUDA call inside a function that returns a code: leave with ECUDA when it fails.
-#define CK(what, x)                                                                    \
-    if (cudaError_t status_of_call = (x); status_of_call != cudaSuccess)               \
-        return fail_cuda(what, status_of_call)
+#include "host_error.inl"
 
 static int device_ready()
 {

@@ -1,32 +1,17 @@
 // Checks of csrc/host_io.inl over a stand-in for the CUDA runtime (cuda_runtime.h beside this file).
 // argv[1] names the check; exit status 0 = it held.
-#include <atomic>
-#include <cstdarg>
 #include <cstdint>
 #include <cstdio>
-#include <mutex>
 #include <string>
 #include <vector>
+
+#include <sys/resource.h>
 
 #include "cuda_runtime.h"
 #include "../../include/lmz_b200.h"
 
 #define API extern "C"
-static thread_local char g_err[256];
-static int report(int code, const char *fmt, ...)
-{
-    va_list ap;
-    va_start(ap, fmt);
-    vsnprintf(g_err, sizeof g_err, fmt, ap);
-    va_end(ap);
-    return code;
-}
-static int fail_msg(int rc, const char *what) { return report(rc, "%s", what); }
-static int fail_cuda(const char *what, cudaError_t e) { return report(LMZ_GPU_ECUDA, "%s: %s", what, cudaGetErrorString(e)); }
-#define CK(what, x)                                                                    \
-    if (cudaError_t status_of_call = (x); status_of_call != cudaSuccess)               \
-        return fail_cuda(what, status_of_call)
-
+#include "../../lmz_b200/csrc/host_error.inl"
 #include "../../lmz_b200/csrc/host_io.inl"
 
 #define NEED(c)                                                          \
@@ -83,6 +68,34 @@ static int failed_range_is_not_waited_for(bool up, int *call)
     return 0;
 }
 
+// Threads that cannot be started (no room for their stacks) are an error, or the caller's own work; never
+// the end of the process.
+static int no_room_for_threads()
+{
+    constexpr size_t N = 4096, WIDTH = 32;
+    std::vector<uint8_t> from(N * 40), got(N * WIDTH);
+    std::vector<uint64_t> offs(N);
+    for (size_t i = 0; i < from.size(); i++) from[i] = (uint8_t)(i * 11);
+    for (size_t i = 0; i < N; i++) offs[i] = i * 40;
+    struct rlimit was, now;
+    NEED(getrlimit(RLIMIT_AS, &was) == 0);
+    long pages = 0;
+    FILE *f = fopen("/proc/self/statm", "r");
+    NEED(f && fscanf(f, "%ld", &pages) == 1);
+    fclose(f);
+    now = was;
+    now.rlim_cur = (rlim_t)pages * 4096 + (20 << 20);        // two stacks of eight MiB
+    NEED(setrlimit(RLIMIT_AS, &now) == 0);
+    void *staging = lmz_gpu_staging_new(64, 200, 100);
+    const bool said = strstr(g_err, "host resources") != nullptr;
+    const int rc = lmz_host_gather(-1, from.data(), from.size(), offs.data(), N, WIDTH, got.data());
+    NEED(setrlimit(RLIMIT_AS, &was) == 0);
+    NEED(!staging && said);
+    NEED(rc == LMZ_GPU_OK);
+    for (size_t i = 0; i < N; i++) NEED(memcmp(got.data() + i * WIDTH, from.data() + i * 40, WIDTH) == 0);
+    return 0;
+}
+
 int main(int argc, char **argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
@@ -91,6 +104,7 @@ int main(int argc, char **argv)
     if (what == "upload without an event") return failed_range_is_not_waited_for(true, &fake::fail_event_create);
     if (what == "download without an event") return failed_range_is_not_waited_for(false, &fake::fail_event_create);
     if (what == "download without a record") return failed_range_is_not_waited_for(false, &fake::fail_event_record);
+    if (what == "no room for threads") return no_room_for_threads();
     fprintf(stderr, "no such check\n");
     return 2;
 }

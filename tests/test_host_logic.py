@@ -461,3 +461,13 @@ def test_an_archives_file_goes_with_its_mapping(shard, tmp_path):
         assert other.fd == -1 and (other.blob == ar.blob).all() and (other.records == ar.records).all()
     assert copy.copy(ar).fd == ar.fd
     assert archive.Archive(ar.blob[:]).fd == -1 and archive.Archive(path.read_bytes()).fd == -1
+
+
+def test_native_planner_declines_what_it_has_no_memory_for(lib_path):
+    """A C++ exception must not leave the entry point: the answer is the one for archives it does not take."""
+    code = ("import ctypes, sys; lib = ctypes.CDLL(sys.argv[1]); f = lib.lmz_host_plan;"
+            "f.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int,"
+            " ctypes.c_uint] + [ctypes.c_void_p] * 8; r = (ctypes.c_uint64 * 4)();"
+            "print(f(None, None, 1 << 60, r, None, 1, 0, *[None] * 8))")
+    out = subprocess.run([sys.executable, "-c", code, lib_path], capture_output=True, text=True)
+    assert out.stdout.strip() == "1", out.stderr

@@ -25,7 +25,7 @@ def host_io(tmp_path_factory):
 
 
 @pytest.mark.parametrize("check", ["arrived unwaited", "arrived waited", "upload without an event",
-                                   "download without an event", "download without a record"])
+                                   "download without an event", "download without a record", "no room for threads"])
 def test_transfers(host_io, check):
     done = subprocess.run([host_io, check], capture_output=True, text=True, timeout=20)
     assert done.returncode == 0, done.stderr
