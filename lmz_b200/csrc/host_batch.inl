@@ -25,13 +25,6 @@ constexpr size_t LENT_HEAD = 64, VERDICT = 16;
 // together.
 constexpr size_t SMALL_BYTES = (size_t)256 << 10;
 
-size_t size_class(size_t bytes)
-{
-    size_t c = 4096;
-    while (c < bytes) c <<= 1;
-    return c;
-}
-
 struct Workspace {
     int device = -1;
     cudaStream_t stream = nullptr;
@@ -156,7 +149,9 @@ bool is_lent(const void *p, size_t bytes)
 
 API void *lmz_gpu_host_alloc(size_t bytes)
 {
-    const size_t c = size_class(bytes + LENT_HEAD);
+    if (bytes > SIZE_MAX - LENT_HEAD) return nullptr;
+    // (what is too large to be kept is taken as large as it is)
+    const size_t c = bytes + LENT_HEAD <= KEPT_HOST_BYTES ? size_class(bytes + LENT_HEAD) : bytes + LENT_HEAD;
     return guarded<void *>(nullptr, [&]() -> void * {
         HostPool &p = host_pool();
         {

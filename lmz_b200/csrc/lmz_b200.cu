@@ -313,6 +313,7 @@ API int lmz_gpu_decode_batch_dev(const void *d_hdr, const void *d_streams, const
     return launch_rans(a, (cudaStream_t)cuda_stream);
 }
 
+#include "host_rules.inl"
 #include "host_batch.inl"
 #include "host_io.inl"
 #include "host_plan.inl"

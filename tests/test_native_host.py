@@ -3,6 +3,7 @@ runtime (tests/native/cuda_runtime.h) whose streams run their work as late as th
 import os
 import shutil
 import subprocess
+import sys
 
 import pytest
 
@@ -29,6 +30,26 @@ def host_io(tmp_path_factory):
 def test_transfers(host_io, check):
     done = subprocess.run([host_io, check], capture_output=True, text=True, timeout=20)
     assert done.returncode == 0, done.stderr
+
+
+@pytest.fixture(scope="module")
+def host_rules(tmp_path_factory):
+    return _compiled(tmp_path_factory, "host_rules_check")
+
+
+@pytest.mark.parametrize("check", ["size classes"])
+def test_rules(host_rules, check):
+    done = subprocess.run([host_rules, check], capture_output=True, text=True, timeout=20)
+    assert done.returncode == 0, done.stderr
+
+
+def test_no_result_memory_is_an_answer():
+    """More than there is, up to what no class could hold: NULL at once."""
+    from lmz_b200 import build
+    code = ("import ctypes, sys; lib = ctypes.CDLL(sys.argv[1]); f = lib.lmz_gpu_host_alloc; f.restype = ctypes.c_void_p;"
+            "f.argtypes = [ctypes.c_size_t]; print([f(n) for n in (1 << 62, (1 << 63) + 1, (1 << 64) - 65, (1 << 64) - 1)])")
+    out = subprocess.run([sys.executable, "-c", code, build.build()], capture_output=True, text=True, timeout=60)
+    assert out.stdout.strip() == "[None, None, None, None]", out.stderr
 
 
 def test_a_mapping_that_is_not_written_through_is_given_back(monkeypatch):
