@@ -76,6 +76,9 @@ def save_archive(path, members, chunk_size: int = 64 << 10, mapped: bool = True,
         raise ValueError("chunk_size must be even, at least 64 KiB and below 2 MiB")
     fd = os.open(path, os.O_RDWR | os.O_CREAT, 0o666)
     try:
+        # whatever ends this save early, down to the end of the process, must not leave a file that opens:
+        # an archive that is overwritten loses its header first, and gets the new one last
+        _put(fd, bytes(fmt.HEADER.size), 0)
         try:
             return _write_archive(fd, members, chunk_size, mapped, stats)
         except BaseException:
@@ -217,8 +220,8 @@ def _write_archive(fd, members, chunk_size, mapped, stats):
                 errors.append(exc)
     if errors:
         raise errors[0]
+    os.ftruncate(fd, end)                                    # (the end of a longer file before is a footer, too)
     _put(fd, fmt.HEADER.pack(fmt.MAGIC, 6, fmt.FLAG_PAGE_MAPPED if mapped else 0, base, 0, 0), 0)
-    os.ftruncate(fd, end)
     if stats is not None:
         stats.update(device_s=sum(e0.elapsed_time(e1) + e2.elapsed_time(e3) for e0, e1, e2, e3 in timed) / 1e3,
                      payload_bytes=off - fmt.HEADER.size)
