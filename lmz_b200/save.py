@@ -25,6 +25,7 @@ from __future__ import annotations
 import ctypes
 import json
 import os
+import stat
 import struct
 import zlib
 
@@ -74,7 +75,10 @@ def save_archive(path, members, chunk_size: int = 64 << 10, mapped: bool = True,
     the file system's side of that.  An existing file is overwritten in place and cut to length."""
     if chunk_size < (64 << 10) or chunk_size >= COND_MIN_BYTES or chunk_size % 2:
         raise ValueError("chunk_size must be even, at least 64 KiB and below 2 MiB")
-    fd = os.open(path, os.O_RDWR | os.O_CREAT, 0o666)
+    try:
+        fd = os.open(path, os.O_RDWR | os.O_CREAT, 0o666)
+    except PermissionError:                                  # a file that may be written only: no mapping, then
+        fd = os.open(path, os.O_WRONLY | os.O_CREAT, 0o666)
     try:
         # whatever ends this save early, down to the end of the process, must not leave a file that opens:
         # an archive that is overwritten loses its header first, and gets the new one last
@@ -82,10 +86,16 @@ def save_archive(path, members, chunk_size: int = 64 << 10, mapped: bool = True,
         try:
             return _write_archive(fd, members, chunk_size, mapped, stats)
         except BaseException:
-            os.ftruncate(fd, 0)
+            _cut(fd, 0)
             raise
     finally:
         os.close(fd)
+
+
+def _cut(fd, size: int) -> None:
+    """Make a file `size` bytes long; a device (os.devnull) has no length."""
+    if stat.S_ISREG(os.fstat(fd).st_mode):
+        os.ftruncate(fd, size)
 
 
 class _FileWriter:
@@ -220,7 +230,7 @@ def _write_archive(fd, members, chunk_size, mapped, stats):
                 errors.append(exc)
     if errors:
         raise errors[0]
-    os.ftruncate(fd, end)                                    # (the end of a longer file before is a footer, too)
+    _cut(fd, end)                                            # (the end of a longer file before is a footer, too)
     _put(fd, fmt.HEADER.pack(fmt.MAGIC, 6, fmt.FLAG_PAGE_MAPPED if mapped else 0, base, 0, 0), 0)
     if stats is not None:
         stats.update(device_s=sum(e0.elapsed_time(e1) + e2.elapsed_time(e3) for e0, e1, e2, e3 in timed) / 1e3,

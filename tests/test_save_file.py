@@ -1,7 +1,6 @@
 """What save_archive does to the file, on the CPU: the device's part is stood in for."""
 import os
 
-import numpy as np
 import pytest
 
 from oracle import archive as oa, synth
@@ -48,3 +47,25 @@ def test_a_shorter_archive_over_a_longer_one(old, monkeypatch):
     n = save.save_archive(str(old), [])
     assert n == old.stat().st_size < before and archive.Archive(str(old)).total == 0
     assert order[-2:] == ["cut", "header"], order
+
+
+@pytest.mark.parametrize("where", ["a device", "a file that may be written only"])
+def test_where_only_writing_goes(old, monkeypatch, where):
+    from lmz_b200 import archive, gpu, save
+    monkeypatch.setattr(gpu, "library", lambda: None)
+    if where == "a device":
+        assert save.save_archive(os.devnull, []) > 0
+        with pytest.raises(ValueError, match="CUDA"):
+            save.save_archive(os.devnull, [("m", None)])
+        return
+    real = os.open
+
+    def as_its_writer_may(path, flags, *mode):
+        if flags & os.O_RDWR:
+            raise PermissionError(13, "made to fail")
+        return real(path, flags, *mode)
+
+    monkeypatch.setattr(os, "open", as_its_writer_may)
+    assert save.save_archive(str(old), []) == old.stat().st_size
+    monkeypatch.undo()
+    assert archive.Archive(str(old)).total == 0
