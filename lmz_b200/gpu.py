@@ -311,7 +311,9 @@ def _decode_batch_cuda(lib, streams, offsets, nstr, plane, out, header):
 
     dev = streams.device
     with torch.cuda.device(dev):
-        flat = streams.reshape(-1).view(torch.uint8)
+        flat = streams.reshape(-1)
+        if flat.dtype != torch.uint8:
+            flat = flat.to(torch.uint8)                      # (by value)
         if _is_cuda_tensor(offsets):
             offs = offsets.reshape(-1).view(torch.int64)
         else:

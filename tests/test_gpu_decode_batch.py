@@ -194,3 +194,22 @@ def test_device_batches_wherever_they_lie(gpu, orc, lead, tail, table_mode):
         bad[at] = value
         with pytest.raises(ValueError):
             gpu.decode_batch(t, bad.tobytes(), 9, 1001)
+
+
+@pytest.mark.parametrize("kind", ["int8", "int32", "int64", "strided"])
+def test_device_batches_of_bytes_in_other_tensors(gpu, orc, kind, table_mode):
+    """Byte values in a tensor of another type are taken by value, a strided tensor in its own order."""
+    if table_mode != -1:
+        pytest.skip("what the bytes come in does not depend on the table layout")
+    import torch
+    plains = [shaped("skewed", 1001, i) for i in range(9)]
+    blob, offs = pack_streams([orc.rans_encode(p) for p in plains])
+    t = torch.frombuffer(bytearray(blob), dtype=torch.uint8).cuda()
+    if kind == "strided":
+        two = torch.zeros(t.numel(), 2, dtype=torch.uint8, device="cuda")
+        two[:, 1] = t
+        t = two[:, 1]
+    else:
+        t = t.to(getattr(torch, kind))
+    out = gpu.decode_batch(t, offs, 9, 1001)
+    assert out.cpu().numpy().tobytes() == b"".join(p.tobytes() for p in plains)
