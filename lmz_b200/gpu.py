@@ -324,9 +324,13 @@ def _decode_batch_cuda(lib, streams, offsets, nstr, plane, out, header):
         if offs.numel() < 2 * nstr:
             raise ValueError("offsets is too short")
         offs = offs.contiguous()
+        size = nstr * plane
+        dst = out if (out is not None and _is_cuda_tensor(out) and out.numel() >= size) \
+            else torch.empty(size, dtype=torch.uint8, device=dev)
         # the kernel reads a little past the last stream: only a tensor that ends where its memory
-        # does has to be copied for that
-        if flat.untyped_storage().nbytes() - flat.storage_offset() - flat.numel() < _READ_AHEAD:
+        # does has to be copied for that, or one that the result goes over
+        if flat.untyped_storage().nbytes() - flat.storage_offset() - flat.numel() < _READ_AHEAD or \
+                (dst.data_ptr() < flat.data_ptr() + flat.numel() and flat.data_ptr() < dst.data_ptr() + size):
             buf = torch.empty(flat.numel() + _READ_AHEAD, dtype=torch.uint8, device=dev)
             buf[:flat.numel()].copy_(flat)
         else:
@@ -335,9 +339,6 @@ def _decode_batch_cuda(lib, streams, offsets, nstr, plane, out, header):
         if header is not None:
             hdr = header if _is_cuda_tensor(header) else \
                 torch.frombuffer(bytearray(header), dtype=torch.uint8).to(dev)
-        size = nstr * plane
-        dst = out if (out is not None and _is_cuda_tensor(out) and out.numel() >= size) \
-            else torch.empty(size, dtype=torch.uint8, device=dev)
         work = torch.empty(nstr * 32 + 256, dtype=torch.uint8, device=dev)
         # (synchronous, which also keeps the inputs alive until the kernels have read them)
         rc = lib.lmz_gpu_decode_batch_checked_dev(hdr.data_ptr() if hdr is not None else None, buf.data_ptr(), flat.numel(),

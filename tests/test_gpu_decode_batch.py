@@ -213,3 +213,21 @@ def test_device_batches_of_bytes_in_other_tensors(gpu, orc, kind, table_mode):
         t = t.to(getattr(torch, kind))
     out = gpu.decode_batch(t, offs, 9, 1001)
     assert out.cpu().numpy().tobytes() == b"".join(p.tobytes() for p in plains)
+
+
+@pytest.mark.parametrize("where", ["on its start", "on its end", "on what is read ahead", "beside it"])
+def test_device_batches_decoded_over_their_own_streams(gpu, orc, where, table_mode):
+    """`out` may share memory with the streams: they are read as they were."""
+    if table_mode != -1:
+        pytest.skip("where the result goes does not depend on the table layout")
+    import torch
+    plains = [shaped("flat", 4097, i) for i in range(40)]
+    blob, offs = pack_streams([orc.rans_encode(p) for p in plains])
+    n, size = len(blob), 40 * 4097
+    whole = torch.zeros(3 * n + 4096, dtype=torch.uint8, device="cuda")
+    at = n + 512
+    whole[at:at + n] = torch.frombuffer(bytearray(blob), dtype=torch.uint8).cuda()
+    lo = {"on its start": at - size + 1000, "on its end": at + n - 1000, "on what is read ahead": at + n + 3, "beside it": at - size}[where]
+    out = gpu.decode_batch(whole[at:at + n], offs, 40, 4097, out=whole[lo:lo + size])
+    assert out.data_ptr() == whole.data_ptr() + lo
+    assert out.cpu().numpy().tobytes() == b"".join(p.tobytes() for p in plains)
