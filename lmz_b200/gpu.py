@@ -401,6 +401,7 @@ def encode_batch(planes, nstr: int, plane: int):
         rc = lib.lmz_gpu_pack_streams_dev(slots.data_ptr(), plane, offs.data_ptr(), nstr, out.data_ptr(), cs)
         if rc != OK:
             return None
+        torch.cuda.current_stream(dev).synchronize()         # (they may be read on any stream from here on)
         if on_device:
             return out[:total], offs
         return out[:total].cpu().numpy().tobytes(), offs.cpu().numpy().astype("<u8").tobytes()

@@ -95,3 +95,19 @@ def test_counts_past_one_stretch_of_the_lanes_counters(gpu, orc, dist, plane):
     """Planes around the lengths at which the encoder sums its 16-bit counters: all of one
     symbol (a lane's counter at its fullest), next to all of one, and every symbol."""
     _check(gpu, orc, [distribution(dist, plane, 5 * i + plane) for i in range(3)])
+
+
+def test_device_results_are_there_when_they_are_returned(gpu, orc):
+    """Streams and offsets may be read at once on any stream, in any thread."""
+    import torch
+    plain = distribution("exponent", 65536, 3)
+    want = torch.frombuffer(bytearray(orc.rans_encode(plain)), dtype=torch.uint8).cuda()
+    t = torch.from_numpy(np.tile(plain, 2000)).cuda()
+    other = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(3):
+        streams, offs = gpu.encode_batch(t, 2000, 65536)
+        assert torch.cuda.current_stream().query()
+        with torch.cuda.stream(other):
+            same = torch.equal(streams.reshape(2000, -1), want.expand(2000, -1))
+        assert same and offs.numel() == 4000
