@@ -280,6 +280,8 @@ def decode_batch(streams, offsets, nstr: int, plane: int, out=None, header=None)
         raise ValueError("nstr is negative")
     if plane < 1:
         raise ValueError("plane must be at least 1")
+    if nstr >> 32 or plane >> 32:
+        raise ValueError("nstr and plane must fit 32 bits")
     if header is not None and len(header) != header_bytes():
         raise ValueError(f"a shared table is {header_bytes()} bytes, not {len(header)}")
     if _is_cuda_tensor(streams):

@@ -231,3 +231,18 @@ def test_device_batches_decoded_over_their_own_streams(gpu, orc, where, table_mo
     out = gpu.decode_batch(whole[at:at + n], offs, 40, 4097, out=whole[lo:lo + size])
     assert out.data_ptr() == whole.data_ptr() + lo
     assert out.cpu().numpy().tobytes() == b"".join(p.tobytes() for p in plains)
+
+
+@pytest.mark.parametrize("on_device", [False, True])
+def test_sizes_beyond_32_bits_are_refused(gpu, orc, on_device, table_mode):
+    """Never taken modulo 2^32: the stream would decode, to a part of what was asked for."""
+    if table_mode != -1:
+        pytest.skip("refused before any table")
+    import torch
+    blob, offs = pack_streams([orc.rans_encode(shaped("skewed", 64, 1))])
+    src = torch.frombuffer(bytearray(blob), dtype=torch.uint8).cuda() if on_device else blob
+    for plane in ((1 << 32) + 64, (1 << 63) + 1, 1 << 70):
+        with pytest.raises(ValueError):
+            gpu.decode_batch(src, offs, 1, plane)
+    with pytest.raises(ValueError):
+        gpu.decode_batch(src, offs, (1 << 32) + 1, 64)
