@@ -89,6 +89,9 @@ int lmz_gpu_set_device(int device);
  * free it. */
 void *lmz_gpu_host_alloc(size_t bytes);
 void lmz_gpu_host_free(void *p);
+/* Whether p is such memory, not yet freed, with room for `bytes`: whether a refused batch may leave its
+ * mark in it. */
+int lmz_gpu_host_lent(const void *p, size_t bytes);
 
 /* No counterpart in the reference.  Give back what the host-memory entry points keep
  * between calls: idle result memory, and per device up to four idle workspaces with

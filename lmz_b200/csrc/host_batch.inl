@@ -204,6 +204,8 @@ API void lmz_gpu_host_free(void *q)
     cudaFreeHost(q);
 }
 
+API int lmz_gpu_host_lent(const void *q, size_t bytes) { return is_lent(q, bytes); }
+
 API void lmz_gpu_trim(void)
 {
     HostPool &p = host_pool();

@@ -52,6 +52,7 @@ _SIGNATURES = {
     "lmz_gpu_pack_offsets_dev": (_C.c_int, [_C.c_void_p, _C.c_uint] + [_C.c_void_p] * 5),
     "lmz_gpu_host_alloc": (_C.c_void_p, [_C.c_size_t]),
     "lmz_gpu_host_free": (None, [_C.c_void_p]),
+    "lmz_gpu_host_lent": (_C.c_int, [_C.c_void_p, _C.c_size_t]),
     "lmz_gpu_trim": (None, []),
     "lmz_gpu_set_table_mode": (_C.c_int, [_C.c_int]),
     "lmz_gpu_decode_streams_dev": (_C.c_int, [_C.c_void_p, _C.c_uint] + [_C.c_void_p] * 6),
@@ -292,13 +293,17 @@ def decode_batch(streams, offsets, nstr: int, plane: int, out=None, header=None)
     src, shared = _host_view(streams), _host_view(header)
     size = nstr * plane
     if out is not None and len(out) >= size:
-        held, dst = out, _host_view(out, writable=True)
+        held, keep = out, _host_view(out, writable=True)
+        # (an earlier result, brought back: its owner's until the batch is known to be good)
+        dst = result_memory(lib, size) if lib.lmz_gpu_host_lent(_addr(keep), size) else keep
     else:
-        held = dst = result_memory(lib, size)
+        held = keep = dst = result_memory(lib, size)
     rc = lib.lmz_gpu_decode_batch(_addr(shared), _addr(src), src.size, _addr(table), nstr, plane,
                                   _addr(dst))
     if rc == EBADSTREAM:
         raise ValueError("malformed rANS stream")
+    if rc == OK and dst is not keep:
+        keep[:size] = dst
     return memoryview(held)[:size] if rc == OK else None
 
 

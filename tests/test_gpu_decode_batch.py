@@ -246,3 +246,25 @@ def test_sizes_beyond_32_bits_are_refused(gpu, orc, on_device, table_mode):
             gpu.decode_batch(src, offs, 1, plane)
     with pytest.raises(ValueError):
         gpu.decode_batch(src, offs, (1 << 32) + 1, 64)
+
+
+@pytest.mark.parametrize("nstr,plane", [(5, 4097), (40, 65537)])
+def test_a_refused_batch_leaves_out_alone(gpu, orc, nstr, plane, table_mode):
+    """Whatever the caller's buffer is: its own, or an earlier result brought back."""
+    if table_mode != -1:
+        pytest.skip("the memory does not depend on the table layout")
+    plains = [shaped("skewed", plane, i) for i in range(nstr)]
+    want = b"".join(p.tobytes() for p in plains)
+    others = [shaped("flat", plane, 77 + i) for i in range(nstr)]
+    blob, offs = pack_streams([orc.rans_encode(p) for p in plains])
+    streams = [orc.rans_encode(p) for p in others]
+    good, good_offs = pack_streams(streams)
+    bad, bad_offs = pack_streams(streams[:-1] + [streams[-1][:-200]])
+    for out in (gpu.decode_batch(blob, offs, nstr, plane), bytearray(want)):
+        with pytest.raises(ValueError):
+            gpu.decode_batch(bad, bad_offs, nstr, plane, out=out)
+        assert bytes(out) == want
+        got = gpu.decode_batch(good, good_offs, nstr, plane, out=out)
+        assert bytes(got) == bytes(out) == b"".join(p.tobytes() for p in others)
+        if not isinstance(out, bytearray):
+            assert gpu.decode_batch(blob, offs, nstr, plane, out=out[1:]) is not None       # too short: memory of its own
