@@ -321,6 +321,7 @@ def _decode_batch_cuda(lib, streams, offsets, nstr, plane, out, header):
         flat = streams.reshape(-1)
         if flat.dtype != torch.uint8:
             flat = flat.to(torch.uint8)                      # (by value)
+        flat = flat.contiguous()
         if _is_cuda_tensor(offsets):
             offs = offsets.reshape(-1).view(torch.int64)
         else:
@@ -380,7 +381,7 @@ def encode_batch(planes, nstr: int, plane: int):
                 torch.empty(0, dtype=torch.int64, device=planes.device)) if on_device else (b"", b"")
     dev = planes.device if on_device else torch.device(f"cuda:{torch.cuda.current_device()}")
     with torch.cuda.device(dev):
-        src = planes.reshape(-1) if on_device else \
+        src = planes.reshape(-1).contiguous() if on_device else \
             torch.frombuffer(bytearray(planes[:nstr * plane]), dtype=torch.uint8).to(dev)
         if src.numel() < nstr * plane:
             raise ValueError("planes is too short")

@@ -176,7 +176,7 @@ def _write_archive(fd, members, chunk_size, mapped, stats):
         for mpath, data in members:
             if not (type(data).__module__.startswith("torch") and data.is_cuda and data.dtype == torch.uint8):
                 raise ValueError("a member must be a CUDA uint8 tensor")
-            flat = data.reshape(-1)
+            flat = data.reshape(-1).contiguous()
             size = int(flat.numel())
             head = bytes(flat[:min(size, 8)].cpu().numpy())
             hlen = struct.unpack("<Q", head)[0] if len(head) == 8 else 0

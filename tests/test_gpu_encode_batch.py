@@ -111,3 +111,12 @@ def test_device_results_are_there_when_they_are_returned(gpu, orc):
         with torch.cuda.stream(other):
             same = torch.equal(streams.reshape(2000, -1), want.expand(2000, -1))
         assert same and offs.numel() == 4000
+
+
+def test_strided_device_planes(gpu, orc):
+    import torch
+    plains = [distribution("exponent", 5000, i) for i in range(3)]
+    two = torch.zeros(15000, 2, dtype=torch.uint8, device="cuda")
+    two[:, 1] = torch.from_numpy(np.concatenate(plains)).cuda()
+    streams, _offs = gpu.encode_batch(two[:, 1], 3, 5000)
+    assert streams.cpu().numpy().tobytes() == b"".join(orc.rans_encode(p) for p in plains)
