@@ -30,10 +30,33 @@ static int size_classes()
     return 0;
 }
 
+// Streams of `plane` symbols, a byte in for each byte out: slices share one stream's time or hide it.
+static int slices()
+{
+    constexpr unsigned SMS = 148;
+    for (unsigned nstr : {1u, 2u, 7u, 8u, 9u, 16u, 63u, 64u, 257u, 512u, 1183u, 1184u, 1185u, 1600u, 3199u, 3200u, 11248u, 40000u})
+        for (uint64_t plane : {1ull, 640ull, 32768ull, 65537ull, 1ull << 20, 1ull << 22, 1ull << 29}) {
+            const unsigned s = batch_slices(2 * nstr * plane, nstr, SMS);
+            NEED(s >= 1 && s <= MOST_SLICES && s <= nstr);
+            if (s == 1) continue;
+            NEED(2 * nstr * plane / s >= SLICE_BYTES);
+            // the launcher's one-warp CTAs of four streams, two to an SM
+            unsigned ctas = 0;
+            for (unsigned j = 0; j < s; j++) ctas += (unsigned)(((uint64_t)nstr * (j + 1) / s - (uint64_t)nstr * j / s + 3) / 4);
+            const double chain = plane / 8 * 64e-9, out = (double)nstr / s * plane / 50e9;
+            NEED(ctas <= 2 * SMS || out >= chain);
+        }
+    NEED(batch_slices(2ull * 16 << 22, 16, SMS) == 8);
+    NEED(batch_slices(28ull << 20, 512, SMS) == 7);
+    NEED(batch_slices(2ull * 1500 << 20, 1500, SMS) == 3);
+    return 0;
+}
+
 int main(int argc, char **argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "size classes") return size_classes();
+    if (what == "slices") return slices();
     fprintf(stderr, "no such check\n");
     return 2;
 }

@@ -37,7 +37,7 @@ def host_rules(tmp_path_factory):
     return _compiled(tmp_path_factory, "host_rules_check")
 
 
-@pytest.mark.parametrize("check", ["size classes"])
+@pytest.mark.parametrize("check", ["size classes", "slices"])
 def test_rules(host_rules, check):
     done = subprocess.run([host_rules, check], capture_output=True, text=True, timeout=20)
     assert done.returncode == 0, done.stderr
