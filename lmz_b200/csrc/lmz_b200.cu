@@ -314,6 +314,7 @@ API int lmz_gpu_decode_batch_dev(const void *d_hdr, const void *d_streams, const
 }
 
 #include "host_rules.inl"
+#include "host_pool.inl"
 #include "host_batch.inl"
 #include "host_io.inl"
 #include "host_plan.inl"

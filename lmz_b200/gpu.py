@@ -173,6 +173,11 @@ def _host_view(buf, writable: bool = False):
     return arr
 
 
+# Page-locking a gigabyte takes 0.4 s: worth it for memory that is kept between calls, as the library does up to this
+# size (csrc/host_pool.inl), but not for one result (one B200, 550 MiB: 294 ms page-locked, 164 not; kept 55).
+_LENT_MAX = (512 << 20) - 64
+
+
 def result_memory(lib, size: int):
     """A writable numpy uint8 array of `size` bytes for a result.  Page-locked where the
     library has some to lend (the copy engine then writes it, and a fresh result costs no
@@ -180,7 +185,7 @@ def result_memory(lib, size: int):
     import weakref
 
     import numpy as np
-    at = lib.lmz_gpu_host_alloc(size)
+    at = lib.lmz_gpu_host_alloc(size) if size <= _LENT_MAX else None
     if not at:
         return np.zeros(size, dtype=np.uint8)
     block = (ctypes.c_uint8 * size).from_address(at)

@@ -24,6 +24,8 @@ inline std::recursive_mutex mu;
 inline FakeStream legacy;
 inline std::map<FakeStream *, size_t> ran;              // operations of a stream that have run
 inline std::set<FakeStream *> streams;                  // alive
+inline std::map<void *, size_t> host;                   // page-locked blocks that are alive
+inline size_t host_allocs = 0;
 inline size_t dropped = 0;                              // operations queued when their stream was destroyed
 inline int fail_event_create = 0, fail_event_record = 0;     // calls from now until one fails, 0 = never
 inline bool due(int &n) { return n > 0 && --n == 0; }
@@ -45,8 +47,25 @@ inline const char *cudaGetErrorString(cudaError_t) { return "made to fail"; }
 inline cudaError_t cudaGetLastError() { return cudaSuccess; }
 inline cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
 inline cudaError_t cudaSetDevice(int) { return cudaSuccess; }
-inline cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { *p = malloc(n); return *p ? cudaSuccess : cudaErrorUnknown; }
-inline cudaError_t cudaFreeHost(void *p) { free(p); return cudaSuccess; }
+inline cudaError_t cudaHostAlloc(void **p, size_t n, unsigned)
+{
+    FAKE_LOCK;
+    *p = malloc(n);                                      // (pages nobody touches cost nothing)
+    if (!*p) return cudaErrorUnknown;
+    fake::host[*p] = n;
+    fake::host_allocs++;
+    return cudaSuccess;
+}
+inline cudaError_t cudaMallocHost(void **p, size_t n) { return cudaHostAlloc(p, n, 0); }
+inline cudaError_t cudaFreeHost(void *p)
+{
+    FAKE_LOCK;
+    fake::host.erase(p);
+    free(p);
+    return cudaSuccess;
+}
+inline cudaError_t cudaMalloc(void **p, size_t n) { *p = malloc(n); return *p ? cudaSuccess : cudaErrorUnknown; }
+inline cudaError_t cudaFree(void *p) { free(p); return cudaSuccess; }
 inline cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned)
 {
     FAKE_LOCK;

@@ -43,6 +43,17 @@ def test_rules(host_rules, check):
     assert done.returncode == 0, done.stderr
 
 
+@pytest.fixture(scope="module")
+def host_pool(tmp_path_factory):
+    return _compiled(tmp_path_factory, "host_pool_check")
+
+
+@pytest.mark.parametrize("check", ["old sizes make room", "random use"])
+def test_result_memory(host_pool, check):
+    done = subprocess.run([host_pool, check], capture_output=True, text=True, timeout=20)
+    assert done.returncode == 0, done.stderr
+
+
 def test_no_result_memory_is_an_answer():
     """More than there is, up to what no class could hold: NULL at once."""
     from lmz_b200 import build
