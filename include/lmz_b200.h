@@ -341,6 +341,8 @@ typedef struct lmz_decode_plan {
  * plaintext once.  Asynchronous on cuda_stream; the caller reads d_any_bad and
  * the status arrays after synchronising. */
 int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *plan, void *cuda_stream);
+/* How many kernels this thread's last lmz_gpu_decode_chunks_dev launched. */
+unsigned lmz_gpu_plan_launches(void);
 
 #ifdef __cplusplus
 }

@@ -41,6 +41,7 @@ def bind(lib) -> None:
             ("lmz_host_gather", _int, [_int, _v, _u64, _v, ctypes.c_size_t, _uns, _v]),
             ("lmz_host_map_file", _v, [_int, _u64, _u64]),
             ("lmz_host_unmap_file", _int, [_v, _u64]),
+            ("lmz_gpu_plan_launches", _uns, []),
             ("lmz_host_plan_head_bytes", _int, []),
             ("lmz_host_plan", _int, [_v, _v, ctypes.c_size_t, _v, _v, _int, _uns] + [_v] * 8)):
         fn = getattr(lib, name)

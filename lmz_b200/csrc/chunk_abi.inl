@@ -41,6 +41,7 @@ static int launch_finish(const FinishArgs &fa, int sms, cudaStream_t cs)
     unsigned n = (fa.piece_end - fa.piece_begin + SUBS - 1) / SUBS;
     unsigned grid = n < (unsigned)sms ? n : (unsigned)sms;
     k_finish<SUBS><<<grid, FINISH_THREADS * SUBS, shm, cs>>>(fa);
+    g_launches++;
     cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) return fail_cuda("launch k_finish", le);
     return LMZ_GPU_OK;
@@ -59,6 +60,7 @@ static int launch_cond_finish(const FinishArgs &fa, int sms, cudaStream_t cs)
     unsigned n = (fa.piece_end - fa.piece_begin + CF_SUBS - 1) / CF_SUBS;
     unsigned grid = n < (unsigned)sms ? n : (unsigned)sms;
     k_cond_finish<<<grid, CF_THREADS, shm, cs>>>(fa);
+    g_launches++;
     cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) return fail_cuda("launch k_cond_finish", le);
     return LMZ_GPU_OK;
@@ -177,6 +179,7 @@ static int launch_two_plane(const lmz_decode_plan *p, uint32_t first, uint32_t c
     StreamArgs ca = da;
     ca.njobs = count;
     k_classify<<<(count + 7) / 8, 256, 0, cs>>>(ca, F_SMALL_LIVE, order, counts);
+    g_launches++;
     cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) return fail_cuda("launch k_classify", le);
     da.order = order;
@@ -200,6 +203,7 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
     rc = sm_count(&sms);
     if (rc) return rc;
 
+    g_launches = 0;
     // `phases` selects parts of the sequence (for timing one kernel alone); 0 runs it all.
     const uint32_t ph = p->phases ? p->phases : 0x1fu;
 
@@ -278,6 +282,7 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
                     if (rc) return rc;
                 } else if (sa.njobs) {
                     k_classify<<<(sa.njobs + 7) / 8, 256, 0, fs>>>(sa, F_SMALL_LIVE, order, counts);
+                    g_launches++;
                     cudaError_t le = cudaGetLastError();
                     if (le != cudaSuccess) return fail_cuda("launch k_classify", le);
                     sa.order = order;
@@ -378,7 +383,9 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
         c.scratch = (const uint8_t *)p->d_scratch;
         CK("memset hist", cudaMemsetAsync(p->d_hist, 0, (size_t)p->n_cond * 1024, cs));
         k_cond_hist<<<p->n_cond_pieces, 256, 0, cs>>>(c);
+        g_launches++;
         k_cond_plan<<<(p->n_cond + 63) / 64, 64, 0, cs>>>(c);
+        g_launches++;
         RansArgs a{};
         a.src = (const uint8_t *)p->d_payload;
         a.jobs = (const StreamJob *)p->d_seg_jobs;
@@ -400,7 +407,9 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
             ks = aux->stream;
         }
         k_cond_count<<<p->n_cond_pieces, 256, 0, ks>>>(c);
+        g_launches++;
         k_cond_scan<<<(p->n_cond * 8 + 127) / 128, 128, 0, ks>>>(c.chunks, c.cond_jobs, c.ncond, c.piece_cnt);
+        g_launches++;
         cudaError_t le = cudaGetLastError();
         if (le != cudaSuccess) return fail_cuda("launch cond kernels", le);
         rc = launch_rans(a, cs);
@@ -455,8 +464,11 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
         k.chunk_crc = (uint32_t *)p->d_chunk_crc;
         k.any_bad = (uint32_t *)p->d_any_bad;
         k_crc_check<<<(p->n_chunks + 127) / 128, 128, 0, cs>>>(k);
+        g_launches++;
         cudaError_t le = cudaGetLastError();
         if (le != cudaSuccess) return fail_cuda("launch k_crc_check", le);
     }
     return LMZ_GPU_OK;
 }
+
+API unsigned lmz_gpu_plan_launches(void) { return g_launches; }

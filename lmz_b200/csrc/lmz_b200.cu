@@ -75,6 +75,9 @@ static int stream_smem_ok()
 
 static int sm_count(int *out);
 
+// Kernels this thread has launched for the plan it was last given (lmz_gpu_plan_launches).
+static thread_local unsigned g_launches;
+
 template <int SINK, bool CRC, int CFN, int MODE>
 static int launch_stream_as(const StreamArgs &a, uint32_t grid, uint32_t W, cudaStream_t cs)
 {
@@ -83,6 +86,7 @@ static int launch_stream_as(const StreamArgs &a, uint32_t grid, uint32_t W, cuda
     int rc = opt_in_smem(k_stream<SINK, CRC, CFN, MODE>, F_SMEM_DYN, done);
     if (rc) return rc;
     k_stream<SINK, CRC, CFN, MODE><<<grid, W * 32, shm, cs>>>(a);
+    g_launches++;
     cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) return fail_cuda("launch k_stream", le);
     return LMZ_GPU_OK;
@@ -212,6 +216,7 @@ static int launch_compact_sorted(const RansArgs &a, cudaStream_t cs)
     do {
         if (cudaMemsetAsync(counts, 0, 8, cs) != cudaSuccess) { rc = fail_msg(LMZ_GPU_ECUDA, "cudaMemsetAsync failed"); break; }
         k_classify<<<(a.njobs + 7) / 8, 256, 0, cs>>>(sa, F_SMALL_LIVE, order, counts);
+        g_launches++;
         cudaError_t le = cudaGetLastError();
         if (le != cudaSuccess) { rc = fail_cuda("launch k_classify", le); break; }
         sa.order = order;

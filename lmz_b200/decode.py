@@ -220,22 +220,7 @@ class ArchiveDecoder:
         for i in range(6):
             c.piece_split[i] = int(p.piece_split[i])
         self._c = c
-        # kernels launched by one run(): stream decode; histogram, bucket map, counting, running
-        # totals and the segment decode of conditioned chunks; up to four finish launches; the
-        # verdict kernel
-        nbf = p.n_fused - p.n_fused_f32
-        # (few enough streams for wide tables: one launch, nothing counted or sorted)
-        few = (8 if checksum else 12) * torch.cuda.get_device_properties(d).multi_processor_count
-        if p.device_classify:                # per group: the count kernel and both instances
-            fused_launches = (0 if not nbf else 1 if nbf <= few else 3) + (3 if p.n_fused_f32 else 0)
-        else:
-            fused_launches = (1 if p.n_fused_small else 0) + (1 if nbf > p.n_fused_small else 0) + \
-                (1 if p.n_fused_f32_small else 0) + (1 if p.n_fused_f32 > p.n_fused_f32_small else 0)
-        fused_launches += (1 if p.n_fused_t else 0) + sum(0 if not n else 1 if 2 * n <= few else 3 for n in (
-            p.n_delta_plain, p.delta_jobs.size - p.n_delta_plain))
-        self.launches_per_run = (1 if p.stream_jobs.size else 0) + \
-            ((4 + (1 if p.seg_jobs.size else 0)) if ncond else 0) + fused_launches + \
-            int(sum(p.piece_split[i + 1] > p.piece_split[i] for i in (0, 1, 3, 4))) + 1
+        self.launches_per_run = 0            # kernels launched by one run(); known after the first
 
     def upload(self, pinned=None, non_blocking: bool = False):
         """Copy the archive's payload region host -> device (from `pinned`, a host
@@ -271,6 +256,8 @@ class ArchiveDecoder:
             rc = self.lib.lmz_gpu_decode_chunks_dev(ctypes.byref(self._c), s.cuda_stream)
         if rc != gpu.OK:
             raise RuntimeError(f"decode launch failed ({rc}): {gpu.last_error()}")
+        if not self.launches_per_run and not phases:
+            self.launches_per_run = self.lib.lmz_gpu_plan_launches()
         return self.output
 
     @property
@@ -364,7 +351,10 @@ class PipelinedDecoder:
         self.d_out = out
         self.copy_stream = torch.cuda.Stream(self.device)
         self.h2d_bytes = sum(hi - lo for lo, hi in self.ranges)
-        self.launches_per_run = sum(s.launches_per_run for s in self.slices)
+
+    @property
+    def launches_per_run(self) -> int:
+        return sum(s.launches_per_run for s in self.slices)
 
     def run_from_host(self, pinned, stream=None):
         """`pinned`: a pinned uint8 host tensor over the archive's bytes (offset 0 =

@@ -618,3 +618,54 @@ def test_a_plan_of_another_mapping_of_the_file(shard, tmp_path):
         dec.check()
         assert (dec.output.cpu().numpy() == shard).all()
         dec.upload()
+
+
+@pytest.mark.parametrize("what", ["shard", "shard, mapped", "many plain two-plane chunks beside fused ones", "f32", "deltas"])
+@pytest.mark.parametrize("checksum", [True, False])
+def test_launches_are_counted_as_they_happen(gpu, shard, what, checksum):
+    """`launches_per_run` against the kernel nodes of the same run captured into a graph, and the graph's output
+    against the source."""
+    import torch
+    from cuda.bindings import runtime
+    from lmz_b200 import archive, decode, plan
+    if what.startswith("shard"):
+        src = shard
+        blob = oa.write_archive([("m.safetensors", src)], mapped="mapped" in what)
+    elif what == "f32":
+        rng = np.random.default_rng(4)
+        src = synth.safetensors_bytes([("w", "F32", (300_000,), (rng.standard_normal(300_000) * 0.02).astype("<f4").view(np.uint8))])
+        blob = oa.write_archive([("m.safetensors", src)], mapped=True)
+    elif what == "deltas":
+        first = synth.normal_bf16((600_000,), 1)
+        files = [synth.safetensors_bytes([("w", "BF16", (600_000,), d)]) for d in (first, synth.perturbed_bf16(first, 2))]
+        src = np.concatenate(files)
+        blob = oa.write_archive([(f"{i}.safetensors", f) for i, f in enumerate(files)], mapped=True)
+    else:                                        # 40 of them, 16 to a CTA: more than those CTAs have wide tables for
+        n = 40 * 32768
+        src = synth.safetensors_bytes([("n", "BF16", (n,), np.repeat(synth.normal_bf16((n // 64,), 5).view("<u2"), 64).view(np.uint8)),
+                                       ("w", "BF16", (n,), synth.normal_bf16((n,), 6))])
+        blob = oa.write_archive([("m.safetensors", src)], mapped=True)
+    ar = archive.Archive(blob)
+    dec = decode.ArchiveDecoder(ar, checksum=checksum, plan=plan.build_plan(ar, fuse="all"))
+    if what.startswith("many"):
+        assert dec.plan.n_delta_plain > 32 and dec.plan.n_fused
+    dec.run()
+    dec.check()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        dec.run(stream=torch.cuda.current_stream())
+
+    def ok(answer):
+        assert int(answer[0]) == 0
+        return answer[1:] if len(answer) > 2 else answer[1]
+
+    raw = runtime.cudaGraph_t(graph.raw_cuda_graph())
+    count = ok(runtime.cudaGraphGetNodes(raw))[-1]
+    nodes = ok(runtime.cudaGraphGetNodes(raw, count))[0]
+    kernels = sum(ok(runtime.cudaGraphNodeGetType(nd)) == runtime.cudaGraphNodeType.cudaGraphNodeTypeKernel for nd in nodes[:count])
+    assert kernels == dec.launches_per_run > 0
+    dec.d_out.zero_()
+    graph.replay()
+    dec.check()
+    assert (dec.output.cpu().numpy() == src).all()
+    del graph
