@@ -268,3 +268,29 @@ def test_a_refused_batch_leaves_out_alone(gpu, orc, nstr, plane, table_mode):
         assert bytes(got) == bytes(out) == b"".join(p.tobytes() for p in others)
         if not isinstance(out, bytearray):
             assert gpu.decode_batch(blob, offs, nstr, plane, out=out[1:]) is not None       # too short: memory of its own
+
+
+@pytest.mark.parametrize("nstr", [148 * 76 + 1, 13024, 28577])
+@pytest.mark.parametrize("wide", ["none", "every seventh", "all"])
+def test_device_batches_sorted_by_alphabet(gpu, orc, nstr, wide, table_mode):
+    """More streams in one launch than full-size tables have room for (the counts are those of 148 SMs): alphabets
+    are counted on the device and each class gets its instance, one of them for none or for all.  A host
+    batch of this size may run in slices that are each below the line."""
+    if table_mode != -1:
+        pytest.skip("sorted only where the library chooses")
+    import torch
+    plane = 331
+    every = {"none": 0, "every seventh": 7, "all": 1}[wide]
+    pool = [distribution("uniform" if every and i % every == 0 else "exponent", plane, 40 + i) for i in range(70)]
+    streams = [orc.rans_encode(p) for p in pool]
+    live = [len(np.unique(p)) for p in pool]
+    assert max(live) > 104 if every else max(live) <= 104
+    blob, offs = pack_streams([streams[i % 70] for i in range(nstr)])
+    t = torch.frombuffer(bytearray(blob), dtype=torch.uint8).cuda()
+    want = torch.from_numpy(np.stack(pool)).cuda()[torch.arange(nstr, device="cuda") % 70].reshape(-1)
+    assert torch.equal(gpu.decode_batch(t, offs, nstr, plane), want)
+    for at in (0, nstr // 2, nstr - 1):                   # one stream's last word is missing
+        bad = np.frombuffer(offs, dtype="<u8").copy()
+        bad[2 * at + 1] -= 2
+        with pytest.raises(ValueError):
+            gpu.decode_batch(t, bad.tobytes(), nstr, plane)

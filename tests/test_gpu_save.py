@@ -68,3 +68,28 @@ def test_two_members_and_what_the_writer_declines(gpu, tmp_path):
         save.save_archive(path, [("f.safetensors", torch.from_numpy(f32).cuda())])
     with pytest.raises(ValueError, match="chunk_size"):
         save.save_archive(path, [("a.safetensors", torch.from_numpy(a).cuda())], chunk_size=8 << 20)
+
+
+@pytest.mark.parametrize("before", ["a longer archive", "a shorter one", "other bytes"])
+def test_over_what_was_there(gpu, tmp_path, before):
+    """A save over an existing file leaves the file that a save to a new one does; one that fails leaves it empty."""
+    import torch
+    from lmz_b200 import archive, decode, save
+    a = synth.llama_shard([0], 5, scale=0.25, vocab=2000, embed=True)
+    b = synth.llama_shard([1], 6, scale=0.125)
+    small, large = (("b.safetensors", b), ("a.safetensors", a))
+    old, new = (large, small) if before == "a longer archive" else (small, large)
+    path, fresh = tmp_path / "over.lmz", tmp_path / "fresh.lmz"
+    if before == "other bytes":
+        path.write_bytes(bytes(range(256)) * 40000)
+    else:
+        save.save_archive(str(path), [(old[0], torch.from_numpy(old[1].copy()).cuda())])
+    member = [(new[0], torch.from_numpy(new[1].copy()).cuda())]
+    assert save.save_archive(str(path), member) == save.save_archive(str(fresh), member) == path.stat().st_size
+    assert path.read_bytes() == fresh.read_bytes()
+    assert (decode.load_archive(str(path)).cpu().numpy() == new[1]).all()
+    with pytest.raises(ValueError):
+        save.save_archive(str(path), member + [("c", torch.zeros(100, device="cuda"))])
+    assert path.stat().st_size == 0
+    with pytest.raises(ValueError):                       # (nothing to map)
+        archive.Archive(str(path))
