@@ -118,9 +118,9 @@ typedef struct lmz_stream_job {
 
 /* Generalises lmz_gpu_decode_batch_dev (lmz/gpu/lmzgpu.cu:412-467) to streams
  * of unequal decoded length written to arbitrary offsets.  d_status (njobs
- * uint32, may be NULL) receives 0, or 1 bad header, 2 truncated, 3 input
- * timeout, 0x100 decoded but with trailing slack; *d_any_bad (uint32, may be
- * NULL, caller zeroes it) is set when any status is 1..3.  Asynchronous. */
+ * uint32, may be NULL) receives 0, or 1 bad header, 2 truncated, 0x100 decoded
+ * but with trailing slack; *d_any_bad (uint32, may be NULL, caller zeroes it) is
+ * set when any status is 1 or 2.  Asynchronous. */
 int lmz_gpu_decode_streams_dev(const void *d_jobs, unsigned njobs, const void *d_src,
                                void *d_dst, const void *d_shared_hdr, void *d_status,
                                void *d_any_bad, void *cuda_stream);
@@ -133,11 +133,10 @@ int lmz_gpu_decode_streams_dev(const void *d_jobs, unsigned njobs, const void *d
  * loads it, held until the process exits); nothing is allocated or freed here.
  *
  * Arguments as lmz_gpu_decode_batch_dev (no tpb).  h_status is host memory for nstr
- * uint32 verdicts (0 ok, 1 bad header, 2 truncated, 3 input timeout, 0x100 trailing
- * slack) or NULL.  The call is synchronous -- it waits for cuda_stream and copies the
- * verdicts to the host before it returns -- and returns LMZ_GPU_EBADSTREAM if
- * any stream failed, LMZ_GPU_EUNSUPPORTED if nstr exceeds the maximum (split the
- * batch).  The first call on each device looks up the array's device address; make
+ * uint32 verdicts (0 ok, 1 bad header, 2 truncated, 0x100 trailing slack) or NULL.
+ * The call is synchronous -- it waits for cuda_stream and copies the verdicts to the
+ * host before it returns -- and returns LMZ_GPU_EBADSTREAM if any stream failed,
+ * LMZ_GPU_EUNSUPPORTED if nstr exceeds the maximum (split the batch).  The first call on each device looks up the array's device address; make
  * that call before starting any stream capture.  All calls on a device share the
  * array: calls that overlap on the GPU race on it, so issue them one at a time. */
 #define LMZ_GPU_NOALLOC_MAX_STREAMS 65536u

@@ -23,7 +23,7 @@ constexpr uint32_t PAD_BYTES = 576;   // readable slack owed after the last stre
 constexpr uint32_t ST_OK = 0;
 constexpr uint32_t ST_BAD_HEADER = 1;   // magic, frequency sum or minimum length
 constexpr uint32_t ST_OVERRUN = 2;      // a refill was needed past the stream's end
-                                        // (3 was an input copy that never landed; no kernel waits on one any more)
+                                        // (3 is the reference's input timeout; no kernel here waits for a copy)
 constexpr uint32_t ST_BAD_SHAPE = 4;    // lengths in a payload disagree with the record
 constexpr uint32_t ST_BAD_CRC = 5;      // decoded chunk does not match the record's crc32
 constexpr uint32_t ST_SLACK = 0x100;    // soft: final states != 2^16 or cursor != length
@@ -71,12 +71,6 @@ __device__ __forceinline__ uint32_t lds_u8(uint32_t a)
     asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a));
     return v;
 }
-__device__ __forceinline__ uint32_t lds_u8_1(uint32_t a)
-{
-    uint32_t v;
-    asm volatile("ld.shared.u8 %0, [%1+1];" : "=r"(v) : "r"(a));
-    return v;
-}
 __device__ __forceinline__ void sts_u8(uint32_t a, uint32_t v)
 {
     asm volatile("st.shared.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory");
@@ -93,10 +87,6 @@ __device__ __forceinline__ uint32_t lds_u16(uint32_t a)
     uint32_t v;
     asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(a));
     return v;
-}
-__device__ __forceinline__ void sts_u16(uint32_t a, uint32_t v)
-{
-    asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
 __device__ __forceinline__ void sts_u32(uint32_t a, uint32_t v)
 {

@@ -200,8 +200,8 @@ __device__ __forceinline__ uint32_t ref_addr(uint32_t ref, uint32_t cf_sa) { ret
 // long ago they were requested, so where warps are few every load in flight is a stall (one B200, 12
 // streams per SM: a third of the time; bulk copies through a raw ring cost as much as they saved).
 // TR_FEW has the L2 fetch words 512 bytes ahead, and the stored bytes that a sink merges four tiles
-// ahead.  On one B200: a 4096 x 14336 BF16 tensor's kernel 583 -> 456 us, the delta kernel of a
-// three-checkpoint chain 1190 -> 1070 us.
+// ahead.  On one B200: a 4096 x 14336 BF16 tensor's kernel 581 -> 458 us, the delta kernel of a
+// three-checkpoint chain 1189 -> 1083 us.
 template <int CFN, int MODE>
 struct Words {
     static constexpr bool TR8 = MODE != TR_4;
@@ -941,26 +941,20 @@ __global__ void k_classify(StreamArgs a, uint32_t small_live, uint32_t *order, u
     if (job >= a.njobs) return;
     // (delta jobs: njobs counts chunks here, and the first plane's alphabet decides: the instance for
     // small ones gives the second plane a full-size table)
-    uint32_t live = 0;
-    for (uint32_t plane = 0; plane < 1u; plane++) {
-        uint64_t soff;
-        uint32_t slen;
-        if (a.djobs) { soff = plane ? a.djobs[job].src_b : a.djobs[job].src_a; slen = plane ? a.djobs[job].len_b : a.djobs[job].len_a; }
-        else if (a.jobs) { soff = a.jobs[job].src_off; slen = a.jobs[job].src_len; }
-        else if (a.sjobs) { soff = a.sjobs[job].src_off; slen = a.sjobs[job].src_len; }
-        else { soff = a.offs[2 * job]; slen = (uint32_t)a.offs[2 * job + 1]; }
-        uint32_t mine = 0;
-        if (slen >= HDR_BYTES + STATE_BYTES) {
-            // this lane's eight frequencies: 16 bytes at any alignment, as aligned words
-            uint32_t w[4];
-            load_words_nc<4>(a.src + soff + 4 + 16 * lane, w);
+    uint64_t soff;
+    uint32_t slen;
+    if (a.djobs) { soff = a.djobs[job].src_a; slen = a.djobs[job].len_a; }
+    else if (a.jobs) { soff = a.jobs[job].src_off; slen = a.jobs[job].src_len; }
+    else if (a.sjobs) { soff = a.sjobs[job].src_off; slen = a.sjobs[job].src_len; }
+    else { soff = a.offs[2 * job]; slen = (uint32_t)a.offs[2 * job + 1]; }
+    uint32_t live = 257;                               // too short: the large instance reports it
+    if (slen >= HDR_BYTES + STATE_BYTES) {
+        // this lane's eight frequencies: 16 bytes at any alignment, as aligned words
+        uint32_t w[4], mine = 0;
+        load_words_nc<4>(a.src + soff + 4 + 16 * lane, w);
 #pragma unroll
-            for (int i = 0; i < 4; i++) mine += ((w[i] & 0xffffu) != 0) + ((w[i] >> 16) != 0);
-            mine = __reduce_add_sync(0xffffffffu, mine);
-        } else {
-            mine = 257;                                // too short: the large instance reports it
-        }
-        live = max(live, mine);
+        for (int i = 0; i < 4; i++) mine += ((w[i] & 0xffffu) != 0) + ((w[i] >> 16) != 0);
+        live = __reduce_add_sync(0xffffffffu, mine);
     }
     if (lane == 0) {
         const bool small = live <= small_live;

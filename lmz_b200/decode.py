@@ -16,7 +16,7 @@ import numpy as np
 from . import _chunks, archive as fmt, gpu, plan as planner
 from .archive import CorruptArchive
 
-_ST_NAMES = {1: "bad stream header", 2: "truncated stream", 3: "input copy timed out",
+_ST_NAMES = {1: "bad stream header", 2: "truncated stream",
              4: "lengths disagree with the record", 5: "checksum mismatch"}
 
 _TORCH_DTYPES = {"BF16": "bfloat16", "F16": "float16", "F32": "float32", "F64": "float64",
@@ -94,12 +94,9 @@ def _crc_tables(lib, device):
     return _tables[key]
 
 
-_layouts_of = set()
-
-
 def _check_layouts(lib):
-    """The library's job layouts are the planner's (asked once)."""
-    if id(lib) in _layouts_of:
+    """The library's job layouts are the planner's (asked once of each)."""
+    if getattr(lib, "layouts_checked", False):
         return
     sizes = (ctypes.c_uint * 5)()
     lib.lmz_gpu_struct_sizes(ctypes.byref(sizes))
@@ -109,7 +106,7 @@ def _check_layouts(lib):
             lib.lmz_gpu_shared_group() != planner.T_GROUP or \
             lib.lmz_gpu_delta_job_bytes() != planner.DELTA_JOB.itemsize:
         raise RuntimeError("the CUDA library and the planner disagree on job layouts")
-    _layouts_of.add(id(lib))
+    lib.layouts_checked = True
 
 
 def _payload_source(ar, plan):

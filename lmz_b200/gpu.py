@@ -24,7 +24,7 @@ import sys
 import threading
 
 __all__ = ["available", "backend", "decode_batch", "grain", "header_bytes",
-           "last_error", "pad_bytes", "state", "verify"]
+           "last_error", "pad_bytes", "state", "trim", "verify"]
 
 ABI_VERSION = 1                      # lmz/gpu/__init__.py:31
 OK, ENODEV, EUNSUPPORTED, EBADSTREAM, ECUDA, EMISMATCH = 0, -1, -2, -3, -4, -5
@@ -251,6 +251,14 @@ def grain() -> int:
 def header_bytes() -> int:
     lib = _loader.get()
     return lib.lmz_gpu_header_bytes() if lib is not None else 516
+
+
+def trim() -> None:
+    """Give back the memory that host calls keep for the next one (csrc/host_pool.inl says how much that may
+    be).  Never probes: a library that is not loaded keeps nothing."""
+    lib = loaded_library()
+    if lib is not None:
+        lib.lmz_gpu_trim()
 
 
 def pad_bytes() -> int:

@@ -169,7 +169,7 @@ def test_results_in_lent_memory_stay_their_callers_own(gpu, orc, nstr, plane, ta
     assert [bytes(h) for h in held] == [sets[0][1], sets[1][1]]
     part = held[0][:1]
     del held
-    gpu.library().lmz_gpu_trim()
+    gpu.trim()
     gpu.decode_batch(*sets[2][0], nstr, plane)
     assert bytes(part) == sets[0][1][:1]
 
