@@ -479,7 +479,7 @@ def _upload_cuts(table_off: int, nslices):
     the other: as many as asked for, or one per 192 MiB, at most eight.  (A range is decoded
     under the upload of the next, but a decode has a smallest duration, that of one stream.)"""
     n = nslices if nslices is not None else min(8, -(-table_off // (192 << 20)))
-    n = max(1, min(int(n), max(1, table_off)))
+    n = max(1, min(int(n), table_off >> 16))             # (of 64 KiB at least: a range has an event and a wait of its own)
     return [table_off * i // n for i in range(n + 1)]
 
 

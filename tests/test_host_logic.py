@@ -471,3 +471,14 @@ def test_native_planner_declines_what_it_has_no_memory_for(lib_path):
             "print(f(None, None, 1 << 60, r, None, 1, 0, *[None] * 8))")
     out = subprocess.run([sys.executable, "-c", code, lib_path], capture_output=True, text=True)
     assert out.stdout.strip() == "1", out.stderr
+
+
+@pytest.mark.parametrize("size", [24, 65535, 65536, 200_000, 10 << 20, 3 << 30])
+@pytest.mark.parametrize("nslices", [None, 0, 1, 5, 8, 10**6])
+def test_uploads_are_cut_into_ranges_worth_having(size, nslices):
+    from lmz_b200 import decode
+    cuts = decode._upload_cuts(size, nslices)
+    assert cuts[0] == 0 and cuts[-1] == size and len(cuts) <= max(8, size // 65536) + 1
+    assert len(cuts) == 2 or min(b - a for a, b in zip(cuts, cuts[1:])) >= 65536
+    if nslices and nslices <= size >> 16:
+        assert len(cuts) == nslices + 1
