@@ -92,7 +92,8 @@ __device__ __forceinline__ void load_words_nc(const uint8_t *p, uint32_t (&w)[N]
     uint32_t sh = (uint32_t)(a & 3u) * 8u;
     uint32_t v[N + 1];
 #pragma unroll
-    for (int i = 0; i <= N; i++) v[i] = __ldg(q + i);
+    for (int i = 0; i < N; i++) v[i] = __ldg(q + i);
+    v[N] = sh ? __ldg(q + N) : 0u;                 // (an aligned read ends where its words do: a buffer may end its mapping there)
 #pragma unroll
     for (int i = 0; i < N; i++) w[i] = __funnelshift_r(v[i], v[i + 1], sh);
 }

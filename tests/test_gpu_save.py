@@ -93,3 +93,23 @@ def test_over_what_was_there(gpu, tmp_path, before):
     assert path.stat().st_size == 0
     with pytest.raises(ValueError):                       # (nothing to map)
         archive.Archive(str(path))
+
+
+@pytest.mark.parametrize("mib", [20, 22])
+def test_checksums_of_a_tensor_that_ends_where_its_memory_does(gpu, mib):
+    """A tensor of whole 2 MiB pages fills an allocation of its own to the last byte: the checksum
+    kernel reads no further."""
+    import ctypes
+    import zlib
+    import torch
+    from lmz_b200 import decode
+    lib = gpu.library()
+    torch.cuda.empty_cache()
+    data = torch.randint(0, 256, (mib << 20,), dtype=torch.uint8, device="cuda")
+    meta = torch.zeros((mib * 16, 4), dtype=torch.int32, device="cuda")
+    tabs = decode._crc_tables(lib, torch.device("cuda", torch.cuda.current_device()))
+    assert lib.lmz_gpu_crc32_chunks_dev(data.data_ptr(), data.numel(), 65536, tabs.data_ptr(), meta.data_ptr(),
+                                        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    got = meta[:, 3].cpu().numpy().view(np.uint32)
+    host = data.cpu().numpy().reshape(-1, 65536)
+    assert [int(v) for v in got] == [zlib.crc32(row) for row in host]
