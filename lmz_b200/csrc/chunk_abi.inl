@@ -172,7 +172,7 @@ static int launch_two_plane(const lmz_decode_plan *p, uint32_t first, uint32_t c
     const bool crc = p->d_piece_crc != nullptr;
     int sms = 0;
     if (int rc = sm_count(&sms)) return rc;
-    const uint32_t per = crc ? wide_per_sm<true>() : wide_per_sm<false>();
+    const uint32_t per = crc ? wide_per_sm<SINK_DELTA, true>() : wide_per_sm<SINK_DELTA, false>();
     if (da.njobs <= per * (most_ctas ? most_ctas : (uint32_t)sms))      // wide tables: nothing to sort by
         return crc ? launch_stream<SINK_DELTA, true, 256>(da, cs) : launch_stream<SINK_DELTA, false, 256>(da, cs);
     CK("memset two-plane counts", cudaMemsetAsync(counts, 0, 8, cs));
@@ -275,12 +275,12 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
                 sa.order = nullptr;
                 sa.count = nullptr;
                 const bool checked = p->d_piece_crc != nullptr;
-                if (solo_fits(sa, checked, sms)) {
-                    // few enough for a warp each: nothing to sort by
-                    if (grp == 0) rc = checked ? launch_solo<SINK_BF16, true>(sa, fs) : launch_solo<SINK_BF16, false>(sa, fs);
-                    else rc = checked ? launch_solo<SINK_F32, true>(sa, fs) : launch_solo<SINK_F32, false>(sa, fs);
+                const uint32_t per = checked ? wide_per_sm<SINK_BF16, true>() : wide_per_sm<SINK_BF16, false>();
+                if (grp == 0 && sa.njobs && sa.njobs <= per * (sa.most_ctas ? sa.most_ctas : (uint32_t)sms)) {
+                    // few enough for wide tables: nothing to sort by
+                    rc = checked ? launch_stream<SINK_BF16, true, 256>(sa, fs) : launch_stream<SINK_BF16, false, 256>(sa, fs);
                     if (rc) return rc;
-                } else {
+                } else if (sa.njobs) {
                     k_classify<<<(sa.njobs + 7) / 8, 256, 0, fs>>>(sa, F_SMALL_LIVE, order, counts);
                     g_launches++;
                     cudaError_t le = cudaGetLastError();
