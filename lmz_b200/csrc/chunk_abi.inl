@@ -172,7 +172,7 @@ static int launch_two_plane(const lmz_decode_plan *p, uint32_t first, uint32_t c
     const bool crc = p->d_piece_crc != nullptr;
     int sms = 0;
     if (int rc = sm_count(&sms)) return rc;
-    const uint32_t per = crc ? wide_per_sm<SINK_DELTA, true>() : wide_per_sm<SINK_DELTA, false>();
+    const uint32_t per = crc ? wide_per_sm<true>() : wide_per_sm<false>();
     if (da.njobs <= per * (most_ctas ? most_ctas : (uint32_t)sms))      // wide tables: nothing to sort by
         return crc ? launch_stream<SINK_DELTA, true, 256>(da, cs) : launch_stream<SINK_DELTA, false, 256>(da, cs);
     CK("memset two-plane counts", cudaMemsetAsync(counts, 0, 8, cs));
@@ -275,12 +275,12 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
                 sa.order = nullptr;
                 sa.count = nullptr;
                 const bool checked = p->d_piece_crc != nullptr;
-                const uint32_t per = checked ? wide_per_sm<SINK_BF16, true>() : wide_per_sm<SINK_BF16, false>();
-                if (grp == 0 && sa.njobs && sa.njobs <= per * (sa.most_ctas ? sa.most_ctas : (uint32_t)sms)) {
-                    // few enough for wide tables: nothing to sort by
-                    rc = checked ? launch_stream<SINK_BF16, true, 256>(sa, fs) : launch_stream<SINK_BF16, false, 256>(sa, fs);
+                if (solo_fits(sa, true, sms)) {
+                    // few enough for a warp each: nothing to sort by
+                    if (grp == 0) rc = checked ? launch_solo<SINK_BF16, true>(sa, fs) : launch_solo<SINK_BF16, false>(sa, fs);
+                    else rc = checked ? launch_solo<SINK_F32, true>(sa, fs) : launch_solo<SINK_F32, false>(sa, fs);
                     if (rc) return rc;
-                } else if (sa.njobs) {
+                } else {
                     k_classify<<<(sa.njobs + 7) / 8, 256, 0, fs>>>(sa, F_SMALL_LIVE, order, counts);
                     g_launches++;
                     cudaError_t le = cudaGetLastError();
@@ -306,22 +306,32 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
             }
             sa.njobs = 0;            // nothing is left for the host-sorted launches below
         } else {
-        sa.njobs = nsmall;
-        rc = p->d_piece_crc ? launch_stream<SINK_BF16, true, F_SMALL_CFN>(sa, fs)
-                            : launch_stream<SINK_BF16, false, F_SMALL_CFN>(sa, fs);
-        if (rc) return rc;
-        part(nbf - nsmall);
-        rc = p->d_piece_crc ? launch_stream<SINK_BF16, true, 256>(sa, fs)
-                            : launch_stream<SINK_BF16, false, 256>(sa, fs);
-        if (rc) return rc;
-        part(nsmall4);
-        rc = p->d_piece_crc ? launch_stream<SINK_F32, true, F_SMALL_CFN>(sa, fs)
-                            : launch_stream<SINK_F32, false, F_SMALL_CFN>(sa, fs);
-        if (rc) return rc;
-        part(p->n_fused_f32 - nsmall4);
-        rc = p->d_piece_crc ? launch_stream<SINK_F32, true, 256>(sa, fs)
-                            : launch_stream<SINK_F32, false, 256>(sa, fs);
-        if (rc) return rc;
+        // (counted by the host: each group's small ones come first)
+        const bool crc = p->d_piece_crc != nullptr;
+        sa.njobs = nbf;
+        if (solo_fits(sa, true, sms)) {
+            rc = crc ? launch_solo<SINK_BF16, true>(sa, fs) : launch_solo<SINK_BF16, false>(sa, fs);
+            if (rc) return rc;
+        } else {
+            sa.njobs = nsmall;
+            rc = crc ? launch_stream<SINK_BF16, true, F_SMALL_CFN>(sa, fs) : launch_stream<SINK_BF16, false, F_SMALL_CFN>(sa, fs);
+            if (rc) return rc;
+            part(nbf - nsmall);
+            rc = crc ? launch_stream<SINK_BF16, true, 256>(sa, fs) : launch_stream<SINK_BF16, false, 256>(sa, fs);
+            if (rc) return rc;
+        }
+        part(p->n_fused_f32);
+        if (solo_fits(sa, true, sms)) {
+            rc = crc ? launch_solo<SINK_F32, true>(sa, fs) : launch_solo<SINK_F32, false>(sa, fs);
+            if (rc) return rc;
+        } else {
+            sa.njobs = nsmall4;
+            rc = crc ? launch_stream<SINK_F32, true, F_SMALL_CFN>(sa, fs) : launch_stream<SINK_F32, false, F_SMALL_CFN>(sa, fs);
+            if (rc) return rc;
+            part(p->n_fused_f32 - nsmall4);
+            rc = crc ? launch_stream<SINK_F32, true, 256>(sa, fs) : launch_stream<SINK_F32, false, 256>(sa, fs);
+            if (rc) return rc;
+        }
         }
         if (p->n_fused_t) {
             // chunks of a shared-table archive: every CTA takes one table's next 80 of them

@@ -51,6 +51,9 @@ struct CrcTables {
     uint32_t mul_gap1984[4][256]; // multiply a state by x^(8 * 1984): from the end of a lane's 64 bytes of one
                                   // 2 KiB warp block to the start of its 64 bytes of the next (k_cond_finish)
     uint32_t lane_mul64[32];      // x^(8 * 64 * (31 - l)): the end of lane l's 64 bytes to the end of the block
+    uint32_t mul_row1024[4][256]; // multiply a state by x^(8 * 1024), one warp's row of BF16 (k_solo)
+    uint32_t mul_row2048[4][256]; // and by x^(8 * 2048), its row of 4-byte elements
+    uint32_t word_pow[513];       // x^(32 * m): the m-th last word of a row to the row's end (k_solo)
 };
 
 // Rows of the piece layout: 256 threads x 16 bytes.
@@ -127,6 +130,13 @@ inline void crc_build_tables(CrcTables &t)
     for (int j = 0; j < 4; j++)
         for (uint32_t i = 0; i < 256; i++) t.mul_gap1984[j][i] = crc_mulmod(gap, i << (8 * j));
     for (uint32_t l = 0; l < 32; l++) t.lane_mul64[l] = crc_xpow(t.x2, 8ull * 64 * (31 - l));
+    const uint32_t row1024 = crc_xpow(t.x2, 8ull * 1024), row2048 = crc_xpow(t.x2, 8ull * 2048);
+    for (int j = 0; j < 4; j++)
+        for (uint32_t i = 0; i < 256; i++) {
+            t.mul_row1024[j][i] = crc_mulmod(row1024, i << (8 * j));
+            t.mul_row2048[j][i] = crc_mulmod(row2048, i << (8 * j));
+        }
+    for (uint32_t m = 0; m < 513; m++) t.word_pow[m] = crc_xpow(t.x2, 32ull * m);
 }
 
 // Feed one little-endian 32-bit word: four table lookups.

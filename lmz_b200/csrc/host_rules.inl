@@ -25,9 +25,9 @@ constexpr unsigned MOST_SLICES = 8;
 constexpr size_t SLICE_BYTES = (size_t)4 << 20;
 
 // How many slices, for `nstr` streams and `bytes` in and out.  A slice takes as long as one of its streams,
-// plane / 8 steps of some 64 ns, however few they are.  Where the slices fit on the device beside each
-// other they share that time (each is a launch of its own, of one-warp CTAs with wide tables: 80 KiB, two to an
-// SM); else they take it in turn, and it must hide under the copies: a slice's plaintext takes plane * streams /
+// plane / 8 steps of some 41 ns, however few they are.  Where the slices fit on the device beside each
+// other they share that time (each is a launch of its own, of CTAs of a warp or two with 34 KiB of tables a warp: six
+// warps to an SM, and a slice that finds no room starts a copy or two later than one that does); else they take it in turn, and it must hide under the copies: a slice's plaintext takes plane * streams /
 // 50 GB/s to come out, its chain plane * 8 ns, so 400 streams and more.  (With four slices at a time, by bytes
 // alone: 16 planes of 4 Mi symbols 66.9 ms, two chains; as here 35.1, in one piece 36.4.)
 unsigned batch_slices(uint64_t bytes, unsigned nstr, unsigned sms)

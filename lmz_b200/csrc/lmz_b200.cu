@@ -18,6 +18,7 @@
 #include "chunk_kernels.cuh"
 #include "cond_kernels.cuh"
 #include "fused_kernel.cuh"
+#include "solo_kernel.cuh"
 #include "encode_kernel.cuh"
 #include "save_kernels.cuh"
 
@@ -92,9 +93,47 @@ static int launch_stream_as(const StreamArgs &a, uint32_t grid, uint32_t W, cuda
     return LMZ_GPU_OK;
 }
 
-// Streams per SM that a sink's wide-table instance takes in one round.
+// Streams per SM that the delta sink's wide-table instance takes in one round.
+template <bool CRC>
+constexpr uint32_t wide_per_sm() { return 4 * stream_warps(0, CRC, SINK_DELTA, TR_FEW); }
+
+template <int SINK, bool CRC, bool WIDE>
+static int launch_solo_as(const StreamArgs &a, uint32_t grid, uint32_t W, cudaStream_t cs)
+{
+    static bool done[64];
+    int rc = opt_in_smem(k_solo<SINK, CRC, WIDE>, F_SMEM_DYN, done);
+    if (rc) return rc;
+    k_solo<SINK, CRC, WIDE><<<grid, W * 32, solo_smem(CRC, WIDE, W).end - F_SMEM_BASE, cs>>>(a);
+    g_launches++;
+    cudaError_t le = cudaGetLastError();
+    if (le != cudaSuccess) return fail_cuda("launch k_solo", le);
+    return LMZ_GPU_OK;
+}
+
+// A warp per stream, whatever the alphabets.
 template <int SINK, bool CRC>
-constexpr uint32_t wide_per_sm() { return 4 * stream_warps(0, CRC, SINK, TR_FEW); }
+static int launch_solo(const StreamArgs &a, cudaStream_t cs)
+{
+    if (a.njobs == 0) return LMZ_GPU_OK;
+    int rc = stream_smem_ok();
+    if (rc) return rc;
+    int sms = 0;
+    rc = sm_count(&sms);
+    if (rc) return rc;
+    // at most one CTA per SM, its warps just enough for as many rounds as the fullest would need
+    const uint32_t room = a.most_ctas ? a.most_ctas : (uint32_t)sms, grid = a.njobs < room ? a.njobs : room;
+    const uint32_t per = (a.njobs + grid - 1) / grid;
+    if (per <= solo_warps(CRC, true)) return launch_solo_as<SINK, CRC, true>(a, grid, per, cs);
+    const uint32_t rounds = (per + solo_warps(CRC, false) - 1) / solo_warps(CRC, false);
+    return launch_solo_as<SINK, CRC, false>(a, grid, (per + rounds - 1) / rounds, cs);
+}
+// Up to so many streams per SM a warp each is faster than four to a warp.  (One B200, exponent planes of 32 KiB:
+// 4 per SM 183 against 281 us, 12 262 against 282, 20 345 against 382, 28 449 against 385.  With the sinks' own work
+// in the same issue slots: 12 64 KiB BF16 chunks with checksums per SM 395 against 489 us, 18 as long either way.)
+static bool solo_fits(const StreamArgs &a, bool sink, int sms)
+{
+    return a.njobs <= (sink ? 16ull : 20ull) * (a.most_ctas ? a.most_ctas : (uint32_t)sms);
+}
 
 // CFN = 128 is for streams the caller knows to have at most F_SMALL_LIVE live symbols;
 // CFN = 0 is the per-stream wide table, CFN = -1 one wide table per CTA.
@@ -123,9 +162,9 @@ static int launch_stream(const StreamArgs &a, cudaStream_t cs)
     // 1535 us).  A wide table's three warps have nothing to gain from the L2 (50.4 ms against 50.2).
     // Up to eight streams per SM (twelve without checksums) a wide table each fits: a step is one lookup and five
     // instructions shorter, whatever the alphabet.
-    if constexpr (CFN > 0 && (SINK == SINK_BF16 || SINK == SINK_DELTA))
-        if (quads * 4 <= grid * wide_per_sm<SINK, CRC>())
-            return launch_stream_as<SINK, CRC, 0, TR_FEW>(a, grid, warps(wide_per_sm<SINK, CRC>() / 4), cs);
+    if constexpr (CFN > 0 && SINK == SINK_DELTA)
+        if (quads * 4 <= grid * wide_per_sm<CRC>())
+            return launch_stream_as<SINK, CRC, 0, TR_FEW>(a, grid, warps(wide_per_sm<CRC>() / 4), cs);
     if constexpr (CFN > 0) {
         constexpr uint32_t few = stream_warps(CFN, CRC, SINK, TR_FEW), most4 = stream_warps(CFN, CRC, SINK, TR_4);
         if constexpr (SINK == SINK_BYTES) {
@@ -235,7 +274,6 @@ static int launch_compact_sorted(const RansArgs &a, cudaStream_t cs)
 // Streams that carry their own table.  Up to 12 per SM a wide table each fits, and a step is one
 // lookup shorter; up to 76 per SM the full-size compact tables take the launch in one round,
 // whatever the alphabets; above that small alphabets go to the denser instance.
-constexpr unsigned WIDE_PER_SM = 4 * stream_warps(0, false, SINK_BYTES, TR_8);
 constexpr unsigned COMPACT_PER_SM = 4 * stream_warps(256, false, SINK_BYTES, TR_8);
 
 static int launch_rans(const RansArgs &a, cudaStream_t cs, bool may_alloc = true)
@@ -247,9 +285,9 @@ static int launch_rans(const RansArgs &a, cudaStream_t cs, bool may_alloc = true
     const StreamArgs sa = as_stream_args(a);
     if (a.shared_hdr) return launch_stream<SINK_BYTES, false, -1>(sa, cs);
     const int forced = g_force_table_mode.load(std::memory_order_relaxed);
-    const bool wide = forced < 0 ? a.njobs <= (unsigned)sms * WIDE_PER_SM : forced == T_WIDE1 || forced == T_WIDE13;
-    if (a.open) return wide ? launch_stream<SINK_OPEN, false, 0>(sa, cs) : launch_stream<SINK_OPEN, false, 256>(sa, cs);
-    if (wide) return launch_stream<SINK_BYTES, false, 0>(sa, cs);
+    const bool solo = forced < 0 ? solo_fits(sa, false, sms) : forced == T_WIDE1 || forced == T_WIDE13;
+    if (a.open) return solo ? launch_solo<SINK_OPEN, false>(sa, cs) : launch_stream<SINK_OPEN, false, 256>(sa, cs);
+    if (solo) return launch_solo<SINK_BYTES, false>(sa, cs);
     if (may_alloc && forced < 0 && a.njobs > (unsigned)sms * COMPACT_PER_SM) {
         rc = launch_compact_sorted(a, cs);
         if (rc != 1) return rc;

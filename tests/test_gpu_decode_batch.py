@@ -294,3 +294,24 @@ def test_device_batches_sorted_by_alphabet(gpu, orc, nstr, wide, table_mode):
         bad[2 * at + 1] -= 2
         with pytest.raises(ValueError):
             gpu.decode_batch(t, bad.tobytes(), nstr, plane)
+
+
+@pytest.mark.parametrize("per_sm", [1, 6, 7, 20, 21])
+@pytest.mark.parametrize("plane", [63, 511, 513, 1031])
+def test_batches_around_the_lines_between_kernels(gpu, orc, per_sm, plane, table_mode):
+    """As many streams per SM as a warp with a table entry per slot each, a warp each and four to a warp take, and one
+    more; planes around the eight steps and the 512 symbols that a warp takes at a time.  Uniform bytes take more
+    words in eight steps than a round translates, a single symbol none."""
+    if table_mode != -1:
+        pytest.skip("the automatic choice")
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    nstr = sms * per_sm - sms // 2
+    kinds = ("exponent", "uniform", "single", "two")
+    pool = [distribution(kinds[i % 4], plane, 31 * i + plane) for i in range(61)]
+    streams = [orc.rans_encode(p) for p in pool]
+    blob, offs = pack_streams([streams[i % 61] for i in range(nstr)])
+    out = np.frombuffer(gpu.decode_batch(blob, offs, nstr, plane), dtype=np.uint8).reshape(nstr, plane)
+    want = np.stack([pool[i % 61] for i in range(nstr)])
+    bad = np.nonzero((out != want).any(axis=1))[0]
+    assert bad.size == 0, bad[:10]
