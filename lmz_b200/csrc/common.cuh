@@ -99,6 +99,11 @@ __device__ __forceinline__ uint2 lds_u64(uint32_t a)
     return v;
 }
 
+__device__ __forceinline__ void red_shared_add(uint32_t a, uint32_t v)
+{
+    asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
 __device__ __forceinline__ void prefetch_l2(const void *p)
 {
     asm volatile("prefetch.global.L2 [%0];" ::"l"(p));

@@ -15,20 +15,24 @@
 //   3. the walk from the last symbol to the first.  Lane k owns state k.  Within a group
 //      of eight symbols the reference visits lane 7 first, so a lane's 16-bit word lands
 //      below those of the lanes above it: one vote and a popcount give its place.  Words
-//      go into a 512-byte ring that mirrors the stream's slot in global memory modulo 512
-//      and leave it in whole, aligned 128-byte pieces;
+//      grow down through a buffer that a piece of 128 bytes of the slot ends; whole pieces leave
+//      it after every tile of 16 steps, and what is left of one moves up to its end;
 //   4. the eight states (lane 0 lowest) and the 516-byte table in front of the words.
 // The stream ends exactly at the end of its slot; its length is reported, so it starts
 // at slot_bytes - length.
 //
-// The walk is a chain through the state: compare, shift, divide, multiply-add.  Everything else is
-// taken out of it: a tile's symbols and, two steps ahead, their table entries are loaded before
-// the state needs them, and the division by the symbol's frequency is exact in one multiply-add
-// and a shift (a multiplier and an addend per frequency: N. Robison's choice between rounding the
-// reciprocal up and rounding it down, of which one always works), with no correction after it.
-// A warp is a CTA: 19 KiB of shared memory, eleven per SM, dealt out one by one, so that a batch
-// spreads evenly.  4096 planes of 32 KiB of BF16 exponents on one B200: 943 -> 518 us
-// (142 -> 259 GB/s of symbols).
+// A batch of 4096 planes is seven warps per SM, so what bounds it is latency: in the walk the chain
+// through the state (compare, shift, divide, multiply-add) and, as long as that, the one from the
+// vote to a word's place, of which a step's is worked out beside the next step's state; in the
+// histogram the loads, the next of which are on their way while these are counted.  A tile's symbols
+// and, two steps ahead, their table entries are loaded before the state needs them, and the division
+// by the symbol's frequency is exact in one multiply-add and a shift (a multiplier and an addend per
+// frequency: N. Robison's choice between rounding the reciprocal up and rounding it down, of which one
+// always works), with no correction after it.  A warp is a CTA: 18 KiB of shared memory, dealt out one
+// by one, so that a batch spreads evenly.
+//
+// One B200, with places and states in one chain and the loads waited for: 4096 planes of 32 KiB of BF16
+// exponents 485 -> 309 us (434 GB/s of symbols), 592 of them 376 -> 219, 28000 of 1 KiB 218 -> 162.
 #pragma once
 #include "common.cuh"
 
@@ -43,9 +47,9 @@ struct EncodeArgs {
     uint32_t *lengths;      // per stream: bytes written at the end of its slot, 0 = failed
 };
 
-constexpr uint32_t E_RING = 512, E_TILE = 128;
+constexpr uint32_t E_BUF = 384, E_TILE = 128;            // a piece of 128 bytes and what a tile can add to it
 constexpr uint32_t E_TABLE = 4096;                    // 256 entries of 16 bytes; until then the group's share of the counters
-constexpr uint32_t E_GROUP_BYTES = E_TABLE + E_RING + E_TILE;
+constexpr uint32_t E_GROUP_BYTES = E_TABLE + E_BUF + E_TILE;
 constexpr uint32_t E_COUNT_MAX = 8u * 64000u;         // symbols counted before the lanes' 16-bit counters are summed
 __host__ __device__ constexpr uint32_t encode_smem_bytes() { return 4 * E_GROUP_BYTES; }
 __host__ __device__ constexpr uint32_t encode_slot_bytes(uint32_t plane)
@@ -67,9 +71,8 @@ __host__ __device__ inline Reciprocal reciprocal_of(uint32_t f)
     while ((2u << s) <= f) s++;
 #endif
     if ((f & (f - 1)) == 0) return {1u << 31, 0, s - 1};
-    // (below 2^32, as f > 2^s; the quotient's fraction is a multiple of 1 / f, so its double rounds to
-    // no other integer)
-    const uint32_t down = (uint32_t)((double)(1ull << (32 + s)) / (double)f);
+    // floor(2^(32 + s) / f), below 2^32 as f > 2^s, sixteen bits at a time
+    const uint32_t top = (1u << (16 + s)) / f, down = (top << 16) + (((1u << (16 + s)) - top * f) << 16) / f;
     const uint32_t rest = 0u - down * f;              // 2^(32 + s) - down * f, below f
     if (f - rest <= (1u << s)) return {down + 1, 0, s};
     return {down, down, s};
@@ -80,12 +83,12 @@ __global__ void __launch_bounds__(32) k_encode(EncodeArgs a)
     extern __shared__ __align__(512) uint8_t esm[];
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t k = lane & 7u, g = lane >> 3;
-    // counters of the whole warp, then the four groups' tables, in the same 16 KiB; rings and tiles behind
+    // counters of the whole warp, then the four groups' tables, in the same 16 KiB; buffers and tiles behind
     uint32_t *counters = reinterpret_cast<uint32_t *>(esm);
     uint8_t *const gp = esm + (size_t)g * E_TABLE;
-    uint8_t *ring = esm + 4 * E_TABLE + g * E_RING;
-    uint8_t *tile = esm + 4 * (E_TABLE + E_RING) + g * E_TILE;
-    const uint32_t ring_sa = smem_addr(ring), tile_sa = smem_addr(tile), tab_sa = smem_addr(gp);
+    uint8_t *buf = esm + 4 * E_TABLE + g * E_BUF;
+    uint8_t *tile = esm + 4 * (E_TABLE + E_BUF) + g * E_TILE;
+    const uint32_t buf_sa = smem_addr(buf), tile_sa = smem_addr(tile), tab_sa = smem_addr(gp);
 
     const uint32_t job = blockIdx.x * 4 + g;
     const bool have = job < a.nstr;
@@ -93,17 +96,22 @@ __global__ void __launch_bounds__(32) k_encode(EncodeArgs a)
     const uint8_t *src = a.src + (size_t)job * a.plane;
 
     // ---- 1. histogram ------------------------------------------------------------------
-    uint32_t c[4][8];                               // [stream of the warp][symbol 8 * lane + j]
+    uint32_t c[4][8];                               // [stream of the warp][symbol_of(j)]
+    auto symbol_of = [&](uint32_t j) { return 4 * lane + j + (j >= 4 ? 124u : 0u); };
 #pragma unroll
     for (int gg = 0; gg < 4; gg++)
 #pragma unroll
         for (int j = 0; j < 8; j++) c[gg][j] = 0;
-    auto count = [&](uint32_t b) { atomicAdd(counters + (b >> 1) * 32 + lane, 1u << (16 * (b & 1u))); };
+    // (symbol b: word b & 127 of the lane's, its low half for b < 128)
+    const uint32_t mine_sa = smem_addr(counters) + 4 * lane;
+    auto count = [&](uint32_t b) { red_shared_add(mine_sa + 128 * (b & 0x7fu), 1u << (16 * (b >> 7))); };
     auto count4 = [&](uint32_t w) {
-        count(w & 0xffu);
-        count(__byte_perm(w, 0u, 0x4441u));
-        count(__byte_perm(w, 0u, 0x4442u));
-        count(w >> 24);
+        // a dot product with one byte of 128 picks a byte, scales it and adds the base
+        const uint32_t low = w & 0x7f7f7f7fu, high = (w >> 3) & 0x10101010u;
+        red_shared_add(__dp4a(low, 0x00000080u, mine_sa), 1u << (high & 0xffu));
+        red_shared_add(__dp4a(low, 0x00008000u, mine_sa), 1u << __byte_perm(high, 0u, 0x4441u));
+        red_shared_add(__dp4a(low, 0x00800000u, mine_sa), 1u << __byte_perm(high, 0u, 0x4442u));
+        red_shared_add(__dp4a(low, 0x80000000u, mine_sa), 1u << (high >> 24));
     };
     for (uint32_t at = 0; at < a.plane; at += E_COUNT_MAX) {
         for (uint32_t i = lane; i < 4096; i += 32) counters[i] = 0;
@@ -118,16 +126,25 @@ __global__ void __launch_bounds__(32) k_encode(EncodeArgs a)
         for (uint32_t i = k; i < head; i += 8) count(p[i]);
         const uint4 *u4 = reinterpret_cast<const uint4 *>(p + head);
         auto count16 = [&](const uint4 &v) { count4(v.x); count4(v.y); count4(v.z); count4(v.w); };
+        // the next four units are on their way while these are counted
         uint32_t u = k;
+        uint4 v[4] = {};
+        auto load4 = [&](uint32_t at4, uint4 (&to)[4]) {
+#pragma unroll
+            for (uint32_t i = 0; i < 4; i++) to[i] = __ldg(u4 + at4 + 8 * i);
+        };
+        if (u + 24 < units) load4(u, v);
         for (; u + 24 < units; u += 32) {
-            const uint4 v0 = __ldg(u4 + u), v1 = __ldg(u4 + u + 8), v2 = __ldg(u4 + u + 16), v3 = __ldg(u4 + u + 24);
-            count16(v0); count16(v1); count16(v2); count16(v3);
+            uint4 w[4] = {};
+            if (u + 56 < units) load4(u + 32, w);
+#pragma unroll
+            for (int i = 0; i < 4; i++) { count16(v[i]); v[i] = w[i]; }
         }
         for (; u < units; u += 8) count16(__ldg(u4 + u));
         for (uint32_t i = head + units * 16 + k; i < m; i += 8) count(p[i]);
         __syncwarp();
-        // lane l sums symbols 8 l .. 8 l + 7 of every stream over that stream's eight lanes; the lanes
-        // start at different copies, which keeps them apart in the banks
+        // lane l sums symbols 4 l .. 4 l + 3 and 128 more of every stream over that stream's eight lanes;
+        // the lanes start at different copies, which keeps them apart in the banks
 #pragma unroll
         for (int j = 0; j < 4; j++)
 #pragma unroll
@@ -142,7 +159,7 @@ __global__ void __launch_bounds__(32) k_encode(EncodeArgs a)
                 // (the rotation by 8 * (lane >> 3) reads stream (gg + lane / 8) & 3)
 #pragma unroll
                 for (int q = 0; q < 4; q++)
-                    if (((gg + (lane >> 3)) & 3u) == (uint32_t)q) { c[q][2 * j] += lo; c[q][2 * j + 1] += hi; }
+                    if (((gg + (lane >> 3)) & 3u) == (uint32_t)q) { c[q][j] += lo; c[q][j + 4] += hi; }
             }
         __syncwarp();
     }
@@ -157,7 +174,7 @@ __global__ void __launch_bounds__(32) k_encode(EncodeArgs a)
         uint64_t best = 0;                              // (count << 8) | (255 - symbol): first index wins
 #pragma unroll
         for (int j = 0; j < 8; j++) {
-            const uint32_t s = lane * 8 + j, cj = c[gg][j];
+            const uint32_t s = symbol_of(j), cj = c[gg][j];
             uint64_t q = nn < (1u << 20) ? (cj * PROB_SCALE) / nn : (uint64_t)cj * PROB_SCALE / nn;
             if (cj && q < 1) q = 1;
             if (q > PROB_SCALE) q = PROB_SCALE;
@@ -175,51 +192,51 @@ __global__ void __launch_bounds__(32) k_encode(EncodeArgs a)
         const uint32_t top = 255u - (uint32_t)(best & 0xffu);
         bool good = true;
         if (sum < PROB_SCALE) {
-            if (top / 8 == lane) {
 #pragma unroll
-                for (int j = 0; j < 8; j++)
-                    if ((uint32_t)j == (top & 7u)) f[j] += PROB_SCALE - sum;
-            }
+            for (int j = 0; j < 8; j++)
+                if (symbol_of(j) == top) f[j] += PROB_SCALE - sum;
         } else {
             uint32_t excess = sum - PROB_SCALE;
             for (uint32_t it = 0; excess && it < 512; it++) {
                 uint32_t bk = 0;                        // (freq << 8) | (255 - symbol), freq > 1 only
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
-                    const uint32_t key = (f[j] << 8) | (255u - (lane * 8 + j));
+                    const uint32_t key = (f[j] << 8) | (255u - symbol_of(j));
                     if (f[j] > 1 && key > bk) bk = key;
                 }
                 bk = __reduce_max_sync(0xffffffffu, bk);
                 if (!bk) { good = false; break; }
                 const uint32_t bi = 255u - (bk & 0xffu), bf = bk >> 8;
                 const uint32_t take = bf - 1 < excess ? bf - 1 : excess;
-                if (bi / 8 == lane) {
 #pragma unroll
-                    for (int j = 0; j < 8; j++)
-                        if ((uint32_t)j == (bi & 7u)) f[j] -= take;
-                }
+                for (int j = 0; j < 8; j++)
+                    if (symbol_of(j) == bi) f[j] -= take;
                 excess -= take;
             }
             if (excess) good = false;
         }
         // cumulative starts, then the entries the walk reads: multiplier, addend, the state from
         // which a word leaves first, and shift | (4096 - f) << 8 | start << 20
+        // (one scan for both halves of the alphabet)
         uint32_t mine = 0;
 #pragma unroll
-        for (int j = 0; j < 8; j++) mine += f[j];
+        for (int j = 0; j < 8; j++) mine += f[j] << (j < 4 ? 0 : 16);
         uint32_t incl = mine;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
             if (lane >= (uint32_t)d) incl += v;
         }
-        if (__shfl_sync(0xffffffffu, incl, 31) != PROB_SCALE) good = false;
-        uint32_t start = incl - mine;
+        const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
+        if ((all & 0xffffu) + (all >> 16) != PROB_SCALE) good = false;
+        const uint32_t low_start = (incl - mine) & 0xffffu, high_start = (all & 0xffffu) + ((incl - mine) >> 16);
+        uint32_t start = low_start;
         const uint32_t t_sa = smem_addr(esm) + gg * E_TABLE;
         bool whole = false;
 #pragma unroll
         for (int j = 0; j < 8; j++) {
-            const uint32_t s = lane * 8 + j;
+            const uint32_t s = symbol_of(j);
+            if (j == 4) start = high_start;
             if ((c[gg][j] != 0) != (f[j] != 0)) good = false;
             const Reciprocal r = reciprocal_of(f[j] ? f[j] : 1u);
             sts_u128_if(1, t_sa + 16 * s, r.mul, r.add, f[j] << 20, r.shift | ((PROB_SCALE - f[j]) << 8) | (start << 20));
@@ -238,7 +255,7 @@ __global__ void __launch_bounds__(32) k_encode(EncodeArgs a)
     const uint32_t T = ok && !single ? (n + 7) / 8 : 0; // groups of eight symbols
     const uint32_t tiles = (T + 15) / 16;
     const uint32_t warp_tiles = __reduce_max_sync(0xffffffffu, tiles);
-    uint32_t x = RANS_LOW, emitted = 0, flushed = 0;    // bytes, counted back from the slot's end
+    uint32_t x = RANS_LOW, flushed = 0, pos = buf_sa + E_BUF;   // words grow down from `pos`; bytes counted back from the slot's end
     // a tile's 128 symbols (lane k: bytes 16 k .. 16 k + 15), requested a tile ahead
     const bool aligned = (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
     auto fetch = [&](uint32_t tt) {
@@ -272,27 +289,38 @@ __global__ void __launch_bounds__(32) k_encode(EncodeArgs a)
         __syncwarp();
         sts_u128_if(1, tile_sa + 16 * k, next.x, next.y, next.z, next.w);
         if (tt) next = fetch(tt - 1);
+        if (tt >= 8 && tt < tiles) prefetch_l2(src + (tt - 8) * 128 + 16 * k);
         __syncwarp();
         uint32_t at[16];
 #pragma unroll
         for (int s = 15; s >= 0; s--) at[s] = tab_sa + 16 * lds_u8(tile_sa + s * 8 + k);
         uint4 e0 = lds_u128(at[15]), e1 = lds_u128(at[14]);
         const bool full = __all_sync(0xffffffffu, mine_tile && tt * 128 + 128 <= n);
+        // A step's words are placed while the next step's states are worked out: the vote's byte, its
+        // popcounts and the address are a chain as long as the state's own.
+        uint32_t votes = 0, word = 0;
+        bool out = false;
+        auto place = [&]() {
+            // (the lanes above this one come before it, counted back from `pos`)
+            sts_u16_if(out, pos - 2 * __popc(votes >> (k + 1)) - 2, word);
+            pos -= 2 * __popc(votes);
+        };
         auto step = [&](int s, bool active) {
             const uint4 e = e0;
             e0 = e1;
             if (s >= 2) e1 = lds_u128(at[s - 2]);
             uint32_t v = x;
             const bool need = active && v >= e.z;
-            const uint32_t vote = __byte_perm(__ballot_sync(0xffffffffu, need), 0u, 0x4440u + g);
-            // (the ring position counts down: bytes before this lane's are those of the lanes above it)
-            const uint32_t before = emitted + 2 * __popc(vote >> (k + 1));
-            sts_u16_if(need, ring_sa + ((0u - before - 2u) & (E_RING - 1)), v);
+            const uint32_t vote = __ballot_sync(0xffffffffu, need);
             if (need) v >>= 16;
-            emitted += 2 * __popc(vote);
-            const uint32_t q = (uint32_t)(((uint64_t)v * e.x + e.y) >> 32) >> (e.w & 31u);
+            const uint64_t p = (uint64_t)v * e.x + e.y;
+            if (s < 15) place();
+            word = x;
+            out = need;
+            const uint32_t q = (uint32_t)(p >> 32) >> (e.w & 31u);
             const uint32_t nx = v + (e.w >> 20) + q * ((e.w >> 8) & 0xfffu);
             if (active) x = nx;
+            votes = __byte_perm(vote, 0u, 0x4440u + g);
         };
         if (full) {
 #pragma unroll
@@ -301,32 +329,38 @@ __global__ void __launch_bounds__(32) k_encode(EncodeArgs a)
 #pragma unroll
             for (int s = 15; s >= 0; s--) step(s, mine_tile && tt * 128 + s * 8 + k < n);
         }
-        // whole 128-byte pieces leave the ring (at most 127 + 256 bytes are ever pending)
-        __syncwarp();
-        while (flushed + 128 <= emitted) {
-            const uint32_t at = flushed + 128;          // piece = [end - at, end - at + 128)
-            const uint4 v = lds_u128(ring_sa + ((0u - at) & (E_RING - 1)) + 16 * k);
-            *reinterpret_cast<uint4 *>(slot + a.slot_bytes - at + 16 * k) = v;
-            flushed = at;
+        place();
+        // whole 128-byte pieces leave the buffer, what is left of one moves up to its end
+        const uint32_t whole = (buf_sa + E_BUF - pos) / 128;
+        if (__any_sync(0xffffffffu, whole != 0)) {
+            __syncwarp();
+            uint8_t *const to = slot + a.slot_bytes - flushed - 128 + 16 * k;
+            const uint4 v0 = lds_u128(buf_sa + 256 + 16 * k), v1 = lds_u128(buf_sa + 128 + 16 * k), v2 = lds_u128(buf_sa + 16 * k);
+            if (whole >= 1) *reinterpret_cast<uint4 *>(to) = v0;
+            if (whole >= 2) *reinterpret_cast<uint4 *>(to - 128) = v1;
+            __syncwarp();
+            const uint4 rest = whole >= 2 ? v2 : v1;
+            sts_u128_if(whole != 0, buf_sa + 256 + 16 * k, rest.x, rest.y, rest.z, rest.w);
+            flushed += 128 * whole;
+            pos += 128 * whole;
         }
     }
+    const uint32_t emitted = flushed + buf_sa + E_BUF - pos;
     __syncwarp();
     if (ok) {
         // the pending tail of the words, byte by byte
-        for (uint32_t j = flushed + k; j < emitted; j += 8)
-            slot[a.slot_bytes - 1 - j] = ring[(0u - 1u - j) & (E_RING - 1)];
+        for (uint32_t j = k; j < buf_sa + E_BUF - pos; j += 8) slot[a.slot_bytes - 1 - flushed - j] = buf[E_BUF - 1 - j];
         // ---- 4. states (lane 0 lowest) and the table, in front of the words -------------
-        uint8_t *p = slot + a.slot_bytes - emitted - STATE_BYTES;
-#pragma unroll
-        for (int b = 0; b < 4; b++) p[4 * k + b] = (uint8_t)(x >> (8 * b));
-        uint8_t *h = p - HDR_BYTES;
-        if (k == 0) { h[0] = 'R'; h[1] = '1'; h[2] = 0; h[3] = 0; }
+        // (an even number of bytes from the slot's end: half words)
+        uint16_t *p = reinterpret_cast<uint16_t *>(slot + a.slot_bytes - emitted - STATE_BYTES), *h = p - HDR_BYTES / 2;
+        p[2 * k] = (uint16_t)x;
+        p[2 * k + 1] = (uint16_t)(x >> 16);
+        if (k == 0) { h[0] = 'R' | '1' << 8; h[1] = 0; }
+#pragma unroll 4
         for (uint32_t s = k; s < 256; s += 8) {
             // (f << 20 is zero for no frequency and for all of it; only the latter leaves the field above the shift empty)
             const uint4 w = lds_u128(tab_sa + 16 * s);
-            const uint32_t f = w.z ? w.z >> 20 : (w.w >> 8 ? 0u : PROB_SCALE);
-            h[4 + 2 * s] = (uint8_t)f;
-            h[5 + 2 * s] = (uint8_t)(f >> 8);
+            h[2 + s] = (uint16_t)(w.z ? w.z >> 20 : (w.w >> 8 ? 0u : PROB_SCALE));
         }
     }
     if (have && k == 0) a.lengths[job] = ok ? HDR_BYTES + STATE_BYTES + emitted : 0u;

@@ -120,3 +120,18 @@ def test_strided_device_planes(gpu, orc):
     two[:, 1] = torch.from_numpy(np.concatenate(plains)).cuda()
     streams, _offs = gpu.encode_batch(two[:, 1], 3, 5000)
     assert streams.cpu().numpy().tobytes() == b"".join(orc.rans_encode(p) for p in plains)
+
+
+@pytest.mark.parametrize("lead", [0, 1, 2, 7])
+@pytest.mark.parametrize("plane", [127, 128, 129, 511, 640, 2049])
+def test_tiles_that_fill_their_buffer(gpu, orc, lead, plane):
+    """Next to each other in a warp: planes whose every tile fills two pieces (each symbol once or twice), one piece every
+    few tiles, none at all; both halves of the alphabet, wherever the planes lie in memory."""
+    import torch
+    rng = np.random.default_rng(plane + lead)
+    plains = [rng.permutation(np.arange(plane) % 256).astype(np.uint8), distribution("exponent", plane, lead),
+              np.full(plane, 255, np.uint8), rng.choice([127, 128], plane).astype(np.uint8), distribution("uniform", plane, 5)]
+    t = torch.zeros(lead + 5 * plane, dtype=torch.uint8, device="cuda")
+    t[lead:] = torch.from_numpy(np.concatenate(plains)).cuda()
+    streams, _offs = gpu.encode_batch(t[lead:], 5, plane)
+    assert streams.cpu().numpy().tobytes() == b"".join(orc.rans_encode(p) for p in plains)
