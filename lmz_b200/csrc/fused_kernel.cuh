@@ -284,10 +284,22 @@ struct Words {
     }
 };
 
+// MULT: the start field is e >> 8 less the bits above it, taken off by the multiplier's pipe, as the integer
+// pipe is the busy one where warps are many.  One B200: four 8B layers 1825 -> 1796 us, 28577 streams of 32 KiB
+// 1588 -> 1574; a delta chain, whose merge keeps the multiplier busy, 1534 -> 1547, so not there.
+template <bool MULT>
 __device__ __forceinline__ uint32_t rans_update(uint32_t x, uint32_t e)
 {
     // f * (x >> 12) + slot - start  ==  x - (x >> 12) * (4096 - f) - start
-    return x - ((x >> PROB_BITS) * (e >> 20) + ((e >> 8) & 0xfffu));
+    if constexpr (MULT) {
+        const uint32_t g = e >> 20;
+        uint32_t start, u;
+        asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(start) : "r"(g), "r"(0u - PROB_SCALE), "r"(e >> 8));
+        asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(u) : "r"(x >> PROB_BITS), "r"(g), "r"(start));
+        return x - u;
+    } else {
+        return x - ((x >> PROB_BITS) * (e >> 20) + ((e >> 8) & 0xfffu));
+    }
 }
 
 // The second half of a step: x2 is the updated state; a lane that needs a refill takes the ring
@@ -315,11 +327,11 @@ __device__ __forceinline__ void refill(uint32_t &x, uint32_t &e, uint32_t x2, bo
 // lane's = bits of the older bytes plus the lanes below it in the newest, so one
 // popcount of hist & below (= 0xffffff00 | lanes below) gives the offset from
 // the block's start.
-template <int CFN, int MODE, bool FIRST>
+template <int CFN, int MODE, bool FIRST, bool MULT>
 __device__ __forceinline__ void stream_step4(uint32_t &x, uint32_t &e, uint32_t &hist, uint32_t base, uint32_t l1_sa,
                                              uint32_t cf_sa, uint32_t below, uint32_t vsel)
 {
-    const uint32_t x2 = rans_update(x, e);
+    const uint32_t x2 = rans_update<MULT>(x, e);
     const bool need = x2 < RANS_LOW;
     const uint32_t vote = __ballot_sync(0xffffffffu, need);
     hist = __byte_perm(vote, FIRST ? 0u : hist, vsel);
@@ -330,11 +342,11 @@ __device__ __forceinline__ void stream_step4(uint32_t &x, uint32_t &e, uint32_t 
 // block's next word lies; returns how many of the block's words had been taken when this lane took
 // one, NONE32 if it took none.
 constexpr uint32_t NONE32 = 0xffffffffu;
-template <int CFN, int MODE>
+template <int CFN, int MODE, bool MULT>
 __device__ __forceinline__ uint32_t stream_step(uint32_t &x, uint32_t &e, uint32_t &base, uint32_t base0, uint32_t l1_sa, uint32_t cf_sa,
                                                 uint32_t lt_mask, uint32_t grp_mask, bool active)
 {
-    const uint32_t x2 = rans_update(x, e);
+    const uint32_t x2 = rans_update<MULT>(x, e);
     const bool need = active && x2 < RANS_LOW;
     const uint32_t vote = __ballot_sync(0xffffffffu, need);
     const uint32_t at = base + tr_entry(MODE) * __popc(vote & lt_mask);
@@ -356,7 +368,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
     constexpr bool ROWMUL = (SINK == SINK_BF16 || SINK == SINK_DELTA) && CRC;
     constexpr int NRA = SINK == SINK_DELTA ? 4 : 8;        // running values per lane: words of its unit of a row
     extern __shared__ __align__(16) uint8_t ssm[];
-    constexpr bool WIDE = CFN <= 0, SHARED = CFN < 0;
+    constexpr bool WIDE = CFN <= 0, SHARED = CFN < 0, MULT = SINK != SINK_DELTA;
     // SINK_DELTA with CFN = 192: the two planes of a chunk have level-2 tables of different sizes, 128
     // entries for the exponent differences (a handful of symbols) and 256 for the sign/mantissa
     // differences, 768 bytes a stream on average.
@@ -616,16 +628,16 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
                 uint32_t base = wd.block(), hist = 0;
                 if (WOVEN) wd.part1();
                 put(s8);
-                stream_step4<CFN, MODE, true>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                stream_step4<CFN, MODE, true, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
                 if (WOVEN) wd.part2(l1_sa);
                 put(s8 + 1);
-                stream_step4<CFN, MODE, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                stream_step4<CFN, MODE, false, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
                 fold(s8 / 2);
                 put(s8 + 2);
-                stream_step4<CFN, MODE, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                stream_step4<CFN, MODE, false, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
                 if (WOVEN) wd.part3(cf_sa, k);
                 put(s8 + 3);
-                stream_step4<CFN, MODE, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                stream_step4<CFN, MODE, false, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
                 fold(s8 / 2 + 1);
                 wd.rd += tr_entry(MODE) * __popc(hist);
                 __syncwarp();
@@ -633,14 +645,14 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
                 base = wd.block();
                 hist = 0;
                 put(s8 + 4);
-                stream_step4<CFN, MODE, true>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                stream_step4<CFN, MODE, true, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
                 put(s8 + 5);
-                stream_step4<CFN, MODE, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                stream_step4<CFN, MODE, false, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
                 fold(s8 / 2 + 2);
                 put(s8 + 6);
-                stream_step4<CFN, MODE, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                stream_step4<CFN, MODE, false, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
                 put(s8 + 7);
-                stream_step4<CFN, MODE, false>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                stream_step4<CFN, MODE, false, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
                 fold(s8 / 2 + 3);
                 wd.rd += tr_entry(MODE) * __popc(hist);
             }
@@ -656,7 +668,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
                 for (uint32_t s = s4; s < s4 + 4; s++) {
                     const bool active = s * NLANES + k < rem;
                     if (active) put(s);
-                    const uint32_t ahead = stream_step<CFN, MODE>(x, e, base, base0, l1_sa, cf_sa, lt_mask, grp_mask, active);
+                    const uint32_t ahead = stream_step<CFN, MODE, MULT>(x, e, base, base0, l1_sa, cf_sa, lt_mask, grp_mask, active);
                     if (SINK == SINK_OPEN) {
                         // the first lane that took a word the stream has not got ends an open stream:
                         // `ahead` words had been taken in this block before it took its own

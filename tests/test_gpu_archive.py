@@ -546,6 +546,30 @@ def test_bf16_chunks_by_how_many_there_are(gpu, tmp_path, nchunks, checksum):
     assert torch.equal(decode.load_archive(path, checksum=checksum), member)
 
 
+@pytest.mark.parametrize("nchunks", [740, 741, 2368, 2369, 3552, 3553])
+def test_bf16_chunks_around_the_lines_between_kernels(gpu, tmp_path, nchunks):
+    """5, 16 and 24 chunks per SM (of 148) and one more: a warp per chunk with a table entry per slot, a warp per chunk,
+    a quarter of one."""
+    test_bf16_chunks_by_how_many_there_are(gpu, tmp_path, nchunks, True)
+
+
+@pytest.mark.parametrize("nchunks", [740, 2368, 2369, 3553, 9500])
+@pytest.mark.parametrize("checksum", [True, False])
+def test_fp32_chunks_by_how_many_there_are(nchunks, checksum):
+    """The same lines for chunks of 4-byte elements, and enough of them for the instance for many warps; the last
+    chunk is cut short."""
+    import torch
+    from lmz_b200 import decode
+    from perf import cases
+    case = dict(path="archive", dtype="F32", layers=0, hidden=4 * nchunks, ffn=4095, kv=0, chunk=65536)
+    dec = decode.ArchiveDecoder(cases._archive(case, nchunks), checksum=checksum)
+    out = dec.run()
+    dec.check()
+    head, data, _meta = cases._checkpoint(case, torch.Generator(device="cuda").manual_seed(nchunks))
+    assert out[:len(head)].cpu().numpy().tobytes() == head
+    assert torch.equal(out[len(head):len(head) + data.numel()], data)
+
+
 @pytest.mark.parametrize("checksum", [True, False])
 def test_many_two_plane_deltas(checksum):
     """More delta chunks than wide tables take: the instances with compact tables for both planes."""
