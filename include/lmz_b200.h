@@ -100,9 +100,9 @@ void lmz_gpu_trim(void);
 
 /* No counterpart in the reference: choose the per-stream decode-table layout for
  * streams that carry their own table.  -1 = by batch size (default), 0 or 2 = compact
- * (1 KiB and a word per symbol, the most streams per SM), 3 or 4 = a wide 16 KiB table
- * per stream (one lookup per symbol; 12 streams per SM, for launches small enough to be
- * bound by per-symbol latency).  A tuning and testing knob; results are identical. */
+ * (1 KiB and a word per symbol, the most streams per SM), 3 or 4 = a warp per stream with an
+ * entry per slot or a byte per slot (for launches small enough to be bound by per-symbol
+ * latency).  A tuning and testing knob; results are identical. */
 int lmz_gpu_set_table_mode(int mode);
 
 /* One stream to decode; mirrors struct lmz::StreamJob.  32 bytes. */

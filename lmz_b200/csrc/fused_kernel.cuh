@@ -1,4 +1,4 @@
-// k_stream: the decode kernel.  One 8-lane group per rANS stream and the stream's consumer
+// k_stream: the decode kernel of launches of many streams (few: solo_kernel.cuh).  One 8-lane group per rANS stream and the stream's consumer
 // fused into the decode loop:
 //
 //   SINK_BYTES  the decoded plane is written as is (decode_batch, scratch planes)
@@ -45,7 +45,7 @@
 //     more than 104 live symbols must be given to the CFN = 256 instance
 //   * a ring entry is word and table entry (8 bytes), or word and level-2 offset (TR_4: 4 bytes, half
 //     the space: more streams per SM for one more lookup in a refilled lane's step)
-//   * CFN = 0: a 16 KiB slot -> entry table per stream; CFN = -1: one such table per CTA, for
+//   * CFN = 0 (few delta chunks): a 16 KiB slot -> entry table per stream; CFN = -1: one such table per CTA, for
 //     batches whose streams share one 516-byte table (lmz_gpu_decode_batch's d_hdr) or for the
 //     chunks of a shared-table archive (StreamArgs.tables); a stream is then states + words
 //   * warps are independent: each takes four streams, then the next four, ...; a launch is

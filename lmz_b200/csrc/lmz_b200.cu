@@ -136,7 +136,7 @@ static bool solo_fits(const StreamArgs &a, bool sink, int sms)
 }
 
 // CFN = 128 is for streams the caller knows to have at most F_SMALL_LIVE live symbols;
-// CFN = 0 is the per-stream wide table, CFN = -1 one wide table per CTA.
+// CFN = -1 is one wide table per CTA.
 template <int SINK, bool CRC, int CFN>
 static int launch_stream(const StreamArgs &a, cudaStream_t cs)
 {
@@ -159,9 +159,9 @@ static int launch_stream(const StreamArgs &a, cudaStream_t cs)
     // round (one B200, 64 KiB BF16 chunks with checksums, TR_8 against TR_4: 180 chunks per SM
     // 2160 against 1880 us, 34 per SM 605 against 675).  Streams of bytes alone, with no checksum tables to
     // make room for, run as many warps of TR_8 as of TR_4, and faster (193 streams per SM 1490 against
-    // 1535 us).  A wide table's three warps have nothing to gain from the L2 (50.4 ms against 50.2).
-    // Up to eight streams per SM (twelve without checksums) a wide table each fits: a step is one lookup and five
-    // instructions shorter, whatever the alphabet.
+    // 1535 us).
+    // Up to eight of the delta sink's streams per SM (twelve without checksums) a wide table each fits (CFN = 0): a
+    // step is one lookup and five instructions shorter, whatever the alphabet.
     if constexpr (CFN > 0 && SINK == SINK_DELTA)
         if (quads * 4 <= grid * wide_per_sm<CRC>())
             return launch_stream_as<SINK, CRC, 0, TR_FEW>(a, grid, warps(wide_per_sm<CRC>() / 4), cs);
@@ -271,8 +271,7 @@ static int launch_compact_sorted(const RansArgs &a, cudaStream_t cs)
     return rc;
 }
 
-// Streams that carry their own table.  Up to 12 per SM a wide table each fits, and a step is one
-// lookup shorter; up to 76 per SM the full-size compact tables take the launch in one round,
+// Streams that carry their own table.  Up to 20 per SM (solo_fits) a warp each; up to 76 per SM the full-size compact tables take the launch in one round,
 // whatever the alphabets; above that small alphabets go to the denser instance.
 constexpr unsigned COMPACT_PER_SM = 4 * stream_warps(256, false, SINK_BYTES, TR_8);
 
