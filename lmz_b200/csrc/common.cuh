@@ -110,6 +110,11 @@ __device__ __forceinline__ void prefetch_l2(const void *p)
 }
 
 // The same where `on`, without a branch.
+__device__ __forceinline__ void sts_u8_if(uint32_t on, uint32_t a, uint32_t v)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.shared.u8 [%0], %1;\n\t}"
+                 ::"r"(a), "r"(v), "r"(on) : "memory");
+}
 __device__ __forceinline__ void sts_u16_if(uint32_t on, uint32_t a, uint32_t v)
 {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.shared.u16 [%0], %1;\n\t}"

@@ -20,7 +20,7 @@
 // Measured on one B200, cycles: multiply-add 4, compare and vote 17, and 4, permute 4, dot product 4,
 // load 23; a popcount is 17, so the lanes below are counted by a byte permute that looks three votes
 // up at a time and a dot product that adds them.  For that the eight lanes sit three to a nibble of
-// the vote; the other twenty-four run along and vote for nothing.
+// the vote; the other twenty-four run along, vote for nothing and write nothing.
 //
 // One B200, k_stream's wide tables against this: a lone stream 61.5 -> 41.2 ns a step, a 4096 x 14336 BF16 tensor in 64 KiB
 // chunks 480 -> 384 us, in 8 MiB chunks 34.1 -> 22.6 ms, seven planes of 4 KiB between host buffers 78 -> 57 us.
@@ -29,12 +29,12 @@
 // Sinks as in fused_kernel.cuh, a tile being 512 symbols: 16 a lane.
 #pragma once
 #include "fused_kernel.cuh"
+#include "solo_layout.cuh"
 
 namespace lmz {
 
 constexpr uint32_t S_TILE = 512;                       // symbols a warp stages, then gives out 16 a lane
 constexpr uint32_t S_ENTRY = 8, S_RING = 128 * S_ENTRY, S_ROUND = 32 * S_ENTRY;   // (and a copy of the ring's first round behind it)
-constexpr uint32_t S_LANES = 0x377u;                   // the lanes that own states: 0-2, 4-6, 8, 9
 constexpr uint32_t S_WIDE_BYTES = PROB_SCALE * S_ENTRY, S_REC_BYTES = 256 * S_ENTRY;
 
 struct SoloSmem {
@@ -122,9 +122,9 @@ __global__ void __launch_bounds__(solo_warps(CRC, WIDE) * 32, 1) k_solo(StreamAr
     extern __shared__ __align__(16) uint8_t ssm[];
     const uint32_t lane = threadIdx.x & 31u, W = blockDim.x >> 5;
     const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);       // (the compiler sees that it is the warp's)
-    const bool owner = S_LANES >> lane & 1u;
-    const uint32_t k = owner ? 3 * (lane >> 2) + (lane & 3u) : 0u;
-    const uint32_t below = S_LANES & ((1u << (owner ? lane : 0u)) - 1u);
+    const SoloLane me = solo_lane(lane);
+    const bool owner = me.owner;
+    const uint32_t k = me.k, below = me.below;
 
     const uint32_t s0 = smem_addr(ssm);
     const SoloSmem m_ = solo_smem(CRC, WIDE, W);
@@ -259,8 +259,11 @@ __global__ void __launch_bounds__(solo_warps(CRC, WIDE) * 32, 1) k_solo(StreamAr
                 c = WIDE ? r.y : ta + r.y;
             }
             uint32_t base = 0;
+            auto put = [&](uint32_t at_stage, bool active) {
+                solo_put(me, at_stage, active, [&](uint32_t on, uint32_t at) { sts_u8_if(on, at, e); });
+            };
             auto step = [&](uint32_t at_stage) {
-                sts_u8(at_stage, e);
+                put(at_stage, true);
                 x2 = y * (e >> 8) + c;
                 const uint32_t ta = slot_at(x2), s = byte_at(ta);
                 const bool need = owner && x2 < RANS_LOW;
@@ -309,7 +312,7 @@ __global__ void __launch_bounds__(solo_warps(CRC, WIDE) * 32, 1) k_solo(StreamAr
                 const uint32_t whole = rem / 64 * 8;
 #pragma unroll 1
                 for (; s < whole && !(SINK == SINK_OPEN && open && left <= 0); s += 8) {
-                    const uint32_t at = stage_sa + s * NLANES + k;
+                    const uint32_t at = stage_sa + s * NLANES;
                     base = ring_sa + (rd & (S_RING - 1));
                     uint32_t base0 = base;
                     part1();
@@ -336,7 +339,7 @@ __global__ void __launch_bounds__(solo_warps(CRC, WIDE) * 32, 1) k_solo(StreamAr
                     if (wr - rd < S_ROUND) { part1(); part2(); part3(); }
                     base = ring_sa + (rd & (S_RING - 1));
                     const bool active = s * NLANES + k < rem;
-                    if (active) sts_u8(stage_sa + s * NLANES + k, e);
+                    put(stage_sa + s * NLANES, active);
                     const uint32_t nx = y * (e >> 8) + c;
                     const bool need = owner && active && nx < RANS_LOW;
                     const uint32_t vote = __ballot_sync(0xffffffffu, need), before = __popc(vote & below);

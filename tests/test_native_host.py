@@ -44,6 +44,17 @@ def test_rules(host_rules, check):
 
 
 @pytest.fixture(scope="module")
+def solo_layout(tmp_path_factory):
+    return _compiled(tmp_path_factory, "solo_layout_check")
+
+
+@pytest.mark.parametrize("check", ["stores"])
+def test_a_warp_per_stream(solo_layout, check):
+    done = subprocess.run([solo_layout, check], capture_output=True, text=True, timeout=20)
+    assert done.returncode == 0, done.stderr
+
+
+@pytest.fixture(scope="module")
 def host_pool(tmp_path_factory):
     return _compiled(tmp_path_factory, "host_pool_check")
 
