@@ -33,7 +33,6 @@
 
 namespace lmz {
 
-constexpr uint32_t S_TILE = 512;                       // symbols a warp stages, then gives out 16 a lane
 constexpr uint32_t S_ENTRY = 8, S_RING = 128 * S_ENTRY, S_ROUND = 32 * S_ENTRY;   // (and a copy of the ring's first round behind it)
 constexpr uint32_t S_WIDE_BYTES = PROB_SCALE * S_ENTRY, S_REC_BYTES = 256 * S_ENTRY;
 
@@ -290,7 +289,8 @@ __global__ void __launch_bounds__(solo_warps(CRC, WIDE) * 32, 1) k_solo(StreamAr
             for (int i = 0; i < NRA; i++) ra[i] = 0;
 
 #pragma unroll 1
-            for (uint32_t t = 0, done = 0; done < n; t++, done += S_TILE) {
+            for (uint32_t t = 0, tiles = tiles_of(n, S_TILE); t < tiles; t++) {
+                const uint32_t done = t * S_TILE;
                 uint32_t rem = min(n - done, S_TILE);
                 uint32_t pr[SINK == SINK_F32 ? 3 : 1][5];
                 if constexpr (SINK == SINK_F32) {
@@ -357,6 +357,7 @@ __global__ void __launch_bounds__(solo_warps(CRC, WIDE) * 32, 1) k_solo(StreamAr
                         if (outs) {
                             n = done + s * NLANES + __popc(S_LANES & ((outs & (0u - outs)) - 1u));
                             rem = n - done;
+                            tiles = t + 1;
                             open = false;
                         }
                     }

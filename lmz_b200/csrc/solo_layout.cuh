@@ -3,14 +3,11 @@
 #pragma once
 #include <cstdint>
 
-#ifdef __CUDACC__
-#define LMZ_HD __host__ __device__
-#else
-#define LMZ_HD
-#endif
+#include "tiles.cuh"
 
 namespace lmz {
 
+constexpr uint32_t S_TILE = 512;                       // symbols a warp stages, then gives out 16 a lane
 constexpr uint32_t S_LANES = 0x377u;                   // the lanes that own states: 0-2, 4-6, 8, 9
 
 // A lane of a warp that decodes one stream.  The lanes that own no state run along: they vote for nothing and

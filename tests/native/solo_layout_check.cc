@@ -46,10 +46,26 @@ static int stores()
     return 0;
 }
 
+// Tiles of any plane of 32 bits: each begins inside the plane, the last one reaches its end, and there are so many.
+static int tiles()
+{
+    for (uint32_t tile : {128u, S_TILE})
+        for (uint64_t edge : {0ull, 1ull << 12, 1ull << 31, 1ull << 32})
+            for (int64_t off = -3 * (int64_t)tile; off <= 3 * (int64_t)tile; off++) {
+                const int64_t n64 = (int64_t)edge + off;
+                if (n64 < 0 || n64 > 0xffffffffll) continue;
+                const uint32_t n = (uint32_t)n64, count = tiles_of(n, tile);
+                NEED((uint64_t)count * tile >= n && (n == 0 ? count == 0 : (uint64_t)(count - 1) * tile < n));
+                NEED(n == 0 || n - (count - 1) * tile <= tile);         // (as the kernels work it out, in 32 bits)
+            }
+    return 0;
+}
+
 int main(int argc, char **argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "stores") return stores();
+    if (what == "tiles") return tiles();
     fprintf(stderr, "no such check\n");
     return 2;
 }

@@ -48,7 +48,7 @@ def solo_layout(tmp_path_factory):
     return _compiled(tmp_path_factory, "solo_layout_check")
 
 
-@pytest.mark.parametrize("check", ["stores"])
+@pytest.mark.parametrize("check", ["stores", "tiles"])
 def test_a_warp_per_stream(solo_layout, check):
     done = subprocess.run([solo_layout, check], capture_output=True, text=True, timeout=20)
     assert done.returncode == 0, done.stderr
