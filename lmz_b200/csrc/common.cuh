@@ -5,6 +5,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "tiles.cuh"
+
 namespace lmz {
 
 // ---- stream format (reference: lmz/native/lmzcore.c:755-767) ---------------
@@ -16,7 +18,6 @@ constexpr uint32_t HDR_BYTES = 516;   // 'R','1',0,0 + 256 x u16 frequencies
 constexpr uint32_t STATE_BYTES = 32;  // 8 x u32 initial states
 
 // ---- kernel geometry --------------------------------------------------------
-constexpr uint32_t TILE = 128;        // symbols one 8-lane group retires per tile (16 steps)
 constexpr uint32_t PAD_BYTES = 576;   // readable slack owed after the last stream
 
 // ---- per-stream status words -------------------------------------------------

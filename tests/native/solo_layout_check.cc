@@ -49,7 +49,7 @@ static int stores()
 // Tiles of any plane of 32 bits: each begins inside the plane, the last one reaches its end, and there are so many.
 static int tiles()
 {
-    for (uint32_t tile : {128u, S_TILE})
+    for (uint32_t tile : {TILE, S_TILE})
         for (uint64_t edge : {0ull, 1ull << 12, 1ull << 31, 1ull << 32})
             for (int64_t off = -3 * (int64_t)tile; off <= 3 * (int64_t)tile; off++) {
                 const int64_t n64 = (int64_t)edge + off;
