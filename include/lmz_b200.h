@@ -99,10 +99,11 @@ int lmz_gpu_host_lent(const void *p, size_t bytes);
 void lmz_gpu_trim(void);
 
 /* No counterpart in the reference: choose the per-stream decode-table layout for
- * streams that carry their own table.  -1 = by batch size (default), 0 or 2 = compact
- * (1 KiB and a word per symbol, the most streams per SM), 3 or 4 = a warp per stream with an
- * entry per slot or a byte per slot (for launches small enough to be bound by per-symbol
- * latency).  A tuning and testing knob; results are identical. */
+ * streams that carry their own table, in batches and in chunks with one coded plane.
+ * -1 = by batch size (default), 0 or 2 = compact (1 KiB and a word per symbol, four streams to
+ * a warp, the most streams per SM), 3 and 4 = a warp per stream (for launches small enough to
+ * be bound by per-symbol latency), 3 with an entry per slot, 4 with a byte per slot and an
+ * entry per symbol.  A tuning and testing knob; results are identical. */
 int lmz_gpu_set_table_mode(int mode);
 
 /* One stream to decode; mirrors struct lmz::StreamJob.  32 bytes. */

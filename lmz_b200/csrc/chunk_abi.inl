@@ -275,7 +275,9 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
                 sa.order = nullptr;
                 sa.count = nullptr;
                 const bool checked = p->d_piece_crc != nullptr;
-                if (solo_fits(sa, true, sms)) {
+                if (sa.njobs == 0) {
+                    // (a group of none)
+                } else if (solo_fits(sa, true, sms)) {
                     // few enough for a warp each: nothing to sort by
                     if (grp == 0) rc = checked ? launch_solo<SINK_BF16, true>(sa, fs) : launch_solo<SINK_BF16, false>(sa, fs);
                     else rc = checked ? launch_solo<SINK_F32, true>(sa, fs) : launch_solo<SINK_F32, false>(sa, fs);

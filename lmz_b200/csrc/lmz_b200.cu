@@ -97,6 +97,9 @@ static int launch_stream_as(const StreamArgs &a, uint32_t grid, uint32_t W, cuda
 template <bool CRC>
 constexpr uint32_t wide_per_sm() { return 4 * stream_warps(0, CRC, SINK_DELTA, TR_FEW); }
 
+// lmz_gpu_set_table_mode's; -1 picks by batch size.
+static std::atomic<int> g_force_table_mode{-1};
+
 template <int SINK, bool CRC, bool WIDE>
 static int launch_solo_as(const StreamArgs &a, uint32_t grid, uint32_t W, cudaStream_t cs)
 {
@@ -120,18 +123,23 @@ static int launch_solo(const StreamArgs &a, cudaStream_t cs)
     int sms = 0;
     rc = sm_count(&sms);
     if (rc) return rc;
-    // at most one CTA per SM, its warps just enough for as many rounds as the fullest would need
+    // at most one CTA per SM, its warps just enough for as many rounds as the fullest would need; an entry per
+    // slot where that is one round
     const uint32_t room = a.most_ctas ? a.most_ctas : (uint32_t)sms, grid = a.njobs < room ? a.njobs : room;
     const uint32_t per = (a.njobs + grid - 1) / grid;
-    if (per <= solo_warps(CRC, true)) return launch_solo_as<SINK, CRC, true>(a, grid, per, cs);
-    const uint32_t rounds = (per + solo_warps(CRC, false) - 1) / solo_warps(CRC, false);
-    return launch_solo_as<SINK, CRC, false>(a, grid, (per + rounds - 1) / rounds, cs);
+    const int forced = g_force_table_mode.load(std::memory_order_relaxed);
+    const bool wide = forced == T_SOLO_WIDE || (forced != T_SOLO_BYTES && per <= solo_warps(CRC, true));
+    const uint32_t most = solo_warps(CRC, wide), rounds = (per + most - 1) / most, W = (per + rounds - 1) / rounds;
+    return wide ? launch_solo_as<SINK, CRC, true>(a, grid, W, cs) : launch_solo_as<SINK, CRC, false>(a, grid, W, cs);
 }
+
 // Up to so many streams per SM a warp each is faster than four to a warp.  (One B200, exponent planes of 32 KiB:
 // 4 per SM 183 against 281 us, 12 262 against 282, 20 345 against 382, 28 449 against 385.  With the sinks' own work
 // in the same issue slots: 12 64 KiB BF16 chunks with checksums per SM 395 against 489 us, 18 as long either way.)
 static bool solo_fits(const StreamArgs &a, bool sink, int sms)
 {
+    const int forced = g_force_table_mode.load(std::memory_order_relaxed);
+    if (forced >= 0) return forced == T_SOLO_WIDE || forced == T_SOLO_BYTES;
     return a.njobs <= (sink ? 16ull : 20ull) * (a.most_ctas ? a.most_ctas : (uint32_t)sms);
 }
 
@@ -178,10 +186,6 @@ static int launch_stream(const StreamArgs &a, cudaStream_t cs)
         return launch_stream_as<SINK, CRC, CFN, TR_8>(a, grid, warps(stream_warps(CFN, CRC, SINK, TR_8)), cs);
     }
 }
-
-// `force_mode` < 0 picks by batch size.
-static std::atomic<int> g_force_table_mode{-1};
-
 
 // A batch of streams to decode to bytes.
 struct RansArgs {
@@ -271,8 +275,8 @@ static int launch_compact_sorted(const RansArgs &a, cudaStream_t cs)
     return rc;
 }
 
-// Streams that carry their own table.  Up to 20 per SM (solo_fits) a warp each; up to 76 per SM the full-size compact tables take the launch in one round,
-// whatever the alphabets; above that small alphabets go to the denser instance.
+// Streams that carry their own table.  Up to 20 per SM (solo_fits) a warp each; up to 76 per SM the full-size compact
+// tables take the launch in one round, whatever the alphabets; above that small alphabets go to the denser instance.
 constexpr unsigned COMPACT_PER_SM = 4 * stream_warps(256, false, SINK_BYTES, TR_8);
 
 static int launch_rans(const RansArgs &a, cudaStream_t cs, bool may_alloc = true)
@@ -284,7 +288,7 @@ static int launch_rans(const RansArgs &a, cudaStream_t cs, bool may_alloc = true
     const StreamArgs sa = as_stream_args(a);
     if (a.shared_hdr) return launch_stream<SINK_BYTES, false, -1>(sa, cs);
     const int forced = g_force_table_mode.load(std::memory_order_relaxed);
-    const bool solo = forced < 0 ? solo_fits(sa, false, sms) : forced == T_WIDE1 || forced == T_WIDE13;
+    const bool solo = solo_fits(sa, false, sms);
     if (a.open) return solo ? launch_solo<SINK_OPEN, false>(sa, cs) : launch_stream<SINK_OPEN, false, 256>(sa, cs);
     if (solo) return launch_solo<SINK_BYTES, false>(sa, cs);
     if (may_alloc && forced < 0 && a.njobs > (unsigned)sms * COMPACT_PER_SM) {
@@ -365,9 +369,9 @@ API int lmz_gpu_decode_batch_dev(const void *d_hdr, const void *d_streams, const
 
 API int lmz_gpu_set_table_mode(int mode)
 {
-    if (mode != -1 && mode != T_NARROW && mode != T_COMPACT && mode != T_WIDE1 && mode != T_WIDE13)
+    if (mode != -1 && mode != T_NARROW && mode != T_COMPACT && mode != T_SOLO_WIDE && mode != T_SOLO_BYTES)
         return fail_msg(LMZ_GPU_EUNSUPPORTED,
-                        "table mode must be -1 (auto), 0 or 2 (compact), 3 or 4 (wide per stream)");
+                        "table mode must be -1 (auto), 0 or 2 (compact), 3 or 4 (a warp per stream)");
     g_force_table_mode.store(mode, std::memory_order_relaxed);
     return LMZ_GPU_OK;
 }

@@ -23,8 +23,8 @@
 
 namespace lmz {
 
-// lmz_gpu_set_table_mode's numbers: 0 and 4 are earlier layouts' and stand for 2 and 3.
-enum : int { T_NARROW = 0, T_COMPACT = 2, T_WIDE1 = 3, T_WIDE13 = 4 };
+// lmz_gpu_set_table_mode's numbers: k_stream's compact tables (0 is an earlier layout's), k_solo's two kinds.
+enum : int { T_NARROW = 0, T_COMPACT = 2, T_SOLO_WIDE = 3, T_SOLO_BYTES = 4 };
 
 // This lane's eight frequencies (symbols 8 * lane ..) of the table whose magic is at `hdr`.
 __device__ __forceinline__ void load_freqs(const uint8_t *hdr, uint32_t lane, uint32_t (&f)[8])

@@ -48,8 +48,8 @@ def test_bf16_shard_layouts(shard, kw):
 
 def test_wide_exponent_alphabets_take_the_large_table_instance():
     """BF16 whose exponent byte takes ~200 values (a skewed draw, so rANS still pays):
-    the planner must list such chunks after the small-alphabet ones, and the
-    256-entry instance of the fused kernel must decode them."""
+    the planner must list such chunks after the small-alphabet ones, and whichever kernel takes
+    them must decode them (so few go to k_solo; the others below, with the layout forced)."""
     from lmz_b200 import archive, plan
     rng = np.random.default_rng(11)
     n = 600_000
@@ -522,11 +522,46 @@ def test_conditioned_chunks_by_number_of_coded_segments(gpu, coded):
         dec.check()
 
 
+@pytest.fixture(params=[2, 3, 4], ids=["compact", "slot entries", "slot bytes"])
+def layout(request, gpu):
+    """k_stream, and k_solo with each kind of table, whatever the number of chunks."""
+    assert gpu.library().lmz_gpu_set_table_mode(request.param) == 0
+    yield request.param
+    gpu.library().lmz_gpu_set_table_mode(-1)
+
+
+def test_wide_exponent_alphabets_in_each_layout(layout):
+    test_wide_exponent_alphabets_take_the_large_table_instance()
+
+
+def test_classifications_agree_in_each_layout(layout, shard):
+    test_host_and_device_classification_agree(shard)
+
+
+@pytest.mark.parametrize("coded", [1, 2, 3])
+def test_conditioned_chunks_in_each_layout(gpu, layout, coded):
+    test_conditioned_chunks_by_number_of_coded_segments(gpu, coded)
+
+
+@pytest.mark.parametrize("classify", ["host", "device"])
+@pytest.mark.parametrize("pad", [0, 1, 2, 3])
+def test_fp32_phases_in_each_layout(layout, pad, classify):
+    """The sinks' stores at every 4-byte phase of 16 bytes, whole tiles and the end of a chunk."""
+    n = 16384 * 5 + 1003
+    w = (np.random.default_rng(pad).standard_normal(n) * 0.02).astype("<f4")
+    src = synth.safetensors_bytes([("lead", "F32", (pad,), np.zeros(pad, "<f4").view(np.uint8)),
+                                   ("w", "F32", (n,), w.view(np.uint8))])
+    blob = oa.write_archive([("f.safetensors", src)], mapped=True)
+    for checksum in (True, False):
+        dec = _roundtrip(blob, src, checksum=checksum, fuse="all", classify=classify)
+        assert dec.plan.n_fused_f32 > 0
+
+
 @pytest.mark.parametrize("nchunks", [1184, 1185, 9473])
 @pytest.mark.parametrize("checksum", [True, False])
 def test_bf16_chunks_by_how_many_there_are(gpu, tmp_path, nchunks, checksum):
-    """Few chunks take wide tables, more of them compact ones in the instance for few warps, many
-    the one for many (the counts are those of 148 SMs); small and large alphabets in each."""
+    """Eight chunks per SM (of 148) and one more, a warp each; and more than 64 per SM, which take the instance for
+    many warps; small and large alphabets in each."""
     import json
     import struct
     import torch

@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.fixture(autouse=True, params=[0, 2, 3, 4, -1], ids=["narrow", "compact", "wide1", "wide13", "auto"])
 def table_mode(request, gpu):
-    """Every test runs with both per-stream table layouts forced."""
+    """Every test runs with each per-stream table layout forced: k_stream's, k_solo's two."""
     lib = gpu.library()
     assert lib.lmz_gpu_set_table_mode(request.param) == 0
     yield request.param
@@ -296,14 +296,13 @@ def test_device_batches_sorted_by_alphabet(gpu, orc, nstr, wide, table_mode):
             gpu.decode_batch(t, bad.tobytes(), nstr, plane)
 
 
+@pytest.mark.parametrize("table_mode", [-1], ids=["auto"], indirect=True)
 @pytest.mark.parametrize("per_sm", [1, 6, 7, 20, 21])
 @pytest.mark.parametrize("plane", [63, 511, 513, 1031])
 def test_batches_around_the_lines_between_kernels(gpu, orc, per_sm, plane, table_mode):
     """As many streams per SM as a warp with a table entry per slot each, a warp each and four to a warp take, and one
     more; planes around the eight steps and the 512 symbols that a warp takes at a time.  Uniform bytes take more
     words in eight steps than a round translates, a single symbol none."""
-    if table_mode != -1:
-        pytest.skip("the automatic choice")
     import torch
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     nstr = sms * per_sm - sms // 2
