@@ -5,13 +5,11 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
-#include "tiles.cuh"
+#include "geometry.cuh"
 
 namespace lmz {
 
 // ---- stream format (reference: lmz/native/lmzcore.c:755-767) ---------------
-constexpr uint32_t PROB_BITS = 12;
-constexpr uint32_t PROB_SCALE = 1u << PROB_BITS;
 constexpr uint32_t RANS_LOW = 1u << 16;
 constexpr uint32_t NLANES = 8;        // interleaved states per stream
 constexpr uint32_t HDR_BYTES = 516;   // 'R','1',0,0 + 256 x u16 frequencies

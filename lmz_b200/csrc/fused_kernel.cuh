@@ -125,10 +125,6 @@ struct StreamArgs {
 constexpr uint32_t F_WIDE_BYTES = PROB_SCALE * 4;   // a slot -> entry table
 constexpr uint32_t F_TABLE_STRIDE = 528;            // 516 rounded up to 16
 constexpr uint32_t F_SHARED_SINK_WARPS = 20;        // chunks of a shared-table archive: 80 per CTA share its table
-constexpr uint32_t F_CRC_BYTES = 32768;             // four slice tables x 256 entries x eight copies (CrcQuarters)
-// The launch's shared memory starts F_SMEM_BASE bytes into the CTA's window (the launcher checks
-// that reservation); at most F_SMEM_DYN bytes of it are to be had.
-constexpr uint32_t F_SMEM_BASE = 1024, F_SMEM_DYN = 232448;
 
 // Where a CTA of W warps keeps what, as addresses in the shared window.  The CRC tables sit on a
 // 32 KiB boundary (a table index is OR-ed onto the base) and level-1 tables on 4 KiB boundaries;

@@ -123,14 +123,10 @@ static int launch_solo(const StreamArgs &a, cudaStream_t cs)
     int sms = 0;
     rc = sm_count(&sms);
     if (rc) return rc;
-    // at most one CTA per SM, its warps just enough for as many rounds as the fullest would need; an entry per
-    // slot where that is one round
-    const uint32_t room = a.most_ctas ? a.most_ctas : (uint32_t)sms, grid = a.njobs < room ? a.njobs : room;
-    const uint32_t per = (a.njobs + grid - 1) / grid;
     const int forced = g_force_table_mode.load(std::memory_order_relaxed);
-    const bool wide = forced == T_SOLO_WIDE || (forced != T_SOLO_BYTES && per <= solo_warps(CRC, true));
-    const uint32_t most = solo_warps(CRC, wide), rounds = (per + most - 1) / most, W = (per + rounds - 1) / rounds;
-    return wide ? launch_solo_as<SINK, CRC, true>(a, grid, W, cs) : launch_solo_as<SINK, CRC, false>(a, grid, W, cs);
+    const SoloLaunch l = solo_launch(a.njobs, a.most_ctas ? a.most_ctas : (uint32_t)sms, CRC,
+                                     forced == T_SOLO_WIDE ? 1 : forced == T_SOLO_BYTES ? 0 : -1);
+    return l.wide ? launch_solo_as<SINK, CRC, true>(a, l.grid, l.warps, cs) : launch_solo_as<SINK, CRC, false>(a, l.grid, l.warps, cs);
 }
 
 // Up to so many streams per SM a warp each is faster than four to a warp.  (One B200, exponent planes of 32 KiB:

@@ -33,34 +33,6 @@
 
 namespace lmz {
 
-constexpr uint32_t S_ENTRY = 8, S_RING = 128 * S_ENTRY, S_ROUND = 32 * S_ENTRY;   // (and a copy of the ring's first round behind it)
-constexpr uint32_t S_WIDE_BYTES = PROB_SCALE * S_ENTRY, S_REC_BYTES = 256 * S_ENTRY;
-
-struct SoloSmem {
-    uint32_t crc, tab, rec, ring, stage, end;
-};
-__host__ __device__ constexpr SoloSmem solo_smem(bool crc, bool wide, uint32_t W)
-{
-    // tables on boundaries of their size, behind the checksum's 32 KiB on theirs; below them what fits
-    SoloSmem m{};
-    uint32_t low = F_SMEM_BASE, high = crc ? 2 * F_CRC_BYTES : wide ? F_CRC_BYTES : 2 * PROB_SCALE;
-    const uint32_t low_end = crc || wide ? F_CRC_BYTES : 2 * PROB_SCALE;
-    m.crc = F_CRC_BYTES;
-    m.tab = high; high += W * (wide ? S_WIDE_BYTES : PROB_SCALE);
-    const uint32_t rec = wide ? 0u : W * S_REC_BYTES, ring = W * (S_RING + S_ROUND), stage = W * S_TILE;
-    if (rec <= low_end - low) { m.rec = low; low += rec; } else { m.rec = high; high += rec; }
-    if (ring <= low_end - low) { m.ring = low; low += ring; } else { m.ring = high; high += ring; }
-    if (stage <= low_end - low) { m.stage = low; low += stage; } else { m.stage = high; high += stage; }
-    m.end = high;
-    return m;
-}
-__host__ __device__ constexpr uint32_t solo_warps(bool crc, bool wide)
-{
-    uint32_t w = wide ? 7 : 28;
-    while (solo_smem(crc, wide, w).end > F_SMEM_BASE + F_SMEM_DYN) w--;
-    return w;
-}
-
 // The stream's tables from its 256 frequencies, eight per lane.  False if the frequencies do not sum
 // to 4096.
 template <bool WIDE>

@@ -3,6 +3,7 @@
 #include <string>
 
 #include "../../lmz_b200/csrc/host_rules.inl"
+#include "../../lmz_b200/csrc/solo_layout.cuh"
 
 #define NEED(c)                                                          \
     do {                                                                 \
@@ -40,12 +41,22 @@ static int slices()
             NEED(s >= 1 && s <= MOST_SLICES && s <= nstr);
             if (s == 1) continue;
             NEED(2 * nstr * plane / s >= SLICE_BYTES);
-            // the launcher's one-warp CTAs of four streams, two to an SM
-            unsigned ctas = 0;
-            for (unsigned j = 0; j < s; j++) ctas += (unsigned)(((uint64_t)nstr * (j + 1) / s - (uint64_t)nstr * j / s + 3) / 4);
-            const double chain = plane / 8 * 64e-9, out = (double)nstr / s * plane / 50e9;
-            NEED(ctas <= 2 * SMS || out >= chain);
+            // the launcher's CTAs: how many wait for how many others, in chains one after the other
+            unsigned ctas = 0, resident = ~0u, warps = 0;
+            for (unsigned j = 0; j < s; j++) {
+                const lmz::SoloLaunch l = lmz::solo_launch((uint32_t)((uint64_t)nstr * (j + 1) / s - (uint64_t)nstr * j / s), SMS, false);
+                ctas += l.grid;
+                resident = std::min(resident, lmz::solo_resident(l, false));
+                warps = std::max(warps, l.warps);
+            }
+            const unsigned chains = (ctas + SMS * resident - 1) / (SMS * resident);
+            const double chain = plane / 8 * 42e-9, out = (double)nstr / s * plane / 50e9;
+            NEED(chains <= (warps == 1 ? 3 : 4) || out >= chain);
         }
+    // what the rule's comment says of the room on an SM
+    NEED(lmz::solo_resident(lmz::solo_launch(SMS, SMS, false), false) == 3);
+    NEED(lmz::solo_resident(lmz::solo_launch(SMS + 1, SMS, false), false) == 2);
+    NEED(lmz::solo_smem(false, true, 1).end == 64 << 10);
     NEED(batch_slices(2ull * 16 << 22, 16, SMS) == 8);
     NEED(batch_slices(28ull << 20, 512, SMS) == 7);
     NEED(batch_slices(2ull * 1500 << 20, 1500, SMS) == 3);
