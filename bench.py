@@ -95,7 +95,7 @@ def archive_key(model: str, layout: str, chunk_size: int, seed: int, shared_tabl
 
 def build_archive(model: str, layout: str, chunk_size: int = 0, seed: int = 1, nproc=None,
                   want_files: bool = False, shared_tables: int = 0):
-    """The synthetic archive of a workload, written by the checker's reference-exact
+    """The synthetic archive of a workload, written by the oracle's reference-exact
     writer.  Returns (archive bytes, files) where files is [(relative path, bytes)] of
     the model's source files when `want_files` (else None)."""
     from oracle import archive as oa, bigwrite, synth
@@ -800,7 +800,7 @@ def run_stress(a, rank: int):
 
 
 def cpu_stress_baseline(a):
-    """`lmz_rans_decode` of the reference's C core (the checker's port where it is absent) over
+    """`lmz_rans_decode` of the reference's C core (the oracle's port where it is absent) over
     64 exponent-like streams of 1 Mi symbols, one worker process per core."""
     import multiprocessing as mp
     from oracle import native

@@ -117,8 +117,8 @@ __global__ void __launch_bounds__(32) k_encode(EncodeArgs a)
         for (uint32_t i = lane; i < 4096; i += 32) counters[i] = 0;
         __syncwarp();
         const uint32_t m = n > at ? min(n - at, E_COUNT_MAX) : 0u;
-        // bytes up to the first 16-byte boundary, whole 16-byte units (two per lane in
-        // flight), then the tail; the lanes' shares differ by a unit and two bytes at most,
+        // bytes up to the first 16-byte boundary, whole 16-byte units (four per lane are counted
+        // while the next four load), then the tail; the lanes' shares differ by a unit and two bytes at most,
         // which the last stretch of E_COUNT_MAX leaves room for
         const uint8_t *p = src + at;
         const uint32_t head = min(m, (uint32_t)((16u - (reinterpret_cast<uintptr_t>(p) & 15u)) & 15u));

@@ -1,5 +1,5 @@
-// k_stream: the decode kernel of launches of many streams (few: solo_kernel.cuh).  One 8-lane group per rANS stream and the stream's consumer
-// fused into the decode loop:
+// k_stream: the decode kernel of launches of many streams (few: solo_kernel.cuh).  One 8-lane group per
+// rANS stream and the stream's consumer fused into the decode loop:
 //
 //   SINK_BYTES  the decoded plane is written as is (decode_batch, scratch planes)
 //   SINK_OPEN   the same where open streams (STREAM_OPEN) may be among them; an instance of its own, as

@@ -2,7 +2,7 @@
 //
 // A file's pages are not page-locked, so its bytes cross through a ring of page-locked blocks.  What
 // bounds that is the host copy: one thread moves 5 GB/s out of the page cache, eight to twelve
-// about 36 (this pool's hosts, 16 cores), against 54 GB/s of the link.  The threads, their blocks
+// about 36 (16 cores), against 54 GB/s of the link.  The threads, their blocks
 // and the CUDA calls are all here: a thread takes a free block, fills it (pread, or memcpy from
 // memory), starts its copy on the transfer's stream and takes the next, so several blocks are
 // being filled while others are on the link and no interpreter lock is involved.  Writing a file
@@ -433,7 +433,7 @@ API int lmz_host_gather(int fd, const void *host, uint64_t size, const uint64_t 
 
 // [off, off + len) of a file on a memory-backed file system (tmpfs) as writable memory, its pages reserved
 // first so that no store can find the file system full.  There write() is one thread's work whatever
-// the number of writers (the file's lock: 300 MB in 80 ms on this pool's hosts), stores through a
+// the number of writers (the file's lock: 300 MB in 80 ms), stores through a
 // mapping are not (38 ms with eight threads, the reservation included; 21 ms over an existing file).
 // NULL: not such a file, or no room -- write() then.
 API void *lmz_host_map_file(int fd, uint64_t off, uint64_t len)

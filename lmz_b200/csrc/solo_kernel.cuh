@@ -22,9 +22,11 @@
 // up at a time and a dot product that adds them.  For that the eight lanes sit three to a nibble of
 // the vote; the other twenty-four run along, vote for nothing and write nothing.
 //
-// One B200, k_stream's wide tables against this: a lone stream 61.5 -> 41.2 ns a step, a 4096 x 14336 BF16 tensor in 64 KiB
-// chunks 480 -> 384 us, in 8 MiB chunks 34.1 -> 22.6 ms, seven planes of 4 KiB between host buffers 78 -> 57 us.
-// Uniform bytes, four words a step, cost no more than exponents with one and a third.
+// One B200, k_stream's wide tables against this: a lone stream 61.5 -> 41.9 ns a step (84 cycles, 25 instructions), a
+// 4096 x 14336 BF16 tensor in 64 KiB chunks 480 -> 382 us (issue slots 67 % busy, 31 instructions a stream's step), in 8 MiB
+// chunks 34.1 -> 23.1 ms, seven planes of 4 KiB between host buffers 78 -> 58 us.  Uniform bytes, four words a
+// step, cost no more than exponents with one and a third.  Where the store of a step's symbols stands matters: behind the
+// vote, or behind the load, a lone stream's 8 MiB took 24.6 ms instead of 23.1.
 //
 // Sinks as in fused_kernel.cuh, a tile being 512 symbols: 16 a lane.
 #pragma once

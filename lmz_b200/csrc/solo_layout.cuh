@@ -10,7 +10,9 @@ namespace lmz {
 constexpr uint32_t S_TILE = 512;                       // symbols a warp stages, then gives out 16 a lane
 constexpr uint32_t S_LANES = 0x377u;                   // the lanes that own states: 0-2, 4-6, 8, 9
 
-constexpr uint32_t S_ENTRY = 8, S_RING = 128 * S_ENTRY, S_ROUND = 32 * S_ENTRY;   // (a copy of the first round lies behind the ring)
+constexpr uint32_t S_ENTRY = 8;                        // bytes of a table's or the ring's entry
+// (a copy of the ring's first round lies behind it)
+constexpr uint32_t S_RING = 128 * S_ENTRY, S_ROUND = 32 * S_ENTRY;
 constexpr uint32_t S_WIDE_BYTES = PROB_SCALE * S_ENTRY, S_REC_BYTES = 256 * S_ENTRY;
 
 struct SoloSmem {

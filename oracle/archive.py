@@ -1,7 +1,7 @@
 """Read, decode and WRITE .lmz archives on the CPU.  Test infrastructure only.
 
 Layout per lmz/format.py:32-66 (header, 32-byte chunk records, compressed
-table + manifest, 40-byte footer).  `decode_archive` is the checker the CUDA
+table + manifest, 40-byte footer).  `decode_archive` is the oracle the CUDA
 path is compared with and the timed CPU baseline; it follows the reference's
 decode driver (lmz/api.py:832-886: refs and deltas resolve through a single
 hop onto plain chunks).  `write_archive` produces inputs where the reference's

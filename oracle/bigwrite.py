@@ -1,7 +1,7 @@
 """Write a large synthetic-model archive with many processes.  Test infrastructure.
 
 Each worker generates the bytes of the chunks it is given from the shard's
-seed, encodes them with the reference's compiled encoder (or the checker's),
+seed, encodes them with the reference's compiled encoder (or the oracle's),
 and parks the payloads in a temporary file; the parent stitches payloads, chunk
 table, manifest and footer together in the reference's layout
 (lmz/format.py:279-322).  Chunk boundaries are those the reference's planner

@@ -1,4 +1,4 @@
-"""Per-chunk decode (the checker) and encode (the input writer).
+"""Per-chunk decode (the oracle) and encode (the input writer).
 
 Test infrastructure only.  The decode side restates what the reference does
 to one chunk payload; the encode side restates the reference's choices closely
@@ -155,7 +155,7 @@ def decode_chunk(payload, codec: int, esize: int, flags: int, rlen: int,
         else:
             out = native.oracle().merge_planes(planes, esize)
     else:
-        raise Corrupt(f"codec {codec} is outside the decode path this checker covers")
+        raise Corrupt(f"codec {codec} is outside the decode path this oracle covers")
     if verify and crc and (zlib.crc32(out) & 0xFFFFFFFF) != crc:
         raise Corrupt("chunk failed its checksum")
     return out

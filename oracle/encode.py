@@ -3,7 +3,7 @@
 Restates the choices of the reference's encoder for byte, float and BF16 data
 (lmz/codec.py: encode_chunk :914-1009, _encode_stream :307-393, _rans_cost
 :410-436, _encode_bf16_cond :456-541, encode_delta :1018-1031) on top of the
-checker's rANS encoder, which writes the reference encoder's exact bytes.  GGUF
+oracle's rANS encoder, which writes the reference encoder's exact bytes.  GGUF
 block codecs are not on the decode path this repository covers and are absent.
 """
 from __future__ import annotations

@@ -1,4 +1,4 @@
-"""ctypes bindings for the checker libraries.  Test infrastructure only.
+"""ctypes bindings for the oracle libraries.  Test infrastructure only.
 
 Two libraries with the same job:
 
@@ -38,7 +38,7 @@ def _p(a: np.ndarray):
 
 
 def build(force: bool = False) -> None:
-    """Compile the checker libraries with ``make`` (a few hundred ms)."""
+    """Compile the oracle libraries with ``make`` (a few hundred ms)."""
     if force or not os.path.exists(os.path.join(HERE, "liblmzoracle.so")):
         subprocess.run(["make", "-C", HERE], check=True, capture_output=True)
 
@@ -348,5 +348,5 @@ def ref() -> Ref | None:
 
 
 def best():
-    """The fastest checker for bulk work: the compiled reference when present."""
+    """The fastest oracle for bulk work: the compiled reference when present."""
     return ref() or oracle()
