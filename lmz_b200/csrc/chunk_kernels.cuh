@@ -135,19 +135,53 @@ constexpr uint32_t PADDED_PIECE = PIECE_ELEMS + (PIECE_ELEMS >> 7) * 4;
 struct CrcQuarters {
     uint32_t b[4], rot;
 };
-__device__ __forceinline__ uint32_t mad128(uint32_t a, uint32_t b)
-{
-    uint32_t v;
-    asm("mad.lo.u32 %0, %1, 128, %2;" : "=r"(v) : "r"(a), "r"(b));
-    return v;
-}
 __device__ __forceinline__ uint32_t crc_feed4q(const CrcQuarters &q, uint32_t s)
 {
-    // (a byte permute and a multiply-add per lookup: half of the work on the multiplier's pipe, where a
-    // shift and a mask would both be the integer pipe's, which is the busy one in k_stream)
+    // (one instruction of the multiplier's pipe picks a byte, scales it and adds its table's base; as a byte permute and a
+    // multiply-add it was two, one of them the integer pipe's: four 8B layers 1761 -> 1718 us)
     const uint32_t r = __byte_perm(s, 0u, q.rot);        // byte i of r = byte i ^ g of s
-    return lds_u32(mad128(__byte_perm(r, 0u, 0x4440u), q.b[0])) ^ lds_u32(mad128(__byte_perm(r, 0u, 0x4441u), q.b[1])) ^
-           lds_u32(mad128(__byte_perm(r, 0u, 0x4442u), q.b[2])) ^ lds_u32(mad128(__byte_perm(r, 0u, 0x4443u), q.b[3]));
+    return lds_u32(byte_mad(r, 0x80u, q.b[0])) ^ lds_u32(byte_mad(r, 0x8000u, q.b[1])) ^ lds_u32(byte_mad(r, 0x800000u, q.b[2])) ^
+           lds_u32(byte_mad(r, 0x80000000u, q.b[3]));
+}
+
+// Four elements of ES bytes to `d` (which differs from lane to lane by multiples of their size), the first `ve` of them; the
+// words of the others become zero.
+template <int ES>
+__device__ __forceinline__ void row_store(uint8_t *d, uint32_t (&w)[ES], uint32_t ve)
+{
+    if (ve == 4) {
+        const uint32_t al = (uint32_t)reinterpret_cast<uintptr_t>(d);
+        if (ES == 4 && (al & 15u) == 0) {
+            *reinterpret_cast<uint4 *>(d) = make_uint4(w[0], w[1], w[ES - 2], w[ES - 1]);
+        } else if ((al & 7u) == 0) {
+#pragma unroll
+            for (int i = 0; i < ES / 2; i++) reinterpret_cast<uint2 *>(d)[i] = make_uint2(w[2 * i], w[2 * i + 1]);
+        } else if ((al & 3u) == 0) {
+#pragma unroll
+            for (int i = 0; i < ES; i++) reinterpret_cast<uint32_t *>(d)[i] = w[i];
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4 * ES; i++) d[i] = (uint8_t)(w[i >> 2] >> (8 * (i & 3)));
+        }
+    } else {
+        const uint32_t vb = ES * ve;
+#pragma unroll
+        for (int i = 0; i < 4 * ES; i++)
+            if ((uint32_t)i < vb) d[i] = (uint8_t)(w[i >> 2] >> (8 * (i & 3)));
+#pragma unroll
+        for (int i = 0; i < ES; i++) {
+            const uint32_t keep = vb > 4u * i ? min(vb - 4u * i, 4u) : 0u;
+            w[i] = keep >= 4 ? w[i] : (keep ? w[i] & ((1u << (8 * keep)) - 1u) : 0u);
+        }
+    }
+}
+// Four 4-byte elements from a word of each of their byte planes, the lowest first.
+__device__ __forceinline__ void interleave4(uint32_t p0, uint32_t p1, uint32_t p2, uint32_t p3, uint32_t (&w)[4])
+{
+    const uint32_t u0 = __byte_perm(p0, p1, 0x5140), u1 = __byte_perm(p0, p1, 0x7362);
+    const uint32_t v0 = __byte_perm(p2, p3, 0x5140), v1 = __byte_perm(p2, p3, 0x7362);
+    w[0] = __byte_perm(u0, v0, 0x5410); w[1] = __byte_perm(u0, v0, 0x7632);
+    w[2] = __byte_perm(u1, v1, 0x5410); w[3] = __byte_perm(u1, v1, 0x7632);
 }
 
 struct FinishArgs {
@@ -203,15 +237,6 @@ __device__ __forceinline__ uint32_t crc_feed4(uint32_t tl, uint32_t s)
     constexpr uint32_t TS = 1024u << LOGR;
     return lds_u32(crc_index<LOGR, 0>(tl, s) + 3 * TS) ^ lds_u32(crc_index<LOGR, 1>(tl, s) + 2 * TS) ^
            lds_u32(crc_index<LOGR, 2>(tl, s) + 1 * TS) ^ lds_u32(crc_index<LOGR, 3>(tl, s));
-}
-
-// The state advanced by a row minus 16 bytes of zeros (tables 4..7 = CrcTables::adv).
-template <int LOGR>
-__device__ __forceinline__ uint32_t crc_advance(uint32_t tl, uint32_t s)
-{
-    constexpr uint32_t TS = 1024u << LOGR;
-    return lds_u32(crc_index<LOGR, 0>(tl, s) + 4 * TS) ^ lds_u32(crc_index<LOGR, 1>(tl, s) + 5 * TS) ^
-           lds_u32(crc_index<LOGR, 2>(tl, s) + 6 * TS) ^ lds_u32(crc_index<LOGR, 3>(tl, s) + 7 * TS);
 }
 
 // SUBS = 256-thread sub-blocks per CTA sharing one table set.  Exponent-conditioned chunks

@@ -98,6 +98,21 @@ __device__ __forceinline__ uint2 lds_u64(uint32_t a)
     return v;
 }
 
+// Sums of products of a's bytes, or a's two halves, with constants, plus c: one instruction of the multiplier's pipe picks a
+// byte or the upper half out of a word, scales it and adds it, where a shift or a permute would be the integer pipe's.
+__device__ __forceinline__ uint32_t byte_mad(uint32_t a, uint32_t weights, uint32_t c)
+{
+    uint32_t v;
+    asm("dp4a.u32.u32 %0, %1, %2, %3;" : "=r"(v) : "r"(a), "r"(weights), "r"(c));
+    return v;
+}
+__device__ __forceinline__ uint32_t high_half_add(uint32_t a, uint32_t c)
+{
+    uint32_t v;
+    asm("dp2a.lo.u32.u32 %0, %1, %2, %3;" : "=r"(v) : "r"(a), "r"(0x0100u), "r"(c));
+    return v;
+}
+
 __device__ __forceinline__ void red_shared_add(uint32_t a, uint32_t v)
 {
     asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");

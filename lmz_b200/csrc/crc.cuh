@@ -33,18 +33,10 @@ __host__ __device__ inline uint32_t crc_mulmod(uint32_t a, uint32_t b)
 
 struct CrcTables {
     uint32_t slice[4][256];   // slice-by-4 byte tables
-    uint32_t adv[4][256];     // advance a state by ADV_BYTES zero bytes, per state byte
     uint32_t lane_mul[256];   // x^(8 * 16 * (255 - t)): thread t's unit to the row's end
     uint32_t x2[32];          // x^(2^k)
-    uint32_t adv_row[4][256]; // advance by a 256-byte group row minus one 32-byte lane unit
-    uint32_t lane_mul8[8];    // x^(8 * 32 * (7 - k)): lane k's unit to the group row's end
-    uint32_t run_mul[256];    // x^(8 * 256 * (255 - t)): thread t's 256-byte run to the piece's end
-    uint32_t adv_row4[4][256];// advance by a 512-byte group row minus one 64-byte lane unit (4-byte elements)
-    uint32_t lane_mul8_4[8];  // x^(8 * 64 * (7 - k))
+    uint32_t mul_row128[4][256]; // multiply a state by x^(8 * 128): a group's row of 4-byte elements (k_stream)
     uint32_t mul_row[4][256]; // multiply a state by x^(8 * 256), one 256-byte group row, per state byte
-    uint32_t word_mul[8][8];  // x^(32 * (64 - 8k - i)): word i of lane k's 32-byte unit to the row's end
-    uint32_t mul_row512[4][256];  // multiply a state by x^(8 * 512): one 512-byte warp row (k_cond_finish)
-    uint32_t word_mul512[32][4];  // x^(32 * (128 - 4l - i)): word i of lane l's 16-byte unit to that row's end
     uint32_t warp_mul8k[8];       // x^(8 * 8192 * (7 - w)): warp w's 8 KiB run to the piece's end
     uint32_t word_mul16[16][4];   // x^(32 * (64 - 4j - i)): word i of the j-th 16-byte unit of a 256-byte row to the row's end (delta sink)
     uint32_t mul_row4096[4][256]; // multiply a state by x^(8 * 4096): one row of a piece (k_finish)
@@ -53,13 +45,12 @@ struct CrcTables {
     uint32_t lane_mul64[32];      // x^(8 * 64 * (31 - l)): the end of lane l's 64 bytes to the end of the block
     uint32_t mul_row1024[4][256]; // multiply a state by x^(8 * 1024), one warp's row of BF16 (k_solo)
     uint32_t mul_row2048[4][256]; // and by x^(8 * 2048), its row of 4-byte elements
-    uint32_t word_pow[513];       // x^(32 * m): the m-th last word of a row to the row's end (k_solo)
+    uint32_t word_pow[513];       // x^(32 * m): the m-th last word of a row to the row's end (k_stream, k_solo)
 };
 
 // Rows of the piece layout: 256 threads x 16 bytes.
 constexpr uint32_t ROW_BYTES = 4096;
 constexpr uint32_t PIECE_BYTES = 65536;
-constexpr uint32_t ADV_BYTES = ROW_BYTES - 16;
 
 // x^e mod P for any exponent (x has order dividing 2^32 - 1, so x2[] wraps).
 __host__ __device__ inline uint32_t crc_xpow(const uint32_t *x2, uint64_t e)
@@ -97,29 +88,13 @@ inline void crc_build_tables(CrcTables &t)
     uint32_t p = 0x40000000u;   // x^1
     t.x2[0] = p;
     for (int k = 1; k < 32; k++) t.x2[k] = p = crc_mulmod(p, p);
-    uint32_t adv = crc_xpow(t.x2, 8ull * ADV_BYTES);
-    for (int j = 0; j < 4; j++)
-        for (uint32_t i = 0; i < 256; i++) t.adv[j][i] = crc_mulmod(adv, i << (8 * j));
     for (uint32_t th = 0; th < 256; th++) t.lane_mul[th] = crc_xpow(t.x2, 8ull * 16 * (255 - th));
-    uint32_t adv2 = crc_xpow(t.x2, 8ull * (256 - 32));
+    const uint32_t row128 = crc_xpow(t.x2, 8ull * 128);
     for (int j = 0; j < 4; j++)
-        for (uint32_t i = 0; i < 256; i++) t.adv_row[j][i] = crc_mulmod(adv2, i << (8 * j));
-    for (uint32_t k = 0; k < 8; k++) t.lane_mul8[k] = crc_xpow(t.x2, 8ull * 32 * (7 - k));
-    for (uint32_t th = 0; th < 256; th++) t.run_mul[th] = crc_xpow(t.x2, 8ull * 256 * (255 - th));
-    uint32_t adv4 = crc_xpow(t.x2, 8ull * (512 - 64));
-    for (int j = 0; j < 4; j++)
-        for (uint32_t i = 0; i < 256; i++) t.adv_row4[j][i] = crc_mulmod(adv4, i << (8 * j));
-    for (uint32_t k = 0; k < 8; k++) t.lane_mul8_4[k] = crc_xpow(t.x2, 8ull * 64 * (7 - k));
+        for (uint32_t i = 0; i < 256; i++) t.mul_row128[j][i] = crc_mulmod(row128, i << (8 * j));
     uint32_t row = crc_xpow(t.x2, 8ull * 256);
     for (int j = 0; j < 4; j++)
         for (uint32_t i = 0; i < 256; i++) t.mul_row[j][i] = crc_mulmod(row, i << (8 * j));
-    for (uint32_t k = 0; k < 8; k++)
-        for (uint32_t i = 0; i < 8; i++) t.word_mul[k][i] = crc_xpow(t.x2, 32ull * (64 - 8 * k - i));
-    uint32_t row512 = crc_xpow(t.x2, 8ull * 512);
-    for (int j = 0; j < 4; j++)
-        for (uint32_t i = 0; i < 256; i++) t.mul_row512[j][i] = crc_mulmod(row512, i << (8 * j));
-    for (uint32_t l = 0; l < 32; l++)
-        for (uint32_t i = 0; i < 4; i++) t.word_mul512[l][i] = crc_xpow(t.x2, 32ull * (128 - 4 * l - i));
     for (uint32_t w = 0; w < 8; w++) t.warp_mul8k[w] = crc_xpow(t.x2, 8ull * 8192 * (7 - w));
     for (uint32_t j = 0; j < 16; j++)
         for (uint32_t i = 0; i < 4; i++) t.word_mul16[j][i] = crc_xpow(t.x2, 32ull * (64 - 4 * j - i));
@@ -144,12 +119,6 @@ __device__ __forceinline__ uint32_t crc_word(const uint32_t (*sl)[256], uint32_t
 {
     s ^= w;
     return sl[3][s & 0xff] ^ sl[2][(s >> 8) & 0xff] ^ sl[1][(s >> 16) & 0xff] ^ sl[0][s >> 24];
-}
-
-// Apply a per-state-byte linear map (the advance tables).
-__device__ __forceinline__ uint32_t crc_apply(const uint32_t (*tb)[256], uint32_t s)
-{
-    return tb[0][s & 0xff] ^ tb[1][(s >> 8) & 0xff] ^ tb[2][(s >> 16) & 0xff] ^ tb[3][s >> 24];
 }
 
 }  // namespace lmz

@@ -62,13 +62,16 @@ enum : int { SINK_BYTES = 0, SINK_BF16 = 1, SINK_F32 = 2, SINK_DELTA = 3, SINK_O
 //   TR_8    8-byte ring entries
 //   TR_4    4-byte ring entries: the most warps
 enum : int { TR_4 = 0, TR_8 = 1, TR_FEW = 2 };
-constexpr uint32_t F_STAGE = 144;                  // a tile's 128 symbols + 16: groups land 4 banks apart
 constexpr uint32_t TR_N = 64, TR_MIRROR = 32;      // ring of translated words; a block of four steps reads at most 32
 constexpr uint32_t TR_ROUND = 16;                  // words translated at a time, two per lane
-constexpr uint32_t F_ROW = 256, F_UNIT = 32;       // bytes of BF16 one group / one lane emits per tile
+constexpr uint32_t F_ROW = 256;                    // bytes of BF16 one group emits per tile
 constexpr int F_SMALL_CFN = 128;                   // level-2 slots of the dense instance
 constexpr int F_HYBRID_CFN = 192;                  // delta sink: 128-entry tables for first planes, 256-entry for second planes
 constexpr uint32_t F_SMALL_LIVE = F_SMALL_CFN - 24; // largest alphabet it takes (the warp's streams sit 0, 8, 16, 24 entries in)
+
+// Bytes of a stream's stage, a tile's 128 symbols and some: groups land four banks apart, or, where a lane takes a word from
+// each of four places, eight.  (With 160 for all, 28577 streams of 32 KiB 1536 -> 1560 us.)
+__host__ __device__ constexpr uint32_t stage_bytes(int sink) { return sink == SINK_BF16 || sink == SINK_F32 ? 160u : 144u; }
 
 struct FusedJob {
     uint64_t src_off;    // rANS stream, bytes from the source base
@@ -130,7 +133,7 @@ constexpr uint32_t F_SHARED_SINK_WARPS = 20;        // chunks of a shared-table 
 // 32 KiB boundary (a table index is OR-ed onto the base) and level-1 tables on 4 KiB boundaries;
 // what fits goes below the CRC tables, chosen so that the whole is shortest.
 struct StreamSmem {
-    uint32_t cf, stage, tr, l1, crc, adv, poison, end;
+    uint32_t cf, stage, tr, l1, crc, poison, end;
 };
 __host__ __device__ constexpr uint32_t tr_entry(int mode) { return mode == TR_4 ? 4u : 8u; }
 __host__ __device__ constexpr uint32_t tr_group(int mode) { return (TR_N + TR_MIRROR) * tr_entry(mode); }
@@ -138,15 +141,14 @@ __host__ __device__ constexpr StreamSmem stream_smem_with(int cfn, bool crc, int
 {
     StreamSmem m{};
     uint32_t p = F_SMEM_BASE;
-    m.poison = p; p += 16;
-    const uint32_t cf = cfn > 0 ? W * 16u * (uint32_t)cfn : 0u, stage = W * 4u * F_STAGE, tr = W * 4u * tr_group(mode);
+    m.poison = p; p += cfn < 0 ? 16u : 0u;
+    const uint32_t cf = cfn > 0 ? W * 16u * (uint32_t)cfn : 0u, stage = W * 4u * stage_bytes(sink), tr = W * 4u * tr_group(mode);
     m.cf = p; p += cf;
     if (low_stage) { m.stage = p; p += stage; }
     if (low_tr) { m.tr = p; p += tr; }
     if (crc) {
         p = (p + F_CRC_BYTES - 1) & ~(F_CRC_BYTES - 1);
         m.crc = p; p += F_CRC_BYTES;
-        if (sink == SINK_F32) { m.adv = p; p += 4096; }
     }
     const uint32_t align = cfn > 0 ? 4096u : F_WIDE_BYTES;
     p = (p + align - 1) & ~(align - 1);
@@ -176,19 +178,24 @@ __host__ __device__ constexpr uint32_t stream_warps(int cfn, bool crc, int sink,
 }
 
 // ---- the ring of translated words ------------------------------------------------------------
-// A slot's table entry: its level-2 byte offset from the stream's first entry (compact), or the
-// address of the entry itself (wide).
+// A slot's table entry (wide: its address), `from` bytes on.  Compact: from its byte offset from the stream's first entry.
 template <int CFN>
-__device__ __forceinline__ uint32_t slot_ref(uint32_t x, uint32_t l1_sa)
+__device__ __forceinline__ uint32_t slot_ref(uint32_t x, uint32_t l1_sa, uint32_t from)
 {
     if (CFN <= 0) return ((x << 2) & 0x3ffcu) | l1_sa;         // the table is 16 KiB aligned
     // the warp's four level-1 tables are interleaved word by word, so bucket b of this group
     // sits 16 * b bytes in -- the slot's bits 4-11, unshifted
     const uint32_t e1 = lds_u32((x & 0xff0u) | l1_sa);
-    return (e1 >> 16) + 4u * __popc(e1 << ((~x & 15u) | 16u));
+    return high_half_add(e1, from + 4u * __popc(e1 << ((~x & 15u) | 16u)));
 }
-template <int CFN>
-__device__ __forceinline__ uint32_t ref_addr(uint32_t ref, uint32_t cf_sa) { return CFN <= 0 ? ref : cf_sa + ref; }
+// Its address.  (TR_4 adds the tables' address last, as a ring entry's is added: four 8B layers 1711 us, 1800 with a sum of three;
+// 28577 streams of 32 KiB of the others 1576 and 1535.)
+template <int CFN, int MODE>
+__device__ __forceinline__ uint32_t slot_addr(uint32_t x, uint32_t l1_sa, uint32_t cf_sa)
+{
+    if (CFN > 0 && MODE == TR_4) return cf_sa + slot_ref<CFN>(x, l1_sa, 0u);
+    return slot_ref<CFN>(x, l1_sa, cf_sa);
+}
 
 // Positions are in bytes of ring entries and only grow; the ring index is the position modulo the ring.
 //
@@ -251,17 +258,17 @@ struct Words {
         room = wr - rd <= RB - TR_ROUND * ES;
         v = __funnelshift_r(lo, hi, sh);
     }
-    __device__ __forceinline__ void part2(uint32_t l1_sa)
+    __device__ __forceinline__ void part2(uint32_t l1_sa, uint32_t cf_sa)
     {
-        r0 = slot_ref<CFN>(v, l1_sa);
-        r1 = slot_ref<CFN>(v >> 16, l1_sa);
+        r0 = slot_ref<CFN>(v, l1_sa, TR8 ? cf_sa : 0u);          // (a 4-byte ring entry has the offset alone)
+        r1 = slot_ref<CFN>(v >> 16, l1_sa, TR8 ? cf_sa : 0u);
     }
-    __device__ __forceinline__ void part3(uint32_t cf_sa, uint32_t k)
+    __device__ __forceinline__ void part3(uint32_t k)
     {
         const uint32_t at = sa + (wr & (RB - 1)) + 2u * ES * k;
         const uint32_t keep = room, again = room && !(wr & LOW);
         if (TR8) {
-            const uint32_t e0 = lds_u32(ref_addr<CFN>(r0, cf_sa)), e1 = lds_u32(ref_addr<CFN>(r1, cf_sa));
+            const uint32_t e0 = lds_u32(r0), e1 = lds_u32(r1);
             sts_u128_if(keep, at, e0, v, e1, v >> 16);
             sts_u128_if(again, at + RB, e0, v, e1, v >> 16);
         } else {
@@ -275,8 +282,8 @@ struct Words {
     __device__ __forceinline__ void round(uint32_t l1_sa, uint32_t cf_sa, uint32_t k)
     {
         part1();
-        part2(l1_sa);
-        part3(cf_sa, k);
+        part2(l1_sa, cf_sa);
+        part3(k);
     }
 };
 
@@ -304,7 +311,7 @@ template <int CFN, int MODE>
 __device__ __forceinline__ void refill(uint32_t &x, uint32_t &e, uint32_t x2, bool need, uint32_t word_sa, uint32_t l1_sa,
                                        uint32_t cf_sa)
 {
-    uint32_t a = ref_addr<CFN>(slot_ref<CFN>(x2, l1_sa), cf_sa);
+    uint32_t a = slot_addr<CFN, MODE>(x2, l1_sa, cf_sa);
     if (MODE != TR_4) {
         e = lds_u32(a);
         const uint2 w = lds_u64(word_sa);
@@ -356,13 +363,12 @@ __device__ __forceinline__ uint32_t stream_step(uint32_t &x, uint32_t &e, uint32
 template <int SINK, bool CRC, int CFN, int MODE>
 __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_stream(StreamArgs a)
 {
-    // SINK_BF16 checksums: lane k keeps one running value per word of its 32-byte unit,
-    // ra[i] = sum over the piece's rows so far of word i * x^(2048 * rows since); a row
-    // costs each of them one multiplication by x^2048 (the same four lookups as feeding a
-    // word) with no chain between the eight and no per-row advance; the constants
-    // word_mul[k][i] carry them to the piece's end.
-    constexpr bool ROWMUL = (SINK == SINK_BF16 || SINK == SINK_DELTA) && CRC;
-    constexpr int NRA = SINK == SINK_DELTA ? 4 : 8;        // running values per lane: words of its unit of a row
+    // Checksums: lane k keeps one running value for each word that it emits of a row (a tile; SINK_F32: a quarter of one),
+    // ra[i] = sum over the piece's rows so far of word i * x^(8 * row * rows since); a row
+    // costs each of them one multiplication by x^(8 * row) (the same four lookups as feeding a
+    // word) with no chain between them and no per-row advance; the constants
+    // word_pow[], word_mul16[] carry them to the piece's end.
+    constexpr int NRA = SINK == SINK_BF16 ? 8 : 4;        // running values per lane: words of its unit of a row
     extern __shared__ __align__(16) uint8_t ssm[];
     constexpr bool WIDE = CFN <= 0, SHARED = CFN < 0, MULT = SINK != SINK_DELTA;
     // SINK_DELTA with CFN = 192: the two planes of a chunk have level-2 tables of different sizes, 128
@@ -377,6 +383,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
     const uint32_t grp_mask = 0xffu << (g * 8), lt_mask = ((1u << k) - 1u) << (g * 8);
     const uint32_t below = 0xffffff00u | ((1u << k) - 1u), vsel = 0x6540u + g;
 
+    constexpr uint32_t F_STAGE = stage_bytes(SINK);
     // ---- shared memory (addresses are 32-bit shared-space addresses) ----------------------
     const uint32_t s0 = smem_addr(ssm);
     const StreamSmem m_ = stream_smem(CFN, CRC, SINK, MODE, W);
@@ -389,12 +396,19 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
                                                : m_.cf + grp * (WIDE ? 0u : 4u * CFN); };
     const uint32_t cf_sa = cf_of(gi);
     const uint32_t stage_sa = m_.stage + gi * F_STAGE;
+    // SINK_BF16, SINK_F32: a tile is given out in units of four elements, unit u by lane u & 7, so that what a group loads
+    // and stores at a time lies in a row; unit u's symbols lie at 16 (u & 7) + 4 (u >> 3), a lane's four units side by side.
+    // (With sixteen consecutive elements to a lane, a warp's 4-byte load took 4.2 wavefronts of the load/store unit and its 8-byte
+    // store 8.2, of 4-byte elements 14.8, where these take 3.4, 3.9 and 4.5: that unit was 83 and 78 % busy, now 76 and 77.
+    // One B200: four 8B layers 1785 -> 1761 us, twelve FP32 layers 893 -> 679; 1704 and 665 with what the multiplier's pipe does
+    // for the addresses.  Rows given out by all 32 lanes take still fewer, and as many more instructions: 1838 instead of 1761.)
+    constexpr bool UNITS = SINK == SINK_BF16 || SINK == SINK_F32;
+    const uint32_t put_sa = stage_sa + 16 * (k >> 2) + (k & 3u);
     // byte i ^ g of a state word goes through slice table 3 - (i ^ g)
     CrcQuarters cq;
 #pragma unroll
     for (uint32_t i = 0; i < 4; i++) cq.b[i] = tab0 + 32u * (3u - (i ^ g)) + 4u * k;
     cq.rot = 0x3210u ^ (0x1111u * g);
-    const uint32_t tla = m_.adv - 4096u;                            // crc_advance<0> adds 4 .. 7 KiB
 
     uint32_t limit = a.njobs;
     if (a.count) limit = SINK == SINK_DELTA ? 2u * *a.count : *a.count;     // (delta: the count is of chunks, two streams each)
@@ -404,17 +418,11 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
     if (blockIdx.x * (by_table ? G : 4u) >= limit) return;          // the whole CTA has nothing to do
 
     if (CRC && fits) {
-        // slice-by-4 tables, eight copies in the bank-quartered layout of CrcQuarters; then
-        // "advance by one row minus one lane unit"
+        // "multiply by a row", eight copies in the bank-quartered layout of CrcQuarters (crc_feed4q sends byte m of a
+        // value through table 3 - m)
         uint32_t *ts = reinterpret_cast<uint32_t *>(gen(tab0));
-        // (crc_feed4q sends byte m of a state through table 3 - m, crc_word's order; the
-        // row multiplication is in crc_apply's order, byte m through table m)
-        for (uint32_t i = threadIdx.x; i < F_CRC_BYTES / 4; i += blockDim.x)
-            ts[i] = ROWMUL ? a.tabs->mul_row[3u - ((i >> 3) & 3u)][i >> 5] : a.tabs->slice[(i >> 3) & 3u][i >> 5];
-        if (SINK == SINK_F32) {
-            uint32_t *ta = reinterpret_cast<uint32_t *>(gen(m_.adv));
-            for (uint32_t i = threadIdx.x; i < 1024u; i += blockDim.x) ta[i] = (&a.tabs->adv_row4[0][0])[i];
-        }
+        const uint32_t(*mul)[256] = SINK == SINK_F32 ? a.tabs->mul_row128 : a.tabs->mul_row;
+        for (uint32_t i = threadIdx.x; i < F_CRC_BYTES / 4; i += blockDim.x) ts[i] = mul[3u - ((i >> 3) & 3u)][i >> 5];
     }
     if (SHARED && fits && warp == 0) {
         // one table for the CTA, built by its first warp: the launch's, or the one this CTA's chunks
@@ -553,7 +561,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
         }
         wd.lo = lo; wd.hi = hi; wd.lo2 = lo2; wd.hi2 = hi2; wd.next = next; wd.left = left;
         if (n == 0) wd.retire();
-        e = lds_u32(ref_addr<CFN>(slot_ref<CFN>(x, l1_sa), cf_sa));
+        e = lds_u32(slot_addr<CFN, MODE>(x, l1_sa, cf_sa));
         __syncwarp();
     }
     uint8_t *out = a.dst + doff;
@@ -564,7 +572,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
     // of output, of which lane k of the chunk's first group takes the 16 from 16 k and lane k
     // of its second group the 16 from 128 + 16 k.
     const uint32_t j16 = 8u * (g & 1u) + k;
-    const uint8_t *mant = SINK == SINK_DELTA ? a.dst + moff + 16 * j16 : a.src + moff + 16 * k;
+    const uint8_t *mant = SINK == SINK_DELTA ? a.dst + moff + 16 * j16 : a.src + moff + 4 * k;
     const uint32_t msh = (uint32_t)(reinterpret_cast<uintptr_t>(mant) & 3u) * 8u;
     const uint32_t *mq = reinterpret_cast<const uint32_t *>(reinterpret_cast<uintptr_t>(mant) & ~uintptr_t(3));
     uint32_t m[5] = {0, 0, 0, 0, 0};
@@ -572,14 +580,20 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
     // measured 0.7 % slower with the other count: four 8B layers 1796 -> 1809 us)
     uint32_t my_tiles = SINK == SINK_BYTES ? tiles_of(n, TS) : (n + TS - 1) / TS;
     const bool has_base = SINK == SINK_DELTA && moff != NONE64;      // (a plain two-plane chunk has none: m stays zero)
-    if ((SINK == SINK_BF16 && my_tiles) || (has_base && n > 8 * j16)) {
+    auto fetch = [&](uint32_t tt) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) m[i] = __ldg(mq + (size_t)tt * (TILE / 4) + 8 * i);
+        if (k == 0) m[4] = __ldg(mq + (size_t)tt * (TILE / 4) + 32);
+    };
+    if (SINK == SINK_BF16 && my_tiles) fetch(0);
+    if (has_base && n > 8 * j16) {
 #pragma unroll
         for (int i = 0; i < 5; i++) m[i] = __ldg(mq + i);
     }
     // SINK_BF16 checksum: the eight running values ra[] are multiplied by x^2048 while the
     // NEXT tile decodes (32 independent table lookups that hide behind the decode chain),
-    // then that tile's words are XORed in.  SINK_F32 keeps one value, `acc`.
-    uint32_t acc = 0, ra[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    // then that tile's words are XORed in.
+    uint32_t ra[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     const bool was_open = open;
     uint32_t last_x = x, taken = 0;               // state and words consumed at the stream's end
 
@@ -593,17 +607,17 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
         uint32_t rem = n > done ? n - done : 0;
         __syncwarp();
         // SINK_F32: the tile's stored bytes are requested before the decode, which hides
-        // their latency (lane k: elements 16k .. 16k+15 of each of the three planes)
+        // their latency: of each plane's 33 words around them every eighth from k on, the last by lane 0
         uint32_t pr[SINK == SINK_F32 ? 3 : 1][5];
         if constexpr (SINK == SINK_F32) {
-            const bool mine = FULL ? rem != 0 : rem > 16 * k;
 #pragma unroll
             for (int j = 0; j < 3; j++) {
-                const uint8_t *pp = a.src + moff + (size_t)j * n + done + 16 * k;
-                const uint32_t *pq = reinterpret_cast<const uint32_t *>(reinterpret_cast<uintptr_t>(pp) & ~uintptr_t(3));
+                const uint8_t *pp = a.src + moff + (size_t)j * n + done;
+                const uint32_t *pq = reinterpret_cast<const uint32_t *>(reinterpret_cast<uintptr_t>(pp) & ~uintptr_t(3)) + k;
 #pragma unroll
-                for (int i = 0; i < 5; i++) pr[j][i] = mine ? __ldg(pq + i) : 0u;
-                if (MODE == TR_FEW && rem > 5 * TS) prefetch_l2(pq + 4 * TS / 4);
+                for (int i = 0; i < 4; i++) pr[j][i] = rem && (FULL || rem + 3 > 4 * (k + 8 * i)) ? __ldg(pq + 8 * i) : 0u;
+                pr[j][4] = k == 0 && rem >= TS ? __ldg(pq + 32) : 0u;
+                if (MODE == TR_FEW && rem > 5 * TS) prefetch_l2(pq + 4 * TS / 4 + 3 * k);
             }
         }
         auto top_up = [&]() {
@@ -612,9 +626,9 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
                 __syncwarp();
             }
         };
-        auto put = [&](uint32_t step) { sts_u8(stage_sa + step * NLANES + k, e); };
+        auto put = [&](uint32_t step) { sts_u8(UNITS ? put_sa + 32 * (step & 3u) + 4 * (step >> 2) : stage_sa + step * NLANES + k, e); };
         auto fold = [&](uint32_t i) {
-            if (ROWMUL && i < NRA) ra[i] = crc_feed4q(cq, ra[i]);
+            if (CRC && i < NRA) ra[i] = crc_feed4q(cq, ra[i]);
         };
         if constexpr (FULL) {
 #pragma unroll
@@ -627,13 +641,13 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
                 if (WOVEN) wd.part1();
                 put(s8);
                 stream_step4<CFN, MODE, true, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
-                if (WOVEN) wd.part2(l1_sa);
+                if (WOVEN) wd.part2(l1_sa, cf_sa);
                 put(s8 + 1);
                 stream_step4<CFN, MODE, false, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
                 fold(s8 / 2);
                 put(s8 + 2);
                 stream_step4<CFN, MODE, false, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
-                if (WOVEN) wd.part3(cf_sa, k);
+                if (WOVEN) wd.part3(k);
                 put(s8 + 3);
                 stream_step4<CFN, MODE, false, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
                 fold(s8 / 2 + 1);
@@ -684,6 +698,23 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
             }
         }
         __syncwarp();
+        uint32_t pw[SINK == SINK_F32 ? 4 : 1][3];
+        if constexpr (SINK == SINK_F32) {
+            // (unit i of this lane: elements 4 (k + 8 i) .. + 3; the words behind are the next lane's, lane 0's of the next unit)
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                const uint32_t sh = (uint32_t)((reinterpret_cast<uintptr_t>(a.src) + moff + (size_t)j * n) & 3u) * 8u;
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    pw[i][j] = __funnelshift_r(pr[j][i], __shfl_sync(0xffffffffu, k == 0 ? pr[j][i + 1] : pr[j][i], (lane & 24u) | ((k + 1) & 7u)), sh);
+            }
+        }
+        uint32_t mw[SINK == SINK_BF16 ? 4 : 1];
+        if constexpr (SINK == SINK_BF16) {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                mw[i] = __funnelshift_r(m[i], __shfl_sync(0xffffffffu, k == 0 ? m[i + 1] : m[i], (lane & 24u) | ((k + 1) & 7u)), msh);
+        }
         if (!rem) return;
         if (SINK == SINK_DELTA) {
             // ---- both planes' symbols of this lane's eight elements, merge, XOR the base, write, checksum
@@ -749,6 +780,39 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
         }
         const uint4 ev = lds_u128(stage_sa + 16 * k);
         const uint32_t ew[4] = {ev.x, ev.y, ev.z, ev.w};
+        if constexpr (SINK == SINK_F32) {
+            // ---- interleave with the three stored planes, write, checksum: eight lanes' units in a row at a time
+#pragma unroll
+            for (uint32_t i = 0; i < 4; i++) {
+                const uint32_t u = k + 8 * i, ve = FULL ? 4u : rem > 4 * u ? min(rem - 4 * u, 4u) : 0u;
+                uint32_t w[4];
+                interleave4(pw[i][0], pw[i][1], pw[i][2], ew[i], w);
+                row_store<4>(out + (size_t)done * 4 + 16 * u, w, ve);
+                if (CRC) {
+#pragma unroll
+                    for (int h = 0; h < 4; h++) ra[h] = (i ? crc_feed4q(cq, ra[h]) : ra[h]) ^ w[h];
+                }
+            }
+            if (CRC && ((t & 127u) == 127u || t + 1 == my_tiles)) {
+                // close the 64 KiB piece: every running value to the row's end, XOR over the group
+                uint32_t v = 0;
+#pragma unroll
+                for (int h = 0; h < 4; h++) {
+                    v ^= crc_mulmod(a.tabs->word_pow[32 - 4 * k - h], ra[h]);
+                    ra[h] = 0;
+                }
+                v ^= __shfl_xor_sync(grp_mask, v, 1);
+                v ^= __shfl_xor_sync(grp_mask, v, 2);
+                v ^= __shfl_xor_sync(grp_mask, v, 4);
+                if (k == 0) {
+                    const uint32_t p = t >> 7, tiles = (t & 127u) + 1;
+                    const uint32_t plen = min(PIECE_BYTES, 4 * n - p * PIECE_BYTES);
+                    if (tiles * 512u != plen) v = crc_unshift(a.tabs->x2, v, tiles * 512u - plen);
+                    a.piece_crc[piece0 + p] = v;
+                }
+            }
+            return;
+        }
         if (SINK == SINK_BYTES || SINK == SINK_OPEN) {
             if ((FULL || rem >= TS) && al == 0) {
                 *reinterpret_cast<uint4 *>(out + done + 16 * k) = ev;
@@ -761,121 +825,26 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
             return;
         }
 
-        if constexpr (SINK == SINK_F32) {
-            // ---- interleave with the three stored planes, write, checksum ------------
-            const uint32_t ve = FULL ? 16u : rem > 16 * k ? min(rem - 16 * k, 16u) : 0u;   // valid elements of this lane
-            uint32_t pw[3][4];
-#pragma unroll
-            for (int j = 0; j < 3; j++) {
-                const uint32_t sh = (uint32_t)((reinterpret_cast<uintptr_t>(a.src) + moff + (size_t)j * n + done) & 3u) * 8u;
-#pragma unroll
-                for (int h = 0; h < 4; h++) pw[j][h] = __funnelshift_r(pr[j][h], pr[j][h + 1], sh);
-            }
-            uint32_t w[16];
-#pragma unroll
-            for (int h = 0; h < 4; h++) {
-                const uint32_t u0 = __byte_perm(pw[0][h], pw[1][h], 0x5140), u1 = __byte_perm(pw[0][h], pw[1][h], 0x7362);
-                const uint32_t v0 = __byte_perm(pw[2][h], ew[h], 0x5140), v1 = __byte_perm(pw[2][h], ew[h], 0x7362);
-                w[4 * h + 0] = __byte_perm(u0, v0, 0x5410); w[4 * h + 1] = __byte_perm(u0, v0, 0x7632);
-                w[4 * h + 2] = __byte_perm(u1, v1, 0x5410); w[4 * h + 3] = __byte_perm(u1, v1, 0x7632);
-            }
-            uint8_t *d = out + (size_t)done * 4 + k * 64;
-            if (ve == 16) {
-                if (al == 0) {
-#pragma unroll
-                    for (int i = 0; i < 4; i++)
-                        reinterpret_cast<uint4 *>(d)[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
-                } else if ((al & 7) == 0) {
-#pragma unroll
-                    for (int i = 0; i < 8; i++) reinterpret_cast<uint2 *>(d)[i] = make_uint2(w[2 * i], w[2 * i + 1]);
-                } else if ((al & 3) == 0) {
-#pragma unroll
-                    for (int i = 0; i < 16; i++) reinterpret_cast<uint32_t *>(d)[i] = w[i];
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 64; i++) d[i] = (uint8_t)(w[i >> 2] >> (8 * (i & 3)));
-                }
-            } else {
-                // whole elements only: a word is either kept or zero
-#pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    if ((uint32_t)i < ve) {
-                        if ((al & 3) == 0) reinterpret_cast<uint32_t *>(d)[i] = w[i];
-                        else
-                            for (int b = 0; b < 4; b++) d[4 * i + b] = (uint8_t)(w[i] >> (8 * b));
-                    } else {
-                        w[i] = 0u;
-                    }
-                }
-            }
-            if (CRC) {
-                acc = crc_advance<0>(tla, acc);
-#pragma unroll
-                for (int i = 0; i < 16; i++) acc = crc_feed4q(cq, acc ^ w[i]);
-                if ((t & 127u) == 127u || t + 1 == my_tiles) {
-                    // close the 64 KiB piece: lane units -> row end, XOR over the group
-                    uint32_t v = crc_mulmod(a.tabs->lane_mul8_4[k], acc);
-                    v ^= __shfl_xor_sync(grp_mask, v, 1);
-                    v ^= __shfl_xor_sync(grp_mask, v, 2);
-                    v ^= __shfl_xor_sync(grp_mask, v, 4);
-                    if (k == 0) {
-                        const uint32_t p = t >> 7, rows = (t & 127u) + 1;
-                        const uint32_t plen = min(PIECE_BYTES, 4 * n - p * PIECE_BYTES);
-                        if (rows * 512u != plen) v = crc_unshift(a.tabs->x2, v, rows * 512u - plen);
-                        a.piece_crc[piece0 + p] = v;
-                    }
-                    acc = 0;
-                }
-            }
-            return;
-        }
-
-        // ---- SINK_BF16: merge with the stored plane, write, checksum ------------------
-        uint32_t w[8];
-#pragma unroll
-        for (int h = 0; h < 4; h++)
-            bf16_merge4(ew[h], __funnelshift_r(m[h], m[h + 1], msh), w[2 * h], w[2 * h + 1]);
+        // ---- SINK_BF16: merge with the stored plane, write, checksum, units as above -----
         if (t + 1 < my_tiles) {                                // next tile's stored bytes
-#pragma unroll
-            for (int i = 0; i < 5; i++) m[i] = __ldg(mq + (size_t)(t + 1) * (TILE / 4) + i);
-            if (MODE == TR_FEW && t + 5 < my_tiles) prefetch_l2(mq + (size_t)(t + 5) * (TILE / 4));
+            fetch(t + 1);
+            if (MODE == TR_FEW && t + 5 < my_tiles) prefetch_l2(mq + (size_t)(t + 5) * (TILE / 4) + 3 * k);
         }
-        uint8_t *d = out + (size_t)done * 2 + k * F_UNIT;
-        const uint32_t ve = FULL ? 16u : rem > 16 * k ? min(rem - 16 * k, 16u) : 0u;   // valid elements of this lane
-        if (ve == 16) {
-            if (al == 0) {
-                reinterpret_cast<uint4 *>(d)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-                reinterpret_cast<uint4 *>(d)[1] = make_uint4(w[4], w[5], w[6], w[7]);
-            } else if ((al & 7) == 0) {
 #pragma unroll
-                for (int i = 0; i < 4; i++) reinterpret_cast<uint2 *>(d)[i] = make_uint2(w[2 * i], w[2 * i + 1]);
-            } else if ((al & 3) == 0) {
-#pragma unroll
-                for (int i = 0; i < 8; i++) reinterpret_cast<uint32_t *>(d)[i] = w[i];
-            } else {
-#pragma unroll
-                for (int i = 0; i < 32; i++) d[i] = (uint8_t)(w[i >> 2] >> (8 * (i & 3)));
-            }
-        } else {
-            const uint32_t vb = 2 * ve;
-#pragma unroll
-            for (int i = 0; i < 32; i++)
-                if ((uint32_t)i < vb) d[i] = (uint8_t)(w[i >> 2] >> (8 * (i & 3)));
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const uint32_t keep = vb > 4u * i ? min(vb - 4u * i, 4u) : 0u;
-                w[i] = keep >= 4 ? w[i] : (keep ? w[i] & ((1u << (8 * keep)) - 1u) : 0u);
-            }
+        for (uint32_t i = 0; i < 4; i++) {
+            const uint32_t u = k + 8 * i, ve = FULL ? 4u : rem > 4 * u ? min(rem - 4 * u, 4u) : 0u;
+            uint32_t w[2];
+            bf16_merge4(ew[i], mw[i], w[0], w[1]);
+            row_store<2>(out + (size_t)done * 2 + 8 * u, w, ve);
+            if (CRC) { ra[2 * i] ^= w[0]; ra[2 * i + 1] ^= w[1]; }
         }
         if (CRC) {
-#pragma unroll
-            for (int i = 0; i < 8; i++) ra[i] ^= w[i];
             if ((t & 255u) == 255u || t + 1 == my_tiles) {
                 // close the 64 KiB piece: every running value to the row's end, XOR over the group
                 uint32_t v = 0;
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
-                    v ^= crc_mulmod(a.tabs->word_mul[k][i], ra[i]);
+                    v ^= crc_mulmod(a.tabs->word_pow[64 - 16 * (i / 2) - 2 * k - i % 2], ra[i]);
                     ra[i] = 0;
                 }
                 v ^= __shfl_xor_sync(grp_mask, v, 1);

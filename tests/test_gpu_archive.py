@@ -557,6 +557,21 @@ def test_fp32_phases_in_each_layout(layout, pad, classify):
         assert dec.plan.n_fused_f32 > 0
 
 
+@pytest.mark.parametrize("tail", [0, 1, 3, 4, 5, 31, 32, 33, 127])
+@pytest.mark.parametrize("lead", [0, 1, 2, 4, 8])
+def test_bf16_rows_in_each_layout(layout, lead, tail):
+    """The BF16 sinks' units of four elements: chunks that end anywhere in one, and output at any alignment (a member of `lead`
+    bytes before); the streams' lengths put the stored planes at theirs."""
+    n = 2 * 32768 + 20480 + tail
+    w = (np.random.default_rng(16 * lead + tail).standard_normal(n) * 0.02).astype("<f4").view("<u4") >> 16
+    src = synth.safetensors_bytes([("w", "BF16", (n,), w.astype("<u2").view(np.uint8))])
+    first = np.full(lead, 7, np.uint8)
+    blob = oa.write_archive(([("a.bin", first)] if lead else []) + [("m.safetensors", src)], mapped=True)
+    for checksum in (True, False):
+        dec = _roundtrip(blob, np.concatenate((first, src)), checksum=checksum, fuse="all")
+        assert dec.plan.fused_jobs.size == 3
+
+
 @pytest.mark.parametrize("nchunks", [1184, 1185, 9473])
 @pytest.mark.parametrize("checksum", [True, False])
 def test_bf16_chunks_by_how_many_there_are(gpu, tmp_path, nchunks, checksum):
