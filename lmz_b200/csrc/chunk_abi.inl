@@ -277,12 +277,14 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
                 const bool checked = p->d_piece_crc != nullptr;
                 if (sa.njobs == 0) {
                     // (a group of none)
-                } else if (solo_fits(sa, true, sms)) {
-                    // few enough for a warp each: nothing to sort by
-                    if (grp == 0) rc = checked ? launch_solo<SINK_BF16, true>(sa, fs) : launch_solo<SINK_BF16, false>(sa, fs);
-                    else rc = checked ? launch_solo<SINK_F32, true>(sa, fs) : launch_solo<SINK_F32, false>(sa, fs);
-                    if (rc) return rc;
                 } else {
+                    // where they are few, there is nothing to sort by
+                    if (grp == 0) rc = checked ? launch_few<SINK_BF16, true>(sa, fs) : launch_few<SINK_BF16, false>(sa, fs);
+                    else rc = checked ? launch_few<SINK_F32, true>(sa, fs) : launch_few<SINK_F32, false>(sa, fs);
+                    if (rc != LMZ_GPU_OK && rc != 1) return rc;
+                }
+                if (rc == 1) {
+                    rc = LMZ_GPU_OK;
                     k_classify<<<(sa.njobs + 7) / 8, 256, 0, fs>>>(sa, F_SMALL_LIVE, order, counts);
                     g_launches++;
                     cudaError_t le = cudaGetLastError();
@@ -311,10 +313,9 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
         // (counted by the host: each group's small ones come first)
         const bool crc = p->d_piece_crc != nullptr;
         sa.njobs = nbf;
-        if (solo_fits(sa, true, sms)) {
-            rc = crc ? launch_solo<SINK_BF16, true>(sa, fs) : launch_solo<SINK_BF16, false>(sa, fs);
-            if (rc) return rc;
-        } else {
+        rc = crc ? launch_few<SINK_BF16, true>(sa, fs) : launch_few<SINK_BF16, false>(sa, fs);
+        if (rc != LMZ_GPU_OK && rc != 1) return rc;
+        if (rc == 1) {
             sa.njobs = nsmall;
             rc = crc ? launch_stream<SINK_BF16, true, F_SMALL_CFN>(sa, fs) : launch_stream<SINK_BF16, false, F_SMALL_CFN>(sa, fs);
             if (rc) return rc;
@@ -323,10 +324,9 @@ API int lmz_gpu_decode_chunks_dev(const lmz_decode_plan *p, void *cuda_stream)
             if (rc) return rc;
         }
         part(p->n_fused_f32);
-        if (solo_fits(sa, true, sms)) {
-            rc = crc ? launch_solo<SINK_F32, true>(sa, fs) : launch_solo<SINK_F32, false>(sa, fs);
-            if (rc) return rc;
-        } else {
+        rc = crc ? launch_few<SINK_F32, true>(sa, fs) : launch_few<SINK_F32, false>(sa, fs);
+        if (rc != LMZ_GPU_OK && rc != 1) return rc;
+        if (rc == 1) {
             sa.njobs = nsmall4;
             rc = crc ? launch_stream<SINK_F32, true, F_SMALL_CFN>(sa, fs) : launch_stream<SINK_F32, false, F_SMALL_CFN>(sa, fs);
             if (rc) return rc;

@@ -45,6 +45,9 @@
 //     more than 104 live symbols must be given to the CFN = 256 instance
 //   * a ring entry is word and table entry (8 bytes), or word and level-2 offset (TR_4: 4 bytes, half
 //     the space: more streams per SM for one more lookup in a refilled lane's step)
+//   * CFN = 1 (F_BYTE_CFN), up to 24 or 28 streams per SM: k_solo's tables of a byte per slot and its 8-byte entries, 7.6 KiB a
+//     stream; a step is two lookups without a popcount between them, and half as many instructions of the integer
+//     pipe, of which a warp that has a scheduler to itself issues one in two cycles
 //   * CFN = 0 (few delta chunks): a 16 KiB slot -> entry table per stream; CFN = -1: one such table per CTA, for
 //     batches whose streams share one 516-byte table (lmz_gpu_decode_batch's d_hdr) or for the
 //     chunks of a shared-table archive (StreamArgs.tables); a stream is then states + words
@@ -53,6 +56,7 @@
 #pragma once
 #include "chunk_kernels.cuh"
 #include "rans.cuh"
+#include "solo_tables.cuh"
 
 namespace lmz {
 
@@ -66,8 +70,13 @@ constexpr uint32_t TR_N = 64, TR_MIRROR = 32;      // ring of translated words; 
 constexpr uint32_t TR_ROUND = 16;                  // words translated at a time, two per lane
 constexpr uint32_t F_ROW = 256;                    // bytes of BF16 one group emits per tile
 constexpr int F_SMALL_CFN = 128;                   // level-2 slots of the dense instance
+constexpr int F_BYTE_CFN = 1;                      // a byte per slot, its symbol, and k_solo's 8-byte entries: a middling number of streams
 constexpr int F_HYBRID_CFN = 192;                  // delta sink: 128-entry tables for first planes, 256-entry for second planes
 constexpr uint32_t F_SMALL_LIVE = F_SMALL_CFN - 24; // largest alphabet it takes (the warp's streams sit 0, 8, 16, 24 entries in)
+
+// F_BYTE_CFN: a stream's 256 entries, and the next one's sixteen banks on, so that two streams' popular symbols lie apart
+// (28 streams of bytes per SM 379 -> 370 us).
+constexpr uint32_t F_REC_STRIDE = S_REC_BYTES + 64;
 
 // Bytes of a stream's stage, a tile's 128 symbols and some: groups land four banks apart, or, where a lane takes a word from
 // each of four places, eight.  (With 160 for all, 28577 streams of 32 KiB 1536 -> 1560 us.)
@@ -136,13 +145,14 @@ struct StreamSmem {
     uint32_t cf, stage, tr, l1, crc, poison, end;
 };
 __host__ __device__ constexpr uint32_t tr_entry(int mode) { return mode == TR_4 ? 4u : 8u; }
-__host__ __device__ constexpr uint32_t tr_group(int mode) { return (TR_N + TR_MIRROR) * tr_entry(mode); }
+__host__ __device__ constexpr uint32_t tr_words(int cfn) { return cfn == F_BYTE_CFN ? 2 * TR_N : TR_N; }
+__host__ __device__ constexpr uint32_t tr_group(int cfn, int mode) { return (tr_words(cfn) + TR_MIRROR) * tr_entry(mode); }
 __host__ __device__ constexpr StreamSmem stream_smem_with(int cfn, bool crc, int sink, int mode, uint32_t W, bool low_stage, bool low_tr)
 {
     StreamSmem m{};
     uint32_t p = F_SMEM_BASE;
     m.poison = p; p += cfn < 0 ? 16u : 0u;
-    const uint32_t cf = cfn > 0 ? W * 16u * (uint32_t)cfn : 0u, stage = W * 4u * stage_bytes(sink), tr = W * 4u * tr_group(mode);
+    const uint32_t cf = cfn == F_BYTE_CFN ? W * 4u * F_REC_STRIDE : cfn > 0 ? W * 16u * (uint32_t)cfn : 0u, stage = W * 4u * stage_bytes(sink), tr = W * 4u * tr_group(cfn, mode);
     m.cf = p; p += cf;
     if (low_stage) { m.stage = p; p += stage; }
     if (low_tr) { m.tr = p; p += tr; }
@@ -152,7 +162,7 @@ __host__ __device__ constexpr StreamSmem stream_smem_with(int cfn, bool crc, int
     }
     const uint32_t align = cfn > 0 ? 4096u : F_WIDE_BYTES;
     p = (p + align - 1) & ~(align - 1);
-    m.l1 = p; p += cfn > 0 ? W * 4096u : cfn == 0 ? W * 4u * F_WIDE_BYTES : F_WIDE_BYTES;
+    m.l1 = p; p += cfn == F_BYTE_CFN ? W * 4u * PROB_SCALE : cfn > 0 ? W * 4096u : cfn == 0 ? W * 4u * F_WIDE_BYTES : F_WIDE_BYTES;
     if (!low_tr) { m.tr = p; p += tr; }
     if (!low_stage) { m.stage = p; p += stage; }
     m.end = p;
@@ -209,7 +219,8 @@ template <int CFN, int MODE>
 struct Words {
     static constexpr bool TR8 = MODE != TR_4;
     static constexpr int AHEAD = MODE == TR_FEW ? 2 : 1;
-    static constexpr uint32_t ES = tr_entry(MODE), RB = TR_N * ES, LOW = TR_MIRROR * ES;
+    static constexpr bool BYTES = CFN == F_BYTE_CFN;
+    static constexpr uint32_t ES = tr_entry(MODE), RB = tr_words(CFN) * ES, LOW = TR_MIRROR * ES;
     static_assert(TR8 || CFN > 0, "a wide table's entry does not fit a 4-byte ring entry");
     uint32_t sa;             // the ring
     uint32_t rd, wr;         // words consumed / translated so far
@@ -239,7 +250,8 @@ struct Words {
         left -= want ? 1 : 0;
     }
     __device__ __forceinline__ uint32_t block() const { return sa + (rd & (RB - 1)); }
-    __device__ __forceinline__ bool low() const { return wr - rd < LOW; }
+    // Fewer than `blocks` of four steps can take.
+    __device__ __forceinline__ bool low(uint32_t blocks = 1) const { return wr - rd < blocks * LOW; }
     // Words consumed so far of a stream of that many bytes.  (Positions are 32-bit bytes of ring entries
     // and wrap in a stream of half a Gi words; the rounds do not.  AHEAD rounds are loaded ahead of `wr`.)
     __device__ __forceinline__ uint32_t taken(uint32_t bytes) const
@@ -252,6 +264,7 @@ struct Words {
 
     // A round in three parts, so that the steps of the decode run between them.
     uint32_t v, r0, r1;
+    uint2 b0, b1;            // F_BYTE_CFN: the entries of the symbols r0, r1
     bool room;
     __device__ __forceinline__ void part1()
     {
@@ -260,14 +273,30 @@ struct Words {
     }
     __device__ __forceinline__ void part2(uint32_t l1_sa, uint32_t cf_sa)
     {
+        if constexpr (BYTES) {
+            r0 = lds_u8((v & (PROB_SCALE - 1)) | l1_sa);
+            r1 = lds_u8((v >> 16 & (PROB_SCALE - 1)) | l1_sa);
+            return;
+        }
         r0 = slot_ref<CFN>(v, l1_sa, TR8 ? cf_sa : 0u);          // (a 4-byte ring entry has the offset alone)
         r1 = slot_ref<CFN>(v >> 16, l1_sa, TR8 ? cf_sa : 0u);
     }
-    __device__ __forceinline__ void part3(uint32_t k)
+    __device__ __forceinline__ void part2b(uint32_t cf_sa)
+    {
+        b0 = lds_u64(cf_sa + S_ENTRY * r0);
+        b1 = lds_u64(cf_sa + S_ENTRY * r1);
+    }
+    __device__ __forceinline__ void part3(uint32_t l1_sa, uint32_t cf_sa, uint32_t k)
     {
         const uint32_t at = sa + (wr & (RB - 1)) + 2u * ES * k;
-        const uint32_t keep = room, again = room && !(wr & LOW);
-        if (TR8) {
+        const uint32_t keep = room, again = room && !(wr & (RB - LOW));
+        if constexpr (BYTES) {
+            const uint2 e0 = b0, e1 = b1;
+            const uint32_t c0 = (v >> PROB_BITS & 15u) * (e0.x >> 8) + e0.y + ((v & (PROB_SCALE - 1)) | l1_sa);
+            const uint32_t c1 = (v >> 28) * (e1.x >> 8) + e1.y + ((v >> 16 & (PROB_SCALE - 1)) | l1_sa);
+            sts_u128_if(keep, at, e0.x, c0, e1.x, c1);
+            sts_u128_if(again, at + RB, e0.x, c0, e1.x, c1);
+        } else if (TR8) {
             const uint32_t e0 = lds_u32(r0), e1 = lds_u32(r1);
             sts_u128_if(keep, at, e0, v, e1, v >> 16);
             sts_u128_if(again, at + RB, e0, v, e1, v >> 16);
@@ -283,7 +312,8 @@ struct Words {
     {
         part1();
         part2(l1_sa, cf_sa);
-        part3(k);
+        if constexpr (BYTES) part2b(cf_sa);
+        part3(l1_sa, cf_sa, k);
     }
 };
 
@@ -360,6 +390,48 @@ __device__ __forceinline__ uint32_t stream_step(uint32_t &x, uint32_t &e, uint32
     return need ? (at - base0) / tr_entry(MODE) : NONE32;
 }
 
+// F_BYTE_CFN's steps, as k_solo's: of a state x only y, e and c are kept, of which the next (unrefilled) one is
+// y * (e >> 8) + c.  (One B200: 83 ns a step up to 16 streams per SM, 90 with 24, where the compact tables take 93 and 107.
+// Two predicated loads instead of the selected one, as k_solo has them: 90 with 16.)
+struct ByteState {
+    uint32_t y, c;
+};
+__device__ __forceinline__ void byte_next(uint32_t &x, uint32_t &e, ByteState &b, uint32_t x2, bool need, uint32_t word_sa,
+                                          uint32_t ta, uint32_t sym, uint32_t rec_sa)
+{
+    const uint2 r = lds_u64(need ? word_sa : rec_sa + S_ENTRY * sym);
+    x = x2;
+    b.y = need ? x2 * 16 : x2 >> PROB_BITS;
+    e = r.x;
+    b.c = r.y + (need ? 0u : ta);
+}
+template <bool FIRST>
+__device__ __forceinline__ void byte_step4(uint32_t &x, uint32_t &e, ByteState &b, uint32_t &hist, uint32_t base, uint32_t tab_sa,
+                                           uint32_t rec_sa, uint32_t below, uint32_t vsel)
+{
+    const uint32_t x2 = b.y * (e >> 8) + b.c;
+    const uint32_t ta = (x2 & (PROB_SCALE - 1)) | tab_sa, sym = lds_u8(ta);
+    const bool need = x2 < RANS_LOW;
+    const uint32_t vote = __ballot_sync(0xffffffffu, need);
+    hist = __byte_perm(vote, FIRST ? 0u : hist, vsel);
+    byte_next(x, e, b, x2, need, base + S_ENTRY * __popc(hist & below), ta, sym, rec_sa);
+}
+__device__ __forceinline__ uint32_t byte_step(uint32_t &x, uint32_t &e, ByteState &b, uint32_t &base, uint32_t base0, uint32_t tab_sa,
+                                              uint32_t rec_sa, uint32_t lt_mask, uint32_t grp_mask, bool active)
+{
+    const uint32_t x2 = b.y * (e >> 8) + b.c;
+    const uint32_t ta = (x2 & (PROB_SCALE - 1)) | tab_sa, sym = lds_u8(ta);
+    const bool need = active && x2 < RANS_LOW;
+    const uint32_t vote = __ballot_sync(0xffffffffu, need);
+    const uint32_t at = base + S_ENTRY * __popc(vote & lt_mask);
+    uint32_t nx = x, ne = e;
+    ByteState nb = b;
+    byte_next(nx, ne, nb, x2, need, at, ta, sym, rec_sa);
+    if (active) { x = nx; e = ne; b = nb; }
+    base += S_ENTRY * __popc(vote & grp_mask);
+    return need ? (at - base0) / S_ENTRY : NONE32;
+}
+
 template <int SINK, bool CRC, int CFN, int MODE>
 __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_stream(StreamArgs a)
 {
@@ -370,7 +442,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
     // word_pow[], word_mul16[] carry them to the piece's end.
     constexpr int NRA = SINK == SINK_BF16 ? 8 : 4;        // running values per lane: words of its unit of a row
     extern __shared__ __align__(16) uint8_t ssm[];
-    constexpr bool WIDE = CFN <= 0, SHARED = CFN < 0, MULT = SINK != SINK_DELTA;
+    constexpr bool WIDE = CFN <= 0, SHARED = CFN < 0, BYTES = CFN == F_BYTE_CFN, MULT = SINK != SINK_DELTA;
     // SINK_DELTA with CFN = 192: the two planes of a chunk have level-2 tables of different sizes, 128
     // entries for the exponent differences (a handful of symbols) and 256 for the sign/mantissa
     // differences, 768 bytes a stream on average.
@@ -390,10 +462,10 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
     const bool fits = s0 == F_SMEM_BASE && m_.end <= s0 + dynamic_smem_bytes();
     auto gen = [&](uint32_t sa) { return ssm + (sa - s0); };
     const uint32_t tab0 = m_.crc;
-    const uint32_t l1_sa = SHARED ? m_.l1 : WIDE ? m_.l1 + gi * F_WIDE_BYTES : m_.l1 + warp * 4096u + g * 4;
+    const uint32_t l1_sa = BYTES ? m_.l1 + gi * PROB_SCALE : SHARED ? m_.l1 : WIDE ? m_.l1 + gi * F_WIDE_BYTES : m_.l1 + warp * 4096u + g * 4;
     // (mixed sizes: the 1 KiB tables of the second planes first, then the half-KiB tables of the first planes)
     auto cf_of = [&](uint32_t grp) { return HYB ? ((grp & 1u) ? m_.cf + (grp >> 1) * 1024u : m_.cf + (G / 2) * 1024u + (grp >> 1) * 512u)
-                                               : m_.cf + grp * (WIDE ? 0u : 4u * CFN); };
+                                               : m_.cf + grp * (WIDE ? 0u : BYTES ? F_REC_STRIDE : 4u * CFN); };
     const uint32_t cf_sa = cf_of(gi);
     const uint32_t stage_sa = m_.stage + gi * F_STAGE;
     // SINK_BF16, SINK_F32: a tile is given out in units of four elements, unit u by lane u & 7, so that what a group loads
@@ -477,7 +549,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
     // the words follow table and states; the first four rounds are requested before the table is
     // built, which hides their latency
     Words<CFN, MODE> wd;
-    wd.sa = m_.tr + gi * tr_group(MODE);
+    wd.sa = m_.tr + gi * tr_group(CFN, MODE);
     wd.rd = wd.wr = 0;
     wd.lo = wd.hi = wd.lo2 = wd.hi2 = 0;
     uint32_t first[4][2];
@@ -522,7 +594,9 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
             uint32_t nlive = 0, max_live = 256;
             bool ok = false;
             uint32_t *tab = reinterpret_cast<uint32_t *>(gen(WIDE ? m_.l1 + (warp * 4 + gg) * F_WIDE_BYTES : m_.l1 + warp * 4096u + gg * 4));
-            if (WIDE) {
+            if (BYTES) {
+                if (on) ok = solo_tables<false>(fr[gg], m_.l1 + (warp * 4 + gg) * PROB_SCALE, cf_of(warp * 4 + gg), lane);
+            } else if (WIDE) {
                 if (on) ok = build_table<true>(fr[gg], tab, nullptr, lane);
             } else {
                 const bool small = HYB ? !(gg & 1u) : CFN < 256;
@@ -548,6 +622,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
         if (partner_n == 0) n = 0;
     }
     uint32_t e = 0;
+    ByteState by{};
     if (__any_sync(0xffffffffu, n != 0)) {
         // the whole ring, so that a group without a stream finds nothing but bounded entries in it
         const uint32_t lo = wd.lo, hi = wd.hi, lo2 = wd.lo2, hi2 = wd.hi2;
@@ -561,7 +636,8 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
         }
         wd.lo = lo; wd.hi = hi; wd.lo2 = lo2; wd.hi2 = hi2; wd.next = next; wd.left = left;
         if (n == 0) wd.retire();
-        e = lds_u32(slot_addr<CFN, MODE>(x, l1_sa, cf_sa));
+        if constexpr (BYTES) byte_next(x, e, by, x, false, 0u, (x & (PROB_SCALE - 1)) | l1_sa, lds_u8((x & (PROB_SCALE - 1)) | l1_sa), cf_sa);
+        else e = lds_u32(slot_addr<CFN, MODE>(x, l1_sa, cf_sa));
         __syncwarp();
     }
     uint8_t *out = a.dst + doff;
@@ -596,11 +672,17 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
     uint32_t ra[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     const bool was_open = open;
     uint32_t last_x = x, taken = 0;               // state and words consumed at the stream's end
+    // (F_BYTE_CFN: as 2^16 unrefilled, or as 1 with a word of zeros, whose entry is slot 0's)
+    auto rest = [&]() {
+        if (!BYTES) return x;
+        return x == RANS_LOW || (x == 1 && by.c == 0 && e == lds_u64(cf_sa + S_ENTRY * lds_u8(l1_sa)).x) ? RANS_LOW : 0u;
+    };
 
     // ---- tiles of 128 symbols ---------------------------------------------------------
     // FULL: every group of the warp that has symbols left has a whole tile of them.  (A group that has no
     // stream, or is done with it, runs along; nothing of its is kept.)
     uint32_t t = 0;
+    bool scarce = true;                           // some stream of the warp may have too few words for the next block
     auto tile = [&](auto full_c) {
         constexpr bool FULL = decltype(full_c)::value;
         const uint32_t done = t * TS;
@@ -620,11 +702,16 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
                 if (MODE == TR_FEW && rem > 5 * TS) prefetch_l2(pq + 4 * TS / 4 + 3 * k);
             }
         }
-        auto top_up = [&]() {
-            while (__any_sync(0xffffffffu, wd.low())) {
+        auto top_up = [&](uint32_t blocks = 1) {
+            while (__any_sync(0xffffffffu, wd.low(blocks))) {
                 wd.round(l1_sa, cf_sa, k);
                 __syncwarp();
             }
+        };
+        auto step4 = [&](auto first_c, uint32_t &hist, uint32_t base) {
+            constexpr bool FIRST = decltype(first_c)::value;
+            if constexpr (BYTES) byte_step4<FIRST>(x, e, by, hist, base, l1_sa, cf_sa, below, vsel);
+            else stream_step4<CFN, MODE, FIRST, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
         };
         auto put = [&](uint32_t step) { sts_u8(UNITS ? put_sa + 32 * (step & 3u) + 4 * (step >> 2) : stage_sa + step * NLANES + k, e); };
         auto fold = [&](uint32_t i) {
@@ -636,35 +723,42 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
                 // eight steps: two blocks, and where warps are few a round of translation between the
                 // steps of the first (where they are many, top_up does all of them: fewer instructions)
                 constexpr bool WOVEN = MODE != TR_4;
-                top_up();
+                // (F_BYTE_CFN has words for two blocks in its ring, and whether that will do for the block behind is asked
+                // while a block runs)
+                if (!BYTES) top_up();
+                else if (scarce) top_up(2);
+                if (BYTES) scarce = __any_sync(0xffffffffu, wd.low(2));
                 uint32_t base = wd.block(), hist = 0;
                 if (WOVEN) wd.part1();
                 put(s8);
-                stream_step4<CFN, MODE, true, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                step4(std::true_type{}, hist, base);
                 if (WOVEN) wd.part2(l1_sa, cf_sa);
                 put(s8 + 1);
-                stream_step4<CFN, MODE, false, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                step4(std::false_type{}, hist, base);
+                if (BYTES) wd.part2b(cf_sa);
                 fold(s8 / 2);
                 put(s8 + 2);
-                stream_step4<CFN, MODE, false, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
-                if (WOVEN) wd.part3(k);
+                step4(std::false_type{}, hist, base);
+                if (WOVEN) wd.part3(l1_sa, cf_sa, k);
                 put(s8 + 3);
-                stream_step4<CFN, MODE, false, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                step4(std::false_type{}, hist, base);
                 fold(s8 / 2 + 1);
                 wd.rd += tr_entry(MODE) * __popc(hist);
                 __syncwarp();
-                top_up();
+                if (!BYTES) top_up();
+                else if (scarce) top_up(2);
+                if (BYTES) scarce = __any_sync(0xffffffffu, wd.low(2));
                 base = wd.block();
                 hist = 0;
                 put(s8 + 4);
-                stream_step4<CFN, MODE, true, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                step4(std::true_type{}, hist, base);
                 put(s8 + 5);
-                stream_step4<CFN, MODE, false, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                step4(std::false_type{}, hist, base);
                 fold(s8 / 2 + 2);
                 put(s8 + 6);
-                stream_step4<CFN, MODE, false, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                step4(std::false_type{}, hist, base);
                 put(s8 + 7);
-                stream_step4<CFN, MODE, false, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
+                step4(std::false_type{}, hist, base);
                 fold(s8 / 2 + 3);
                 wd.rd += tr_entry(MODE) * __popc(hist);
             }
@@ -680,7 +774,9 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
                 for (uint32_t s = s4; s < s4 + 4; s++) {
                     const bool active = s * NLANES + k < rem;
                     if (active) put(s);
-                    const uint32_t ahead = stream_step<CFN, MODE, MULT>(x, e, base, base0, l1_sa, cf_sa, lt_mask, grp_mask, active);
+                    uint32_t ahead;
+                    if constexpr (BYTES) ahead = byte_step(x, e, by, base, base0, l1_sa, cf_sa, lt_mask, grp_mask, active);
+                    else ahead = stream_step<CFN, MODE, MULT>(x, e, base, base0, l1_sa, cf_sa, lt_mask, grp_mask, active);
                     if (SINK == SINK_OPEN) {
                         // the first lane that took a word the stream has not got ends an open stream:
                         // `ahead` words had been taken in this block before it took its own
@@ -696,6 +792,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
                 }
                 wd.rd += base - base0;
             }
+            scarce = true;
         }
         __syncwarp();
         uint32_t pw[SINK == SINK_F32 ? 4 : 1][3];
@@ -870,7 +967,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
             if (__all_sync(0xffffffffu, n <= done || n - done >= TS)) tile(std::true_type{});
             else tile(std::false_type{});
             t++;
-            if (t == my_tiles) { last_x = x; taken = wd.taken(slen - LEAD); wd.retire(); }
+            if (t == my_tiles) { last_x = rest(); taken = wd.taken(slen - LEAD); wd.retire(); }
         }
     } else {
     // Tiles are decoded in runs of whole ones, with nothing to watch inside a run: as many as the
@@ -890,7 +987,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
             tile(std::false_type{});
             t++;
         }
-        if (t == my_tiles) { last_x = x; taken = wd.taken(slen - LEAD); wd.retire(); }
+        if (t == my_tiles) { last_x = rest(); taken = wd.taken(slen - LEAD); wd.retire(); }
     }
     }
 

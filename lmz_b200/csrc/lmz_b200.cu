@@ -129,14 +129,34 @@ static int launch_solo(const StreamArgs &a, cudaStream_t cs)
     return l.wide ? launch_solo_as<SINK, CRC, true>(a, l.grid, l.warps, cs) : launch_solo_as<SINK, CRC, false>(a, l.grid, l.warps, cs);
 }
 
-// Up to so many streams per SM a warp each is faster than four to a warp.  (One B200, exponent planes of 32 KiB:
-// 4 per SM 183 against 281 us, 12 262 against 282, 20 345 against 382, 28 449 against 385.  With the sinks' own work
-// in the same issue slots: 12 64 KiB BF16 chunks with checksums per SM 395 against 489 us, 18 as long either way.)
-static bool solo_fits(const StreamArgs &a, bool sink, int sms)
+// Launches of few streams, with nothing to sort by: a warp each up to so many per SM, then four to a warp as long as
+// byte tables (F_BYTE_CFN) take the launch in one round.  1 when they are more.
+//
+// One B200, us, compact tables / a warp each / byte tables.  Exponent planes of 32 KiB: 16 per SM 382 / 353 / 352, 20 per SM
+// 401 / 405 / 378, 24 per SM 445 / - / 370; uniform bytes 20 per SM - / 417 / 455, 24 per SM 478 / - / 460: a warp each up to 20.
+// With the sinks' own work in the same issue slots, 64 KiB BF16 chunks with checksums: 12 per SM 489 / 362 / 438, 16 per SM
+// 489 / 410 / 440, 20 per SM 521 / - / 458, 24 per SM 521 / - / 454; FP32 ones: 16 per SM - / 307 / 312, 20 per SM
+// 357 / - / 350, 24 per SM 387 / - / 365: a warp each up to 16.  Open streams have no byte-table instance.
+template <int SINK, bool CRC>
+static int launch_few(const StreamArgs &a, cudaStream_t cs)
 {
+    if (a.njobs == 0) return LMZ_GPU_OK;
+    int rc = stream_smem_ok();
+    if (rc) return rc;
+    int sms = 0;
+    rc = sm_count(&sms);
+    if (rc) return rc;
     const int forced = g_force_table_mode.load(std::memory_order_relaxed);
-    if (forced >= 0) return forced == T_SOLO_WIDE || forced == T_SOLO_BYTES;
-    return a.njobs <= (sink ? 16ull : 20ull) * (a.most_ctas ? a.most_ctas : (uint32_t)sms);
+    const uint64_t room = a.most_ctas ? a.most_ctas : (uint32_t)sms;
+    constexpr uint32_t solo = SINK == SINK_BYTES || SINK == SINK_OPEN ? 20 : 16;
+    if (forced >= 0 ? forced == T_SOLO_WIDE || forced == T_SOLO_BYTES : a.njobs <= solo * room) return launch_solo<SINK, CRC>(a, cs);
+    if constexpr (SINK != SINK_OPEN) {
+        if (forced < 0 && a.njobs <= 4 * stream_warps(F_BYTE_CFN, CRC, SINK, TR_FEW) * room) {
+            const uint32_t quads = (a.njobs + 3) / 4, grid = quads < room ? quads : (uint32_t)room;
+            return launch_stream_as<SINK, CRC, F_BYTE_CFN, TR_FEW>(a, grid, (quads + grid - 1) / grid, cs);
+        }
+    }
+    return 1;
 }
 
 // CFN = 128 is for streams the caller knows to have at most F_SMALL_LIVE live symbols;
@@ -271,7 +291,7 @@ static int launch_compact_sorted(const RansArgs &a, cudaStream_t cs)
     return rc;
 }
 
-// Streams that carry their own table.  Up to 20 per SM (solo_fits) a warp each; up to 76 per SM the full-size compact
+// Streams that carry their own table.  Few of them: launch_few; up to 76 per SM the full-size compact
 // tables take the launch in one round, whatever the alphabets; above that small alphabets go to the denser instance.
 constexpr unsigned COMPACT_PER_SM = 4 * stream_warps(256, false, SINK_BYTES, TR_8);
 
@@ -284,9 +304,9 @@ static int launch_rans(const RansArgs &a, cudaStream_t cs, bool may_alloc = true
     const StreamArgs sa = as_stream_args(a);
     if (a.shared_hdr) return launch_stream<SINK_BYTES, false, -1>(sa, cs);
     const int forced = g_force_table_mode.load(std::memory_order_relaxed);
-    const bool solo = solo_fits(sa, false, sms);
-    if (a.open) return solo ? launch_solo<SINK_OPEN, false>(sa, cs) : launch_stream<SINK_OPEN, false, 256>(sa, cs);
-    if (solo) return launch_solo<SINK_BYTES, false>(sa, cs);
+    rc = a.open ? launch_few<SINK_OPEN, false>(sa, cs) : launch_few<SINK_BYTES, false>(sa, cs);
+    if (rc != 1) return rc;
+    if (a.open) return launch_stream<SINK_OPEN, false, 256>(sa, cs);
     if (may_alloc && forced < 0 && a.njobs > (unsigned)sms * COMPACT_PER_SM) {
         rc = launch_compact_sorted(a, cs);
         if (rc != 1) return rc;

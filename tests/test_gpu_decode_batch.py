@@ -314,3 +314,25 @@ def test_batches_around_the_lines_between_kernels(gpu, orc, per_sm, plane, table
     want = np.stack([pool[i % 61] for i in range(nstr)])
     bad = np.nonzero((out != want).any(axis=1))[0]
     assert bad.size == 0, bad[:10]
+
+
+@pytest.mark.parametrize("table_mode", [-1], ids=["auto"], indirect=True)
+@pytest.mark.parametrize("nstr", [148 * 20, 148 * 20 + 1, 148 * 28 - 1, 148 * 28 + 1])
+@pytest.mark.parametrize("plane", [1, 17, 129, 1000, 4097])
+def test_device_batches_around_the_lines_between_kernels(gpu, nstr, plane, table_mode):
+    """20 and 28 streams per SM (of 148) and one more: a warp each, byte tables for four to a warp, compact tables; planes
+    that end anywhere in a tile, alphabets of one symbol to all of them, and one stream a word short."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(nstr + plane)
+    u = torch.rand((nstr, plane), generator=gen, device="cuda")
+    kind = (torch.arange(nstr, device="cuda") % 5)[:, None]
+    flat, few = (u * 256).to(torch.int32), torch.log2(1 / (1 - u)).clamp_(max=40).to(torch.int32)
+    planes = torch.where(kind == 0, flat, torch.where(kind == 1, few + 100, torch.where(kind == 2, torch.full_like(flat, 7),
+                         torch.where(kind == 3, (flat > 250).to(torch.int32), (flat * flat) >> 8)))).to(torch.uint8)
+    streams, offsets = gpu.encode_batch(planes.reshape(-1), nstr, plane)
+    assert torch.equal(gpu.decode_batch(streams, offsets, nstr, plane).view(nstr, plane), planes)
+    if plane >= 129:
+        short = offsets.clone()
+        short[2 * (nstr - nstr % 5 - 5) + 1] -= 2              # (a flat one)
+        with pytest.raises(ValueError):
+            gpu.decode_batch(streams, short, nstr, plane)
