@@ -124,6 +124,11 @@ __device__ __forceinline__ void prefetch_l2(const void *p)
 }
 
 // The same where `on`, without a branch.
+__device__ __forceinline__ void lds_u64_if(uint32_t on, uint32_t a, uint2 &v)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\t@p ld.shared.v2.u32 {%0,%1}, [%2];\n\t}"
+                 : "+r"(v.x), "+r"(v.y) : "r"(a), "r"(on));
+}
 __device__ __forceinline__ void sts_u8_if(uint32_t on, uint32_t a, uint32_t v)
 {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.shared.u8 [%0], %1;\n\t}"

@@ -10,21 +10,24 @@
 //                  word's own, so it is worked out before the word is asked for (32 words at a time,
 //                  one a lane) and waits in a ring
 //
-// Ring and tables hold the same 8-byte entries, {f << 8 | symbol, c}, so that one load serves both kinds of
-// lanes, from an address picked behind the vote.
+// Ring and tables hold the same 8-byte entries, {f << 8 | symbol, c}.
 //
-//   WIDE      an entry per slot: 32 KiB a stream
+//   WIDE      an entry per slot: 32 KiB a stream.  A lane without a refill loads its entry while the vote is under way, one with a
+//             refill behind it: two loads, of which a lane takes part in one, into the same registers, with nothing to pick
+//             between them
 //   else      a byte per slot, its symbol (4 KiB), looked up while the vote is under way, and an entry
-//             per symbol whose c is -start: the slot is added to what was loaded
+//             per symbol whose c is -start: the slot is added to what was loaded.  One load serves both kinds of lanes, from an
+//             address picked behind the vote, as warps are many enough here for a load's slot to count (12 streams
+//             per SM 316 us, 329 with two)
 //
 // Measured on one B200, cycles: multiply-add 4, compare and vote 17, and 4, permute 4, dot product 4,
 // load 23; a popcount is 17, so the lanes below are counted by a byte permute that looks three votes
 // up at a time and a dot product that adds them.  For that the eight lanes sit three to a nibble of
 // the vote; the other twenty-four run along, vote for nothing and write nothing.
 //
-// One B200, k_stream's wide tables against this: a lone stream 61.5 -> 41.9 ns a step (84 cycles, 25 instructions), a
-// 4096 x 14336 BF16 tensor in 64 KiB chunks 480 -> 382 us (issue slots 67 % busy, 31 instructions a stream's step), in 8 MiB
-// chunks 34.1 -> 23.1 ms, seven planes of 4 KiB between host buffers 78 -> 58 us.  Uniform bytes, four words a
+// One B200, k_stream's wide tables against this: a lone stream 61.5 -> 38.5 ns a step (41.9 with one load behind a pick), a
+// 4096 x 14336 BF16 tensor in 64 KiB chunks 480 -> 381 us (issue slots 67 % busy, 31 instructions a stream's step), in 8 MiB
+// chunks 34.1 -> 22.3 ms (23.1 with one load), seven planes of 4 KiB between host buffers 78 -> 58 us.  Uniform bytes, four words a
 // step, cost no more than exponents with one and a third.  Where the store of a step's symbols stands matters: behind the
 // vote, or behind the load, a lone stream's 8 MiB took 24.6 ms instead of 23.1.
 //
@@ -188,9 +191,12 @@ __global__ void __launch_bounds__(solo_warps(CRC, WIDE) * 32, 1) k_solo(StreamAr
                 x2 = y * (e >> 8) + c;
                 const uint32_t ta = slot_at(x2), s = byte_at(ta);
                 const bool need = owner && x2 < RANS_LOW;
+                uint2 r = {0, 0};
+                if (WIDE) lds_u64_if(!need, ta, r);             // (on its way while the vote is)
                 const uint32_t vote = __ballot_sync(0xffffffffu, need);
                 const uint32_t at = __dp4a(__byte_perm(0x02010100u, 0x03020201u, vote & below), S_ENTRY * 0x01010101u, base);
-                const uint2 r = lds_u64(need ? at : entry_at(ta, s));
+                if (WIDE) lds_u64_if(need, at, r);
+                else r = lds_u64(need ? at : entry_at(ta, s));
                 y = need ? x2 * 16 : x2 >> PROB_BITS;
                 e = r.x;
                 c = WIDE ? r.y : r.y + (need ? 0u : ta);
