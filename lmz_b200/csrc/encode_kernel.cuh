@@ -32,7 +32,9 @@
 // by one, so that a batch spreads evenly.
 //
 // One B200, with places and states in one chain and the loads waited for: 4096 planes of 32 KiB of BF16
-// exponents 485 -> 309 us (434 GB/s of symbols), 592 of them 376 -> 219, 28000 of 1 KiB 218 -> 162.
+// exponents 485 -> 309 us, 592 of them 376 -> 219, 28000 of 1 KiB 218 -> 162.  With the groups' tiles in different banks (a third of
+// the load/store unit's wavefronts were conflicts, most of them there) and one popcount a step instead of two, through the
+// public call: 4096 planes 411 -> 384 us, 8288 of them 786 -> 750, 8288 of 4 KiB of uniform bytes 318 -> 289.
 #pragma once
 #include "common.cuh"
 
@@ -48,8 +50,10 @@ struct EncodeArgs {
 };
 
 constexpr uint32_t E_BUF = 384, E_TILE = 128;            // a piece of 128 bytes and what a tile can add to it
+// (the groups' buffers and tiles lie four banks apart: side by side, all four would read the same two banks at every step)
+constexpr uint32_t E_BUF_STRIDE = E_BUF + 16, E_TILE_STRIDE = E_TILE + 16;
 constexpr uint32_t E_TABLE = 4096;                    // 256 entries of 16 bytes; until then the group's share of the counters
-constexpr uint32_t E_GROUP_BYTES = E_TABLE + E_BUF + E_TILE;
+constexpr uint32_t E_GROUP_BYTES = E_TABLE + E_BUF_STRIDE + E_TILE_STRIDE;
 constexpr uint32_t E_COUNT_MAX = 8u * 64000u;         // symbols counted before the lanes' 16-bit counters are summed
 __host__ __device__ constexpr uint32_t encode_smem_bytes() { return 4 * E_GROUP_BYTES; }
 __host__ __device__ constexpr uint32_t encode_slot_bytes(uint32_t plane)
@@ -86,8 +90,8 @@ __global__ void __launch_bounds__(32) k_encode(EncodeArgs a)
     // counters of the whole warp, then the four groups' tables, in the same 16 KiB; buffers and tiles behind
     uint32_t *counters = reinterpret_cast<uint32_t *>(esm);
     uint8_t *const gp = esm + (size_t)g * E_TABLE;
-    uint8_t *buf = esm + 4 * E_TABLE + g * E_BUF;
-    uint8_t *tile = esm + 4 * (E_TABLE + E_BUF) + g * E_TILE;
+    uint8_t *buf = esm + 4 * E_TABLE + g * E_BUF_STRIDE;
+    uint8_t *tile = esm + 4 * (E_TABLE + E_BUF_STRIDE) + g * E_TILE_STRIDE;
     const uint32_t buf_sa = smem_addr(buf), tile_sa = smem_addr(tile), tab_sa = smem_addr(gp);
 
     const uint32_t job = blockIdx.x * 4 + g;
@@ -256,6 +260,7 @@ __global__ void __launch_bounds__(32) k_encode(EncodeArgs a)
     const uint32_t tiles = (T + 15) / 16;
     const uint32_t warp_tiles = __reduce_max_sync(0xffffffffu, tiles);
     uint32_t x = RANS_LOW, flushed = 0, pos = buf_sa + E_BUF;   // words grow down from `pos`; bytes counted back from the slot's end
+    const uint32_t above = 0xffffff00u | (0xfeu << k & 0xffu);
     // a tile's 128 symbols (lane k: bytes 16 k .. 16 k + 15), requested a tile ahead
     const bool aligned = (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
     auto fetch = [&](uint32_t tt) {
@@ -297,13 +302,13 @@ __global__ void __launch_bounds__(32) k_encode(EncodeArgs a)
         uint4 e0 = lds_u128(at[15]), e1 = lds_u128(at[14]);
         const bool full = __all_sync(0xffffffffu, mine_tile && tt * 128 + 128 <= n);
         // A step's words are placed while the next step's states are worked out: the vote's byte, its
-        // popcounts and the address are a chain as long as the state's own.
-        uint32_t votes = 0, word = 0;
+        // popcount and the address are a chain as long as the state's own.  `hist` collects the votes of four steps, the newest
+        // in byte 0: the words before this lane's, counted back from `pos`, are the older bytes' and the lanes' above it.
+        uint32_t hist = 0, word = 0;
         bool out = false;
-        auto place = [&]() {
-            // (the lanes above this one come before it, counted back from `pos`)
-            sts_u16_if(out, pos - 2 * __popc(votes >> (k + 1)) - 2, word);
-            pos -= 2 * __popc(votes);
+        auto place = [&](bool last) {
+            sts_u16_if(out, pos - 2 * __popc(hist & above) - 2, word);
+            if (last) pos -= 2 * __popc(hist);
         };
         auto step = [&](int s, bool active) {
             const uint4 e = e0;
@@ -314,13 +319,13 @@ __global__ void __launch_bounds__(32) k_encode(EncodeArgs a)
             const uint32_t vote = __ballot_sync(0xffffffffu, need);
             if (need) v >>= 16;
             const uint64_t p = (uint64_t)v * e.x + e.y;
-            if (s < 15) place();
+            if (s < 15) place((s & 3) == 3);
             word = x;
             out = need;
-            const uint32_t q = (uint32_t)(p >> 32) >> (e.w & 31u);
+            const uint32_t q = __funnelshift_r((uint32_t)(p >> 32), 0u, e.w);          // (by the low five bits)
             const uint32_t nx = v + (e.w >> 20) + q * ((e.w >> 8) & 0xfffu);
             if (active) x = nx;
-            votes = __byte_perm(vote, 0u, 0x4440u + g);
+            hist = __byte_perm(vote, (s & 3) == 3 ? 0u : hist, 0x6540u + g);
         };
         if (full) {
 #pragma unroll
@@ -329,7 +334,7 @@ __global__ void __launch_bounds__(32) k_encode(EncodeArgs a)
 #pragma unroll
             for (int s = 15; s >= 0; s--) step(s, mine_tile && tt * 128 + s * 8 + k < n);
         }
-        place();
+        place(true);
         // whole 128-byte pieces leave the buffer, what is left of one moves up to its end
         const uint32_t whole = (buf_sa + E_BUF - pos) / 128;
         if (__any_sync(0xffffffffu, whole != 0)) {
