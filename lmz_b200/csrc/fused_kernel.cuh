@@ -198,12 +198,18 @@ __device__ __forceinline__ uint32_t slot_ref(uint32_t x, uint32_t l1_sa, uint32_
     const uint32_t e1 = lds_u32((x & 0xff0u) | l1_sa);
     return high_half_add(e1, from + 4u * __popc(e1 << ((~x & 15u) | 16u)));
 }
-// Its address.  (TR_4 adds the tables' address last, as a ring entry's is added: four 8B layers 1711 us, 1800 with a sum of three;
-// 28577 streams of 32 KiB of the others 1576 and 1535.)
+// Its address.  One B200: TR_4 adds the tables' address last, as a ring entry's is added (four 8B layers 1711 us, 1800 with a sum
+// of three); TR_8 first (28577 streams of 32 KiB 1535 us, 1576 with it last); TR_FEW, whose warps have the integer pipe almost to
+// themselves, takes the offset by a shift (44 BF16 chunks per SM 586 us, 603 by a dot product), but not in the delta sink's
+// mixed tables (a delta chain 1525 and 1519).
 template <int CFN, int MODE>
 __device__ __forceinline__ uint32_t slot_addr(uint32_t x, uint32_t l1_sa, uint32_t cf_sa)
 {
     if (CFN > 0 && MODE == TR_4) return cf_sa + slot_ref<CFN>(x, l1_sa, 0u);
+    if (CFN > 0 && MODE == TR_FEW && CFN != F_HYBRID_CFN) {
+        const uint32_t e1 = lds_u32((x & 0xff0u) | l1_sa);
+        return cf_sa + ((e1 >> 16) + 4u * __popc(e1 << ((~x & 15u) | 16u)));
+    }
     return slot_ref<CFN>(x, l1_sa, cf_sa);
 }
 
@@ -391,8 +397,8 @@ __device__ __forceinline__ uint32_t stream_step(uint32_t &x, uint32_t &e, uint32
 }
 
 // F_BYTE_CFN's steps, as k_solo's: of a state x only y, e and c are kept, of which the next (unrefilled) one is
-// y * (e >> 8) + c.  (One B200: 83 ns a step up to 16 streams per SM, 90 with 24, where the compact tables take 93 and 107.
-// Two predicated loads instead of the selected one, as k_solo has them: 90 with 16.)
+// y * (e >> 8) + c.  (One B200, planes of 32 KiB: 342 us up to 16 streams per SM, 370 with 24, where the compact tables
+// take 382 and 445.  With two predicated loads instead of the picked one, as k_solo has them: 377 and 402.)
 struct ByteState {
     uint32_t y, c;
 };
