@@ -695,7 +695,8 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
         uint32_t rem = n > done ? n - done : 0;
         __syncwarp();
         // SINK_F32: the tile's stored bytes are requested before the decode, which hides
-        // their latency: of each plane's 33 words around them every eighth from k on, the last by lane 0
+        // their latency: of each plane's 33 words around them every eighth from k on, the last by lane 0.  (A plane may start
+        // three bytes into a word: `rem` bytes of it reach into word w where rem + 3 > 4 w.)
         uint32_t pr[SINK == SINK_F32 ? 3 : 1][5];
         if constexpr (SINK == SINK_F32) {
 #pragma unroll
@@ -704,7 +705,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
                 const uint32_t *pq = reinterpret_cast<const uint32_t *>(reinterpret_cast<uintptr_t>(pp) & ~uintptr_t(3)) + k;
 #pragma unroll
                 for (int i = 0; i < 4; i++) pr[j][i] = rem && (FULL || rem + 3 > 4 * (k + 8 * i)) ? __ldg(pq + 8 * i) : 0u;
-                pr[j][4] = k == 0 && rem >= TS ? __ldg(pq + 32) : 0u;
+                pr[j][4] = k == 0 && rem + 3 > TS ? __ldg(pq + 32) : 0u;
                 if (MODE == TR_FEW && rem > 5 * TS) prefetch_l2(pq + 4 * TS / 4 + 3 * k);
             }
         }

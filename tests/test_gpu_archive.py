@@ -572,6 +572,44 @@ def test_bf16_rows_in_each_layout(layout, lead, tail):
         assert dec.plan.fused_jobs.size == 3
 
 
+@pytest.mark.parametrize("tail", [0, 1, 3, 4, 5, 31, 32, 33, 124, 125, 126, 127])
+def test_fp32_rows_in_each_layout(layout, tail):
+    """The FP32 sinks' units of four elements, from stored planes that are read as words: chunks that end anywhere in a unit,
+    their planes starting at each of a word's four bytes."""
+    n, members = 16384 + 8192 + tail, []
+    for i in range(24):
+        w = (np.random.default_rng(100 * i + tail).standard_normal(n) * 0.02).astype("<f4")
+        if i in (8, 16):                         # (moves what follows by a byte: streams are of even length)
+            members.append((f"{i}.bin", np.full(i // 8, 7, np.uint8)))
+        members.append((f"{i}.safetensors", synth.safetensors_bytes([(f"w{i}", "F32", (n,), w.view(np.uint8))])))
+    blob = oa.write_archive(members, mapped=True)
+    source = np.concatenate([m for _name, m in members])
+    for checksum in (True, False):
+        dec = _roundtrip(blob, source, checksum=checksum, fuse="all")
+        jobs = dec.plan.fused_jobs
+        assert dec.plan.n_fused_f32 == 48
+        assert set((jobs["mant_off"][jobs["n"] == 8192 + tail] % 4).tolist()) == {0, 1, 2, 3}
+
+
+@pytest.mark.parametrize("tail", [125, 126, 127])
+@pytest.mark.parametrize("checksum", [True, False])
+def test_fp32_tails_of_a_large_archive(gpu, tail, checksum):
+    """More FP32 chunks than the planner's line, by its own choice, the last one ragged: with 127 elements behind its last whole tile
+    one of the three planes, whatever the first one's phase, reaches into a word of its own."""
+    import torch
+    from lmz_b200 import decode
+    from perf import cases
+    case = dict(path="archive", dtype="F32", layers=0, hidden=378 * 128 + 128 - tail, ffn=4095, kv=0, chunk=65536)
+    whole, rest = divmod(cases._elements(case), 16384)
+    assert rest % 128 == tail and rest > 4096
+    dec = decode.ArchiveDecoder(cases._archive(case, tail), checksum=checksum)
+    assert dec.plan.n_fused_f32 == whole + 1 and dec.plan.fused_jobs["n"].min() == rest
+    out = dec.run()
+    dec.check()
+    head, data, _meta = cases._checkpoint(case, torch.Generator(device="cuda").manual_seed(tail))
+    assert torch.equal(out[len(head):len(head) + data.numel()], data)
+
+
 @pytest.mark.parametrize("nchunks", [1184, 1185, 9473])
 @pytest.mark.parametrize("checksum", [True, False])
 def test_bf16_chunks_by_how_many_there_are(gpu, tmp_path, nchunks, checksum):
