@@ -28,15 +28,17 @@
 // and, two steps ahead, their table entries are loaded before the state needs them, and the division
 // by the symbol's frequency is exact in one multiply-add and a shift (a multiplier and an addend per
 // frequency: N. Robison's choice between rounding the reciprocal up and rounding it down, of which one
-// always works), with no correction after it.  A warp is a CTA: 18 KiB of shared memory, dealt out one
-// by one, so that a batch spreads evenly.
+// always works), with no correction after it.  A warp is a CTA: 17.6 KiB of shared memory (encode_layout.cuh), twelve
+// to an SM, dealt out one by one, so that a batch spreads evenly.
 //
 // One B200, with places and states in one chain and the loads waited for: 4096 planes of 32 KiB of BF16
 // exponents 485 -> 309 us, 592 of them 376 -> 219, 28000 of 1 KiB 218 -> 162.  With the groups' tiles in different banks (a third of
 // the load/store unit's wavefronts were conflicts, most of them there) and one popcount a step instead of two, through the
-// public call: 4096 planes 411 -> 384 us, 8288 of them 786 -> 750, 8288 of 4 KiB of uniform bytes 318 -> 289.
+// public call: 4096 planes 411 -> 384 us, 8288 of them 786 -> 750, 8288 of 4 KiB of uniform bytes 318 -> 289.  (Tiles of their own
+// beside the buffers left room for eleven CTAs per SM: 6800 planes, a round of twelve, 528 us of kernel instead of 369.)
 #pragma once
 #include "common.cuh"
+#include "encode_layout.cuh"
 
 namespace lmz {
 
@@ -49,13 +51,7 @@ struct EncodeArgs {
     uint32_t *lengths;      // per stream: bytes written at the end of its slot, 0 = failed
 };
 
-constexpr uint32_t E_BUF = 384, E_TILE = 128;            // a piece of 128 bytes and what a tile can add to it
-// (the groups' buffers and tiles lie four banks apart: side by side, all four would read the same two banks at every step)
-constexpr uint32_t E_BUF_STRIDE = E_BUF + 16, E_TILE_STRIDE = E_TILE + 16;
-constexpr uint32_t E_TABLE = 4096;                    // 256 entries of 16 bytes; until then the group's share of the counters
-constexpr uint32_t E_GROUP_BYTES = E_TABLE + E_BUF_STRIDE + E_TILE_STRIDE;
 constexpr uint32_t E_COUNT_MAX = 8u * 64000u;         // symbols counted before the lanes' 16-bit counters are summed
-__host__ __device__ constexpr uint32_t encode_smem_bytes() { return 4 * E_GROUP_BYTES; }
 __host__ __device__ constexpr uint32_t encode_slot_bytes(uint32_t plane)
 {
     return (HDR_BYTES + STATE_BYTES + 2u * plane + 64u + 511u) & ~511u;
@@ -87,12 +83,11 @@ __global__ void __launch_bounds__(32) k_encode(EncodeArgs a)
     extern __shared__ __align__(512) uint8_t esm[];
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t k = lane & 7u, g = lane >> 3;
-    // counters of the whole warp, then the four groups' tables, in the same 16 KiB; buffers and tiles behind
+    // counters of the whole warp, then the four groups' tables, in the same 16 KiB; their buffers behind
     uint32_t *counters = reinterpret_cast<uint32_t *>(esm);
     uint8_t *const gp = esm + (size_t)g * E_TABLE;
-    uint8_t *buf = esm + 4 * E_TABLE + g * E_BUF_STRIDE;
-    uint8_t *tile = esm + 4 * (E_TABLE + E_BUF_STRIDE) + g * E_TILE_STRIDE;
-    const uint32_t buf_sa = smem_addr(buf), tile_sa = smem_addr(tile), tab_sa = smem_addr(gp);
+    uint8_t *buf = esm + encode_buffer(g);
+    const uint32_t buf_sa = smem_addr(buf), tile_sa = buf_sa, tab_sa = smem_addr(gp);
 
     const uint32_t job = blockIdx.x * 4 + g;
     const bool have = job < a.nstr;
@@ -299,6 +294,7 @@ __global__ void __launch_bounds__(32) k_encode(EncodeArgs a)
         uint32_t at[16];
 #pragma unroll
         for (int s = 15; s >= 0; s--) at[s] = tab_sa + 16 * lds_u8(tile_sa + s * 8 + k);
+        __syncwarp();                                    // (words may lie where the tile did)
         uint4 e0 = lds_u128(at[15]), e1 = lds_u128(at[14]);
         const bool full = __all_sync(0xffffffffu, mine_tile && tt * 128 + 128 <= n);
         // A step's words are placed while the next step's states are worked out: the vote's byte, its

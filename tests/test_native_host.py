@@ -55,6 +55,17 @@ def test_a_warp_per_stream(solo_layout, check):
 
 
 @pytest.fixture(scope="module")
+def encode_layout(tmp_path_factory):
+    return _compiled(tmp_path_factory, "encode_layout_check")
+
+
+@pytest.mark.parametrize("check", ["residents", "buffers", "banks"])
+def test_the_encoders_shared_memory(encode_layout, check):
+    done = subprocess.run([encode_layout, check], capture_output=True, text=True, timeout=20)
+    assert done.returncode == 0, done.stderr
+
+
+@pytest.fixture(scope="module")
 def host_pool(tmp_path_factory):
     return _compiled(tmp_path_factory, "host_pool_check")
 
