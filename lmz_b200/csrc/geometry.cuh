@@ -20,6 +20,11 @@ constexpr uint32_t F_CRC_BYTES = 32768;             // four slice tables x 256 e
 // counted.
 constexpr uint32_t F_SMEM_BASE = 1024, F_SMEM_DYN = 232448, F_SMEM_SM = F_SMEM_BASE + F_SMEM_DYN;
 
+// Dynamic shared memory of a CTA that needs `bytes`, where no SM is to take two of them while another has none: more than half
+// of what an SM has.
+LMZ_HD constexpr uint32_t alone_on_sm(uint32_t bytes) { return bytes < F_SMEM_SM / 2 ? F_SMEM_SM / 2 : bytes; }
+static_assert(2 * (F_SMEM_BASE + alone_on_sm(0)) > F_SMEM_SM && alone_on_sm(0) <= F_SMEM_DYN, "one, and it can be had");
+
 // Tiles of `tile` symbols that n symbols take.  A plane may have any n of 32 bits, so a kernel counts tiles: n + tile - 1
 // and the offset behind the last tile can be more than 32 bits hold.
 LMZ_HD constexpr uint32_t tiles_of(uint32_t n, uint32_t tile) { return n / tile + (n % tile != 0); }

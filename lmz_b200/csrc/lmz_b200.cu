@@ -83,7 +83,12 @@ template <int SINK, bool CRC, int CFN, int MODE>
 static int launch_stream_as(const StreamArgs &a, uint32_t grid, uint32_t W, cudaStream_t cs)
 {
     static bool done[64];
-    const uint32_t shm = stream_smem(CFN, CRC, SINK, MODE, W).end - F_SMEM_BASE;
+    // A launch is of one CTA per SM at most, and as long as its fullest SM.  Beside the kernel for an archive's other chunks, whose
+    // CTAs with checksum tables hold an SM when this one starts, CTAs of up to seven warps went two to another SM.  (One B200,
+    // chunks with checksums, 28 per SM: BF16 634 -> 491 us, FP32 455 -> 366; 32 per SM, whose CTAs are larger, 494 and 370
+    // either way.  Without checksums, and of planes alone, none were seen to, and launches of several threads may share an SM.)
+    uint32_t shm = stream_smem(CFN, CRC, SINK, MODE, W).end - F_SMEM_BASE;
+    if (CRC && CFN > 0 && SINK != SINK_DELTA) shm = alone_on_sm(shm);
     int rc = opt_in_smem(k_stream<SINK, CRC, CFN, MODE>, F_SMEM_DYN, done);
     if (rc) return rc;
     k_stream<SINK, CRC, CFN, MODE><<<grid, W * 32, shm, cs>>>(a);
@@ -132,11 +137,15 @@ static int launch_solo(const StreamArgs &a, cudaStream_t cs)
 // Launches of few streams, with nothing to sort by: a warp each up to so many per SM, then four to a warp as long as
 // byte tables (F_BYTE_CFN) take the launch in one round.  1 when they are more.
 //
-// One B200, us, compact tables / a warp each / byte tables.  Exponent planes of 32 KiB: 16 per SM 382 / 353 / 352, 20 per SM
-// 401 / 405 / 378, 24 per SM 445 / - / 370; uniform bytes 20 per SM - / 417 / 455, 24 per SM 478 / - / 460: a warp each up to 20.
-// With the sinks' own work in the same issue slots, 64 KiB BF16 chunks with checksums: 12 per SM 489 / 362 / 438, 16 per SM
-// 489 / 410 / 440, 20 per SM 521 / - / 458, 24 per SM 521 / - / 454; FP32 ones: 16 per SM - / 307 / 312, 20 per SM
-// 357 / - / 350, 24 per SM 387 / - / 365: a warp each up to 16.  Open streams have no byte-table instance.
+// One B200, us, compact tables / a warp each / byte tables.  Exponent planes of 32 KiB: 16 per SM - / 301 / 283, 20 per SM
+// - / 347 / 307, 24 per SM 379 / - / 308, 28 per SM 381 / - / 309; uniform bytes 16 per SM - / 306 / 385, 20 per SM - / 358 / 397,
+// 24 per SM 418 / - / 399, 28 per SM 422 / - / 402; planes of 4 KiB, exponents 20 per SM - / 55 / 57, 24 per SM 68 / - / 58, uniform
+// bytes - / 57 / 70 and 72 / - / 70: a warp each up to 20.
+// With the sinks' own work in the same issue slots, 64 KiB BF16 chunks with checksums: 12 per SM - / 325 / 405, 16 per SM
+// - / 373 / 407, 17 per SM 483 / - / 417, 24 per SM 489 / - / 422; FP32 ones: 12 per SM - / 257 / 268, 16 per SM - / 296 / 268,
+// 17 per SM 358 / - / 272, 24 per SM 363 / - / 287; without checksums 28 per SM, BF16 464 / - / 380, FP32 326 / - / 243: a warp each up
+// to 16 (FP32 chunks, which come here only where a caller has few of them fused, share the line of BF16's).
+// Open streams have no byte-table instance.
 template <int SINK, bool CRC>
 static int launch_few(const StreamArgs &a, cudaStream_t cs)
 {

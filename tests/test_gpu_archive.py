@@ -781,3 +781,32 @@ def test_launches_are_counted_as_they_happen(gpu, shard, what, checksum):
     dec.check()
     assert (dec.output.cpu().numpy() == src).all()
     del graph
+
+
+@pytest.mark.parametrize("dtype", ["BF16", "F32"])
+def test_no_multiprocessor_takes_two_ctas_of_a_launch_of_one_each(gpu, dtype):
+    """28 chunks per SM, seven warps to a CTA, of which an SM has room for two, take no longer than 32 per SM (with some SMs taking
+    two and some none they took 1.23 and 1.28 times as long)."""
+    import torch
+    from lmz_b200 import decode
+    from perf import cases
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+
+    def took(per):
+        elements = 65536 // (4 if dtype == "F32" else 2)
+        case = dict(path="archive", dtype=dtype, layers=0, hidden=sms * per, ffn=elements, kv=0, chunk=65536)
+        dec = decode.ArchiveDecoder(cases._archive(case, per), fuse="all")
+        assert dec.plan.n_fused == sms * per
+        each = []
+        for _ in range(20):
+            torch.cuda._sleep(200_000)                    # (the run is queued by the time it starts)
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            dec.run()
+            b.record()
+            b.synchronize()
+            each.append(a.elapsed_time(b))
+        dec.check()
+        return sorted(each)[len(each) // 2]
+
+    assert took(28) < 1.1 * took(32)
