@@ -630,7 +630,8 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
     uint32_t e = 0;
     ByteState by{};
     if (__any_sync(0xffffffffu, n != 0)) {
-        // the whole ring, so that a group without a stream finds nothing but bounded entries in it
+        // the whole ring, so that a group without a stream finds nothing but bounded entries in it.  (F_BYTE_CFN: half of it; such a
+        // group's addresses come from bytes and masked slots alone, whatever its ring and tables hold.)
         const uint32_t lo = wd.lo, hi = wd.hi, lo2 = wd.lo2, hi2 = wd.hi2;
         const uint32_t *next = wd.next;
         const int32_t left = wd.left;

@@ -783,6 +783,69 @@ def test_launches_are_counted_as_they_happen(gpu, shard, what, checksum):
     del graph
 
 
+@pytest.mark.parametrize("nchunks", [740, 2368, 2369, 3552, 3553, 4144, 4145])
+@pytest.mark.parametrize("checksum", [True, False])
+def test_fused_fp32_chunks_by_how_many_there_are(gpu, nchunks, checksum):
+    """5, 16, 24 and 28 FP32 chunks per SM (of 148) and one more, all through the sink, which the planner leaves to the caller
+    for so few; the last one is cut short."""
+    import torch
+    from lmz_b200 import decode
+    from perf import cases
+    case = dict(path="archive", dtype="F32", layers=0, hidden=1024 * nchunks - 3, ffn=16, kv=0, chunk=65536)
+    dec = decode.ArchiveDecoder(cases._archive(case, nchunks), checksum=checksum, fuse="all")
+    assert dec.plan.n_fused_f32 == nchunks
+    out = dec.run()
+    dec.check()
+    head, data, _meta = cases._checkpoint(case, torch.Generator(device="cuda").manual_seed(nchunks))
+    assert torch.equal(out[len(head):len(head) + data.numel()], data)
+
+
+@pytest.fixture(scope="module", params=[("BF16", 17), ("F32", 17), ("BF16", 65), ("F32", 65)], ids=lambda p: f"{p[0]}, {p[1]} per SM")
+def many_small_tensors(request):
+    """(source, archive, element size, chunks): 17 chunks per SM (of 148) and two more take byte tables, four to a warp, 65 the
+    instances for many warps; they end anywhere in a unit of four elements and lie anywhere in a word, and every fifth has
+    a large alphabet."""
+    dtype, per_sm = request.param
+    es = 4 if dtype == "F32" else 2
+    tails, members = (0, 1, 3, 4, 5, 31, 32, 33, 124, 125, 126, 127), []
+    for i in range(148 * per_sm + 2):
+        n = 4480 + 128 * (i % 3) + tails[i % 12]
+        rng = np.random.default_rng(i)
+        w = (rng.standard_normal(n) * 0.02).astype("<f4")
+        if i % 5 == 0:
+            u, some = w.view("<u4"), rng.random(n) < 0.1
+            u[some] = u[some] & 0x807FFFFF | rng.integers(1, 255, int(some.sum())).astype("<u4") << 23
+        raw = w.view(np.uint8) if es == 4 else (w.view("<u4") >> 16).astype("<u2").view(np.uint8)
+        if i % 11 == 0:
+            members.append((f"{i}.bin", np.full(1, i % 256, np.uint8)))
+        members.append((f"{i}.safetensors", synth.safetensors_bytes([(f"w{i}", dtype, (n,), raw)])))
+    return np.concatenate([m for _name, m in members]), oa.write_archive(members, mapped=True, delta=False, workers=8), es, 148 * per_sm + 2
+
+
+@pytest.mark.parametrize("checksum", [True, False])
+@pytest.mark.parametrize("damaged", [0, 9])
+def test_many_small_chunks_in_the_sinks(gpu, many_small_tensors, checksum, damaged):
+    """Every chunk of such a launch; and with tables or states refused, each beside three others in its warp, every other chunk."""
+    from lmz_b200 import archive, decode, plan
+    source, blob, es, count = many_small_tensors
+    jobs = plan.build_plan(archive.Archive(blob), fuse="all").fused_jobs
+    assert jobs.size == count
+    assert set((jobs["mant_off"] % 4).tolist()) == {0, 1, 2, 3} and set((jobs["dst_off"] % 4).tolist()) == {0, 1, 2, 3}
+    bad, keep = bytearray(blob), np.ones(source.size, dtype=bool)
+    for i in range(damaged):
+        job = jobs[277 * i + i % 4]
+        bad[int(job["src_off"]) + (4 + 2 * i if i % 2 else 516 + 4 * (i % 8) + 1)] ^= 0x11
+        keep[int(job["dst_off"]):int(job["dst_off"]) + int(job["n"]) * es] = False
+    dec = decode.ArchiveDecoder(bytes(bad), checksum=checksum, fuse="all")
+    dec.run()
+    if damaged:
+        with pytest.raises(archive.CorruptArchive):
+            dec.check()
+    else:
+        dec.check()
+    assert (dec.output.cpu().numpy()[keep] == source[keep]).all()
+
+
 @pytest.mark.parametrize("dtype", ["BF16", "F32"])
 def test_no_multiprocessor_takes_two_ctas_of_a_launch_of_one_each(gpu, dtype):
     """28 chunks per SM, seven warps to a CTA, of which an SM has room for two, take no longer than 32 per SM (with some SMs taking
