@@ -135,13 +135,21 @@ constexpr uint32_t PADDED_PIECE = PIECE_ELEMS + (PIECE_ELEMS >> 7) * 4;
 struct CrcQuarters {
     uint32_t b[4], rot;
 };
+// A lookup's address: one instruction of the multiplier's pipe picks a byte, scales it and adds its table's base (four 8B layers
+// 1718 us, 1761 with the other form), or, MAD, a byte permute and a multiply-add, one of each pipe (see where it is asked for).
+template <int I>
+__device__ __forceinline__ uint32_t crc_entry4q(bool mad, const CrcQuarters &q, uint32_t r)
+{
+    if (!mad) return lds_u32(byte_mad(r, 0x80u << (8 * I), q.b[I]));
+    uint32_t v;
+    asm("mad.lo.u32 %0, %1, 128, %2;" : "=r"(v) : "r"(__byte_perm(r, 0u, 0x4440u + I)), "r"(q.b[I]));
+    return lds_u32(v);
+}
+template <bool MAD = false>
 __device__ __forceinline__ uint32_t crc_feed4q(const CrcQuarters &q, uint32_t s)
 {
-    // (one instruction of the multiplier's pipe picks a byte, scales it and adds its table's base; as a byte permute and a
-    // multiply-add it was two, one of them the integer pipe's: four 8B layers 1761 -> 1718 us)
     const uint32_t r = __byte_perm(s, 0u, q.rot);        // byte i of r = byte i ^ g of s
-    return lds_u32(byte_mad(r, 0x80u, q.b[0])) ^ lds_u32(byte_mad(r, 0x8000u, q.b[1])) ^ lds_u32(byte_mad(r, 0x800000u, q.b[2])) ^
-           lds_u32(byte_mad(r, 0x80000000u, q.b[3]));
+    return crc_entry4q<0>(MAD, q, r) ^ crc_entry4q<1>(MAD, q, r) ^ crc_entry4q<2>(MAD, q, r) ^ crc_entry4q<3>(MAD, q, r);
 }
 
 // Four elements of ES bytes to `d` (which differs from lane to lane by multiples of their size), the first `ve` of them; the

@@ -200,16 +200,17 @@ __device__ __forceinline__ uint32_t slot_ref(uint32_t x, uint32_t l1_sa, uint32_
 }
 // Its address.  One B200: TR_4 adds the tables' address last, as a ring entry's is added (four 8B layers 1711 us, 1800 with a sum
 // of three); TR_8 first (28577 streams of 32 KiB 1535 us, 1576 with it last); TR_FEW, whose warps have the integer pipe almost to
-// themselves, takes the offset by a shift (44 BF16 chunks per SM 586 us, 603 by a dot product), but not in the delta sink's
-// mixed tables (a delta chain 1525 and 1519).
+// themselves, takes the offset by a shift (44 BF16 chunks per SM 586 us, 603 by a dot product).  The delta sink's mixed tables are
+// the other way round: TR_4 by a shift (a chain of 14.9 K chunks 1934 us, 1945 by a dot product), TR_FEW by a dot product (a chain of
+// 10.3 K 1493 us, 1499 by a shift; one of 6.1 K 936 and 934).
 template <int CFN, int MODE>
 __device__ __forceinline__ uint32_t slot_addr(uint32_t x, uint32_t l1_sa, uint32_t cf_sa)
 {
-    if (CFN > 0 && MODE == TR_4) return cf_sa + slot_ref<CFN>(x, l1_sa, 0u);
-    if (CFN > 0 && MODE == TR_FEW && CFN != F_HYBRID_CFN) {
+    if (CFN > 0 && MODE == (CFN == F_HYBRID_CFN ? TR_4 : TR_FEW)) {
         const uint32_t e1 = lds_u32((x & 0xff0u) | l1_sa);
         return cf_sa + ((e1 >> 16) + 4u * __popc(e1 << ((~x & 15u) | 16u)));
     }
+    if (CFN > 0 && MODE == TR_4) return cf_sa + slot_ref<CFN>(x, l1_sa, 0u);
     return slot_ref<CFN>(x, l1_sa, cf_sa);
 }
 
@@ -482,7 +483,7 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
     // for the addresses.  Rows given out by all 32 lanes take still fewer, and as many more instructions: 1838 instead of 1761.)
     constexpr bool UNITS = SINK == SINK_BF16 || SINK == SINK_F32;
     const uint32_t put_sa = stage_sa + 16 * (k >> 2) + (k & 3u);
-    // byte i ^ g of a state word goes through slice table 3 - (i ^ g)
+    // byte i ^ g of a state word goes through table 3 - (i ^ g)
     CrcQuarters cq;
 #pragma unroll
     for (uint32_t i = 0; i < 4; i++) cq.b[i] = tab0 + 32u * (3u - (i ^ g)) + 4u * k;
@@ -722,8 +723,9 @@ __global__ void __launch_bounds__(stream_warps(CFN, CRC, SINK, MODE) * 32, 1) k_
             else stream_step4<CFN, MODE, FIRST, MULT>(x, e, hist, base, l1_sa, cf_sa, below, vsel);
         };
         auto put = [&](uint32_t step) { sts_u8(UNITS ? put_sa + 32 * (step & 3u) + 4 * (step >> 2) : stage_sa + step * NLANES + k, e); };
+        // (the delta sink with many warps adds up addresses on both pipes: a chain of 14.9 K chunks 1934 -> 1922 us)
         auto fold = [&](uint32_t i) {
-            if (CRC && i < NRA) ra[i] = crc_feed4q(cq, ra[i]);
+            if (CRC && i < NRA) ra[i] = crc_feed4q<SINK == SINK_DELTA && MODE == TR_4>(cq, ra[i]);
         };
         if constexpr (FULL) {
 #pragma unroll

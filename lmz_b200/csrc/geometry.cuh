@@ -14,7 +14,7 @@ constexpr uint32_t PROB_BITS = 12;
 constexpr uint32_t PROB_SCALE = 1u << PROB_BITS;
 constexpr uint32_t TILE = 128;        // symbols one 8-lane group retires per tile (16 steps)
 
-constexpr uint32_t F_CRC_BYTES = 32768;             // four slice tables x 256 entries x eight copies (CrcQuarters)
+constexpr uint32_t F_CRC_BYTES = 32768;             // four tables of a byte's 256 entries, eight copies (CrcQuarters)
 // The launch's shared memory starts F_SMEM_BASE bytes into the CTA's window (the launcher checks
 // that reservation); at most F_SMEM_DYN bytes of it are to be had, and F_SMEM_SM by all CTAs of an SM, reservations
 // counted.
