@@ -137,13 +137,13 @@ static int launch_solo(const StreamArgs &a, cudaStream_t cs)
 // Launches of few streams, with nothing to sort by: a warp each up to so many per SM, then four to a warp as long as
 // byte tables (F_BYTE_CFN) take the launch in one round.  1 when they are more.
 //
-// One B200, us, compact tables / a warp each / byte tables.  Exponent planes of 32 KiB: 16 per SM - / 301 / 283, 20 per SM
-// - / 347 / 307, 24 per SM 379 / - / 308, 28 per SM 381 / - / 309; uniform bytes 16 per SM - / 306 / 385, 20 per SM - / 358 / 397,
-// 24 per SM 418 / - / 399, 28 per SM 422 / - / 402; planes of 4 KiB, exponents 20 per SM - / 55 / 57, 24 per SM 68 / - / 58, uniform
-// bytes - / 57 / 70 and 72 / - / 70: a warp each up to 20.
-// With the sinks' own work in the same issue slots, 64 KiB BF16 chunks with checksums: 12 per SM - / 325 / 405, 16 per SM
-// - / 373 / 407, 17 per SM 483 / - / 417, 24 per SM 489 / - / 422; FP32 ones: 12 per SM - / 257 / 268, 16 per SM - / 296 / 268,
-// 17 per SM 358 / - / 272, 24 per SM 363 / - / 287; without checksums 28 per SM, BF16 464 / - / 380, FP32 326 / - / 243: a warp each up
+// One B200, us, compact tables / a warp each / byte tables.  Exponent planes of 32 KiB: 16 per SM - / 291 / 278, 20 per SM
+// - / 338 / 301, 24 per SM 379 / - / 303, 28 per SM 381 / - / 303; uniform bytes 16 per SM - / 297 / 383, 20 per SM - / 352 / 395,
+// 24 per SM 418 / - / 397, 28 per SM 420 / - / 399; planes of 4 KiB, exponents 20 per SM - / 53 / 53, 24 per SM 68 / - / 55, uniform
+// bytes - / 55 / 66 and 72 / - / 66: a warp each up to 20.
+// With the sinks' own work in the same issue slots, 64 KiB BF16 chunks with checksums: 12 per SM - / 327 / 403, 16 per SM
+// - / 376 / 405, 17 per SM 483 / - / 411, 24 per SM 489 / - / 417; FP32 ones: 12 per SM - / 255 / 264, 16 per SM - / 294 / 264,
+// 17 per SM 358 / - / 269, 24 per SM 362 / - / 284; without checksums 28 per SM, BF16 463 / - / 374, FP32 325 / - / 239: a warp each up
 // to 16 (FP32 chunks, which come here only where a caller has few of them fused, share the line of BF16's).
 // Open streams have no byte-table instance.
 template <int SINK, bool CRC>

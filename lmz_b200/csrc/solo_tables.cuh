@@ -24,10 +24,11 @@ __device__ __forceinline__ bool solo_tables(const uint32_t (&f)[8], uint32_t tab
     uint32_t start = incl - tot;
     if constexpr (!WIDE) {
         // A symbol's first slot gets what the symbol is above the one before it, every other slot zero: a slot's symbol is the sum up
-        // to it.  Lane k sums words 33 k .. 33 k + 32 (the lanes' in different banks; the last lane has one), four bytes
-        // by one multiplication, as no sum is above 255.  What this takes does not depend on the alphabet, where the lanes or the
-        // warp filling the symbols' slots one symbol after the other did.  (One B200, four of them to a warp, us: 24
-        // planes per SM of 331 uniform bytes 65.5 -> 28.6, of 4096 79.9 -> 69.7; of 331 exponents 32.2 -> 26.6.)
+        // to it.  Lane k sums words 36 k .. 36 k + 35 (sixteen bytes at a time, eight lanes' in different banks; the last three lanes have
+        // none), four bytes by one multiplication, as no sum is above 255.  What this takes does not depend on the alphabet, where
+        // the lanes or the warp filling the symbols' slots one symbol after the other did.  (One B200, us, compact tables / filled
+        // / summed up: four to a warp, 24 planes per SM of 256 uniform bytes 19 / 52 / 15, of 4 KiB 72 / 80 / 66, of 256
+        // exponents 19 / 21 / 15, of 4 KiB 70 / 66 / 55; a warp each, 20 per SM, of 256 uniform bytes - / 19 / 11.)
         for (uint32_t i = 0; i < PROB_SCALE; i += 512) sts_u128_if(1, tab_sa + i + 16 * lane, 0, 0, 0, 0);
         uint32_t last = 0;
 #pragma unroll
@@ -38,20 +39,25 @@ __device__ __forceinline__ bool solo_tables(const uint32_t (&f)[8], uint32_t tab
         if (!lower) before = 0;
         __syncwarp();
 #pragma unroll
-        for (uint32_t i = 0; i < 8; i++) {
-            const uint32_t s = lane * 8 + i, fi = f[i];
+        for (uint32_t i = 0; i < 8; i += 2) {
+            const uint32_t s = lane * 8 + i, f0 = f[i], f1 = f[i + 1];
             // (the table's address goes with start: c = -(tab_sa + start) + the address of the slot)
-            sts_u64_if(1, rec_sa + S_ENTRY * s, fi << 8 | s, 0u - (start + tab_sa));
-            sts_u8_if(fi, tab_sa + start, s - before);
-            if (fi) before = s;
-            start += fi;
+            sts_u128_if(1, rec_sa + S_ENTRY * s, f0 << 8 | s, 0u - (start + tab_sa), f1 << 8 | (s + 1), 0u - (start + f0 + tab_sa));
+            sts_u8_if(f0, tab_sa + start, s - before);
+            if (f0) before = s;
+            sts_u8_if(f1, tab_sa + start + f0, s + 1 - before);
+            if (f1) before = s + 1;
+            start += f0 + f1;
         }
         __syncwarp();
-        const uint32_t mine = tab_sa + 33 * 4 * lane, words = lane < 31 ? 33 : 1;
+        const uint32_t first = 36 * lane, mine = tab_sa + 4 * first;
         uint32_t sum = 0;
 #pragma unroll
-        for (uint32_t j = 0; j < 33; j++)
-            if (j < words) sum = byte_mad(lds_u32(mine + 4 * j), 0x01010101u, sum);
+        for (uint32_t j = 0; j < 36; j += 4)
+            if (first + j < PROB_SCALE / 4) {
+                const uint4 w = lds_u128(mine + 4 * j);
+                sum = byte_mad(w.w, 0x01010101u, byte_mad(w.z, 0x01010101u, byte_mad(w.y, 0x01010101u, byte_mad(w.x, 0x01010101u, sum))));
+            }
         uint32_t upto = sum;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
@@ -60,11 +66,15 @@ __device__ __forceinline__ bool solo_tables(const uint32_t (&f)[8], uint32_t tab
         }
         uint32_t at = (upto - sum) * 0x01010101u;
 #pragma unroll
-        for (uint32_t j = 0; j < 33; j++)
-            if (j < words) {
-                const uint32_t v = lds_u32(mine + 4 * j) * 0x01010101u + at;
-                sts_u32(mine + 4 * j, v);
-                at = __byte_perm(v, 0u, 0x3333);
+        for (uint32_t j = 0; j < 36; j += 4)
+            if (first + j < PROB_SCALE / 4) {
+                uint4 w = lds_u128(mine + 4 * j);
+                w.x = w.x * 0x01010101u + at;
+                w.y = w.y * 0x01010101u + __byte_perm(w.x, 0u, 0x3333);
+                w.z = w.z * 0x01010101u + __byte_perm(w.y, 0u, 0x3333);
+                w.w = w.w * 0x01010101u + __byte_perm(w.z, 0u, 0x3333);
+                sts_u128_if(1, mine + 4 * j, w.x, w.y, w.z, w.w);
+                at = __byte_perm(w.w, 0u, 0x3333);
             }
         __syncwarp();
         return true;

@@ -342,7 +342,7 @@ def test_device_batches_around_the_lines_between_kernels(gpu, nstr, plane, table
 @pytest.mark.parametrize("plane", [331, 2048])
 def test_byte_tables_of_any_alphabet_are_built_in_little_time(gpu, plane, table_mode):
     """24 streams per SM of short planes with large alphabets, where a stream's table is most of what it takes: as long as with
-    compact tables or less, and half as much again at the very most (with symbols filled in one by one 2.3 and 1.3 times it)."""
+    compact tables or less, and half as much again at the very most (with symbols filled in one by one 2.3 and 1.3 times)."""
     import torch
     lib, nstr = gpu.library(), 24 * torch.cuda.get_device_properties(0).multi_processor_count
     planes = torch.randint(0, 256, (nstr * plane,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(plane)).to(torch.uint8)
