@@ -75,7 +75,7 @@ constexpr int F_HYBRID_CFN = 192;                  // delta sink: 128-entry tabl
 constexpr uint32_t F_SMALL_LIVE = F_SMALL_CFN - 24; // largest alphabet it takes (the warp's streams sit 0, 8, 16, 24 entries in)
 
 // F_BYTE_CFN: a stream's 256 entries, and the next one's sixteen banks on, so that two streams' popular symbols lie apart
-// (28 streams of bytes per SM 379 -> 370 us).
+// (28 streams of bytes per SM 379 -> 370 us through the public call, tables filled one symbol after the other).
 constexpr uint32_t F_REC_STRIDE = S_REC_BYTES + 64;
 
 // Bytes of a stream's stage, a tile's 128 symbols and some: groups land four banks apart, or, where a lane takes a word from
@@ -398,8 +398,8 @@ __device__ __forceinline__ uint32_t stream_step(uint32_t &x, uint32_t &e, uint32
 }
 
 // F_BYTE_CFN's steps, as k_solo's: of a state x only y, e and c are kept, of which the next (unrefilled) one is
-// y * (e >> 8) + c.  (One B200, planes of 32 KiB: 342 us up to 16 streams per SM, 370 with 24, where the compact tables
-// take 382 and 445.  With two predicated loads instead of the picked one, as k_solo has them: 377 and 402.)
+// y * (e >> 8) + c.  (One B200, planes of 32 KiB: 278 us up to 16 streams per SM, 303 with 24, where the compact tables take 379.
+// With two predicated loads instead of the picked one, as k_solo has them, it took a tenth longer.)
 struct ByteState {
     uint32_t y, c;
 };

@@ -29,9 +29,9 @@ constexpr size_t SLICE_BYTES = (size_t)4 << 20;
 // a launch of its own, of one CTA per SM at most, of which an SM has room for three of one warp (64 KiB: a table of
 // 32 KiB on a boundary of its size) or two of two, and a CTA that finds none waits for one of an earlier slice to
 // end, which came in with an earlier copy.  At most three chains in turn for slices of one-warp CTAs, four for the others,
-// most of them under the copies.  (One B200, steps of 42 ns, us, new inputs, as here against slices only where all are resident: 444 of
-// 32 KiB 840 either way, 600 of 32 KiB 1100 against 1190, 600 of 64 KiB 1830 against 2300, 1184 of 64 KiB 3400 against
-// 3800, 600 of 256 KiB 7200 against 9500.)  Beyond that slices take their chains in turn, and one must hide under
+// most of them under the copies.  (One B200, steps of 42 ns, us, new inputs, as here against slices only where all are
+// resident: 444 of 32 KiB 840 either way, 600 of 32 KiB 1100 against 1190, 600 of 64 KiB 1830 against 2300, 1184 of 64 KiB
+// 3400 against 3800, 600 of 256 KiB 7200 against 9500.)  Beyond that slices take their chains in turn, and one must hide under
 // the copies: a slice's plaintext takes plane * streams / 50 GB/s to come out, its chain plane * 4.8 ns, and more
 // where streams share an SM, so 400 streams and more.  (With four slices at a time, by bytes alone, and steps of
 // 64 ns: 16 planes of 4 Mi symbols 66.9 ms, two chains; as here 35.1, in one piece 36.4.)

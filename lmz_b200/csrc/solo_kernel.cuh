@@ -27,7 +27,7 @@
 //
 // One B200, k_stream's wide tables against this: a lone stream 61.5 -> 38.5 ns a step (41.9 with one load behind a pick), a
 // 4096 x 14336 BF16 tensor in 64 KiB chunks 480 -> 381 us (issue slots 67 % busy, 31 instructions a stream's step), in 8 MiB
-// chunks 34.1 -> 22.3 ms (23.1 with one load), seven planes of 4 KiB between host buffers 78 -> 58 us.  Uniform bytes, four words a
+// chunks 34.1 -> 22.4 ms (23.1 with one load), seven planes of 4 KiB between host buffers 78 -> 55 us.  Uniform bytes, four words a
 // step, cost no more than exponents with one and a third.  Where the store of a step's symbols stands matters: behind the
 // vote, or behind the load, a lone stream's 8 MiB took 24.6 ms instead of 23.1.
 //

@@ -114,9 +114,11 @@ def _gather(ar: fmt.Archive, lo: int, offs: np.ndarray, width: int) -> np.ndarra
     return ar.blob[lo:][offs[:, None] + np.arange(width, dtype=np.int64)[None, :]]
 
 
-# Fewest 4-byte-element chunks worth the fused kernel: a launch that cannot fill the SMs'
-# stream slots (148 x 76) is bound by each warp's own instruction stream, and there the
-# two-pass path (lean stream kernel, then the merge kernel) measured faster.
+# Fewest 4-byte-element chunks that the fused kernel is chosen for: a launch that cannot fill the SMs'
+# stream slots is bound by each warp's own instruction stream, and up to 16 chunks per SM the
+# two-pass path (lean stream kernel, then the merge kernel) is faster.  One B200 of 148 SMs, us, fused / two passes,
+# 64 KiB chunks with checksums: 8 per SM 285 / 194, 16 per SM 294 / 272, 20 per SM 277 / 317, 28 per SM 366 / 347,
+# 32 per SM 370 / 408, 54 per SM 470 / 575.  (The line is that of a fused kernel that took a third longer.)
 FUSE_F32_MIN = 8192
 SMALL_LIVE = 104       # largest alphabet the denser fused-kernel instance takes (csrc/fused_kernel.cuh)
 
